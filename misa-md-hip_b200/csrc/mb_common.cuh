@@ -34,6 +34,18 @@ __device__ __forceinline__ double4 ldg4(const double4 *p) {
   return make_double4(a.x, a.y, b.x, b.y);
 }
 
+// 32-byte record of a site in one load / store (32-byte aligned).  The load may be moved
+// across stores: only for positions that the kernel does not write (and F' only where the
+// kernel does not write it).
+__device__ __forceinline__ double4 ld_site(const double4 *p) {
+  double4 v;
+  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void st_site(double4 *p, double x, double y, double z, double w) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(w) : "memory");
+}
+
 // ----------------------------------------------------------------- tracing
 // NVTX range around an entry point's work (shows in Nsight timelines; costs nothing
 // when no tool is attached).
@@ -75,6 +87,9 @@ struct DevPot {
   const double4 *phi_val; // [np][nr]
   const double4 *phi_der; // [np][nr]
   const double2 *force1;  // single type: [nr][3] {f d0, phi d0}, {f d1, phi d1}, {f d2, phi d2}
+  // single type, knot form: an interval reads its d0 and d2 and the next knot's d0
+  const double2 *f_ys;    // [nr] {y, s} of f (a cubic Hermite piece takes two knots)
+  const double2 *force2;  // [nr][2] {f d0, phi d0}, {f d2, phi d2}
   // single precision copies for the mixed path
   const float4 *f_val32;   // [nt][nr]  {y, s, c2, c3}
   const float2 *force32;   // single type: [nr][3] {f d0, phi d0}, {f d1, phi d1}, {f d2, phi d2}
@@ -128,17 +143,46 @@ int stencil_from_linear(const int64_t *even, size_t n_even, const int64_t *odd, 
 int stencil_generate(double a0, double reach, int ext_x, int ext_y, int64_t *even, int64_t *odd, int cap, int *n,
                      int *reach_x, int *reach_y, int *reach_z);
 int stencil_sort_by_distance(double a0, double cutoff, int ext_x, int ext_y, int64_t *even, int64_t *odd, int n,
-                             int *n_near);
+                             int *n_near, double *dist = nullptr);
+
+// Shell windows and summation runs of a one-type stencil whose near entries are BCC shells
+// (mb_pair64.cuh, mb_shell64.cu): near shell h looks up the table intervals lo[h] ..
+// lo[h] + cnt[h] - 1 of the density window and of the force window; run r holds the
+// entries [kb[r], kb[r + 1]), the first near_runs of them near ones of shell[r].
+#define MB_NEAR_SHELLS 6
+#define MB_RUNS_MAX 16
+#define MB_RUN 8      // near entries per run
+#define MB_OUT_RUN 16 // outer entries per run
+struct Windows64 {
+  int lo[MB_NEAR_SHELLS], cnt[MB_NEAR_SHELLS];
+};
+struct Shells64 {
+  int n, runs, near_runs;
+  Windows64 rho, force;
+  short kb[MB_RUNS_MAX + 1], shell[MB_RUNS_MAX];
+};
+struct Plan64 {
+  bool ok; // the stencil and tables suit the shell-window and entry-split kernels
+  Shells64 sh;
+  int *sites; // site list of the work items
+};
+// R: ideal distance of the entries of `st` (sorted).  False when the kernels do not apply.
+struct StencilSet;
+bool plan64_shells(const DevPot &P, const Geom &g, double a0, double cutoff, const double *R, const StencilSet &st,
+                   Shells64 &S);
+int plan64_plane_items(const Geom &g); // work items of one (z, sublattice) plane
+int plan64_items(const Geom &g);       // ... of the box
+int plan64_sites(const Geom &g, int *sites, cudaStream_t s);
+bool split64_fits(const Shells64 &sh);
 
 // ------------------------------------------------------ kernel arguments
 struct Lattice64 {
-  double *px, *py, *pz; // positions (ext)
+  double4 *p;           // {x, y, z, F'(rho)} of every site (ext), 32-byte aligned
   int8_t *code;         // type, < 0 vacant, MB_FLAG_ITL marks sites near an interstitial
-  double *df;           // F'(rho) (ext)
   double *rho;          // optional rho output (ext) or nullptr
   double *vx, *vy, *vz; // velocities (box sites used)
   double *fx, *fy, *fz; // forces (box sites used)
-  double *nx, *ny, *nz; // positions written by the drift (ext) or nullptr
+  double4 *n;           // records whose positions the drift writes (ext) or nullptr
 };
 
 struct Itl64 {
@@ -192,10 +236,10 @@ __host__ __device__ __forceinline__ void site_ideal(int s, int cx, int y, int z,
 // (null: the force pass walks every entry).
 int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, double rc2,
                  double *e_partial, int energy, int skip_flagged, cudaStream_t s, int z0 = 0, int z1 = -1,
-                 uint2 *outer = nullptr);
+                 uint2 *outer = nullptr, const Plan64 *plan = nullptr);
 int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, const StepParams &sp,
                    double *e_partial, int energy, int skip_flagged, cudaStream_t s, int z0 = 0, int z1 = -1,
-                   const uint2 *outer = nullptr);
+                   const uint2 *outer = nullptr, const Plan64 *plan = nullptr);
 // Work items (32-site row chunks) of the whole box: the length of the outer masks.
 inline long long items_per_box(const Geom &g) { return (long long)((g.bcx + 31) / 32) * g.by * 2 * g.bz; }
 // Outer-entry masks on (default), or off when MB_OUTER_MASKS=0 (the force passes then walk
@@ -236,20 +280,19 @@ int launch_pack_ext(const Geom &g, mb_atom_element *aos, int ext_x, int ext_y, c
                     cudaStream_t s, int z0 = 0, int z1 = -1); // what: 1 rho+df, 2 force, 3 df only
 int launch_unpack_box(const Geom &g, const mb_atom_element *aos, Lattice64 L, int with_f, int *bad_type,
                       int n_types, cudaStream_t s);
-int launch_pack_box(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double *px, const double *py,
-                    const double *pz, double h, int unkick, cudaStream_t s);
+int launch_pack_box(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double4 *pos, double h, int unkick,
+                    cudaStream_t s);
 int launch_unpack_box_ids(const Geom &g, const mb_atom_element *aos, Lattice64 L, int with_f, int *bad_type,
                           int64_t *ids, int n_types, cudaStream_t s, int z0 = 0, int z1 = -1);
-int launch_pack_box_ids(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double *px, const double *py,
-                        const double *pz, double h, int unkick, const int64_t *ids, cudaStream_t s, int z0 = 0,
-                        int z1 = -1);
+int launch_pack_box_ids(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double4 *pos, double h,
+                        int unkick, const int64_t *ids, cudaStream_t s, int z0 = 0, int z1 = -1);
 int launch_df_from_rho(const Geom &g, const DevPot &pot, const Lattice64 &L, cudaStream_t s);
 // z-slab halo layers (mb_layout.cu): sites of one message, and the pack (box layers ->
-// buf) / unpack (buf -> ghost layers, z positions + z_shift) of one field: what 1 positions
-// (c0, c1, c2), 2 df (c0), 3 site codes.
+// buf) / unpack (buf -> ghost layers, z positions + z_shift) of one field: what 1 positions,
+// 2 df (both of the records p), 3 site codes.
 long long halo_sites(const Geom &g);
-int launch_halo(const Geom &g, int what, int pack, int side, double *c0, double *c1, double *c2, int8_t *code,
-                void *buf, double z_shift, cudaStream_t s);
+int launch_halo(const Geom &g, int what, int pack, int side, double4 *p, int8_t *code, void *buf, double z_shift,
+                cudaStream_t s);
 
 // Half-neighbour hook passes (mb_half.cu): a decoded half-stencil offset.
 struct HalfOff {
@@ -263,5 +306,16 @@ int launch_half64(bool force, mb_atom_element *aos, const mb_device_domain &d, c
 
 // ------------------------------------------------------------ utilities
 int device_sm_count();
+#define MB_SMEM_MAX (227 * 1024)
+// Lets two kernels use `bytes` of dynamic shared memory (once per process).
+#define MB_SMEM_ATTR(k0, k1, bytes)                                                                            \
+  do {                                                                                                         \
+    static bool done_ = false;                                                                                 \
+    if (!done_) {                                                                                              \
+      MB_CUDA(cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes)));            \
+      MB_CUDA(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes)));            \
+      done_ = true;                                                                                            \
+    }                                                                                                          \
+  } while (0)
 
 } // namespace mb

@@ -98,9 +98,10 @@ int stencil_from_linear(const int64_t *even, size_t n_even, const int64_t *odd, 
 }
 
 // Reorders both parities' doubled-x linear stencils by ideal distance (stable) and
-// returns how many lead entries lie inside `cutoff` (equal for both parities).
+// returns how many lead entries lie inside `cutoff` (equal for both parities) and, with
+// `dist`, the sorted ideal distances.
 int stencil_sort_by_distance(double a0, double cutoff, int ext_x, int ext_y, int64_t *even, int64_t *odd, int n,
-                             int *n_near) {
+                             int *n_near, double *dist) {
   const long long plane = (long long)ext_x * ext_y;
   int near[2] = {0, 0};
   for (int par = 0; par < 2; par++) {
@@ -119,6 +120,7 @@ int stencil_sort_by_distance(double a0, double cutoff, int ext_x, int ext_y, int
     std::stable_sort(ord.begin(), ord.end(), [](const std::pair<double, int64_t> &x,
                                                  const std::pair<double, int64_t> &y) { return x.first < y.first; });
     for (int k = 0; k < n; k++) src[k] = ord[k].second;
+    for (int k = 0; k < n && dist; k++) dist[k] = ord[k].first;
   }
   if (near[0] != near[1]) return fail(MB_ERR_STATE, "even and odd stencils differ inside the cutoff");
   *n_near = near[0];

@@ -43,7 +43,8 @@ struct HookCtx {
   // device buffers sized for the ext lattice
   size_t n_ext = 0;
   mb_atom_element *aos = nullptr;
-  double *px = nullptr, *py = nullptr, *pz = nullptr, *df = nullptr, *rho = nullptr, *fx = nullptr, *fy = nullptr,
+  double4 *p = nullptr; // {x, y, z, F'(rho)}
+  double *rho = nullptr, *fx = nullptr, *fy = nullptr,
          *fz = nullptr;
   int8_t *code = nullptr;
   int *bad = nullptr;
@@ -63,11 +64,12 @@ static std::mutex g_mu;
 static unsigned char *g_noalloc_dev[MB_NOALLOC_MAX_DEVICES] = {};
 
 static void free_buffers(HookCtx &c) {
-  void *ptrs[] = {c.aos, c.px, c.py, c.pz, c.df, c.rho, c.fx, c.fy, c.fz, c.code, c.bad};
+  void *ptrs[] = {c.aos, c.p, c.rho, c.fx, c.fy, c.fz, c.code, c.bad};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   c.aos = nullptr;
-  c.px = c.py = c.pz = c.df = c.rho = c.fx = c.fy = c.fz = nullptr;
+  c.p = nullptr;
+  c.rho = c.fx = c.fy = c.fz = nullptr;
   c.code = nullptr;
   c.bad = nullptr;
   c.n_ext = 0;
@@ -78,7 +80,8 @@ static int ensure_buffers(HookCtx &c) {
   if (c.n_ext == n && c.aos) return MB_OK;
   free_buffers(c);
   MB_CUDA(cudaMalloc(&c.aos, n * sizeof(mb_atom_element)));
-  double **dp[] = {&c.px, &c.py, &c.pz, &c.df, &c.rho, &c.fx, &c.fy, &c.fz};
+  MB_CUDA(cudaMalloc(&c.p, n * sizeof(double4)));
+  double **dp[] = {&c.rho, &c.fx, &c.fy, &c.fz};
   for (double **p : dp) MB_CUDA(cudaMalloc(p, n * sizeof(double)));
   MB_CUDA(cudaMalloc(&c.code, (n + 3) & ~(size_t)3));
   MB_CUDA(cudaMalloc(&c.bad, sizeof(int)));
@@ -88,11 +91,8 @@ static int ensure_buffers(HookCtx &c) {
 
 static Lattice64 lattice_view(HookCtx &c) {
   Lattice64 L{};
-  L.px = c.px;
-  L.py = c.py;
-  L.pz = c.pz;
+  L.p = c.p;
   L.code = c.code;
-  L.df = c.df;
   L.rho = c.rho;
   L.fx = c.fx;
   L.fy = c.fy;
@@ -511,7 +511,8 @@ static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 // Bytes of scratch one ext site needs (AoS copy + positions + code + df + rho),
 // each array rounded up to 256 B, plus the error flag.
 static size_t noalloc_bytes(size_t n) {
-  return align256(n * sizeof(mb_atom_element)) + 5 * align256(n * sizeof(double)) + align256(n) + 256;
+  return align256(n * sizeof(mb_atom_element)) + align256(n * sizeof(double4)) + align256(n * sizeof(double)) +
+         align256(n) + 256;
 }
 
 static size_t noalloc_max_sites() {
@@ -564,10 +565,7 @@ extern "C" int mb_eam_rho_calc_noalloc(mb_atom_element *atoms, double cutoff_rad
   };
   mb_atom_element *aos = (mb_atom_element *)carve(n * sizeof(mb_atom_element));
   Lattice64 L{};
-  L.px = (double *)carve(n * sizeof(double));
-  L.py = (double *)carve(n * sizeof(double));
-  L.pz = (double *)carve(n * sizeof(double));
-  L.df = (double *)carve(n * sizeof(double));
+  L.p = (double4 *)carve(n * sizeof(double4));
   L.rho = (double *)carve(n * sizeof(double));
   L.code = (int8_t *)carve(n);
   int *bad = (int *)carve(sizeof(int));

@@ -24,9 +24,11 @@
 #include <limits.h>
 #include <stdio.h>
 #include <stdlib.h>
+#include <string.h>
 
 #include "mb_common.cuh"
 #include "mb_device.cuh"
+#include "mb_pair64.cuh"
 
 namespace mb {
 
@@ -39,19 +41,6 @@ __device__ __forceinline__ int z_layer(const Geom &g, double a0, double z) {
   const double c = floor(w / a0);
   return c < 0.0 ? 0 : (c >= (double)(g.bz - 1) ? g.bz - 1 : (int)c);
 }
-
-// Lists the box site of a drifted lattice atom that left its site (conversion on).
-__device__ __forceinline__ void conv_check(const Geom &g, const StepParams &sp, int s, int cx, int y, int z, double nx,
-                                           double ny, double nz) {
-  if (!(sp.conv2 > 0.0)) return;
-  double X, Y, Z;
-  site_ideal(s, cx, y, z, sp.a0, X, Y, Z);
-  const double ux = nx - X, uy = ny - Y, uz = nz - Z;
-  if (ux * ux + uy * uy + uz * uz <= sp.conv2) return;
-  const int slot = atomicAdd(sp.cand_n, 1);
-  if (slot < MB_CAND_CAP) sp.cand[slot] = ((long long)z * g.by + y) * (2LL * g.bcx) + 2LL * cx + s;
-}
-
 
 #define MB_EPART_CAP 4096 // CTA partial sums per energy region
 #ifndef MB_RHO_THREADS
@@ -128,7 +117,8 @@ struct RhoArgs {
 template <bool BF>
 __device__ __forceinline__ double rho_term(const RhoArgs &a, const Lattice64 &L, const double2 *s_f2, long long j,
                                            double xi, double yi, double zi, bool *near = nullptr) {
-  const double dx = xi - L.px[j], dy = yi - L.py[j], dz = zi - L.pz[j];
+  const double4 pj = ld_site(L.p + j);
+  const double dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
   const double d2 = dx * dx + dy * dy + dz * dz;
   const bool in = d2 < a.rc2;
   if (!BF) *near = d2 < a.rc2m;
@@ -162,7 +152,7 @@ __device__ __forceinline__ unsigned long long rho_site(const StencilSet &st, con
   const int code = L.code[i];
   if (code < 0 || (a.skip_flagged && (code & MB_FLAG_ITL))) return 0;
   const int ti = code & 0x3F;
-  const double xi = L.px[i], yi = L.py[i], zi = L.pz[i];
+  const double xi = L.p[i].x, yi = L.p[i].y, zi = L.p[i].z;
   const int *off = st.off[s];
   double rho = 0.0;
   unsigned long long near = 0;
@@ -185,7 +175,8 @@ __device__ __forceinline__ unsigned long long rho_site(const StencilSet &st, con
 #pragma unroll 4
     for (int k = 0; k < st.n; k++) {
       const long long j = i + off[k];
-      const double dx = xi - L.px[j], dy = yi - L.py[j], dz = zi - L.pz[j];
+      const double4 pj = ld_site(L.p + j);
+      const double dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
       const double d2 = dx * dx + dy * dy + dz * dz;
       if (d2 < a.rc2) {
         const double r = d2 * rsqrt(d2);
@@ -198,9 +189,9 @@ __device__ __forceinline__ unsigned long long rho_site(const StencilSet &st, con
     }
   }
   const double df = dF64(P, ti, rho);
-  L.df[i] = df;
+  L.p[i].w = df;
   if (L.rho) L.rho[i] = rho;
-  if (g.images) for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.df[idx] = df; });
+  if (g.images) for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.p[idx].w = df; });
   if (ENERGY) e_acc += F64(P, ti, rho);
   return near;
 }
@@ -267,13 +258,14 @@ template <bool ENERGY, bool BF>
 __device__ __forceinline__ void force_term(const ForceArgs &a, const Lattice64 &L, const double2 *s_f1, long long j,
                                            double xi, double yi, double zi, double dfi, double &fx, double &fy,
                                            double &fz, double &ep) {
-  const double dx = xi - L.px[j], dy = yi - L.py[j], dz = zi - L.pz[j];
+  const double4 pj = ld_site(L.p + j);
+  const double dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
   const double d2 = dx * dx + dy * dy + dz * dz;
   const bool in = d2 < a.sp.rc2;
   if (!BF && !in) return;
   const double rinv = rsqrt(d2);
   const double r = d2 * rinv;
-  const double dfj = L.df[j];
+  const double dfj = pj.w;
   int m;
   double p;
   spl_locate_in(r, a.P.rdr, a.P.nr, m, p);
@@ -337,8 +329,8 @@ __global__ void __launch_bounds__(MB_FORCE_THREADS, 1)
     const int code = L.code[i];
     if (code < 0 || (a.skip_flagged && (code & MB_FLAG_ITL))) continue;
     const int ti = code & 0x3F;
-    const double xi = L.px[i], yi = L.py[i], zi = L.pz[i];
-    const double dfi = L.df[i];
+    const double xi = L.p[i].x, yi = L.p[i].y, zi = L.p[i].z;
+    const double dfi = L.p[i].w;
     const int *off = st.off[s];
     double fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0;
     if (ONE_TYPE) {
@@ -385,12 +377,13 @@ __global__ void __launch_bounds__(MB_FORCE_THREADS, 1)
 #pragma unroll 4
       for (int k = 0; k < st.n; k++) {
         const long long j = i + off[k];
-        const double dx = xi - L.px[j], dy = yi - L.py[j], dz = zi - L.pz[j];
+        const double4 pj = ld_site(L.p + j);
+        const double dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
         const double d2 = dx * dx + dy * dy + dz * dz;
         if (d2 < sp.rc2) {
           const double rinv = rsqrt(d2);
           const double r = d2 * rinv;
-          const double dfj = L.df[j];
+          const double dfj = pj.w;
           const int tj = L.code[j] & 0x3F;
           double ph = 0.0;
           const double psip = pair_psip(P, ti, tj, r, dfi, dfj, ENERGY ? &ph : nullptr);
@@ -420,15 +413,11 @@ __global__ void __launch_bounds__(MB_FORCE_THREADS, 1)
         vy += sp.h * fy;
         vz += sp.h * fz;
         const double nx = xi + sp.dt * vx, ny = yi + sp.dt * vy, nz = zi + sp.dt * vz;
-        L.nx[i] = nx;
-        L.ny[i] = ny;
-        L.nz[i] = nz;
+        st_site(L.n + i, nx, ny, nz, 0.0);
         conv_check(g, sp, s, cx, y, z, nx, ny, nz);
         if (g.images)
           for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
-            L.nx[idx] = nx + ox;
-            L.ny[idx] = ny + oy;
-            L.nz[idx] = nz + oz;
+            st_site(L.n + idx, nx + ox, ny + oy, nz + oz, 0.0);
           });
       }
       L.vx[i] = vx;
@@ -479,13 +468,17 @@ static void brick_override(const char *name, int *shape) {
   }
 }
 
-static void set_walk(const Geom &g, int z0, int z1, const int *brick, ItemWalk &wk, long long &w0, long long &n1) {
+static void read_bricks() {
   static bool read = false;
   if (!read) {
     brick_override("MB_RHO_BRICK", kRhoBrick);
     brick_override("MB_FORCE_BRICK", kForceBrick);
     read = true;
   }
+}
+
+static void set_walk(const Geom &g, int z0, int z1, const int *brick, ItemWalk &wk, long long &w0, long long &n1) {
+  read_bricks();
   wk.chunks = (g.bcx + 31) / 32;
   const bool whole = z0 == 0 && z1 == g.bz;
   if (whole && brick[0] > 0 && brick[1] > 0) {
@@ -517,8 +510,57 @@ static int smem_knots(const DevPot &pot, int bytes_per_knot) {
 // Per-item outer-entry masks fit in 64 bits.
 static bool outer_masks_fit(const StencilSet &st) { return st.n - st.n_near <= 64; }
 
+int launch_shell_rho64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s);
+int launch_shell_force64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s);
+int launch_split_rho64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s);
+int launch_split_force64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s);
+
+// Launches of up to this many items per SM split each item over several warps
+// (mb_split64.cu); larger ones take shell windows (mb_shell64.cu).  Measured on one B200 (a
+// pass, launch gap included): density 20 us a split round of 4 items per SM and 8.7 us each
+// further one against 44-52 us for up to 32 items per SM in shell windows, so the line lies
+// at 5 rounds; force 20 + 11.7 us against 47-57 us, 4 rounds.  The environment variables
+// MB_SPLIT_RHO_ITEMS and MB_SPLIT_FORCE_ITEMS override the lines (0: shell windows always).
+#define MB_SPLIT_RHO_ITEMS 20
+#define MB_SPLIT_FORCE_ITEMS 16
+static bool split_launch(const char *name, int per_sm, const LatticeArgs &a) {
+  if (const char *v = getenv(name)) per_sm = atoi(v);
+  return a.n_items - a.w0 <= per_sm * device_sm_count();
+}
+
+// Arguments of a planned pass over box layers [z0, z1).
+static LatticeArgs lattice_args(const Geom &g, const DevPot &pot, const Lattice64 &L, double rc2, int skip_flagged,
+                                uint2 *outer, const Plan64 &plan, int z0, int z1) {
+  LatticeArgs a{};
+  a.g = g;
+  a.P = pot;
+  a.L = L;
+  a.sh = plan.sh;
+  a.sites = plan.sites;
+  const int per_layer = 2 * plan64_plane_items(g);
+  a.w0 = z0 * per_layer;
+  a.n_items = z1 * per_layer;
+  a.rc2 = rc2;
+  a.rc2m = rc2 * (1.0 + 1e-9);
+  long long bits;
+  memcpy(&bits, &rc2, sizeof(bits));
+  a.rc2_hi = (int)(bits >> 32);
+  a.skip_flagged = skip_flagged;
+  a.outer = outer;
+  return a;
+}
+
 int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, double rc2,
-                 double *e_partial, int energy, int skip_flagged, cudaStream_t s, int z0, int z1, uint2 *outer) {
+                 double *e_partial, int energy, int skip_flagged, cudaStream_t s, int z0, int z1, uint2 *outer,
+                 const Plan64 *plan) {
+  if (plan && plan->ok && L.rho && cutoff_in_table(pot, rc2)) {
+    if (z1 < 0) z1 = g.bz;
+    if (z0 < 0 || z0 >= z1 || z1 > g.bz) return z0 == z1 ? MB_OK : fail(MB_ERR_ARG, "z-slab outside the box");
+    LatticeArgs a = lattice_args(g, pot, L, rc2, skip_flagged, outer, *plan, z0, z1);
+    a.e0 = e_partial;
+    if (split_launch("MB_SPLIT_RHO_ITEMS", MB_SPLIT_RHO_ITEMS, a)) return launch_split_rho64(st, a, energy, s);
+    return launch_shell_rho64(st, a, energy, s);
+  }
   RhoArgs a;
   a.g = g;
   a.P = pot;
@@ -560,7 +602,18 @@ int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const L
 
 int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, const StepParams &sp,
                    double *e_partial, int energy, int skip_flagged, cudaStream_t s, int z0, int z1,
-                   const uint2 *outer) {
+                   const uint2 *outer, const Plan64 *plan) {
+  if (plan && plan->ok && L.fx && cutoff_in_table(pot, sp.rc2)) {
+    if (z1 < 0) z1 = g.bz;
+    if (z0 < 0 || z0 >= z1 || z1 > g.bz) return z0 == z1 ? MB_OK : fail(MB_ERR_ARG, "z-slab outside the box");
+    LatticeArgs a =
+        lattice_args(g, pot, L, sp.rc2, skip_flagged, const_cast<uint2 *>(outer), *plan, z0, z1);
+    a.sp = sp;
+    a.e0 = e_partial ? e_partial + MB_EPART_CAP : nullptr;
+    a.e1 = e_partial ? e_partial + 2 * MB_EPART_CAP : nullptr;
+    if (split_launch("MB_SPLIT_FORCE_ITEMS", MB_SPLIT_FORCE_ITEMS, a)) return launch_split_force64(st, a, energy, s);
+    return launch_shell_force64(st, a, energy, s);
+  }
   ForceArgs a;
   a.g = g;
   a.P = pot;
@@ -679,18 +732,16 @@ __device__ __forceinline__ void window_pairs64(const Geom &g, const Lattice64 &L
         ok[t] = k < n && window_site(g, win, list[k], qx, qy, qz, I.a0, I.reach, j[t], sx[t], sy[t], sz[t]);
       }
       int cj[4];
-      double xj[4], yj[4], zj[4], dj[4];
+      double4 pj[4];
 #pragma unroll
       for (int t = 0; t < 4; t++) {
         cj[t] = ok[t] ? (int)L.code[j[t]] : -1;
-        xj[t] = ok[t] ? L.px[j[t]] : 0.0;
-        yj[t] = ok[t] ? L.py[j[t]] : 0.0;
-        zj[t] = ok[t] ? L.pz[j[t]] : 0.0;
-        dj[t] = (DF && ok[t]) ? L.df[j[t]] : 0.0;
+        pj[t] = ok[t] ? ld_site(L.p + j[t]) : make_double4(0.0, 0.0, 0.0, 0.0);
       }
 #pragma unroll
       for (int t = 0; t < 4; t++)
-        if (cj[t] >= 0) pair(qx - (xj[t] + sx[t]), qy - (yj[t] + sy[t]), qz - (zj[t] + sz[t]), cj[t] & 0x3F, dj[t]);
+        if (cj[t] >= 0)
+          pair(qx - (pj[t].x + sx[t]), qy - (pj[t].y + sy[t]), qz - (pj[t].z + sz[t]), cj[t] & 0x3F, DF ? pj[t].w : 0.0);
     }
     return;
   }
@@ -701,7 +752,8 @@ __device__ __forceinline__ void window_pairs64(const Geom &g, const Lattice64 &L
     if (!window_site(g, win, c, qx, qy, qz, I.a0, I.reach, j, sx, sy, sz)) continue;
     const int cj = L.code[j];
     if (cj < 0) continue;
-    pair(qx - (L.px[j] + sx), qy - (L.py[j] + sy), qz - (L.pz[j] + sz), cj & 0x3F, DF ? L.df[j] : 0.0);
+    const double4 pj = ld_site(L.p + j);
+    pair(qx - (pj.x + sx), qy - (pj.y + sy), qz - (pj.z + sz), cj & 0x3F, DF ? pj.w : 0.0);
   }
 }
 
@@ -727,11 +779,12 @@ __global__ void __launch_bounds__(MB_ITL_THREADS)
       decode_ext(g, i, s, cx, y, z);
       if (!all_z && (z < z0 || z >= z1)) continue;
       const int ti = L.code[i] & 0x3F;
-      const double xi = L.px[i], yi = L.py[i], zi = L.pz[i];
+      const double xi = L.p[i].x, yi = L.p[i].y, zi = L.p[i].z;
       double rho = 0.0;
       for (int k = lane; k < st.n; k += 32) {
         const long long j = i + st.off[s][k];
-        const double dx = xi - L.px[j], dy = yi - L.py[j], dz = zi - L.pz[j];
+        const double4 pj = ld_site(L.p + j);
+        const double dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
         const double d2 = dx * dx + dy * dy + dz * dz;
         if (d2 < rc2) rho += rho_of_r(P, L.code[j] & 0x3F, d2 * rsqrt(d2));
       }
@@ -744,9 +797,9 @@ __global__ void __launch_bounds__(MB_ITL_THREADS)
       rho = warp_sum(rho);
       if (lane == 0) {
         const double df = dF64(P, ti, rho);
-        L.df[i] = df;
+        L.p[i].w = df;
         if (L.rho) L.rho[i] = rho;
-        if (g.images) for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.df[idx] = df; });
+        if (g.images) for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.p[idx].w = df; });
         if (ENERGY) e_acc += F64(P, ti, rho);
       }
     } else {
@@ -805,10 +858,10 @@ __global__ void __launch_bounds__(MB_ITL_THREADS)
       i = I.flag_list[w - n_itl];
       decode_ext(g, i, s, cx, y, z);
       ti = L.code[i] & 0x3F;
-      xi = L.px[i];
-      yi = L.py[i];
-      zi = L.pz[i];
-      dfi = L.df[i];
+      xi = L.p[i].x;
+      yi = L.p[i].y;
+      zi = L.p[i].z;
+      dfi = L.p[i].w;
     } else {
       it = (int)w;
       ti = I.type[it];
@@ -839,7 +892,8 @@ __global__ void __launch_bounds__(MB_ITL_THREADS)
         const long long j = i + st.off[s][k];
         const int cj = L.code[j];
         if (cj < 0) continue;
-        add_pair(xi - L.px[j], yi - L.py[j], zi - L.pz[j], cj & 0x3F, L.df[j]);
+        const double4 pj = ld_site(L.p + j);
+        add_pair(xi - pj.x, yi - pj.y, zi - pj.z, cj & 0x3F, pj.w);
       }
     } else {
       window_pairs64<true>(g, L, I, xi, yi, zi, list, add_pair);
@@ -882,15 +936,11 @@ __global__ void __launch_bounds__(MB_ITL_THREADS)
           vz += sp.h * fz;
           const double nx = xi + sp.dt * vx, ny = yi + sp.dt * vy, nz = zi + sp.dt * vz;
           if (is_site) {
-            L.nx[i] = nx;
-            L.ny[i] = ny;
-            L.nz[i] = nz;
+            st_site(L.n + i, nx, ny, nz, 0.0);
             conv_check(g, sp, s, cx, y, z, nx, ny, nz);
             if (g.images)
               for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
-                L.nx[idx] = nx + ox;
-                L.ny[idx] = ny + oy;
-                L.nz[idx] = nz + oz;
+                st_site(L.n + idx, nx + ox, ny + oy, nz + oz, 0.0);
               });
           } else {
             I.nx[it] = nx;
@@ -1009,12 +1059,12 @@ __global__ void __launch_bounds__(MB_CONV_THREADS, 1)
     decode_box(g, t, s, cx, y, z);
     const long long i = ext_index(g, s, cx, y, z);
     const int k = n0 + r;
-    I.nx[k] = L.nx[i];
-    I.ny[k] = L.ny[i];
-    I.nz[k] = L.nz[i];
-    I.px[k] = L.px[i];
-    I.py[k] = L.py[i];
-    I.pz[k] = L.pz[i];
+    I.nx[k] = L.n[i].x;
+    I.ny[k] = L.n[i].y;
+    I.nz[k] = L.n[i].z;
+    I.px[k] = L.p[i].x;
+    I.py[k] = L.p[i].y;
+    I.pz[k] = L.p[i].z;
     I.vx[k] = L.vx[i];
     I.vy[k] = L.vy[i];
     I.vz[k] = L.vz[i];
@@ -1022,20 +1072,20 @@ __global__ void __launch_bounds__(MB_CONV_THREADS, 1)
     I.fy[k] = L.fy[i];
     I.fz[k] = L.fz[i];
     I.rho[k] = L.rho ? L.rho[i] : 0.0;
-    I.df[k] = L.df[i];
+    I.df[k] = L.p[i].w;
     I.type[k] = (int8_t)(L.code[i] & 0x3F);
     I.id[k] = site_id[t];
     // vacant: both position buffers far away (the pair loops reject vacancies by
     // position, and the buffer of this step comes back as the next step's drift target)
     L.code[i] = -1;
-    L.nx[i] = L.ny[i] = L.nz[i] = MB_VACANT_POS;
-    L.px[i] = L.py[i] = L.pz[i] = MB_VACANT_POS;
+    L.n[i].x = L.n[i].y = L.n[i].z = MB_VACANT_POS;
+    L.p[i].x = L.p[i].y = L.p[i].z = MB_VACANT_POS;
     L.vx[i] = L.vy[i] = L.vz[i] = 0.0;
     L.fx[i] = L.fy[i] = L.fz[i] = 0.0;
     for_images(g, s, cx, y, z, [&](long long idx, double, double, double) {
       L.code[idx] = -1;
-      L.nx[idx] = L.ny[idx] = L.nz[idx] = MB_VACANT_POS;
-      L.px[idx] = L.py[idx] = L.pz[idx] = MB_VACANT_POS;
+      L.n[idx].x = L.n[idx].y = L.n[idx].z = MB_VACANT_POS;
+      L.p[idx].x = L.p[idx].y = L.p[idx].z = MB_VACANT_POS;
     });
   }
   const int n1 = n0 + nconv;
@@ -1101,27 +1151,23 @@ __global__ void __launch_bounds__(MB_CONV_THREADS, 1)
     const double px = nx + (I.px[k] - I.nx[k]), py = ny + (I.py[k] - I.ny[k]), pz = nz + (I.pz[k] - I.nz[k]);
     const int8_t ty = I.type[k];
     L.code[i] = ty;
-    L.nx[i] = nx;
-    L.ny[i] = ny;
-    L.nz[i] = nz;
-    L.px[i] = px;
-    L.py[i] = py;
-    L.pz[i] = pz;
+    st_site(L.n + i, nx, ny, nz, 0.0);
+    L.p[i].x = px;
+    L.p[i].y = py;
+    L.p[i].z = pz;
     L.vx[i] = I.vx[k];
     L.vy[i] = I.vy[k];
     L.vz[i] = I.vz[k];
     L.fx[i] = I.fx[k];
     L.fy[i] = I.fy[k];
     L.fz[i] = I.fz[k];
-    L.df[i] = I.df[k];
+    L.p[i].w = I.df[k];
     for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
       L.code[idx] = ty;
-      L.nx[idx] = nx + ox;
-      L.ny[idx] = ny + oy;
-      L.nz[idx] = nz + oz;
-      L.px[idx] = px + ox;
-      L.py[idx] = py + oy;
-      L.pz[idx] = pz + oz;
+      st_site(L.n + idx, nx + ox, ny + oy, nz + oz, 0.0);
+      L.p[idx].x = px + ox;
+      L.p[idx].y = py + oy;
+      L.p[idx].z = pz + oz;
     });
     site_id[t] = I.id[k];
     atomicOr(&removed[k >> 5], 1u << (k & 31));
@@ -1199,18 +1245,18 @@ __global__ void k_images64(const Geom g, const Lattice64 L, int what, long long 
     const int z = (int)(r >> 1);
     const long long i = ext_index(g, s, cx, y, z);
     if (what & 1) {
-      const double x0 = L.px[i], y0 = L.py[i], z0 = L.pz[i];
+      const double x0 = L.p[i].x, y0 = L.p[i].y, z0 = L.p[i].z;
       const int8_t c = L.code[i];
       for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
-        L.px[idx] = x0 + ox;
-        L.py[idx] = y0 + oy;
-        L.pz[idx] = z0 + oz;
+        L.p[idx].x = x0 + ox;
+        L.p[idx].y = y0 + oy;
+        L.p[idx].z = z0 + oz;
         L.code[idx] = (int8_t)(c < 0 ? c : (c & 0x3F));
       });
     }
     if (what & 2) {
-      const double d = L.df[i];
-      for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.df[idx] = d; });
+      const double d = L.p[i].w;
+      for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.p[idx].w = d; });
     }
   }
 }
@@ -1257,17 +1303,17 @@ __global__ void k_kick_drift64(const Geom g, const Lattice64 L, const Itl64 I, c
     const long long i = ext_index(g, s, cx, y, z);
     if (L.code[i] < 0) continue;
     const double vx = L.vx[i] + sp.h * L.fx[i], vy = L.vy[i] + sp.h * L.fy[i], vz = L.vz[i] + sp.h * L.fz[i];
-    const double x0 = L.px[i] + sp.dt * vx, y0 = L.py[i] + sp.dt * vy, z0 = L.pz[i] + sp.dt * vz;
+    const double x0 = L.p[i].x + sp.dt * vx, y0 = L.p[i].y + sp.dt * vy, z0 = L.p[i].z + sp.dt * vz;
     L.vx[i] = vx;
     L.vy[i] = vy;
     L.vz[i] = vz;
-    L.px[i] = x0;
-    L.py[i] = y0;
-    L.pz[i] = z0;
+    L.p[i].x = x0;
+    L.p[i].y = y0;
+    L.p[i].z = z0;
     for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
-      L.px[idx] = x0 + ox;
-      L.py[idx] = y0 + oy;
-      L.pz[idx] = z0 + oz;
+      L.p[idx].x = x0 + ox;
+      L.p[idx].y = y0 + oy;
+      L.p[idx].z = z0 + oz;
     });
   }
 }

@@ -27,10 +27,10 @@ __global__ void k_unpack_ext(const Geom g, const mb_atom_element *aos, int ext_x
     }
     const bool vac = type < 0;
     L.code[i] = (int8_t)(vac ? -1 : type);
-    L.px[i] = vac ? MB_VACANT_POS : a.x[0];
-    L.py[i] = vac ? MB_VACANT_POS : a.x[1];
-    L.pz[i] = vac ? MB_VACANT_POS : a.x[2];
-    if (with_df == 1) L.df[i] = a.df;
+    L.p[i].x = vac ? MB_VACANT_POS : a.x[0];
+    L.p[i].y = vac ? MB_VACANT_POS : a.x[1];
+    L.p[i].z = vac ? MB_VACANT_POS : a.x[2];
+    if (with_df == 1) L.p[i].w = a.df;
     if (with_df == 2 && L.rho) L.rho[i] = a.rho;
   }
 }
@@ -52,13 +52,13 @@ __global__ void k_pack_ext(const Geom g, mb_atom_element *aos, int ext_x, int ex
     mb_atom_element &a = aos[((long long)ez * ext_y + ey) * ext_x + ex];
     if (what == 1) {
       a.rho = L.rho[i];
-      a.df = L.df[i];
+      a.df = L.p[i].w;
     } else if (what == 2) {
       a.f[0] = L.fx[i];
       a.f[1] = L.fy[i];
       a.f[2] = L.fz[i];
     } else {
-      a.df = L.df[i];
+      a.df = L.p[i].w;
     }
   }
 }
@@ -83,9 +83,9 @@ __global__ void k_unpack_box(const Geom g, const mb_atom_element *aos, Lattice64
     }
     const bool vac = type < 0;
     L.code[i] = (int8_t)(vac ? -1 : type);
-    L.px[i] = vac ? MB_VACANT_POS : a.x[0];
-    L.py[i] = vac ? MB_VACANT_POS : a.x[1];
-    L.pz[i] = vac ? MB_VACANT_POS : a.x[2];
+    L.p[i].x = vac ? MB_VACANT_POS : a.x[0];
+    L.p[i].y = vac ? MB_VACANT_POS : a.x[1];
+    L.p[i].z = vac ? MB_VACANT_POS : a.x[2];
     L.vx[i] = vac ? 0.0 : a.v[0];
     L.vy[i] = vac ? 0.0 : a.v[1];
     L.vz[i] = vac ? 0.0 : a.v[2];
@@ -98,11 +98,9 @@ __global__ void k_unpack_box(const Geom g, const mb_atom_element *aos, Lattice64
   }
 }
 
-// Box-order records of the synchronised state.  px/py/pz: positions of the
-// step; unkick: v is stored half a step ahead and is brought back by h*f.
-__global__ void k_pack_box(const Geom g, mb_atom_element *aos, const Lattice64 L, const double *px,
-                           const double *py, const double *pz, double h, int unkick, const int64_t *ids, long long t0,
-                           long long t1) {
+// Box-order records of the synchronised state.  pos: positions and F' of the step; unkick: v is stored half a step ahead and is brought back by h*f.
+__global__ void k_pack_box(const Geom g, mb_atom_element *aos, const Lattice64 L, const double4 *pos, double h,
+                           int unkick, const int64_t *ids, long long t0, long long t1) {
   const int bxd = 2 * g.bcx;
   for (long long t = t0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; t < t1;
        t += (long long)gridDim.x * blockDim.x) {
@@ -120,9 +118,10 @@ __global__ void k_pack_box(const Geom g, mb_atom_element *aos, const Lattice64 L
       for (int k = 0; k < 3; k++) a.x[k] = a.v[k] = a.f[k] = 0.0;
       a.rho = a.df = 0.0;
     } else {
-      a.x[0] = px[i];
-      a.x[1] = py[i];
-      a.x[2] = pz[i];
+      const double4 p = ld_site(pos + i);
+      a.x[0] = p.x;
+      a.x[1] = p.y;
+      a.x[2] = p.z;
       a.f[0] = L.fx[i];
       a.f[1] = L.fy[i];
       a.f[2] = L.fz[i];
@@ -130,7 +129,7 @@ __global__ void k_pack_box(const Geom g, mb_atom_element *aos, const Lattice64 L
       a.v[1] = L.vy[i] - (unkick ? h * a.f[1] : 0.0);
       a.v[2] = L.vz[i] - (unkick ? h * a.f[2] : 0.0);
       a.rho = L.rho ? L.rho[i] : 0.0;
-      a.df = L.df[i];
+      a.df = p.w;
     }
     aos[t] = a;
   }
@@ -164,7 +163,7 @@ __global__ void k_df_from_rho(const Geom g, const DevPot P, Lattice64 L) {
     double p;
     spl_loc(L.rho[i], P.rdrho, P.nrho, m, p);
     const double4 d = ldg4(&P.F_der[(size_t)(c & 0x3F) * P.nrho + m]);
-    L.df[i] = (d.z * p + d.y) * p + d.x;
+    L.p[i].w = (d.z * p + d.y) * p + d.x;
   }
 }
 
@@ -213,20 +212,19 @@ int launch_unpack_box(const Geom &g, const mb_atom_element *aos, Lattice64 L, in
   return launch_unpack_box_ids(g, aos, L, with_f, bad_type, nullptr, n_types, s);
 }
 
-int launch_pack_box_ids(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double *px, const double *py,
-                        const double *pz, double h, int unkick, const int64_t *ids, cudaStream_t s, int z0, int z1) {
+int launch_pack_box_ids(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double4 *pos, double h,
+                        int unkick, const int64_t *ids, cudaStream_t s, int z0, int z1) {
   if (z1 < 0) z1 = g.bz;
   const long long layer = 2LL * g.bcx * g.by;
   if (z1 <= z0) return MB_OK;
-  k_pack_box<<<flat_grid(layer * (z1 - z0)), 256, 0, s>>>(g, aos, L, px, py, pz, h, unkick, ids, layer * z0,
-                                                           layer * z1);
+  k_pack_box<<<flat_grid(layer * (z1 - z0)), 256, 0, s>>>(g, aos, L, pos, h, unkick, ids, layer * z0, layer * z1);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }
 
-int launch_pack_box(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double *px, const double *py,
-                    const double *pz, double h, int unkick, cudaStream_t s) {
-  return launch_pack_box_ids(g, aos, L, px, py, pz, h, unkick, nullptr, s);
+int launch_pack_box(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double4 *pos, double h, int unkick,
+                    cudaStream_t s) {
+  return launch_pack_box_ids(g, aos, L, pos, h, unkick, nullptr, s);
 }
 
 int launch_df_from_rho(const Geom &g, const DevPot &pot, const Lattice64 &L, cudaStream_t s) {
@@ -248,8 +246,8 @@ int launch_df_from_rho(const Geom &g, const DevPot &pot, const Lattice64 &L, cud
 // first slab).
 namespace mb {
 
-__global__ void k_halo(const Geom g, int what, int pack, int ez0, double *c0, double *c1, double *c2, int8_t *code,
-                       void *buf, double z_shift) {
+__global__ void k_halo(const Geom g, int what, int pack, int ez0, double4 *p, int8_t *code, void *buf,
+                       double z_shift) {
   const long long plane = (long long)g.ey * g.ecx;
   const long long per_s = plane * g.gz, n = 2 * per_s;
   const int ncomp = what == 1 ? 3 : 1;
@@ -267,20 +265,20 @@ __global__ void k_halo(const Geom g, int what, int pack, int ez0, double *c0, do
       else
         code[idx] = b[r];
     } else {
-      double *col = c == 0 ? c0 : (c == 1 ? c1 : c2);
+      double *v = reinterpret_cast<double *>(p + idx) + (what == 2 ? 3 : c);
       double *b = static_cast<double *>(buf);
       if (pack)
-        b[t] = col[idx];
+        b[t] = *v;
       else
-        col[idx] = c == 2 ? b[t] + z_shift : b[t];
+        *v = c == 2 ? b[t] + z_shift : b[t];
     }
   }
 }
 
 long long halo_sites(const Geom &g) { return 2LL * g.gz * g.ey * g.ecx; }
 
-int launch_halo(const Geom &g, int what, int pack, int side, double *c0, double *c1, double *c2, int8_t *code,
-                void *buf, double z_shift, cudaStream_t s) {
+int launch_halo(const Geom &g, int what, int pack, int side, double4 *p, int8_t *code, void *buf, double z_shift,
+                cudaStream_t s) {
   if (what < 1 || what > 3) return fail(MB_ERR_ARG, "halo field must be 1 (positions), 2 (df) or 3 (site codes)");
   if (side != 0 && side != 1) return fail(MB_ERR_ARG, "halo side must be 0 (below) or 1 (above)");
   if (!buf) return fail(MB_ERR_ARG, "null halo buffer");
@@ -289,8 +287,7 @@ int launch_halo(const Geom &g, int what, int pack, int side, double *c0, double 
   const long long n = halo_sites(g) * (what == 1 ? 3 : 1);
   long long grid = (n + 255) / 256;
   if (grid > 8LL * device_sm_count()) grid = 8LL * device_sm_count();
-  k_halo<<<(int)(grid > 0 ? grid : 1), 256, 0, s>>>(g, what, pack, ez0, c0, c1, c2, code, buf,
-                                                     what == 1 ? z_shift : 0.0);
+  k_halo<<<(int)(grid > 0 ? grid : 1), 256, 0, s>>>(g, what, pack, ez0, p, code, buf, what == 1 ? z_shift : 0.0);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }

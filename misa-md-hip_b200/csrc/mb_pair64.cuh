@@ -1,0 +1,329 @@
+// One-type FP64 pair terms of the lattice passes, shared by the shell-window kernels
+// (mb_shell64.cu, large launches) and the entry-split kernels (mb_split64.cu, small ones).
+//
+// Both sum a site's stencil in the same fixed order, so a lattice gives the same bits
+// whichever of them runs (a z-slab of a large lattice may be a small launch):
+//   * near entries (inside the cutoff at the ideal lattice, by distance) in runs of up to
+//     MB_RUN entries of one shell; then runs of MB_OUT_RUN outer entries;
+//   * within a near run first the pairs inside the shell's table window, in entry order,
+//     then the others (strongly displaced atoms) that are inside the cutoff, in entry order;
+//   * the site's total takes the run sums in order.
+// Every rounding is spelled out (__fma_rn and friends), so that the two kernels cannot
+// differ in what the compiler contracts.
+#pragma once
+
+#include "mb_device.cuh"
+#include "mb_ensemble_shells.cuh"
+
+namespace mb {
+
+// Work items: 32 consecutive sites of one (z, sublattice) plane; a lane's entry of the site
+// list (Plan64::sites) is its ext index, with MB_SITE_FACE where the site has periodic
+// images, or negative (no site).  Items of box layers [z0, z1) are a contiguous range.
+#define MB_SITE_FACE 0x40000000
+#define MB_SITE_INDEX 0x3fffffff
+
+// Everything the two kinds of kernel need.
+struct LatticeArgs {
+  Geom g;
+  DevPot P;
+  Lattice64 L;
+  Shells64 sh;
+  const int *sites;
+  int w0, n_items;       // items [w0, n_items)
+  double rc2, rc2m;      // squared cutoff; a hair above it for the outer-entry masks
+  int rc2_hi;            // high word of rc2
+  int skip_flagged;
+  uint2 *outer;          // per item: the outer entries some lane has inside rc2m (or null)
+  double *e0, *e1;       // CTA partials: density pass F(rho); force pass pair and kinetic energy
+  StepParams sp;
+};
+
+// ------------------------------------------------------------- pair terms
+// sqrt(d2) and 1 / sqrt(d2): the hardware's seed y and one step of Householder's iteration
+// of order 3, y (1 + e (1/2 + 3/8 e)) with e = 1 - d2 y^2.
+__device__ __forceinline__ void root64(double d2, double &r, double &rinv) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d2));
+  const double t = __dmul_rn(d2, y), e = __fma_rn(-t, y, 1.0), h = __dmul_rn(e, __fma_rn(0.375, e, 0.5));
+  r = __fma_rn(t, h, t);
+  rinv = __fma_rn(y, h, y);
+}
+
+// Interval of r in a table window that starts at knot lo, given base = MB_FLOOR - lo:
+// rounding base + r / dr down to a whole number leaves it in the low word.  True inside
+// the window (n intervals, all inside the cutoff): then k is the interval's place in it
+// and p the local coordinate.
+#define MB_FLOOR 6755399441055744.0 // 1.5 * 2^52
+#define MB_FLOOR_HI 0x43380000      // its high word
+__device__ __forceinline__ bool window_locate(double r, double rdr, double base, unsigned n, unsigned &k, double &p) {
+  const double s = __fma_rd(r, rdr, base);
+  k = (unsigned)__double2loint(s);
+  p = __fma_rn(r, rdr, __dsub_rn(base, s));
+  return __double2hiint(s) == MB_FLOOR_HI && k < n;
+}
+
+// The same in the whole table, for the pairs outside their window (r < cutoff).
+__device__ __forceinline__ void table_locate(double r, const DevPot &P, int &m, double &p) {
+  m = min((int)__dmul_rd(r, P.rdr), P.nr - 2);
+  p = __fma_rn(r, P.rdr, -(double)m);
+}
+
+// Squared length of d, summed as x, y, z.
+__device__ __forceinline__ double len2(double dx, double dy, double dz) {
+  return __fma_rn(dz, dz, __fma_rn(dy, dy, __dmul_rn(dx, dx)));
+}
+
+// Spline value between the knots k0 = {y, s} and k1: cubic Hermite piece.
+__device__ __forceinline__ double hermite64(double2 k0, double2 k1, double p) {
+  const double dy = __dsub_rn(k1.x, k0.x), u = __dsub_rn(dy, k0.y), c3 = __dsub_rn(__dsub_rn(k1.y, dy), u);
+  return __fma_rn(__fma_rn(__fma_rn(c3, p, __dsub_rn(u, c3)), p, k0.y), p, k0.x);
+}
+
+// {f', phi'} on an interval from its end values d0, d1 and quadratic coefficients c.
+__device__ __forceinline__ double2 slopes(double2 d0, double2 c, double2 d1, double p) {
+  return make_double2(__fma_rn(__fma_rn(c.x, p, __dsub_rn(__dsub_rn(d1.x, d0.x), c.x)), p, d0.x),
+                      __fma_rn(__fma_rn(c.y, p, __dsub_rn(__dsub_rn(d1.y, d0.y), c.y)), p, d0.y));
+}
+
+// Table window in shared memory: one (density) or two (force) 16-byte words per knot,
+// COPIES interleaved copies of every word, lane l reading copy l % COPIES; k0 is the window's first knot.  With 8 copies
+// the 8 lanes that a wavefront of 16-byte loads serves read 8 different bank groups,
+// whatever their knots.
+template <int COPIES>
+struct Window64 {
+  const double2 *w; // this lane's copy of the window's first knot
+  double base;      // MB_FLOOR - first knot
+  unsigned n;       // intervals
+};
+
+// Whether a pair outside its window may be inside the cutoff (vacant sites are far away).
+__device__ __forceinline__ bool maybe_in(const LatticeArgs &a, double d2) { return __double2hiint(d2) <= a.rc2_hi; }
+
+// Density term of a pair; false outside the window.
+template <int COPIES>
+__device__ __forceinline__ bool rho_pair64(const Window64<COPIES> &W, const DevPot &P, double d2, double &v) {
+  double r, rinv, p;
+  unsigned k;
+  root64(d2, r, rinv);
+  const bool ok = window_locate(r, P.rdr, W.base, W.n, k, p);
+  const double2 *q = W.w + min(k, W.n - 1) * COPIES;
+  v = hermite64(q[0], q[COPIES], p);
+  return ok;
+}
+__device__ __forceinline__ double rho_table64(const DevPot &P, double d2) {
+  double r, rinv, p;
+  int m;
+  root64(d2, r, rinv);
+  table_locate(r, P, m, p);
+  return hermite64(__ldg(P.f_ys + m), __ldg(P.f_ys + m + 1), p);
+}
+
+// fpair = -((df_i + df_j) f'(r) + phi'(r)) / r of a pair; false outside the window.  With
+// ENERGY e is half its pair energy (inside the window).
+template <bool ENERGY>
+__device__ __forceinline__ double half_phi64(const DevPot &P, int m, double p) {
+  const double4 v = ldg4(P.phi_val + m);
+  return __dmul_rn(0.5, __fma_rn(__fma_rn(__fma_rn(v.w, p, v.z), p, v.y), p, v.x));
+}
+template <int COPIES, bool ENERGY>
+__device__ __forceinline__ bool force_pair64(const Window64<COPIES> &W, const DevPot &P, double d2, double dfs,
+                                             double &f, double &e) {
+  double r, rinv, p;
+  unsigned k;
+  root64(d2, r, rinv);
+  const bool ok = window_locate(r, P.rdr, W.base, W.n, k, p);
+  const double2 *q = W.w + min(k, W.n - 1) * (2 * COPIES);
+  const double2 s = slopes(q[0], q[COPIES], q[2 * COPIES], p);
+  f = __dmul_rn(-__fma_rn(dfs, s.x, s.y), rinv);
+  if (ENERGY && ok) e = half_phi64<true>(P, (int)k + (int)(MB_FLOOR - W.base), p);
+  return ok;
+}
+template <bool ENERGY>
+__device__ __forceinline__ double force_table64(const DevPot &P, double d2, double dfs, double &e) {
+  double r, rinv, p;
+  int m;
+  root64(d2, r, rinv);
+  table_locate(r, P, m, p);
+  const double2 *t = P.force2 + 2 * (size_t)m;
+  const double2 s = slopes(__ldg(t), __ldg(t + 1), __ldg(t + 2), p);
+  if (ENERGY) e = half_phi64<true>(P, m, p);
+  return __dmul_rn(-__fma_rn(dfs, s.x, s.y), rinv);
+}
+
+// A site at work: its record, F' and stencil offsets.
+struct Site64 {
+  const double4 *p;  // its record
+  const int *off;    // the stencil of its sublattice
+  double x, y, z, w; // position and F'
+};
+
+// ------------------------------------------------------------------ runs
+// The pairs of a run that fell outside their window: entries k0 + b for the bits b of `far`.
+__device__ __forceinline__ void rho_far(const LatticeArgs &a, const Site64 &c, int k0, unsigned far, double &t) {
+  while (far) {
+    const int k = k0 + __ffs(far) - 1;
+    far &= far - 1;
+    const double4 q = ld_site(c.p + c.off[k]);
+    const double d2 = len2(c.x - q.x, c.y - q.y, c.z - q.z);
+    if (d2 < a.rc2) t = __dadd_rn(t, rho_table64(a.P, d2));
+  }
+}
+template <bool ENERGY>
+__device__ __forceinline__ void force_far(const LatticeArgs &a, const Site64 &c, int k0, unsigned far, double &fx,
+                                          double &fy, double &fz, double &ep) {
+  while (far) {
+    const int k = k0 + __ffs(far) - 1;
+    far &= far - 1;
+    const double4 q = ld_site(c.p + c.off[k]);
+    const double dx = c.x - q.x, dy = c.y - q.y, dz = c.z - q.z, d2 = len2(dx, dy, dz);
+    if (d2 < a.rc2) {
+      double e;
+      const double f = force_table64<ENERGY>(a.P, d2, __dadd_rn(c.w, q.w), e);
+      fx = __fma_rn(dx, f, fx);
+      fy = __fma_rn(dy, f, fy);
+      fz = __fma_rn(dz, f, fz);
+      if (ENERGY) ep += e;
+    }
+  }
+}
+
+// One near entry of a run (bit: its place in the run), q the neighbour's record.
+template <int COPIES>
+__device__ __forceinline__ void rho_near(const LatticeArgs &a, const Window64<COPIES> &W, const Site64 &c,
+                                         const double4 &q, int bit, double &t, unsigned &far) {
+  const double d2 = len2(c.x - q.x, c.y - q.y, c.z - q.z);
+  double v;
+  const bool ok = rho_pair64(W, a.P, d2, v);
+  if (ok) t = __dadd_rn(t, v);
+  if (!ok && maybe_in(a, d2)) far |= 1u << bit;
+}
+template <int COPIES, bool ENERGY>
+__device__ __forceinline__ void force_near(const LatticeArgs &a, const Window64<COPIES> &W, const Site64 &c,
+                                           const double4 &q, int bit, double &fx, double &fy, double &fz,
+                                           double &ep, unsigned &far) {
+  const double dx = c.x - q.x, dy = c.y - q.y, dz = c.z - q.z, d2 = len2(dx, dy, dz);
+  double f, e;
+  const bool ok = force_pair64<COPIES, ENERGY>(W, a.P, d2, __dadd_rn(c.w, q.w), f, e);
+  if (ok) {
+    fx = __fma_rn(dx, f, fx);
+    fy = __fma_rn(dy, f, fy);
+    fz = __fma_rn(dz, f, fz);
+    if (ENERGY) ep += e;
+  }
+  if (!ok && maybe_in(a, d2)) far |= 1u << bit;
+}
+
+// The outer entries [k0, k1) of a density sum; near: bit k - k0 set when entry k lies
+// inside the margin of the masks.
+__device__ __forceinline__ double rho_outer(const LatticeArgs &a, const Site64 &c, int k0, int k1, unsigned &near) {
+  double t = 0.0;
+#pragma unroll 4
+  for (int k = k0; k < k1; k++) {
+    const double4 q = ld_site(c.p + c.off[k]);
+    const double d2 = len2(c.x - q.x, c.y - q.y, c.z - q.z);
+    near |= (unsigned)(d2 < a.rc2m) << (k - k0);
+  }
+  // inside the margin: nearly always inside the cutoff too
+  rho_far(a, c, k0, near, t);
+  return t;
+}
+
+// The outer entries [k0, k1) of a force whose bit k - k0 of `bits` is set (the others are
+// beyond the cutoff for every lane of the item).
+template <bool ENERGY>
+__device__ __forceinline__ void force_outer(const LatticeArgs &a, const Site64 &c, int k0, int k1, unsigned bits,
+                                            double &fx, double &fy, double &fz, double &ep) {
+  fx = fy = fz = 0.0;
+  bits &= (1u << (k1 - k0)) - 1u;
+  unsigned in = 0;
+  while (bits) {
+    const int b = __ffs(bits) - 1;
+    bits &= bits - 1;
+    const double4 q = ld_site(c.p + c.off[k0 + b]);
+    in |= (unsigned)(len2(c.x - q.x, c.y - q.y, c.z - q.z) < a.rc2) << b;
+  }
+  force_far<ENERGY>(a, c, k0, in, fx, fy, fz, ep);
+}
+
+// --------------------------------------------------------- ends of a site
+__device__ __forceinline__ void decode_site(const Geom &g, int i, int &s, int &cx, int &y, int &z) {
+  const unsigned E = (unsigned)g.E, u = (unsigned)i;
+  s = u >= E;
+  const unsigned r = u - (s ? E : 0u), row = r / (unsigned)g.ecx;
+  cx = (int)(r - row * (unsigned)g.ecx) - g.gcx;
+  const unsigned ez = row / (unsigned)g.ey;
+  z = (int)ez - g.gz;
+  y = (int)(row - ez * (unsigned)g.ey) - g.gy;
+}
+
+// df = F'(rho), its ghost images; returns F(rho) with ENERGY.
+template <bool ENERGY>
+__device__ __forceinline__ double rho_finish64(const Geom &g, const DevPot &P, const Lattice64 &L, int ti, int ref,
+                                               double rho) {
+  const int i = ref & MB_SITE_INDEX;
+  const double df = dF64(P, ti, rho);
+  L.p[i].w = df;
+  L.rho[i] = rho;
+  if (g.images && (ref & MB_SITE_FACE)) {
+    int s, cx, y, z;
+    decode_site(g, i, s, cx, y, z);
+    for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.p[idx].w = df; });
+  }
+  return ENERGY ? F64(P, ti, rho) : 0.0;
+}
+
+// Lists the box site of a drifted lattice atom that left its site (conversion on).
+__device__ __forceinline__ void conv_check(const Geom &g, const StepParams &sp, int s, int cx, int y, int z, double nx,
+                                           double ny, double nz) {
+  if (!(sp.conv2 > 0.0)) return;
+  double X, Y, Z;
+  site_ideal(s, cx, y, z, sp.a0, X, Y, Z);
+  const double ux = nx - X, uy = ny - Y, uz = nz - Z;
+  if (ux * ux + uy * uy + uz * uz <= sp.conv2) return;
+  const int slot = atomicAdd(sp.cand_n, 1);
+  if (slot < MB_CAND_CAP) sp.cand[slot] = ((long long)z * g.by + y) * (2LL * g.bcx) + 2LL * cx + s;
+}
+
+// Force of a site: stores it, closes the previous step, drifts to the next positions (and
+// their ghost images); returns the kinetic energy with ENERGY.
+template <bool ENERGY>
+__device__ __forceinline__ double force_finish64(const Geom &g, const Lattice64 &L, const StepParams &sp, int ref,
+                                                 const Site64 &c, double fx, double fy, double fz) {
+  double ek = 0.0;
+  const int i = ref & MB_SITE_INDEX;
+  L.fx[i] = fx;
+  L.fy[i] = fy;
+  L.fz[i] = fz;
+  if (!L.vx) return ek;
+  double vx = L.vx[i], vy = L.vy[i], vz = L.vz[i];
+  if (sp.kick_pre) {
+    vx = __fma_rn(sp.h, fx, vx);
+    vy = __fma_rn(sp.h, fy, vy);
+    vz = __fma_rn(sp.h, fz, vz);
+  }
+  if (ENERGY) ek = 0.5 * sp.mass * (vx * vx + vy * vy + vz * vz) * MB_MVV2E;
+  if (sp.drift) {
+    vx = __fma_rn(sp.h, fx, vx);
+    vy = __fma_rn(sp.h, fy, vy);
+    vz = __fma_rn(sp.h, fz, vz);
+    const double nx = __fma_rn(sp.dt, vx, c.x), ny = __fma_rn(sp.dt, vy, c.y), nz = __fma_rn(sp.dt, vz, c.z);
+    st_site(L.n + i, nx, ny, nz, 0.0);
+    const bool face = g.images && (ref & MB_SITE_FACE);
+    if (face || sp.conv2 > 0.0) {
+      int s, cx, y, z;
+      decode_site(g, i, s, cx, y, z);
+      conv_check(g, sp, s, cx, y, z, nx, ny, nz);
+      if (face)
+        for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
+          st_site(L.n + idx, nx + ox, ny + oy, nz + oz, 0.0);
+        });
+    }
+  }
+  L.vx[i] = vx;
+  L.vy[i] = vy;
+  L.vz[i] = vz;
+  return ek;
+}
+
+} // namespace mb

@@ -142,7 +142,7 @@ int pot_build(const mb_eam_tables *t, PotHost **out) {
 
   std::vector<double4> f_val((size_t)nt * nr), f_der((size_t)nt * nr), F_val((size_t)nt * nrho),
       F_der((size_t)nt * nrho), phi_val((size_t)np * nr), phi_der((size_t)np * nr);
-  std::vector<double2> force1((size_t)nr * 3);
+  std::vector<double2> force1((size_t)nr * 3), force2((size_t)nr * 2), f_ys((size_t)nr);
   std::vector<float4> f_val32((size_t)nt * nr), phi_val32((size_t)nr);
   std::vector<float2> force32((size_t)nr * 3);
   std::vector<double> c7;
@@ -172,6 +172,9 @@ int pot_build(const mb_eam_tables *t, PotHost **out) {
     force32[(size_t)m * 3 + 0] = make_float2((float)fd.x, (float)pd.x);
     force32[(size_t)m * 3 + 1] = make_float2((float)fd.y, (float)pd.y);
     force32[(size_t)m * 3 + 2] = make_float2((float)fd.z, (float)pd.z);
+    f_ys[m] = make_double2(f_val[m].x, f_val[m].y);
+    force2[2 * (size_t)m] = make_double2(fd.x, pd.x);
+    force2[2 * (size_t)m + 1] = make_double2(fd.z, pd.z);
     const double4 pv = phi_val[m];
     phi_val32[m] = make_float4((float)pv.x, (float)pv.y, (float)pv.z, (float)pv.w);
   }
@@ -197,7 +200,8 @@ int pot_build(const mb_eam_tables *t, PotHost **out) {
                o_f1 = reserve(force1.size() * sizeof(double2)), o_fv32 = reserve(f_val32.size() * sizeof(float4)),
                o_f32 = reserve(force32.size() * sizeof(float2)), o_pv32 = reserve(phi_val32.size() * sizeof(float4)),
                o_fs = reserve(fs.size() * sizeof(float2)), o_ab = reserve(ab.size() * sizeof(float2)),
-               o_ps = reserve(ps.size() * sizeof(float4));
+               o_ps = reserve(ps.size() * sizeof(float4)),
+               o_ys = reserve(f_ys.size() * sizeof(double2)), o_f2 = reserve(force2.size() * sizeof(double2));
   PotHost *p = new PotHost();
   cudaError_t e = cudaMalloc(&p->blob, off);
   if (e != cudaSuccess) {
@@ -213,6 +217,8 @@ int pot_build(const mb_eam_tables *t, PotHost **out) {
   memcpy(&staging[o_pv], phi_val.data(), phi_val.size() * sizeof(double4));
   memcpy(&staging[o_pd], phi_der.data(), phi_der.size() * sizeof(double4));
   memcpy(&staging[o_f1], force1.data(), force1.size() * sizeof(double2));
+  memcpy(&staging[o_ys], f_ys.data(), f_ys.size() * sizeof(double2));
+  memcpy(&staging[o_f2], force2.data(), force2.size() * sizeof(double2));
   memcpy(&staging[o_fv32], f_val32.data(), f_val32.size() * sizeof(float4));
   memcpy(&staging[o_f32], force32.data(), force32.size() * sizeof(float2));
   memcpy(&staging[o_pv32], phi_val32.data(), phi_val32.size() * sizeof(float4));
@@ -242,6 +248,8 @@ int pot_build(const mb_eam_tables *t, PotHost **out) {
   d.phi_val = (const double4 *)(b + o_pv);
   d.phi_der = (const double4 *)(b + o_pd);
   d.force1 = (const double2 *)(b + o_f1);
+  d.f_ys = (const double2 *)(b + o_ys);
+  d.force2 = (const double2 *)(b + o_f2);
   d.f_val32 = (const float4 *)(b + o_fv32);
   d.force32 = (const float2 *)(b + o_f32);
   d.phi_val32 = (const float4 *)(b + o_pv32);

@@ -1,0 +1,398 @@
+// FP64 lattice passes with one-type tables for large launches: shell by shell, each with
+// its own replicated table window in shared memory.
+//
+// What bounds a pass with one copy of the table is the SM's 128-byte/clock data stage: in
+// a thermally disordered lattice the 32 lanes of a stencil entry look up random knots, and
+// a 16-byte shared load, served 8 lanes at a time, waits for the most-used of 8 bank
+// groups (2.6 lanes on average).  Here the stencil is walked shell by shell: the knots of
+// one shell's distances are few enough for 8 copies, one per bank group, so that a lookup
+// always takes the least number of wavefronts.  A CTA runs a batch of its items through
+// one shell after the other; the partial sums of the sites rest in their rho / force
+// arrays (L2) in between.  The shells are built into the code (mb_ensemble_shells.cuh), so
+// that a neighbour costs one 32-byte load with an immediate column offset.
+// Measured on one B200, 96^3 cells at 300 K: step 1.04 -> 0.79 ms; bank conflicts 94 M + 141
+// M -> none, instructions per 32-site item 6,250 -> 3,290 (density) and 5,460 -> 3,800
+// (force).  The density pass is now at 88% of the L1TEX data stage, the force pass waits on
+// neighbour loads (24 warps per SM, 80 registers).
+#include <math.h>
+
+#include "mb_pair64.cuh"
+
+namespace mb {
+
+#ifndef MB_SHELL_RHO_THREADS
+#define MB_SHELL_RHO_THREADS 1024 // 896: step at 96^3 cells 2% slower
+#endif
+#ifndef MB_SHELL_FORCE_THREADS
+#define MB_SHELL_FORCE_THREADS 768 // 896 and 1024 (spills): step at 96^3 cells 1% and 4% slower
+#endif
+#ifndef MB_SHELL_ROUNDS
+#define MB_SHELL_ROUNDS 12 // items per warp in a batch (6: 3%, 24: 1% slower)
+#endif
+#define MB_AHEAD 4 // neighbour loads issued ahead (1, 2, 8: the same within 1%)
+#define MB_COPIES 8
+// Intervals of a window.  Density: 8 copies of 16 bytes per knot, 131 KB (860: 1% slower at
+// 300 K, 2.5% at 900 K).  Force: 8 copies of 32 bytes, 162 KB, +-0.36 A with 5,000 knots
+// (520: 2% slower at 300 K; 720 and more leave too little L1).
+#ifndef MB_RHO_WINDOW
+#define MB_RHO_WINDOW 1024
+#endif
+#ifndef MB_FORCE_WINDOW
+#define MB_FORCE_WINDOW 648
+#endif
+
+// The density pass visits neighbouring shells that share a window together: first shell of
+// each visit (the force pass, with twice the bytes per knot, visits them one by one).
+template <int NEAR>
+struct RhoVisits {
+  static constexpr int n = NEAR == 5 ? 3 : 4;
+  static constexpr int first[5] = {0, 2, 3, 5, 6};
+};
+
+// Fills the window with knots [lo, lo + n] of PER 16-byte words each, every word 8 times:
+// a thread reads a word once and lane l starts with copy l % 8, so that the stores of 8
+// lanes fall into 8 bank groups.
+template <int PER>
+__device__ __forceinline__ void fill_window(double2 *w, const double2 *tab, int lo, int n) {
+  const double2 *src = tab + PER * (size_t)lo;
+  const int words = (n + 1) * PER;
+#pragma unroll 2
+  for (int k = threadIdx.x; k < words; k += blockDim.x) {
+    const double2 v = __ldg(src + k);
+#pragma unroll
+    for (int c = 0; c < MB_COPIES; c++) w[k * MB_COPIES + ((c + threadIdx.x) & (MB_COPIES - 1))] = v;
+  }
+}
+
+// Bases of a site's neighbours: even vectors, and odd ones (on the other sublattice).
+struct Bases64 {
+  const double4 *be, *bo;
+};
+__device__ __forceinline__ Bases64 site_bases(const Geom &g, const double4 *p, int i) {
+  const int odd = i < (int)g.E ? (int)g.E : -(int)g.E + g.ey * g.ecx + g.ecx + 1;
+  return Bases64{p + i, p + i + odd};
+}
+template <int K>
+__device__ __forceinline__ double4 ld_neighbour(const Bases64 &b, int pl, int rw) {
+  using T = HStore<K>;
+  return ld_site((T::odd ? b.bo : b.be) + (T::dz * pl + T::dy * rw) + T::dx);
+}
+
+// A warp's items of a batch: w_lo, w_lo + stride, ... below w_hi.
+struct BatchItems {
+  int lo, hi, stride;
+};
+__device__ __forceinline__ int batch_count(const LatticeArgs &a, int &rounds) {
+  const int stride = gridDim.x * (blockDim.x >> 5);
+  rounds = (a.n_items - a.w0 + stride - 1) / stride;
+  return (rounds + MB_SHELL_ROUNDS - 1) / MB_SHELL_ROUNDS;
+}
+__device__ __forceinline__ BatchItems batch_items(const LatticeArgs &a, int b, int batches, int rounds) {
+  const int warps = blockDim.x >> 5, stride = gridDim.x * warps;
+  return BatchItems{a.w0 + (rounds * b / batches) * stride + (int)blockIdx.x * warps + (int)(threadIdx.x >> 5),
+                    min(a.n_items, a.w0 + (rounds * (b + 1) / batches) * stride), stride};
+}
+
+// This lane's entry of item w in the site list (none past the end of the batch).
+__device__ __forceinline__ int item_ref(const LatticeArgs &a, int w, int hi) {
+  return w < hi ? __ldg(a.sites + 32 * (size_t)w + (threadIdx.x & 31)) : -1;
+}
+
+// Density sums of shell SH's runs.
+template <int SH>
+__device__ __forceinline__ void rho_shell(const LatticeArgs &a, const Window64<MB_COPIES> &W, const Site64 &c,
+                                          const Bases64 &b, int pl, int rw, double &rho) {
+  constexpr int first = kBcc.start[SH], end = kBcc.start[SH + 1];
+  static_for<0, (end - first + MB_RUN - 1) / MB_RUN>([&](auto rc) {
+    constexpr int k0 = first + decltype(rc)::value * MB_RUN, k1 = k0 + MB_RUN < end ? k0 + MB_RUN : end;
+    double t = 0.0;
+    unsigned far = 0;
+    static_for<0, (k1 - k0 + MB_AHEAD - 1) / MB_AHEAD>([&](auto cc) {
+      constexpr int c0 = k0 + decltype(cc)::value * MB_AHEAD, c1 = c0 + MB_AHEAD < k1 ? c0 + MB_AHEAD : k1;
+      double4 q[MB_AHEAD];
+      static_for<c0, c1>([&](auto kc) { q[decltype(kc)::value - c0] = ld_neighbour<decltype(kc)::value>(b, pl, rw); });
+      static_for<c0, c1>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        rho_near(a, W, c, q[k - c0], k - k0, t, far);
+      });
+    });
+    rho_far(a, c, k0, far, t);
+    rho = __dadd_rn(rho, t);
+  });
+}
+
+template <int SH, bool ENERGY>
+__device__ __forceinline__ void force_shell(const LatticeArgs &a, const Window64<MB_COPIES> &W, const Site64 &c,
+                                            const Bases64 &b, int pl, int rw, double &fx, double &fy, double &fz,
+                                            double &ep) {
+  constexpr int first = kBcc.start[SH], end = kBcc.start[SH + 1];
+  static_for<0, (end - first + MB_RUN - 1) / MB_RUN>([&](auto rc) {
+    constexpr int k0 = first + decltype(rc)::value * MB_RUN, k1 = k0 + MB_RUN < end ? k0 + MB_RUN : end;
+    double tx = 0.0, ty = 0.0, tz = 0.0;
+    unsigned far = 0;
+    static_for<0, (k1 - k0 + MB_AHEAD - 1) / MB_AHEAD>([&](auto cc) {
+      constexpr int c0 = k0 + decltype(cc)::value * MB_AHEAD, c1 = c0 + MB_AHEAD < k1 ? c0 + MB_AHEAD : k1;
+      double4 q[MB_AHEAD];
+      static_for<c0, c1>([&](auto kc) { q[decltype(kc)::value - c0] = ld_neighbour<decltype(kc)::value>(b, pl, rw); });
+      static_for<c0, c1>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        force_near<MB_COPIES, ENERGY>(a, W, c, q[k - c0], k - k0, tx, ty, tz, ep, far);
+      });
+    });
+    force_far<ENERGY>(a, c, k0, far, tx, ty, tz, ep);
+    fx = __dadd_rn(fx, tx);
+    fy = __dadd_rn(fy, ty);
+    fz = __dadd_rn(fz, tz);
+  });
+}
+
+// NEAR: shells inside the cutoff at the ideal lattice.
+template <bool ENERGY, int NEAR>
+__global__ void __launch_bounds__(MB_SHELL_RHO_THREADS, 1)
+    k_shell_rho64(const __grid_constant__ StencilSet st, const __grid_constant__ LatticeArgs a) {
+  extern __shared__ double2 s_w[];
+  const Lattice64 &L = a.L;
+  constexpr int n_near = kBcc.start[NEAR];
+  const int lane = threadIdx.x & 31, pl = a.g.ey * a.g.ecx, rw = a.g.ecx;
+  int rounds;
+  const int batches = batch_count(a, rounds);
+  double e_acc = 0.0;
+  for (int b = 0; b < batches; b++) {
+    const BatchItems it = batch_items(a, b, batches, rounds);
+    static_for<0, RhoVisits<NEAR>::n>([&](auto vc) {
+      constexpr int V = decltype(vc)::value, SH = RhoVisits<NEAR>::first[V], END = RhoVisits<NEAR>::first[V + 1];
+      const int lo = a.sh.rho.lo[SH], cnt = a.sh.rho.cnt[SH];
+      __syncthreads();
+      fill_window<1>(s_w, a.P.f_ys, lo, cnt);
+      __syncthreads();
+      const Window64<MB_COPIES> W{s_w + (lane & (MB_COPIES - 1)), MB_FLOOR - lo, (unsigned)cnt};
+      int next = item_ref(a, it.lo, it.hi);
+      for (int w = it.lo; w < it.hi; w += it.stride) {
+        const int ref = next, i = ref & MB_SITE_INDEX;
+        next = item_ref(a, w + it.stride, it.hi); // under way while this item is worked on
+        int code = -1;
+        double4 own;
+        double rho = 0.0;
+        if (ref >= 0) { // three loads at once, before the code is looked at
+          code = L.code[i];
+          own = ld_site(L.p + i);
+          if (SH) rho = L.rho[i];
+        }
+        unsigned long long near = 0;
+        if (!(code < 0 || (a.skip_flagged && (code & MB_FLAG_ITL)))) {
+          const Site64 c{L.p + i, st.off[i >= (int)a.g.E], own.x, own.y, own.z, 0.0};
+          const Bases64 bs = site_bases(a.g, L.p, i);
+          static_for<SH, END>([&](auto hc) { rho_shell<decltype(hc)::value>(a, W, c, bs, pl, rw, rho); });
+          if (END < NEAR) {
+            L.rho[i] = rho;
+          } else {
+            for (int k0 = n_near; k0 < st.n; k0 += MB_OUT_RUN) {
+              unsigned m = 0;
+              rho = __dadd_rn(rho, rho_outer(a, c, k0, min(k0 + MB_OUT_RUN, st.n), m));
+              near |= (unsigned long long)m << (k0 - n_near);
+            }
+            const double e = rho_finish64<ENERGY>(a.g, a.P, L, code & 0x3F, ref, rho);
+            if (ENERGY) e_acc += e;
+          }
+        }
+        if (END == NEAR && a.outer) {
+          const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)near);
+          const unsigned hi = __reduce_or_sync(0xffffffffu, (unsigned)(near >> 32));
+          if (lane == 0) a.outer[w] = make_uint2(lo, hi);
+        }
+      }
+    });
+  }
+  if (ENERGY) {
+    const double t = block_sum(e_acc);
+    if (threadIdx.x == 0) a.e0[blockIdx.x] = t;
+  }
+}
+
+template <bool ENERGY, int NEAR>
+__global__ void __launch_bounds__(MB_SHELL_FORCE_THREADS, 1)
+    k_shell_force64(const __grid_constant__ StencilSet st, const __grid_constant__ LatticeArgs a) {
+  extern __shared__ double2 s_w[];
+  const Lattice64 &L = a.L;
+  constexpr int n_near = kBcc.start[NEAR];
+  const int lane = threadIdx.x & 31, pl = a.g.ey * a.g.ecx, rw = a.g.ecx;
+  int rounds;
+  const int batches = batch_count(a, rounds);
+  double e_pair = 0.0, e_kin = 0.0;
+  for (int b = 0; b < batches; b++) {
+    const BatchItems it = batch_items(a, b, batches, rounds);
+    static_for<0, NEAR>([&](auto shc) {
+      constexpr int SH = decltype(shc)::value;
+      __syncthreads();
+      const int lo = a.sh.force.lo[SH], cnt = a.sh.force.cnt[SH];
+      __syncthreads();
+      fill_window<2>(s_w, a.P.force2, lo, cnt);
+      __syncthreads();
+      const Window64<MB_COPIES> W{s_w + (lane & (MB_COPIES - 1)), MB_FLOOR - lo, (unsigned)cnt};
+      int next = item_ref(a, it.lo, it.hi);
+      for (int w = it.lo; w < it.hi; w += it.stride) {
+        const int ref = next, i = ref & MB_SITE_INDEX;
+        next = item_ref(a, w + it.stride, it.hi);
+        if (ref < 0) continue;
+        const int code = L.code[i];
+        const double4 own = ld_site(L.p + i);
+        double fx = 0.0, fy = 0.0, fz = 0.0;
+        if (SH) {
+          fx = L.fx[i];
+          fy = L.fy[i];
+          fz = L.fz[i];
+        }
+        if (code < 0 || (a.skip_flagged && (code & MB_FLAG_ITL))) continue;
+        const Site64 c{L.p + i, st.off[i >= (int)a.g.E], own.x, own.y, own.z, own.w};
+        force_shell<SH, ENERGY>(a, W, c, site_bases(a.g, L.p, i), pl, rw, fx, fy, fz, e_pair);
+        if (SH + 1 < NEAR) {
+          L.fx[i] = fx;
+          L.fy[i] = fy;
+          L.fz[i] = fz;
+        } else {
+          unsigned long long mask = ~0ull;
+          if (a.outer) {
+            const uint2 m2 = a.outer[w];
+            mask = (unsigned long long)m2.x | ((unsigned long long)m2.y << 32);
+          }
+          for (int k0 = n_near; k0 < st.n; k0 += MB_OUT_RUN) {
+            const unsigned bits = (unsigned)(mask >> (k0 - n_near)) & ((1u << MB_OUT_RUN) - 1u);
+            if (!bits) continue;
+            double tx, ty, tz;
+            force_outer<ENERGY>(a, c, k0, min(k0 + MB_OUT_RUN, st.n), bits, tx, ty, tz, e_pair);
+            fx = __dadd_rn(fx, tx);
+            fy = __dadd_rn(fy, ty);
+            fz = __dadd_rn(fz, tz);
+          }
+          const double ek = force_finish64<ENERGY>(a.g, L, a.sp, ref, c, fx, fy, fz);
+          if (ENERGY) e_kin += ek;
+        }
+      }
+    });
+  }
+  if (ENERGY) {
+    const double t1 = block_sum(e_pair);
+    if (threadIdx.x == 0) a.e0[blockIdx.x] = t1;
+    const double t2 = block_sum(e_kin);
+    if (threadIdx.x == 0) a.e1[blockIdx.x] = t2;
+  }
+}
+
+static size_t window_bytes(const Windows64 &w, int n, int words) {
+  int knots = 0;
+  for (int h = 0; h < n; h++) knots = w.cnt[h] + 1 > knots ? w.cnt[h] + 1 : knots;
+  return (size_t)knots * words * MB_COPIES * sizeof(double2);
+}
+
+template <int NEAR>
+static int shell_rho(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
+  MB_SMEM_ATTR((k_shell_rho64<false, NEAR>), (k_shell_rho64<true, NEAR>), MB_SMEM_MAX - 1024);
+  const size_t smem = window_bytes(a.sh.rho, a.sh.n, 1);
+  if (energy)
+    k_shell_rho64<true, NEAR><<<device_sm_count(), MB_SHELL_RHO_THREADS, smem, s>>>(st, a);
+  else
+    k_shell_rho64<false, NEAR><<<device_sm_count(), MB_SHELL_RHO_THREADS, smem, s>>>(st, a);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+template <int NEAR>
+static int shell_force(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
+  MB_SMEM_ATTR((k_shell_force64<false, NEAR>), (k_shell_force64<true, NEAR>), MB_SMEM_MAX - 1024);
+  const size_t smem = window_bytes(a.sh.force, a.sh.n, 2);
+  if (energy)
+    k_shell_force64<true, NEAR><<<device_sm_count(), MB_SHELL_FORCE_THREADS, smem, s>>>(st, a);
+  else
+    k_shell_force64<false, NEAR><<<device_sm_count(), MB_SHELL_FORCE_THREADS, smem, s>>>(st, a);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
+int launch_shell_rho64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
+  return a.sh.n == 5 ? shell_rho<5>(st, a, energy, s) : shell_rho<6>(st, a, energy, s);
+}
+int launch_shell_force64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
+  return a.sh.n == 5 ? shell_force<5>(st, a, energy, s) : shell_force<6>(st, a, energy, s);
+}
+
+// ------------------------------------------------------------------ plan
+// Least margin of a window around its shells' ideal distances: atoms displaced by 0.07 A
+// per component (300 K) put a pair 0.1 A (rms) off its ideal distance.
+#define MB_WINDOW_MARGIN 0.25 // A
+
+// Window of `cap` intervals around the distances r0 .. r1; false when it cannot hold the
+// least margin.  It ends inside the cutoff, so that a pair in the window is inside it too.
+static bool shell_window(const DevPot &P, double cutoff, double r0, double r1, int cap, int &lo, int &cnt) {
+  const int inside = (int)floor(cutoff * P.rdr) - 1; // knots inside the cutoff
+  const int mid = (int)(0.5 * (r0 + r1) * P.rdr);
+  int hi = mid + cap / 2;
+  lo = mid - cap / 2;
+  if (lo < 0) lo = 0;
+  if (hi > inside) hi = inside;
+  if (hi > P.nr - 1) hi = P.nr - 1;
+  cnt = hi - lo;
+  return cnt > 0 && 0.5 * cap >= (0.5 * (r1 - r0) + MB_WINDOW_MARGIN) * P.rdr;
+}
+
+__global__ void k_site_list(const Geom g, int cpp, int *sites) {
+  const long long n = 64LL * g.bz * cpp;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    const int p = (int)(t / (32LL * cpp)), b = (int)(t - (long long)p * 32 * cpp);
+    const int y = b / g.bcx, cx = b - y * g.bcx, s = p & 1, z = p >> 1;
+    int ref = -1;
+    if (y < g.by) {
+      ref = (int)ext_index(g, s, cx, y, z);
+      if (cx < g.gcx || cx >= g.bcx - g.gcx || y < g.gy || y >= g.by - g.gy || z < g.gz || z >= g.bz - g.gz)
+        ref |= MB_SITE_FACE;
+    }
+    sites[t] = ref;
+  }
+}
+
+int plan64_items(const Geom &g) { return 2 * g.bz * plan64_plane_items(g); }
+int plan64_plane_items(const Geom &g) { return (g.bcx * g.by + 31) / 32; }
+
+// R: the ideal distances of the (sorted) entries.  The plan applies when the near entries
+// are exactly BCC shells 1-5 or 1-6 in the order of mb_ensemble_shells.cuh, the ghost
+// frame is 2 cells wide, and the knots are coarse enough for windows of at least the least
+// margin (finer tables would read global memory too often).
+bool plan64_shells(const DevPot &P, const Geom &g, double a0, double cutoff, const double *R, const StencilSet &st,
+                   Shells64 &S) {
+  S = Shells64{};
+  S.n = st.n_near == kBcc.start[5] ? 5 : st.n_near == kBcc.start[6] ? 6 : 0;
+  if (P.n_types != 1 || !S.n || st.n - st.n_near > 64 || g.E > 0x1fffffffLL) return false;
+  double r[MB_NEAR_SHELLS];
+  for (int h = 0; h < S.n; h++) {
+    r[h] = 0.5 * a0 * sqrt((double)kBcc.n2[h]);
+    for (int k = kBcc.start[h]; k < kBcc.start[h + 1]; k++) {
+      const HVec v = kBcc.v[k];
+      if (fabs(R[k] - r[h]) > 1e-9 * r[h]) return false;
+      for (int s = 0; s < 2; s++) { // the offsets are those built into the code
+        const int s2 = (s + v.hx) & 1;
+        const int dx = (v.hx + s - s2) / 2, dy = (v.hy + s - s2) / 2, dz = (v.hz + s - s2) / 2;
+        if (st.off[s][k] != (s2 - s) * (int)g.E + (dz * g.ey + dy) * g.ecx + dx) return false;
+      }
+    }
+    if (!shell_window(P, cutoff, r[h], r[h], MB_FORCE_WINDOW, S.force.lo[h], S.force.cnt[h])) return false;
+    for (int k = kBcc.start[h]; k < kBcc.start[h + 1]; k += MB_RUN) {
+      S.shell[S.runs] = (short)h;
+      S.kb[S.runs++] = (short)k;
+    }
+  }
+  const int *first = RhoVisits<5>::first; // the visits of NEAR = 6 begin with the same shells
+  for (int v = 0; first[v] < S.n; v++)
+    for (int h = first[v]; h < first[v + 1]; h++)
+      if (!shell_window(P, cutoff, r[first[v]], r[first[v + 1] - 1], MB_RHO_WINDOW, S.rho.lo[h], S.rho.cnt[h]))
+        return false;
+  S.near_runs = S.runs;
+  for (int k = st.n_near; k < st.n; k += MB_OUT_RUN) S.kb[S.runs++] = (short)k;
+  S.kb[S.runs] = (short)st.n;
+  return split64_fits(S);
+}
+
+int plan64_sites(const Geom &g, int *sites, cudaStream_t s) {
+  k_site_list<<<8 * device_sm_count(), 256, 0, s>>>(g, plan64_plane_items(g), sites);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
+} // namespace mb

@@ -22,15 +22,16 @@ struct mb_sim {
   mb::PotHost *pot = nullptr;
   mb::Geom g{};
   mb::StencilSet st{};
+  mb::Plan64 plan{};
   std::vector<int64_t> st_even, st_odd;
   int ext_x = 0, ext_y = 0, ext_z = 0;
   long long n_ext = 0, n_box = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[8] = {};
   // lattice
-  double *pos[2][3] = {};
+  double4 *pos[2] = {}; // {x, y, z, F'(rho)} of every site, two buffers
   int8_t *code = nullptr;
-  double *df = nullptr, *rho = nullptr, *v[3] = {}, *f[3] = {};
+  double *rho = nullptr, *v[3] = {}, *f[3] = {};
   int64_t *id = nullptr;
   // per-item masks of the outer stencil entries in the cutoff: written by each density
   // pass, read by the force pass at the same positions (outer_ok: the phase-wise steps of
@@ -94,14 +95,9 @@ static int dalloc(mb_sim *s, void **p, size_t bytes) {
 
 Lattice64 sim_lattice(mb_sim *s, int which) {
   Lattice64 L{};
-  L.px = s->pos[which][0];
-  L.py = s->pos[which][1];
-  L.pz = s->pos[which][2];
-  L.nx = s->pos[which ^ 1][0];
-  L.ny = s->pos[which ^ 1][1];
-  L.nz = s->pos[which ^ 1][2];
+  L.p = s->pos[which];
+  L.n = s->pos[which ^ 1];
   L.code = s->code;
-  L.df = s->df;
   L.rho = s->rho;
   L.vx = s->v[0];
   L.vy = s->v[1];
@@ -173,11 +169,11 @@ static int step64(mb_sim *s, int energy, int kick_pre, int drift, int timed) {
   const int itl = itl_active(s);
   if (itl) MB_TRY(launch_itl_mark64(s->g, L, I, s->stream));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[4], s->stream));
-  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, ep, energy, itl, s->stream, 0, -1, s->outer));
+  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, ep, energy, itl, s->stream, 0, -1, s->outer, &s->plan));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[5], s->stream));
   if (itl) MB_TRY(launch_itl_rho64(s->g, s->st, P, L, I, sp.rc2, ep, energy, s->stream));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[6], s->stream));
-  MB_TRY(launch_force64(s->g, s->st, P, L, sp, ep, energy, itl, s->stream, 0, -1, s->outer));
+  MB_TRY(launch_force64(s->g, s->st, P, L, sp, ep, energy, itl, s->stream, 0, -1, s->outer, &s->plan));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[7], s->stream));
   if (itl) MB_TRY(launch_itl_force64(s->g, s->st, P, L, I, sp, ep, energy, s->stream));
   if (sp.conv2 > 0.0)
@@ -414,10 +410,13 @@ static int create_sim(const mb_sim_config *cfg, const mb_eam_tables *pot, int z_
   rc = stencil_generate(cfg->lattice_const, reach, s->ext_x, s->ext_y, even, odd, MB_MAX_STENCIL, &n, &rx, &ry, &rz);
   const int par[2] = {0, 1};
   int n_near = 0;
+  double dist[MB_MAX_STENCIL] = {};
   if (rc == MB_OK && pot->n_types == 1)
-    rc = stencil_sort_by_distance(cfg->lattice_const, cfg->cutoff, s->ext_x, s->ext_y, even, odd, n, &n_near);
+    rc = stencil_sort_by_distance(cfg->lattice_const, cfg->cutoff, s->ext_x, s->ext_y, even, odd, n, &n_near, dist);
   if (rc == MB_OK) rc = stencil_from_linear(even, n, odd, n, s->ext_x, s->ext_y, g, par, &s->st);
   s->st.n_near = n_near;
+  if (rc == MB_OK)
+    s->plan.ok = plan64_shells(pot_dev(s->pot), g, cfg->lattice_const, cfg->cutoff, dist, s->st, s->plan.sh);
   if (rc != MB_OK) {
     pot_free(s->pot);
     delete s;
@@ -436,13 +435,19 @@ static int create_sim(const mb_sim_config *cfg, const mb_eam_tables *pot, int z_
     if (cudaEventCreate(&e) != cudaSuccess) return cleanup(fail(MB_ERR_CUDA, "event creation failed"));
   const size_t ne = (size_t)s->n_ext;
   const bool fp64 = cfg->precision == MB_PREC_FP64;
-  for (int b = 0; b < 2; b++)
-    for (int c = 0; c < 3; c++)
-      if ((rc = dalloc(s, (void **)&s->pos[b][c], ne * sizeof(double))) != MB_OK) return cleanup(rc);
+  for (int b = 0; b < 2; b++) {
+    if ((rc = dalloc(s, (void **)&s->pos[b], ne * sizeof(double4))) != MB_OK) return cleanup(rc);
+    if (cudaMemsetAsync(s->pos[b], 0, ne * sizeof(double4), s->stream) != cudaSuccess)
+      return cleanup(fail(MB_ERR_CUDA, "memset failed"));
+  }
   if ((rc = dalloc(s, (void **)&s->code, (ne + 3) & ~(size_t)3)) != MB_OK) return cleanup(rc);
   if (fp64) {
-    if ((rc = dalloc(s, (void **)&s->df, ne * sizeof(double))) != MB_OK) return cleanup(rc);
     if ((rc = dalloc(s, (void **)&s->rho, ne * sizeof(double))) != MB_OK) return cleanup(rc);
+    if (s->plan.ok) {
+      if ((rc = dalloc(s, (void **)&s->plan.sites, 32 * sizeof(int) * (size_t)plan64_items(s->g))) != MB_OK)
+        return cleanup(rc);
+      if ((rc = plan64_sites(s->g, s->plan.sites, s->stream)) != MB_OK) return cleanup(rc);
+    }
     if (outer_masks_on() &&
         (rc = dalloc(s, (void **)&s->outer, (size_t)items_per_box(s->g) * sizeof(uint2))) != MB_OK)
       return cleanup(rc);
@@ -501,15 +506,15 @@ int mb_sim_destroy(mb_sim *s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   drop_graph(s);
   if (s->ens) mb_ensemble_destroy(s->ens);
-  void *ptrs[] = {s->code, s->df, s->rho, s->outer, s->id, s->epart, s->eout, s->stage, s->bad, s->irho, s->idf, s->itype,
+  void *ptrs[] = {s->code, s->rho, s->outer, s->plan.sites, s->id, s->epart, s->eout, s->stage, s->bad, s->irho, s->idf, s->itype,
                   s->iid, s->flag_list, s->flag_count, s->d_nitl, s->d_cand, s->d_cand_n, s->d_conv_counters};
   for (void *p : ptrs)
     if (p) cudaFree(p);
-  for (int b = 0; b < 2; b++)
-    for (int c = 0; c < 3; c++) {
-      if (s->pos[b][c]) cudaFree(s->pos[b][c]);
+  for (int b = 0; b < 2; b++) {
+    if (s->pos[b]) cudaFree(s->pos[b]);
+    for (int c = 0; c < 3; c++)
       if (s->ipos[b][c]) cudaFree(s->ipos[b][c]);
-    }
+  }
   for (int c = 0; c < 3; c++) {
     if (s->v[c]) cudaFree(s->v[c]);
     if (s->f[c]) cudaFree(s->f[c]);
@@ -663,8 +668,7 @@ int mb_sim_download(mb_sim *s, mb_atom_element *box_atoms, mb_atom_element *itl,
   const int which = s->primed ? (s->cur ^ 1) : s->cur;
   const int unkick = s->primed ? 1 : 0;
   Lattice64 L = sim_lattice(s, s->cur);
-  MB_TRY(launch_pack_box_ids(s->g, s->stage, L, s->pos[which][0], s->pos[which][1], s->pos[which][2],
-                             sim_params(s, 0, 0).h, unkick, s->id, s->stream));
+  MB_TRY(launch_pack_box_ids(s->g, s->stage, L, s->pos[which], sim_params(s, 0, 0).h, unkick, s->id, s->stream));
   MB_CUDA(cudaMemcpyAsync(box_atoms, s->stage, (size_t)s->n_box * sizeof(mb_atom_element), cudaMemcpyDeviceToHost,
                           s->stream));
   MB_CUDA(cudaStreamSynchronize(s->stream));
@@ -811,7 +815,7 @@ static int step_host_whole(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
   MB_CUDA(cudaMemcpyAsync(s->stage, box_atoms, (size_t)s->n_box * sizeof(mb_atom_element), cudaMemcpyHostToDevice,
                           s->stream));
   Lattice64 L = sim_lattice(s, 0);
-  L.nx = L.ny = L.nz = nullptr;
+  L.n = nullptr;
   MB_TRY(launch_unpack_box_ids(s->g, s->stage, L, 1, s->bad, s->id, pot_dev(s->pot).n_types, s->stream));
   MB_TRY(launch_images64(s->g, L, 1, s->stream));
   MB_TRY(upload_itl(s, itl, n_itl, 1));
@@ -821,11 +825,11 @@ static int step_host_whole(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
   const DevPot &P = pot_dev(s->pot);
   const int it = s->n_itl > 0;
   if (it) MB_TRY(launch_itl_mark64(s->g, L, I, s->stream));
-  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, nullptr, 0, it, s->stream, 0, -1, s->outer));
+  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, nullptr, 0, it, s->stream, 0, -1, s->outer, &s->plan));
   if (it) MB_TRY(launch_itl_rho64(s->g, s->st, P, L, I, sp.rc2, nullptr, 0, s->stream));
-  MB_TRY(launch_force64(s->g, s->st, P, L, sp, nullptr, 0, it, s->stream, 0, -1, s->outer));
+  MB_TRY(launch_force64(s->g, s->st, P, L, sp, nullptr, 0, it, s->stream, 0, -1, s->outer, &s->plan));
   if (it) MB_TRY(launch_itl_force64(s->g, s->st, P, L, I, sp, nullptr, 0, s->stream));
-  MB_TRY(launch_pack_box_ids(s->g, s->stage, L, L.px, L.py, L.pz, sp.h, 0, s->id, s->stream));
+  MB_TRY(launch_pack_box_ids(s->g, s->stage, L, L.p, sp.h, 0, s->id, s->stream));
   MB_CUDA(cudaMemcpyAsync(box_atoms, s->stage, (size_t)s->n_box * sizeof(mb_atom_element), cudaMemcpyDeviceToHost,
                           s->stream));
   MB_CUDA(cudaStreamSynchronize(s->stream));
@@ -863,7 +867,7 @@ static int step_host_slabs(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
     return urc;
   }
   Lattice64 L = sim_lattice(s, 0);
-  L.nx = L.ny = L.nz = nullptr;
+  L.n = nullptr;
   Itl64 I = sim_itl(s, 0);
   const StepParams sp = sim_params(s, 1, 0);
   const DevPot &P = pot_dev(s->pot);
@@ -882,14 +886,14 @@ static int step_host_slabs(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
     return MB_OK;
   };
   auto rho = [&](int k) -> int {
-    MB_TRY(launch_rho64(g, s->st, P, L, sp.rc2, nullptr, 0, it, cs, zb[k], zb[k + 1], s->outer));
+    MB_TRY(launch_rho64(g, s->st, P, L, sp.rc2, nullptr, 0, it, cs, zb[k], zb[k + 1], s->outer, &s->plan));
     if (it) MB_TRY(launch_itl_rho64(g, s->st, P, L, I, sp.rc2, nullptr, 0, cs, zb[k], zb[k + 1]));
     return MB_OK;
   };
   auto force = [&](int k) -> int {
-    MB_TRY(launch_force64(g, s->st, P, L, sp, nullptr, 0, it, cs, zb[k], zb[k + 1], s->outer));
+    MB_TRY(launch_force64(g, s->st, P, L, sp, nullptr, 0, it, cs, zb[k], zb[k + 1], s->outer, &s->plan));
     if (it) MB_TRY(launch_itl_force64(g, s->st, P, L, I, sp, nullptr, 0, cs, zb[k], zb[k + 1]));
-    MB_TRY(launch_pack_box_ids(g, s->stage, L, L.px, L.py, L.pz, sp.h, 0, s->id, cs, zb[k], zb[k + 1]));
+    MB_TRY(launch_pack_box_ids(g, s->stage, L, L.p, sp.h, 0, s->id, cs, zb[k], zb[k + 1]));
     MB_CUDA(cudaEventRecord(s->ev_out[k], cs));
     MB_CUDA(cudaStreamWaitEvent(s->cp_out, s->ev_out[k], 0));
     const long long r0 = zb[k] * layer, r1 = zb[k + 1] * layer;
@@ -1017,9 +1021,8 @@ int mb_sim_halo_bytes(mb_sim *s, int32_t what, int64_t *bytes) {
 static int halo(mb_sim *s, int what, int pack, int side, void *buf, double z_shift) {
   if (!s || s->ens) return fail(MB_ERR_ARG, "bad arguments");
   if (!s->slab) return fail(MB_ERR_STATE, "halo layers belong to z-slab runs (mb_sim_create_slab)");
-  double *c0 = what == 1 ? s->pos[s->cur][0] : s->df, *c1 = s->pos[s->cur][1], *c2 = s->pos[s->cur][2];
   if (!pack && what != 2) s->outer_ok = false; // new ghost positions or codes: the masks are stale
-  MB_TRY(launch_halo(s->g, what, pack, side, c0, c1, c2, s->code, buf, z_shift, s->stream));
+  MB_TRY(launch_halo(s->g, what, pack, side, s->pos[s->cur], s->code, buf, z_shift, s->stream));
   MB_CUDA(cudaStreamSynchronize(s->stream));
   return MB_OK;
 }
@@ -1044,13 +1047,14 @@ int mb_sim_slab_phase(mb_sim *s, int32_t phase, int32_t energy) {
   if (phase == 0) {
     if (energy) MB_CUDA(cudaMemsetAsync(s->epart, 0, sizeof(double) * energy_partials_needed(), s->stream));
     MB_TRY(launch_rho64(s->g, s->st, P, L, s->cfg.cutoff * s->cfg.cutoff, ep, energy, 0, s->stream, 0, -1,
-                        s->outer));
+                        s->outer, &s->plan));
     s->outer_ok = true;
     return MB_OK;
   }
   // forces at pos[cur], closing kick of the previous step (once primed), drift to pos[cur ^ 1]
   const StepParams sp = sim_params(s, s->primed ? 1 : 0, 1);
-  MB_TRY(launch_force64(s->g, s->st, P, L, sp, ep, energy, 0, s->stream, 0, -1, s->outer_ok ? s->outer : nullptr));
+  MB_TRY(launch_force64(s->g, s->st, P, L, sp, ep, energy, 0, s->stream, 0, -1, s->outer_ok ? s->outer : nullptr,
+                        &s->plan));
   s->outer_ok = false;
   const long long n = s->primed ? s->step + 1 : 0;
   s->step = n;
