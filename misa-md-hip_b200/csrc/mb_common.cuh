@@ -23,7 +23,11 @@
 #define MB_FTM2V 9.64853321233e-3 // (eV/A)/amu -> A/fs^2
 #define MB_MVV2E (1.0 / MB_FTM2V) // amu A^2/fs^2 -> eV
 #define MB_VACANT_POS 1.0e30      // position given to vacant sites: every r^2 test rejects them
-#define MB_FLAG_ITL 0x40          // site code bit: an interstitial is within reach
+// Site code: type, or negative for a vacancy; two bits mark a site that has an interstitial
+// within reach, one for the steps at either position buffer (a step's marks can be set while
+// the last step's come off).
+#define MB_TYPE_MASK 0x1F
+#define MB_FLAG_ITL(cur) ((cur) ? 0x20 : 0x40)
 
 namespace mb {
 
@@ -178,7 +182,7 @@ bool split64_fits(const Shells64 &sh);
 // ------------------------------------------------------ kernel arguments
 struct Lattice64 {
   double4 *p;           // {x, y, z, F'(rho)} of every site (ext), 32-byte aligned
-  int8_t *code;         // type, < 0 vacant, MB_FLAG_ITL marks sites near an interstitial
+  int8_t *code;         // type, < 0 vacant, MB_FLAG_ITL bits
   double *rho;          // optional rho output (ext) or nullptr
   double *vx, *vy, *vz; // velocities (box sites used)
   double *fx, *fy, *fz; // forces (box sites used)
@@ -195,8 +199,10 @@ struct Itl64 {
   double *vx, *vy, *vz, *fx, *fy, *fz, *rho, *df;
   int8_t *type;
   int64_t *id;
-  int *flag_list;          // flagged box sites (ext index)
-  int *flag_count;         // [0] this step, [1] overflow marker
+  int flag;                // this step's mark in the site codes
+  int *flag_list, *flag_count; // sites marked this step (ext index)
+  int *old_list, *old_count;   // ... and last step, whose marks are the other bit
+  int *overflow;               // set when a list is too short
   double a0, reach;        // window radius in A (cutoff + skin)
 };
 
@@ -226,6 +232,8 @@ __host__ __device__ __forceinline__ void site_ideal(int s, int cx, int y, int z,
 }
 
 // kernels (mb_kernels64.cu)
+// flag: the code bit of sites near an interstitial (0: none): a lattice pass leaves the sums
+// over lattice atoms in rho / force of such a site and the interstitial pass finishes it.
 // [z0, z1): the box layers a launch covers (z1 < 0: up to the last layer).  The
 // interstitial passes then take the flagged sites in those layers and the
 // interstitials whose wrapped z lies in them.
@@ -235,10 +243,10 @@ __host__ __device__ __forceinline__ void site_ideal(int s, int cx, int y, int z,
 // those entries, so it must run on the positions of the density pass that wrote them
 // (null: the force pass walks every entry).
 int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, double rc2,
-                 double *e_partial, int energy, int skip_flagged, cudaStream_t s, int z0 = 0, int z1 = -1,
+                 double *e_partial, int energy, int flag, cudaStream_t s, int z0 = 0, int z1 = -1,
                  uint2 *outer = nullptr, const Plan64 *plan = nullptr);
 int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, const StepParams &sp,
-                   double *e_partial, int energy, int skip_flagged, cudaStream_t s, int z0 = 0, int z1 = -1,
+                   double *e_partial, int energy, int flag, cudaStream_t s, int z0 = 0, int z1 = -1,
                    const uint2 *outer = nullptr, const Plan64 *plan = nullptr);
 // Work items (32-site row chunks) of the whole box: the length of the outer masks.
 inline long long items_per_box(const Geom &g) { return (long long)((g.bcx + 31) / 32) * g.by * 2 * g.bz; }
@@ -249,14 +257,16 @@ inline bool outer_masks_on() {
   const char *v = getenv("MB_OUTER_MASKS");
   return !(v && v[0] == '0');
 }
-int launch_itl_mark64(const Geom &g, const Lattice64 &L, const Itl64 &I, cudaStream_t s);
-// Flags the sites of layers [z0, z1) near an interstitial, without clearing or
-// resetting the list first.
-int launch_itl_mark_slab64(const Geom &g, const Lattice64 &L, const Itl64 &I, int z0, int z1, cudaStream_t s);
-int launch_itl_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, const Itl64 &I,
-                     double rc2, double *e_partial, int energy, cudaStream_t s, int z0 = 0, int z1 = -1);
-int launch_itl_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, const Itl64 &I,
-                       const StepParams &sp, double *e_partial, int energy, cudaStream_t s, int z0 = 0, int z1 = -1);
+// Marks the sites of layers [z0, z1) near an interstitial; with clear set, last step's marks
+// come off.  This step's list must be empty: a force pass empties the other one.
+int launch_itl_mark64(const Geom &g, const Lattice64 &L, const Itl64 &I, int clear, cudaStream_t s, int z0 = 0,
+                      int z1 = -1);
+// Takes off the marks of both lists and empties them.
+int launch_itl_reset64(const Lattice64 &L, const Itl64 &I, cudaStream_t s);
+int launch_itl_rho64(const Geom &g, const DevPot &pot, const Lattice64 &L, const Itl64 &I, double rc2,
+                     double *e_partial, int energy, cudaStream_t s, int z0 = 0, int z1 = -1);
+int launch_itl_force64(const Geom &g, const DevPot &pot, const Lattice64 &L, const Itl64 &I, const StepParams &sp,
+                       double *e_partial, int energy, cudaStream_t s, int z0 = 0, int z1 = -1);
 int launch_images64(const Geom &g, const Lattice64 &L, int what, cudaStream_t s, int z0 = 0,
                     int z1 = -1); // what: 1 pos+code, 2 df
 // Lattice <-> interstitial bookkeeping after a drift (one CTA): candidates of

@@ -179,44 +179,6 @@ __device__ __forceinline__ bool window_site(const Geom &g, const Window &w, int 
   return true;
 }
 
-// The reach test of candidate c alone (the same arithmetic as window_site /
-// window_site_rel, so the same candidates pass).
-__device__ __forceinline__ bool window_in_reach(const Window &w, int c, double qx, double qy, double qz, double a0,
-                                                double R) {
-  const int ix = c % w.nx;
-  const int rest = c / w.nx;
-  const int iy = rest % w.ny;
-  const int iz = rest / w.ny;
-  const int gx = w.gx0 + ix, gy = w.gy0 + iy, gz = w.gz0 + iz;
-  const double h = 0.5 * (double)(gx & 1);
-  const double ox = 0.5 * a0 * gx - qx, oy = a0 * (gy + h) - qy, oz = a0 * (gz + h) - qz;
-  return ox * ox + oy * oy + oz * oz < R * R;
-}
-
-// In-reach candidates of a window, listed by one warp in candidate order: list[k] for
-// k < the returned count (list: this warp's cap entries of shared memory).  The reach
-// test is cheap arithmetic and about 1 candidate in 8 passes (a sphere in its bounding
-// box of sites), so the walk that follows loads only real sites, several per lane at
-// once, instead of one dependent load chain per round of 32 candidates.  Returns -1
-// when more than cap candidates pass (the caller then walks every candidate).
-__device__ __forceinline__ int window_compact(const Window &w, double qx, double qy, double qz, double a0, double R,
-                                              int *list, int cap) {
-  const int lane = threadIdx.x & 31;
-  const int ncand = w.nx * w.ny * w.nz;
-  int n = 0;
-  for (int base = 0; base < ncand; base += 32) {
-    const int c = base + lane;
-    const bool in = c < ncand && window_in_reach(w, c, qx, qy, qz, a0, R);
-    const unsigned m = __ballot_sync(0xffffffffu, in);
-    const int k = n + __popc(m & ((1u << lane) - 1u));
-    if (in && k < cap) list[k] = c;
-    n += __popc(m);
-  }
-  __syncwarp();
-  return n <= cap ? n : -1;
-}
-#define MB_WIN_LIST 256 // compacted window entries per warp
-
 // Appends this lane's entry (when `add`) to list[0 .. cap) with one atomicAdd on *count
 // per warp instead of one per lane (many lanes appending at once would serialise on the
 // counter); every lane of the warp must call it.  Entries past cap are dropped and
@@ -234,6 +196,26 @@ __device__ __forceinline__ void warp_append(bool add, int value, int *count, int
     list[slot] = value;
   else
     *overflow = 1;
+}
+
+// Sets a bit of a site code, or takes it off, while other threads change neighbouring codes
+// or other bits; code_bit_on returns whether it was off.
+__device__ __forceinline__ bool code_bit_on(int8_t *code, int bit) {
+  const uintptr_t addr = (uintptr_t)code;
+  const unsigned int m = (unsigned int)bit << (8 * (addr & 3));
+  return !(atomicOr((unsigned int *)(addr & ~(uintptr_t)3), m) & m);
+}
+__device__ __forceinline__ void code_bit_off(int8_t *code, int bits) {
+  const uintptr_t addr = (uintptr_t)code;
+  atomicAnd((unsigned int *)(addr & ~(uintptr_t)3), ~((unsigned int)bits << (8 * (addr & 3))));
+}
+
+// Sum over the 8 lanes of a group (lanes 8g .. 8g + 7), in a fixed order.
+__device__ __forceinline__ double group8_sum(double v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v;
 }
 
 // Same candidate walk, returning the ideal image position relative to the query point

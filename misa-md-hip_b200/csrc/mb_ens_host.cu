@@ -117,7 +117,7 @@ __global__ void k_ens_pack(LatDesc d, mb_atom_element *aos, const int64_t *ids, 
     mb_atom_element a;
     const int c = d.code[i];
     a.id = ids[t];
-    a.type = c < 0 ? -1 : (c & 0x3F);
+    a.type = c < 0 ? -1 : (c & MB_TYPE_MASK);
     a.pad_ = 0;
     if (c < 0) {
       for (int k = 0; k < 3; k++) a.x[k] = a.v[k] = a.f[k] = 0.0;
@@ -1012,7 +1012,7 @@ int mb_ensemble_add(mb_ensemble *e, const mb_lattice_spec *spec, const mb_atom_e
   d.steps_target = steps;
   const size_t n = 2 * (size_t)d.E, nb = 2 * (size_t)cx * cy * cz, ci = (size_t)std::max(1, L.cap_itl);
   const int per = 2 * 4 * 64 + 64;
-  d.cap_flag = std::max(1, L.cap_itl * per);
+  d.cap_flag = std::max(1, L.cap_itl * (per / 2)); // of either list (a step's and the last one's)
   char *p = (char *)block;
   auto take = [&](size_t b) {
     char *q = p;
@@ -1048,7 +1048,7 @@ int mb_ensemble_add(mb_ensemble *e, const mb_lattice_spec *spec, const mb_atom_e
   d.idf = (double *)take(ci * 8);
   L.iids = (int64_t *)take(ci * 8);
   d.itype = (int8_t *)take(ci);
-  d.flag_list = (int *)take((size_t)d.cap_flag * 4);
+  d.flag_list = (int *)take((size_t)std::max(2, L.cap_itl * per) * 4);
   d.flag_count = (int *)take(16); // [count parity 0, count parity 1, overflow, -]
   d.cand = (long long *)take(MB_CAND_CAP * 8);
   d.cand_n = (int *)take(16);

@@ -171,18 +171,18 @@ __device__ void rho_tiles(const EnsParams &P, TileCtx &T, const float4 *s_fv) {
     __syncwarp();
     if (lane == 0) mbar_arrive(&T.empty[b]); // tile data no longer needed by this warp
     if (warp == 0) producer_issue(P, T, pr);  // tile i + 2 into this buffer
-    if (work && (code & MB_FLAG_ITL)) {
+    if (work && (code & MB_FLAG_ITL(d.cur))) {
       d.rho[me.i] = (float)(((double)rs0 + (double)rs1) + ((double)rc0 + (double)rc1));
     } else if (work) {
       const double rho = ((double)rs0 + (double)rs1) + ((double)rc0 + (double)rc1);
-      const double df = dF64(P.P, code & 0x3F, rho);
+      const double df = dF64(P.P, code & MB_TYPE_MASK, rho);
       float4 *u4 = d.u4[d.cur];
       reinterpret_cast<float *>(u4 + me.i)[3] = (float)df;
       d.rho[me.i] = (float)rho;
       const Geom g = lat_geom(d);
       for_images(g, me.s, me.bcx, me.by, me.bz,
                  [&](long long idx, double, double, double) { reinterpret_cast<float *>(u4 + idx)[3] = (float)df; });
-      if (ENERGY) e_site = F64(P.P, code & 0x3F, rho);
+      if (ENERGY) e_site = F64(P.P, code & MB_TYPE_MASK, rho);
     }
     if (ENERGY) {
       const double tsum = block_sum(e_site);
@@ -289,7 +289,7 @@ __device__ void force_tiles(const EnsParams &P, TileCtx &T, const float2 *s_fd) 
       d.fz[i] = (float)fz;
       if (ENERGY) e_pair = ((double)ps0 + (double)ps1) + ((double)pc0 + (double)pc1);
     }
-    if (work && !(code & MB_FLAG_ITL)) { // flagged sites are integrated by the interstitial items
+    if (work && !(code & MB_FLAG_ITL(d.cur))) { // flagged sites are integrated by the interstitial items
       const long long i = me.i;
       const double fx = ((double)fs0.x + (double)fs1.x) + ((double)fc0.x + (double)fc1.x);
       const double fy = ((double)fs0.y + (double)fs1.y) + ((double)fc0.y + (double)fc1.y);
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(ENS_THREADS, 1) k_ens_step(const __grid_consta
   if (P.n_itl_lats > 0) {
     for (int q = 0; q < P.n_itl_lats; q++) {
       const LatDesc &d = P.lats[P.itl_lats[q]];
-      if (lat_active(d)) itl_clear_flags(d);
+      if (lat_active(d)) itl_clear_flags(d, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     }
     if (!grid_sync(P.bar, P.err, P.bar_spins)) return;
     const int warps = gridDim.x * (blockDim.x >> 5);
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(ENS_THREADS, 1) k_ens_step(const __grid_consta
     for (int q = 0; q < P.n_itl_lats; q++) {
       const LatDesc &d = P.lats[P.itl_lats[q]];
       if (!lat_active(d)) continue;
-      for (int it = gw; it < d.n_itl; it += warps) itl_mark_one(P, d, it);
+      for (int it = gw; it < d.n_itl; it += warps) itl_mark_one(P, d, it, threadIdx.x & 31, 32);
     }
     if (!grid_sync(P.bar, P.err, P.bar_spins)) return;
   }
@@ -393,6 +393,7 @@ __global__ void __launch_bounds__(ENS_THREADS, 1) k_ens_step(const __grid_consta
     for (int l = threadIdx.x; l < P.n_lats; l += blockDim.x) {
       LatDesc *d = const_cast<LatDesc *>(&P.lats[l]);
       if (!lat_active(*d)) continue;
+      d->flag_count[d->cur ^ 1] = 0; // last step's marks are off: its list takes the next step's
       d->cur ^= 1;
       if (d->primed)
         d->steps_done++;

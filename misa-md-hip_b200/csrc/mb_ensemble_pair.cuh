@@ -115,45 +115,36 @@ __device__ __forceinline__ void force_pair(const EnsParams &P, const float4 &u, 
 }
 
 // ------------------------------------------------------- interstitial items
-// Sites flagged at the previous step of lattice d lose their flag (all CTAs share
-// the old list); the count this step will fill starts at zero.  Counts alternate
-// with the buffer parity: count[cur] is this step's list, count[cur ^ 1] the last.
-__device__ __forceinline__ void itl_clear_flags(const LatDesc &d) {
-  const int cur = d.cur;
-  const int nold = min(d.flag_count[cur ^ 1], d.cap_flag);
-  const int stride = gridDim.x * blockDim.x;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nold; k += stride) {
-    const int idx = d.flag_list[k];
-    d.code[idx] = (int8_t)(d.code[idx] & ~MB_FLAG_ITL);
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) d.flag_count[cur] = 0;
+// Sites marked at the previous step of lattice d lose their mark (threads t, t + n, ...).
+// Lists, counts and mark bits alternate with the buffer parity: list cur holds this step's
+// sites, list cur ^ 1 last step's.  The bookkeeping at the end of a step empties the latter.
+__device__ __forceinline__ int *flag_list_of(const LatDesc &d, int parity) {
+  return d.flag_list + (size_t)parity * d.cap_flag;
+}
+__device__ __forceinline__ void itl_clear_flags(const LatDesc &d, int t, int n) {
+  const int old = d.cur ^ 1;
+  const int nold = min(d.flag_count[old], d.cap_flag);
+  const int *list = flag_list_of(d, old);
+  for (int k = t; k < nold; k += n) code_bit_off(d.code + list[k], MB_FLAG_ITL(old));
 }
 
-// One warp flags the lattice sites within reach of interstitial `it`.  With
-// `list` (this warp's MB_WIN_LIST entries of shared memory) the in-reach candidates are
-// listed first and the lanes then flag only those.
-__device__ __forceinline__ void itl_mark_one(const EnsParams &P, const LatDesc &d, int it, int *list = nullptr) {
+// `n` threads (whole warps; this one is number t) mark the lattice sites within reach of
+// interstitial `it`.
+__device__ __forceinline__ void itl_mark_one(const EnsParams &P, const LatDesc &d, int it, int t, int n) {
   const Geom g = lat_geom(d);
-  const int lane = threadIdx.x & 31;
   const int cur = d.cur;
+  int *list = flag_list_of(d, cur);
   const double qx = d.ipx[cur][it], qy = d.ipy[cur][it], qz = d.ipz[cur][it];
   const Window w = make_window(qx, qy, qz, P.a0, P.reach);
-  const int nlist = list ? window_compact(w, qx, qy, qz, P.a0, P.reach, list, MB_WIN_LIST) : -1;
-  const int ncand = nlist >= 0 ? nlist : w.nx * w.ny * w.nz;
-  for (int base = 0; base < ncand; base += 32) { // whole warp per round (warp_append)
-    const int k = base + lane;
+  const int ncand = w.nx * w.ny * w.nz;
+  for (int base = 0; base < ncand; base += n) { // whole warps per round (warp_append)
+    const int k = base + t;
     long long idx = 0;
-    bool fresh = false;
     double sx, sy, sz;
-    if (k < ncand && window_site(g, w, nlist >= 0 ? list[k] : k, qx, qy, qz, P.a0, P.reach, idx, sx, sy, sz) &&
-        d.code[idx] >= 0) {
-      const uintptr_t addr = (uintptr_t)(d.code + idx);
-      unsigned int *word = (unsigned int *)(addr & ~(uintptr_t)3);
-      const unsigned int bit = (unsigned int)MB_FLAG_ITL << (8 * (addr & 3));
-      fresh = !(atomicOr(word, bit) & bit);
-    }
+    const bool fresh = k < ncand && window_site(g, w, k, qx, qy, qz, P.a0, P.reach, idx, sx, sy, sz) &&
+                       d.code[idx] >= 0 && code_bit_on(d.code + idx, MB_FLAG_ITL(cur));
     // flag_count[2]: overflow, reported by the host
-    warp_append(fresh, (int)idx, &d.flag_count[cur], d.flag_list, d.cap_flag, &d.flag_count[2]);
+    warp_append(fresh, (int)idx, &d.flag_count[cur], list, d.cap_flag, &d.flag_count[2]);
   }
 }
 
@@ -295,62 +286,23 @@ __device__ __forceinline__ void itl_finish(const EnsParams &P, const LatDesc &d,
   }
 }
 
-// Sum over the 8 lanes of a group (lanes 8g .. 8g + 7), in a fixed order.
-__device__ __forceinline__ double group8_sum(double v) {
-  v += __shfl_xor_sync(0xffffffffu, v, 4);
-  v += __shfl_xor_sync(0xffffffffu, v, 2);
-  v += __shfl_xor_sync(0xffffffffu, v, 1);
-  return v;
-}
-
-// Pairs of interstitial it (position xi, yi, zi) with the lattice sites of its window,
-// one warp, handed to pair (which sums them per lane).  With `list` (this warp's MB_WIN_LIST entries of shared
-// memory) the in-reach sites are listed first and each lane then loads up to four of
-// them at once; without it (or when more than MB_WIN_LIST sites are in reach) every
-// candidate of the window is visited in rounds of 32.
+// Pairs of an interstitial at (xi, yi, zi) with the lattice sites of its window: candidates
+// t, t + n, ..., handed to pair (which sums them per thread).
 template <class Pair>
 __device__ __forceinline__ void itl_window_pairs(const EnsParams &P, const LatDesc &d, const Geom &g,
-                                                 const float4 *u4, double xi, double yi, double zi, int *list,
+                                                 const float4 *u4, double xi, double yi, double zi, int t, int n,
                                                  bool with_df, Pair pair) {
-  const int lane = threadIdx.x & 31;
   const Window win = make_window(xi, yi, zi, P.a0, P.reach);
-  const int n = list ? window_compact(win, xi, yi, zi, P.a0, P.reach, list, MB_WIN_LIST) : -1;
-  if (n >= 0) {
-    for (int k0 = 0; k0 < n; k0 += 128) {
-      long long j[4];
-      double ox[4], oy[4], oz[4];
-      bool ok[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int k = k0 + 32 * t + lane;
-        j[t] = 0;
-        ox[t] = oy[t] = oz[t] = 0.0;
-        ok[t] = k < n && window_site_rel(g, win, list[k], xi, yi, zi, P.a0, P.reach, j[t], ox[t], oy[t], oz[t]);
-      }
-      int cj[4];
-      float4 uj[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        cj[t] = ok[t] ? (int)d.code[j[t]] : -1;
-        uj[t] = ok[t] ? u4[j[t]] : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int t = 0; t < 4; t++)
-        if (cj[t] >= 0)
-          pair(-(ox[t] + (double)uj[t].x), -(oy[t] + (double)uj[t].y), -(oz[t] + (double)uj[t].z), cj[t] & 0x3F,
-               with_df ? (double)uj[t].w : 0.0);
-    }
-    return;
-  }
   const int ncand = win.nx * win.ny * win.nz;
-  for (int c = lane; c < ncand; c += 32) {
+  for (int c = t; c < ncand; c += n) {
     long long j;
     double ox, oy, oz;
     if (!window_site_rel(g, win, c, xi, yi, zi, P.a0, P.reach, j, ox, oy, oz)) continue;
     const int cj = d.code[j];
-    if (cj < 0) continue;
     const float4 uj = u4[j];
-    pair(-(ox + (double)uj.x), -(oy + (double)uj.y), -(oz + (double)uj.z), cj & 0x3F, with_df ? (double)uj.w : 0.0);
+    if (cj >= 0)
+      pair(-(ox + (double)uj.x), -(oy + (double)uj.y), -(oz + (double)uj.z), cj & MB_TYPE_MASK,
+           with_df ? (double)uj.w : 0.0);
   }
 }
 
@@ -359,9 +311,8 @@ __device__ __forceinline__ void itl_window_pairs(const EnsParams &P, const LatDe
 // flagged site's lattice-pair part comes from the lattice kernels (rho / f of the site);
 // its interstitial pairs, df, integration and ghost images are done here.  An
 // interstitial's pairs (lattice window and other interstitials) are all done here, FP64.
-// `list`: see itl_window_pairs.
-template <bool FORCE, bool ENERGY, bool CELLS>
-__device__ void itl_item(const EnsParams &P, const LatDesc &d, int w, int nflag, int *list = nullptr) {
+template <bool FORCE, bool ENERGY>
+__device__ void itl_item(const EnsParams &P, const LatDesc &d, int w, int nflag) {
   const int lane = threadIdx.x & 31;
   const Geom g = lat_geom(d);
   const int cur = d.cur;
@@ -371,9 +322,9 @@ __device__ void itl_item(const EnsParams &P, const LatDesc &d, int w, int nflag,
   int s = 0, cx = 0, y = 0, z = 0, it = 0, ti;
   double xi, yi, zi, dfi = 0.0;
   if (is_site) {
-    i = d.flag_list[w];
+    i = flag_list_of(d, cur)[w];
     decode_ext(g, i, s, cx, y, z);
-    ti = d.code[i] & 0x3F;
+    ti = d.code[i] & MB_TYPE_MASK;
     double X, Y, Z;
     ideal_pos(s, cx, y, z, P.a0, X, Y, Z);
     xi = X + d.ux[i];
@@ -405,9 +356,9 @@ __device__ void itl_item(const EnsParams &P, const LatDesc &d, int w, int nflag,
       }
     }
   } else {
-    itl_window_pairs(P, d, g, u4, xi, yi, zi, list, FORCE, pair);
+    itl_window_pairs(P, d, g, u4, xi, yi, zi, lane, 32, FORCE, pair);
   }
-  itl_pairs<CELLS>(d, g, cur, xi, yi, zi, is_site ? -1 : it, lane, pair, FORCE);
+  itl_pairs<false>(d, g, cur, xi, yi, zi, is_site ? -1 : it, lane, pair, FORCE);
   if (!FORCE) {
     acc0 = warp_sum(acc0);
   } else {
@@ -440,9 +391,9 @@ __device__ void itl_site_group(const EnsParams &P, const LatDesc &d, int w, bool
     itl_pair<FORCE, ENERGY>(P, ti, dfi, dx, dy, dz, tj, dfj, acc0, fx, fy, fz, ep);
   };
   if (valid) {
-    i = d.flag_list[w];
+    i = flag_list_of(d, cur)[w];
     decode_ext(g, i, s, cx, y, z);
-    ti = d.code[i] & 0x3F;
+    ti = d.code[i] & MB_TYPE_MASK;
     double X, Y, Z;
     ideal_pos(s, cx, y, z, P.a0, X, Y, Z);
     xi = X + d.ux[i];
@@ -491,33 +442,76 @@ __device__ void itl_site_group(const EnsParams &P, const LatDesc &d, int w, bool
     itl_finish<FORCE, ENERGY>(P, d, g, true, i, s, cx, y, z, 0, ti, xi, yi, zi, acc0, fx, fy, fz, ep);
 }
 
-// Items of every lattice that holds interstitials.  Split kernels (CELLS: their per-step
-// interstitial cell list applies; `list`: this warp's window list): the interstitials
-// first, one warp each, so that their window walks (the longest items) start at once,
-// then the flagged sites four to a warp.  Persistent kernel: one item per warp, whole
-// interstitial lists.
-template <bool FORCE, bool ENERGY, bool CELLS = false>
-__device__ void itl_items(const EnsParams &P, int *list = nullptr) {
+// Interstitial `it` of lattice d, worked by a whole block: its window's candidates are spread
+// over the threads (3 or 4 each instead of 22 rounds of one warp), the first warp adds the
+// other interstitials, and thread 0 sums in a fixed order and finishes.  red: 4 x 32 doubles
+// of shared memory.
+template <bool FORCE, bool ENERGY>
+__device__ void itl_block_item(const EnsParams &P, const LatDesc &d, int it, double (*red)[32]) {
+  const Geom g = lat_geom(d);
+  const int cur = d.cur, ti = d.itype[it], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double xi = d.ipx[cur][it], yi = d.ipy[cur][it], zi = d.ipz[cur][it], dfi = FORCE ? d.idf[it] : 0.0;
+  double acc0 = 0.0, fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0;
+  auto pair = [&](double dx, double dy, double dz, int tj, double dfj) {
+    itl_pair<FORCE, ENERGY>(P, ti, dfi, dx, dy, dz, tj, dfj, acc0, fx, fy, fz, ep);
+  };
+  itl_window_pairs(P, d, g, d.u4[cur], xi, yi, zi, threadIdx.x, blockDim.x, FORCE, pair);
+  if (warp == 0) itl_pairs<true>(d, g, cur, xi, yi, zi, it, lane, pair, FORCE);
+  double *vals[4] = {FORCE ? &fx : &acc0, &fy, &fz, &ep};
+  const int n = FORCE ? (ENERGY ? 4 : 3) : 1;
+  __syncthreads(); // the sums of the block's last item are read
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    if (q >= n) break;
+    const double v = warp_sum(*vals[q]);
+    if (lane == 0) red[q][warp] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (q >= n) break;
+      double v = 0.0;
+      for (int k = 0; k < (int)(blockDim.x >> 5); k++) v += red[q][k];
+      *vals[q] = v;
+    }
+    itl_finish<FORCE, ENERGY>(P, d, g, false, 0, 0, 0, 0, 0, it, ti, xi, yi, zi, acc0, fx, fy, fz, ep);
+  }
+}
+
+// Items of every lattice that holds interstitials, split kernels: a block takes one
+// interstitial or blockDim / 8 marked sites (8 lanes each), the interstitials first; the
+// blocks start at another place of each lattice's items.
+template <bool FORCE, bool ENERGY>
+__device__ void itl_block_items(const EnsParams &P, double (*red)[32]) {
+  const int per = blockDim.x >> 3;
+  for (int q = 0; q < P.n_itl_lats; q++) {
+    const LatDesc &d = P.lats[P.itl_lats[q]];
+    if (!lat_active(d)) continue;
+    const int nflag = min(d.flag_count[d.cur], d.cap_flag), n_itl = d.n_itl;
+    const int jobs = n_itl + (nflag + per - 1) / per;
+    for (int job = (blockIdx.x + 61u * (unsigned)q) % gridDim.x; job < jobs; job += gridDim.x) {
+      if (job < n_itl) {
+        itl_block_item<FORCE, ENERGY>(P, d, job, red);
+      } else {
+        const int f = (job - n_itl) * per + (int)(threadIdx.x >> 3);
+        itl_site_group<FORCE, ENERGY>(P, d, f, f < nflag);
+      }
+    }
+  }
+}
+
+// The same in the persistent kernel: one item per warp, whole interstitial lists.
+template <bool FORCE, bool ENERGY>
+__device__ void itl_items(const EnsParams &P) {
   const int warps = gridDim.x * (blockDim.x >> 5);
   const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   for (int q = 0; q < P.n_itl_lats; q++) {
     const LatDesc &d = P.lats[P.itl_lats[q]];
     if (!lat_active(d)) continue;
     const int nflag = min(d.flag_count[d.cur], d.cap_flag);
-    if (CELLS) {
-      const int n = d.n_itl + (nflag + 3) / 4;
-      for (int w = gw; w < n; w += warps) {
-        if (w < d.n_itl) {
-          itl_item<FORCE, ENERGY, true>(P, d, nflag + w, nflag, list);
-        } else {
-          const int f = 4 * (w - d.n_itl) + (int)((threadIdx.x & 31) >> 3);
-          itl_site_group<FORCE, ENERGY>(P, d, f, f < nflag);
-        }
-      }
-    } else {
-      const int n = nflag + d.n_itl;
-      for (int w = gw; w < n; w += warps) itl_item<FORCE, ENERGY, false>(P, d, w, nflag);
-    }
+    const int n = nflag + d.n_itl;
+    for (int w = gw; w < n; w += warps) itl_item<FORCE, ENERGY>(P, d, w, nflag);
   }
 }
 

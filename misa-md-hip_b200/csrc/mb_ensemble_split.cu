@@ -280,15 +280,15 @@ __device__ __forceinline__ double mx_rho_site(const EnsParams &P, const MxStenci
   }
   const double rho = (double)rs + (double)rc;
   d.rho[i] = (float)rho;
-  if (code & MB_FLAG_ITL) return 0.0; // lattice part only: the interstitial items finish the site
-  const double df = dF64(P.P, code & 0x3F, rho);
+  if (code & MB_FLAG_ITL(d.cur)) return 0.0; // lattice part only: the interstitial items finish the site
+  const double df = dF64(P.P, code & MB_TYPE_MASK, rho);
   reinterpret_cast<float *>(uw + i)[3] = (float)df;
   int sx, cx, y, z;
   mx_unpack(pos, sx, cx, y, z);
   const Geom g = lat_geom(d);
   for_images(g, sx, cx, y, z,
              [&](long long idx, double, double, double) { reinterpret_cast<float *>(uw + idx)[3] = (float)df; });
-  return ENERGY ? F64(P.P, code & 0x3F, rho) : 0.0;
+  return ENERGY ? F64(P.P, code & MB_TYPE_MASK, rho) : 0.0;
 }
 
 // Force + velocity-Verlet of one site; adds pair energy and kinetic energy.  Pair terms
@@ -385,7 +385,7 @@ __device__ __forceinline__ void mx_force_site(const EnsParams &P, const MxStenci
   d.fy[i] = (float)fy;
   d.fz[i] = (float)fz;
   if (ENERGY) e_pair += (double)ps + (double)pc;
-  if (code & MB_FLAG_ITL) return; // lattice part only: the interstitial items integrate the site
+  if (code & MB_FLAG_ITL(d.cur)) return; // lattice part only: the interstitial items integrate the site
   double vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
   if (d.primed) {
     vx += P.h * fx;
@@ -488,23 +488,21 @@ __global__ void __launch_bounds__(MX_FORCE_THREADS, 1)
   }
 }
 
-// Interstitial phases and step bookkeeping of split mode, one kernel each (the
-// phases the persistent kernel separates with grid barriers).
-__global__ void k_mx_itl_clear(const __grid_constant__ EnsParams P) {
-  for (int q = 0; q < P.n_itl_lats; q++) {
-    const LatDesc &d = P.lats[P.itl_lats[q]];
-    if (lat_active(d)) itl_clear_flags(d);
-  }
-}
+// Interstitial phases and step bookkeeping of split mode.
 
-// Interstitial cell list of one lattice per CTA, from this step's positions: the counts
+// One launch before the density pass: block q < n_itl_lats bins the interstitials of lattice
+// q into cells; the others mark the sites near interstitials (MX_MARK_THREADS threads each)
+// and take last step's marks off.  The three do not depend on one another: this step's marks
+// are another bit and another list than last step's.
+//
+// Interstitial cell list of one lattice, from this step's positions: the counts
 // of the previous build are cleared, (cell, index) keys sorted in shared memory, and each
 // occupied cell gets its start and count.  The order (cell, index) does not depend on
 // thread timing.
 #define MX_BIN_THREADS 1024
-__global__ void __launch_bounds__(MX_BIN_THREADS, 1) k_mx_itl_bin(const __grid_constant__ EnsParams P) {
+#define MX_MARK_THREADS 256
+__device__ void mx_itl_bin(const LatDesc &d) {
   __shared__ long long key[MX_ICELL_MAX];
-  const LatDesc &d = P.lats[P.itl_lats[blockIdx.x]];
   if (!lat_active(d) || !d.icount) return; // uniform per block
   const int tid = threadIdx.x, n = d.n_itl, cur = d.cur;
   const int nold = d.iflag[1];
@@ -548,24 +546,28 @@ __global__ void __launch_bounds__(MX_BIN_THREADS, 1) k_mx_itl_bin(const __grid_c
   }
 }
 
-// The interstitial kernels run MX_ITL_THREADS threads per block; each warp keeps its list
-// of in-reach window sites (window_compact) in shared memory.
-#define MX_ITL_THREADS 256
-__global__ void __launch_bounds__(MX_ITL_THREADS) k_mx_itl_mark(const __grid_constant__ EnsParams P) {
-  __shared__ int s_list[MX_ITL_THREADS / 32][MB_WIN_LIST];
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+__global__ void __launch_bounds__(MX_BIN_THREADS, 1) k_mx_itl_prep(const __grid_constant__ EnsParams P) {
+  const int bins = P.n_itl_lats;
+  if ((int)blockIdx.x < bins) {
+    mx_itl_bin(P.lats[P.itl_lats[blockIdx.x]]);
+    return;
+  }
+  const int per = MX_BIN_THREADS / MX_MARK_THREADS, groups = ((int)gridDim.x - bins) * per;
+  const int block = (int)blockIdx.x - bins, group = block * per + (int)threadIdx.x / MX_MARK_THREADS;
   for (int q = 0; q < P.n_itl_lats; q++) {
     const LatDesc &d = P.lats[P.itl_lats[q]];
     if (!lat_active(d)) continue;
-    for (int it = gw; it < d.n_itl; it += warps) itl_mark_one(P, d, it, s_list[threadIdx.x >> 5]);
+    itl_clear_flags(d, block * MX_BIN_THREADS + threadIdx.x, ((int)gridDim.x - bins) * MX_BIN_THREADS);
+    for (int it = (int)((group + 61u * (unsigned)q) % (unsigned)groups); it < d.n_itl; it += groups)
+      itl_mark_one(P, d, it, (int)threadIdx.x % MX_MARK_THREADS, MX_MARK_THREADS);
   }
 }
 
+#define MX_ITL_THREADS 256
 template <bool FORCE, bool ENERGY>
-__global__ void __launch_bounds__(MX_ITL_THREADS, 2) k_mx_itl_items(const __grid_constant__ EnsParams P) {
-  __shared__ int s_list[MX_ITL_THREADS / 32][MB_WIN_LIST];
-  itl_items<FORCE, ENERGY, true>(P, s_list[threadIdx.x >> 5]);
+__global__ void __launch_bounds__(MX_ITL_THREADS, 3) k_mx_itl_items(const __grid_constant__ EnsParams P) {
+  __shared__ double red[4][32];
+  itl_block_items<FORCE, ENERGY>(P, red);
 }
 
 // Lattice <-> interstitial bookkeeping after the drift, one CTA per lattice that can
@@ -617,7 +619,7 @@ __global__ void __launch_bounds__(MX_CONV_THREADS, 1) k_mx_convert(const __grid_
     d.ifz[k] = (double)d.fz[i];
     d.irho[k] = (double)d.rho[i];
     d.idf[k] = (double)d.u4[c0][i].w;
-    d.itype[k] = (int8_t)(d.code[i] & 0x3F);
+    d.itype[k] = (int8_t)(d.code[i] & MB_TYPE_MASK);
     d.iids[k] = d.ids[t];
     // vacant: far away in both float4 buffers (the pair loops reject vacancies by position)
     d.code[i] = -1;
@@ -765,6 +767,7 @@ __global__ void k_mx_bookkeeping(const __grid_constant__ EnsParams P) {
   for (int l = threadIdx.x; l < P.n_lats; l += blockDim.x) {
     LatDesc *d = const_cast<LatDesc *>(&P.lats[l]);
     if (!lat_active(*d)) continue;
+    d->flag_count[d->cur ^ 1] = 0; // last step's marks are off: its list takes the next step's
     d->cur ^= 1;
     if (d->primed)
       d->steps_done++;
@@ -851,12 +854,8 @@ int mx_launch_step(const EnsParams &P, const MxStencil &S, int lat, int energy, 
     MB_TRY((mx_set_attrs<8, 1>()));
     attr = true;
   }
-  const int itl_grid = 2 * sms;
-  if (P.n_itl_lats > 0) {
-    k_mx_itl_clear<<<itl_grid, 256, 0, s>>>(P);
-    k_mx_itl_bin<<<P.n_itl_lats, MX_BIN_THREADS, 0, s>>>(P);
-    k_mx_itl_mark<<<itl_grid, MX_ITL_THREADS, 0, s>>>(P);
-  }
+  const int itl_grid = 3 * sms;
+  if (P.n_itl_lats > 0) k_mx_itl_prep<<<P.n_itl_lats + sms, MX_BIN_THREADS, 0, s>>>(P);
   if (ev) MB_CUDA(cudaEventRecord(ev[0], s));
   mx_passes(P, S, lat, energy, s, 0, rho_smem);
   if (ev) MB_CUDA(cudaEventRecord(ev[1], s));

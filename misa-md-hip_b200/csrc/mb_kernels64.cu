@@ -102,7 +102,7 @@ struct RhoArgs {
   Lattice64 L;
   double rc2;
   double *e_partial;
-  int skip_flagged;
+  int flag;
   int m_lo;      // first knot kept in shared memory
   ItemWalk walk;
   long long w0, n_items; // items [w0, n_items): a z-slab of the box (z slowest) or every brick
@@ -150,8 +150,8 @@ __device__ __forceinline__ unsigned long long rho_site(const StencilSet &st, con
   const DevPot &P = a.P;
   const long long i = ext_index(g, s, cx, y, z);
   const int code = L.code[i];
-  if (code < 0 || (a.skip_flagged && (code & MB_FLAG_ITL))) return 0;
-  const int ti = code & 0x3F;
+  if (code < 0) return 0;
+  const int ti = code & MB_TYPE_MASK;
   const double xi = L.p[i].x, yi = L.p[i].y, zi = L.p[i].z;
   const int *off = st.off[s];
   double rho = 0.0;
@@ -183,14 +183,15 @@ __device__ __forceinline__ unsigned long long rho_site(const StencilSet &st, con
         int m;
         double p;
         spl_locate(r, P.rdr, P.nr, m, p);
-        const int tj = L.code[j] & 0x3F;
+        const int tj = L.code[j] & MB_TYPE_MASK;
         rho += cubic(ldg4(&P.f_val[(size_t)tj * P.nr + m]), p);
       }
     }
   }
+  if (L.rho) L.rho[i] = rho;
+  if (code & a.flag) return near; // the interstitial pass adds its pairs to this sum
   const double df = dF64(P, ti, rho);
   L.p[i].w = df;
-  if (L.rho) L.rho[i] = rho;
   if (g.images) for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.p[idx].w = df; });
   if (ENERGY) e_acc += F64(P, ti, rho);
   return near;
@@ -245,7 +246,7 @@ struct ForceArgs {
   StepParams sp;
   double *e_pair;    // CTA partials of 1/2 sum phi
   double *e_kin;     // CTA partials of kinetic energy
-  int skip_flagged;
+  int flag;
   int m_lo;
   ItemWalk walk;
   long long w0, n_items; // items [w0, n_items)
@@ -327,8 +328,8 @@ __global__ void __launch_bounds__(MB_FORCE_THREADS, 1)
     if (cx >= g.bcx) continue;
     const long long i = ext_index(g, s, cx, y, z);
     const int code = L.code[i];
-    if (code < 0 || (a.skip_flagged && (code & MB_FLAG_ITL))) continue;
-    const int ti = code & 0x3F;
+    if (code < 0) continue;
+    const int ti = code & MB_TYPE_MASK;
     const double xi = L.p[i].x, yi = L.p[i].y, zi = L.p[i].z;
     const double dfi = L.p[i].w;
     const int *off = st.off[s];
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(MB_FORCE_THREADS, 1)
           const double rinv = rsqrt(d2);
           const double r = d2 * rinv;
           const double dfj = pj.w;
-          const int tj = L.code[j] & 0x3F;
+          const int tj = L.code[j] & MB_TYPE_MASK;
           double ph = 0.0;
           const double psip = pair_psip(P, ti, tj, r, dfi, dfj, ENERGY ? &ph : nullptr);
           if (ENERGY) ep += 0.5 * ph;
@@ -400,7 +401,7 @@ __global__ void __launch_bounds__(MB_FORCE_THREADS, 1)
       L.fy[i] = fy;
       L.fz[i] = fz;
     }
-    if (L.vx) {
+    if (L.vx && !(code & a.flag)) { // flagged: the interstitial pass adds its pairs and integrates
       double vx = L.vx[i], vy = L.vy[i], vz = L.vz[i];
       if (sp.kick_pre) {
         vx += sp.h * fx;
@@ -529,7 +530,7 @@ static bool split_launch(const char *name, int per_sm, const LatticeArgs &a) {
 }
 
 // Arguments of a planned pass over box layers [z0, z1).
-static LatticeArgs lattice_args(const Geom &g, const DevPot &pot, const Lattice64 &L, double rc2, int skip_flagged,
+static LatticeArgs lattice_args(const Geom &g, const DevPot &pot, const Lattice64 &L, double rc2, int flag,
                                 uint2 *outer, const Plan64 &plan, int z0, int z1) {
   LatticeArgs a{};
   a.g = g;
@@ -545,18 +546,18 @@ static LatticeArgs lattice_args(const Geom &g, const DevPot &pot, const Lattice6
   long long bits;
   memcpy(&bits, &rc2, sizeof(bits));
   a.rc2_hi = (int)(bits >> 32);
-  a.skip_flagged = skip_flagged;
+  a.flag = flag;
   a.outer = outer;
   return a;
 }
 
 int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, double rc2,
-                 double *e_partial, int energy, int skip_flagged, cudaStream_t s, int z0, int z1, uint2 *outer,
+                 double *e_partial, int energy, int flag, cudaStream_t s, int z0, int z1, uint2 *outer,
                  const Plan64 *plan) {
   if (plan && plan->ok && L.rho && cutoff_in_table(pot, rc2)) {
     if (z1 < 0) z1 = g.bz;
     if (z0 < 0 || z0 >= z1 || z1 > g.bz) return z0 == z1 ? MB_OK : fail(MB_ERR_ARG, "z-slab outside the box");
-    LatticeArgs a = lattice_args(g, pot, L, rc2, skip_flagged, outer, *plan, z0, z1);
+    LatticeArgs a = lattice_args(g, pot, L, rc2, flag, outer, *plan, z0, z1);
     a.e0 = e_partial;
     if (split_launch("MB_SPLIT_RHO_ITEMS", MB_SPLIT_RHO_ITEMS, a)) return launch_split_rho64(st, a, energy, s);
     return launch_shell_rho64(st, a, energy, s);
@@ -568,7 +569,7 @@ int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const L
   a.rc2 = rc2;
   a.rc2m = rc2 * (1.0 + 1e-9);
   a.e_partial = e_partial;
-  a.skip_flagged = skip_flagged;
+  a.flag = flag;
   const bool one = pot.n_types == 1 && cutoff_in_table(pot, rc2);
   a.outer = one && outer_masks_fit(st) ? outer : nullptr;
   int nsm = smem_knots(pot, (int)sizeof(double4));
@@ -601,13 +602,13 @@ int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const L
 }
 
 int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, const StepParams &sp,
-                   double *e_partial, int energy, int skip_flagged, cudaStream_t s, int z0, int z1,
+                   double *e_partial, int energy, int flag, cudaStream_t s, int z0, int z1,
                    const uint2 *outer, const Plan64 *plan) {
   if (plan && plan->ok && L.fx && cutoff_in_table(pot, sp.rc2)) {
     if (z1 < 0) z1 = g.bz;
     if (z0 < 0 || z0 >= z1 || z1 > g.bz) return z0 == z1 ? MB_OK : fail(MB_ERR_ARG, "z-slab outside the box");
     LatticeArgs a =
-        lattice_args(g, pot, L, sp.rc2, skip_flagged, const_cast<uint2 *>(outer), *plan, z0, z1);
+        lattice_args(g, pot, L, sp.rc2, flag, const_cast<uint2 *>(outer), *plan, z0, z1);
     a.sp = sp;
     a.e0 = e_partial ? e_partial + MB_EPART_CAP : nullptr;
     a.e1 = e_partial ? e_partial + 2 * MB_EPART_CAP : nullptr;
@@ -621,7 +622,7 @@ int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const
   a.sp = sp;
   a.e_pair = e_partial ? e_partial + MB_EPART_CAP : nullptr;
   a.e_kin = e_partial ? e_partial + 2 * MB_EPART_CAP : nullptr;
-  a.skip_flagged = skip_flagged;
+  a.flag = flag;
   const bool one = pot.n_types == 1 && cutoff_in_table(pot, sp.rc2);
   a.outer = one && outer_masks_fit(st) ? outer : nullptr;
   int nsm = smem_knots(pot, (int)(3 * sizeof(double2)));
@@ -654,231 +655,113 @@ int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const
 }
 
 // ----------------------------------------------------- interstitial passes
-// Lattice sites whose IDEAL position lies within reach of an interstitial are
-// flagged (site code bit MB_FLAG_ITL) and skipped by the lattice passes; the
-// warp-per-item kernels below recompute them in full (stencil + interstitials)
-// together with the interstitials themselves.  Every pair with r < cutoff is thus
-// seen from both sides as long as no lattice atom strays more than
-// (reach - cutoff) from its site.
+// Lattice sites whose IDEAL position lies within reach of an interstitial are marked.  The
+// lattice passes leave a marked site's sums over lattice atoms in its rho / force; the
+// kernels below add its interstitial pairs and finish it, and do the interstitials
+// themselves.  Every pair with r < cutoff is thus seen from both sides as long as no lattice
+// atom strays more than (reach - cutoff) from its site.
+//
+// All of this is short chains of dependent loads: a block of MB_ITL_THREADS takes one
+// interstitial (its window of ~600 candidate sites is 3 candidates a thread) or 32 marked
+// sites, 8 lanes each.  With one warp per interstitial, 22 rounds of candidates each, and
+// one warp per marked site's whole stencil, the marking, density and force kernels of 24
+// interstitials on 37 x 52 x 45 cells took 14 / 14 / 14 us on one B200.
 
-// Last step's flags come off (grid-stride over the old list) ...
-__global__ void k_itl_clear(const Lattice64 L, const Itl64 I) {
-  const int nold = min(I.flag_count[0], I.cap_flag);
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nold; k += gridDim.x * blockDim.x) {
-    const int idx = I.flag_list[k];
-    L.code[idx] = (int8_t)(L.code[idx] & ~MB_FLAG_ITL);
-  }
-}
-
-// ... then one warp per interstitial flags the sites within reach (the count was
-// reset in between); only sites in box layers [z0, z1) when that is not the whole box.
-// The in-reach sites of the window are listed first (window_compact), so the lanes then
-// flag only those, several at once.
+// Blocks below n_mark mark the sites near interstitials blockIdx, blockIdx + n_mark, ...
+// (only sites in box layers [z0, z1) when that is not the whole box); the others take last
+// step's marks, which are another bit, off.
 __global__ void __launch_bounds__(MB_ITL_THREADS)
-    k_itl_mark(const Geom g, const Lattice64 L, const Itl64 I, int z0, int z1) {
-  __shared__ int s_list[MB_ITL_THREADS / 32][MB_WIN_LIST];
-  const bool all_z = z0 <= 0 && z1 >= g.bz;
-  const int lane = threadIdx.x & 31;
-  const int it = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
-  if (it >= itl_n(I)) return; // the same for the whole warp
-  const double qx = I.px[it], qy = I.py[it], qz = I.pz[it];
-  const Window w = make_window(qx, qy, qz, I.a0, I.reach);
-  int *list = s_list[threadIdx.x >> 5];
-  const int nlist = window_compact(w, qx, qy, qz, I.a0, I.reach, list, MB_WIN_LIST);
-  const int ncand = nlist >= 0 ? nlist : w.nx * w.ny * w.nz;
-  for (int base = 0; base < ncand; base += 32) { // whole warp per round (warp_append)
-    const int k = base + lane;
-    long long idx = 0;
-    bool fresh = false;
-    double sx, sy, sz;
-    bool site = k < ncand && window_site(g, w, nlist >= 0 ? list[k] : k, qx, qy, qz, I.a0, I.reach, idx, sx, sy, sz);
-    if (site && !all_z) {
-      int ss, scx, sy_, sz_;
-      decode_ext(g, idx, ss, scx, sy_, sz_);
-      site = sz_ >= z0 && sz_ < z1;
-    }
-    if (site && L.code[idx] >= 0) {
-      const uintptr_t addr = (uintptr_t)(L.code + idx);
-      unsigned int *word = (unsigned int *)(addr & ~(uintptr_t)3);
-      const unsigned int bit = (unsigned int)MB_FLAG_ITL << (8 * (addr & 3));
-      fresh = !(atomicOr(word, bit) & bit);
-    }
-    // flag_count[1]: overflow, reported by the host
-    warp_append(fresh, (int)idx, &I.flag_count[0], I.flag_list, I.cap_flag, &I.flag_count[1]);
-  }
-}
-
-// Lattice sites of the window of interstitial q, one warp: pair(dx, dy, dz, type, df)
-// for every occupied site in reach, d = q - (x_j + its periodic image shift), df only with
-// DF.  The in-reach sites are listed first (window_compact, list: this warp's shared
-// memory) and each lane then loads up to four of them at once: one round of dependent
-// loads instead of one per 32 candidates.
-template <bool DF, class Pair>
-__device__ __forceinline__ void window_pairs64(const Geom &g, const Lattice64 &L, const Itl64 &I, double qx,
-                                               double qy, double qz, int *list, Pair pair) {
-  const int lane = threadIdx.x & 31;
-  const Window win = make_window(qx, qy, qz, I.a0, I.reach);
-  const int n = window_compact(win, qx, qy, qz, I.a0, I.reach, list, MB_WIN_LIST);
-  if (n >= 0) {
-    for (int k0 = 0; k0 < n; k0 += 128) {
-      long long j[4];
-      double sx[4], sy[4], sz[4];
-      bool ok[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int k = k0 + 32 * t + lane;
-        j[t] = 0;
-        sx[t] = sy[t] = sz[t] = 0.0;
-        ok[t] = k < n && window_site(g, win, list[k], qx, qy, qz, I.a0, I.reach, j[t], sx[t], sy[t], sz[t]);
-      }
-      int cj[4];
-      double4 pj[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        cj[t] = ok[t] ? (int)L.code[j[t]] : -1;
-        pj[t] = ok[t] ? ld_site(L.p + j[t]) : make_double4(0.0, 0.0, 0.0, 0.0);
-      }
-#pragma unroll
-      for (int t = 0; t < 4; t++)
-        if (cj[t] >= 0)
-          pair(qx - (pj[t].x + sx[t]), qy - (pj[t].y + sy[t]), qz - (pj[t].z + sz[t]), cj[t] & 0x3F, DF ? pj[t].w : 0.0);
-    }
+    k_itl_mark(const Geom g, const Lattice64 L, const Itl64 I, int n_mark, int z0, int z1) {
+  if ((int)blockIdx.x >= n_mark) {
+    const int n = min(*I.old_count, I.cap_flag);
+    const int old = MB_FLAG_ITL(0) ^ MB_FLAG_ITL(1) ^ I.flag;
+    for (int k = (blockIdx.x - n_mark) * blockDim.x + threadIdx.x; k < n; k += (gridDim.x - n_mark) * blockDim.x)
+      code_bit_off(L.code + I.old_list[k], old);
     return;
   }
-  const int ncand = win.nx * win.ny * win.nz;
-  for (int c = lane; c < ncand; c += 32) {
-    long long j;
-    double sx, sy, sz;
-    if (!window_site(g, win, c, qx, qy, qz, I.a0, I.reach, j, sx, sy, sz)) continue;
-    const int cj = L.code[j];
-    if (cj < 0) continue;
-    const double4 pj = ld_site(L.p + j);
-    pair(qx - (pj.x + sx), qy - (pj.y + sy), qz - (pj.z + sz), cj & 0x3F, DF ? pj.w : 0.0);
-  }
-}
-
-// Items of the interstitial passes: the interstitials first (w < n_itl), so that their
-// window walks (the longest items) start at once, then the flagged sites.
-template <bool ENERGY>
-__global__ void __launch_bounds__(MB_ITL_THREADS)
-    k_itl_rho64(const __grid_constant__ StencilSet st, const Geom g, const DevPot P, const Lattice64 L, const Itl64 I,
-                double rc2, double *e_partial, int z0, int z1) {
-  const int lane = threadIdx.x & 31;
-  const bool all_z = z0 <= 0 && z1 >= g.bz; // else only items in box layers [z0, z1)
-  const int nflag = min(I.flag_count[0], I.cap_flag);
-  const int n_itl = itl_n(I);
-  const long long n_items = (long long)nflag + n_itl;
-  const long long wstride = (long long)gridDim.x * (blockDim.x >> 5);
-  __shared__ int s_list[MB_ITL_THREADS / 32][MB_WIN_LIST];
-  int *list = s_list[threadIdx.x >> 5];
-  double e_acc = 0.0;
-  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n_items; w += wstride) {
-    if (w >= n_itl) {
-      const long long i = I.flag_list[w - n_itl];
-      int s, cx, y, z;
-      decode_ext(g, i, s, cx, y, z);
-      if (!all_z && (z < z0 || z >= z1)) continue;
-      const int ti = L.code[i] & 0x3F;
-      const double xi = L.p[i].x, yi = L.p[i].y, zi = L.p[i].z;
-      double rho = 0.0;
-      for (int k = lane; k < st.n; k += 32) {
-        const long long j = i + st.off[s][k];
-        const double4 pj = ld_site(L.p + j);
-        const double dx = xi - pj.x, dy = yi - pj.y, dz = zi - pj.z;
-        const double d2 = dx * dx + dy * dy + dz * dz;
-        if (d2 < rc2) rho += rho_of_r(P, L.code[j] & 0x3F, d2 * rsqrt(d2));
+  const bool all_z = z0 <= 0 && z1 >= g.bz;
+  for (int it = blockIdx.x; it < itl_n(I); it += n_mark) {
+    const double qx = I.px[it], qy = I.py[it], qz = I.pz[it];
+    const Window w = make_window(qx, qy, qz, I.a0, I.reach);
+    const int ncand = w.nx * w.ny * w.nz;
+    for (int base = 0; base < ncand; base += blockDim.x) { // whole warps per round (warp_append)
+      const int k = base + threadIdx.x;
+      long long idx = 0;
+      double sx, sy, sz;
+      bool site = k < ncand && window_site(g, w, k, qx, qy, qz, I.a0, I.reach, idx, sx, sy, sz);
+      if (site && !all_z) {
+        int ss, scx, sy_, sz_;
+        decode_ext(g, idx, ss, scx, sy_, sz_);
+        site = sz_ >= z0 && sz_ < z1;
       }
-      for (int K = lane; K < n_itl; K += 32) {
-        const double dx = min_image(xi - I.px[K], g.Lx, g.iLx), dy = min_image(yi - I.py[K], g.Ly, g.iLy),
-                     dz = min_image(zi - I.pz[K], g.Lz, g.iLz);
-        const double d2 = dx * dx + dy * dy + dz * dz;
-        if (d2 < rc2) rho += rho_of_r(P, I.type[K], d2 * rsqrt(d2));
-      }
-      rho = warp_sum(rho);
-      if (lane == 0) {
-        const double df = dF64(P, ti, rho);
-        L.p[i].w = df;
-        if (L.rho) L.rho[i] = rho;
-        if (g.images) for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.p[idx].w = df; });
-        if (ENERGY) e_acc += F64(P, ti, rho);
-      }
-    } else {
-      const int it = (int)w;
-      const double qx = I.px[it], qy = I.py[it], qz = I.pz[it];
-      if (!all_z) {
-        const int lz = z_layer(g, I.a0, qz);
-        if (lz < z0 || lz >= z1) continue;
-      }
-      double rho = 0.0;
-      window_pairs64<false>(g, L, I, qx, qy, qz, list, [&](double dx, double dy, double dz, int tj, double) {
-        const double d2 = dx * dx + dy * dy + dz * dz;
-        if (d2 < rc2) rho += rho_of_r(P, tj, d2 * rsqrt(d2));
-      });
-      for (int K = lane; K < n_itl; K += 32) {
-        if (K == it) continue;
-        const double dx = min_image(qx - I.px[K], g.Lx, g.iLx), dy = min_image(qy - I.py[K], g.Ly, g.iLy),
-                     dz = min_image(qz - I.pz[K], g.Lz, g.iLz);
-        const double d2 = dx * dx + dy * dy + dz * dz;
-        if (d2 < rc2) rho += rho_of_r(P, I.type[K], d2 * rsqrt(d2));
-      }
-      rho = warp_sum(rho);
-      if (lane == 0) {
-        const int t = I.type[it];
-        I.rho[it] = rho;
-        I.df[it] = dF64(P, t, rho);
-        if (ENERGY) e_acc += F64(P, t, rho);
-      }
+      const bool fresh = site && L.code[idx] >= 0 && code_bit_on(L.code + idx, I.flag);
+      warp_append(fresh, (int)idx, I.flag_count, I.flag_list, I.cap_flag, I.overflow);
     }
   }
-  if (ENERGY) {
-    const double t = block_sum(e_acc);
-    if (threadIdx.x == 0) e_partial[blockIdx.x] = t;
-  }
 }
 
-template <bool ENERGY>
+// Sum of v over the block in a fixed order, in thread 0 (its warp sums in `red`).
+__device__ __forceinline__ double itl_block_sum(double v, double *red) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x == 0)
+    for (int k = 0; k < MB_ITL_THREADS / 32; k++) t += red[k];
+  return t;
+}
+
+// Density (FORCE = 0) or force pass of the interstitials and of the marked sites' pairs with
+// them.  e0, e1: CTA partials of F(rho), or of the pair and kinetic energies.
+template <bool FORCE, bool ENERGY>
 __global__ void __launch_bounds__(MB_ITL_THREADS)
-    k_itl_force64(const __grid_constant__ StencilSet st, const Geom g, const DevPot P, const Lattice64 L,
-                  const Itl64 I, const StepParams sp, double *e_pair, double *e_kin, int z0, int z1) {
-  const int lane = threadIdx.x & 31;
+    k_itl_items64(const Geom g, const DevPot P, const Lattice64 L, const Itl64 I, const StepParams sp, double *e0,
+                  double *e1, int z0, int z1) {
+  __shared__ double red[4][MB_ITL_THREADS / 32];
   const bool all_z = z0 <= 0 && z1 >= g.bz; // else only items in box layers [z0, z1)
-  const int nflag = min(I.flag_count[0], I.cap_flag);
-  const int n_itl = itl_n(I);
-  const long long n_items = (long long)nflag + n_itl;
-  const long long wstride = (long long)gridDim.x * (blockDim.x >> 5);
-  __shared__ int s_list[MB_ITL_THREADS / 32][MB_WIN_LIST];
-  int *list = s_list[threadIdx.x >> 5];
-  double ep_acc = 0.0, ek_acc = 0.0;
-  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n_items; w += wstride) {
-    const bool is_site = w >= n_itl;
+  const int nflag = min(*I.flag_count, I.cap_flag), n_itl = itl_n(I), l8 = threadIdx.x & 7;
+  const int jobs = n_itl + (nflag + MB_ITL_THREADS / 8 - 1) / (MB_ITL_THREADS / 8);
+  double acc0 = 0.0, acc1 = 0.0;
+  for (int job = blockIdx.x; job < jobs; job += gridDim.x) {
+    const bool is_site = job >= n_itl;
     long long i = 0;
-    int s = 0, cx = 0, y = 0, z = 0, it = 0, ti;
-    double xi, yi, zi, dfi;
+    int s = 0, cx = 0, y = 0, z = 0, ti = 0;
+    bool on = true;
+    double xi = 0.0, yi = 0.0, zi = 0.0, dfi = 0.0;
     if (is_site) {
-      i = I.flag_list[w - n_itl];
-      decode_ext(g, i, s, cx, y, z);
-      ti = L.code[i] & 0x3F;
-      xi = L.p[i].x;
-      yi = L.p[i].y;
-      zi = L.p[i].z;
-      dfi = L.p[i].w;
+      const int w = (job - n_itl) * (MB_ITL_THREADS / 8) + (threadIdx.x >> 3);
+      on = w < nflag;
+      if (on) {
+        i = I.flag_list[w];
+        const double4 own = ld_site(L.p + i);
+        ti = L.code[i] & MB_TYPE_MASK;
+        xi = own.x;
+        yi = own.y;
+        zi = own.z;
+        if (FORCE) dfi = own.w;
+        decode_ext(g, i, s, cx, y, z);
+        on = all_z || (z >= z0 && z < z1);
+      }
     } else {
-      it = (int)w;
-      ti = I.type[it];
-      xi = I.px[it];
-      yi = I.py[it];
-      zi = I.pz[it];
-      dfi = I.df[it];
+      ti = I.type[job];
+      xi = I.px[job];
+      yi = I.py[job];
+      zi = I.pz[job];
+      if (FORCE) dfi = I.df[job];
+      if (!all_z) {
+        const int lz = z_layer(g, I.a0, zi);
+        if (lz < z0 || lz >= z1) continue; // the whole block
+      }
     }
-    if (!all_z) {
-      const int lz = is_site ? z : z_layer(g, I.a0, zi);
-      if (lz < z0 || lz >= z1) continue;
-    }
-    double fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0;
-    auto add_pair = [&](double dx, double dy, double dz, int tj, double dfj) {
+    double rho = 0.0, fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0;
+    auto pair = [&](double dx, double dy, double dz, int tj, double dfj) {
       const double d2 = dx * dx + dy * dy + dz * dz;
       if (d2 >= sp.rc2) return;
       const double rinv = rsqrt(d2);
+      if (!FORCE) {
+        rho += rho_of_r(P, tj, d2 * rinv);
+        return;
+      }
       double ph = 0.0;
       const double psip = pair_psip(P, ti, tj, d2 * rinv, dfi, dfj, ENERGY ? &ph : nullptr);
       const double fpair = -psip * rinv;
@@ -887,137 +770,172 @@ __global__ void __launch_bounds__(MB_ITL_THREADS)
       fz += dz * fpair;
       if (ENERGY) ep += 0.5 * ph;
     };
-    if (is_site) {
-      for (int k = lane; k < st.n; k += 32) {
-        const long long j = i + st.off[s][k];
+    if (!is_site) {
+      const Window win = make_window(xi, yi, zi, I.a0, I.reach);
+      const int ncand = win.nx * win.ny * win.nz;
+      for (int c = threadIdx.x; c < ncand; c += MB_ITL_THREADS) {
+        long long j;
+        double sx, sy, sz;
+        if (!window_site(g, win, c, xi, yi, zi, I.a0, I.reach, j, sx, sy, sz)) continue;
         const int cj = L.code[j];
-        if (cj < 0) continue;
         const double4 pj = ld_site(L.p + j);
-        add_pair(xi - pj.x, yi - pj.y, zi - pj.z, cj & 0x3F, pj.w);
+        if (cj >= 0)
+          pair(xi - (pj.x + sx), yi - (pj.y + sy), zi - (pj.z + sz), cj & MB_TYPE_MASK, FORCE ? pj.w : 0.0);
       }
-    } else {
-      window_pairs64<true>(g, L, I, xi, yi, zi, list, add_pair);
     }
-    for (int K = lane; K < n_itl; K += 32) {
-      if (!is_site && K == it) continue;
-      add_pair(min_image(xi - I.px[K], g.Lx, g.iLx), min_image(yi - I.py[K], g.Ly, g.iLy), min_image(zi - I.pz[K], g.Lz, g.iLz),
-               I.type[K], I.df[K]);
-    }
-    fx = warp_sum(fx);
-    fy = warp_sum(fy);
-    fz = warp_sum(fz);
-    if (ENERGY) ep = warp_sum(ep);
-    if (lane == 0) {
-      double *vxp = is_site ? L.vx : I.vx;
-      const long long vi = is_site ? i : it;
-      if (is_site) {
-        if (L.fx) {
-          L.fx[i] = fx;
-          L.fy[i] = fy;
-          L.fz[i] = fz;
-        }
+    if (on)
+      for (int K = is_site ? l8 : threadIdx.x; K < n_itl; K += is_site ? 8 : MB_ITL_THREADS) {
+        if (!is_site && K == job) continue;
+        pair(min_image(xi - I.px[K], g.Lx, g.iLx), min_image(yi - I.py[K], g.Ly, g.iLy),
+             min_image(zi - I.pz[K], g.Lz, g.iLz), I.type[K], FORCE ? I.df[K] : 0.0);
+      }
+    if (is_site) {
+      if (!FORCE) {
+        rho = group8_sum(rho);
       } else {
-        I.fx[it] = fx;
-        I.fy[it] = fy;
-        I.fz[it] = fz;
+        fx = group8_sum(fx);
+        fy = group8_sum(fy);
+        fz = group8_sum(fz);
+        if (ENERGY) ep = group8_sum(ep);
       }
-      if (vxp) {
-        double *vyp = is_site ? L.vy : I.vy, *vzp = is_site ? L.vz : I.vz;
-        double vx = vxp[vi], vy = vyp[vi], vz = vzp[vi];
-        if (sp.kick_pre) {
-          vx += sp.h * fx;
-          vy += sp.h * fy;
-          vz += sp.h * fz;
-        }
-        if (ENERGY) ek_acc += 0.5 * sp.mass * (vx * vx + vy * vy + vz * vz) * MB_MVV2E;
-        if (sp.drift) {
-          vx += sp.h * fx;
-          vy += sp.h * fy;
-          vz += sp.h * fz;
-          const double nx = xi + sp.dt * vx, ny = yi + sp.dt * vy, nz = zi + sp.dt * vz;
-          if (is_site) {
-            st_site(L.n + i, nx, ny, nz, 0.0);
-            conv_check(g, sp, s, cx, y, z, nx, ny, nz);
-            if (g.images)
-              for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
-                st_site(L.n + idx, nx + ox, ny + oy, nz + oz, 0.0);
-              });
-          } else {
-            I.nx[it] = nx;
-            I.ny[it] = ny;
-            I.nz[it] = nz;
-          }
-        }
-        vxp[vi] = vx;
-        vyp[vi] = vy;
-        vzp[vi] = vz;
+      if (!on || l8) continue; // the first lane of the group finishes
+    } else {
+      __syncthreads(); // the last job's sums are read
+      if (!FORCE) {
+        rho = itl_block_sum(rho, red[0]);
+      } else {
+        fx = itl_block_sum(fx, red[0]);
+        fy = itl_block_sum(fy, red[1]);
+        fz = itl_block_sum(fz, red[2]);
+        if (ENERGY) ep = itl_block_sum(ep, red[3]);
       }
-      if (ENERGY) ep_acc += ep;
+      if (threadIdx.x) continue;
+    }
+    if (!FORCE) {
+      if (is_site) rho = L.rho[i] + rho;
+      const double df = dF64(P, ti, rho);
+      if (is_site) {
+        L.rho[i] = rho;
+        L.p[i].w = df;
+        if (g.images) for_images(g, s, cx, y, z, [&](long long idx, double, double, double) { L.p[idx].w = df; });
+      } else {
+        I.rho[job] = rho;
+        I.df[job] = df;
+      }
+      if (ENERGY) acc0 += F64(P, ti, rho);
+      continue;
+    }
+    const long long vi = is_site ? i : job;
+    double *fxp = is_site ? L.fx : I.fx, *fyp = is_site ? L.fy : I.fy, *fzp = is_site ? L.fz : I.fz;
+    if (is_site) {
+      fx = fxp[vi] + fx;
+      fy = fyp[vi] + fy;
+      fz = fzp[vi] + fz;
+    }
+    fxp[vi] = fx;
+    fyp[vi] = fy;
+    fzp[vi] = fz;
+    if (ENERGY) acc0 += ep;
+    double *vxp = is_site ? L.vx : I.vx, *vyp = is_site ? L.vy : I.vy, *vzp = is_site ? L.vz : I.vz;
+    if (!vxp) continue;
+    double vx = vxp[vi], vy = vyp[vi], vz = vzp[vi];
+    if (sp.kick_pre) {
+      vx += sp.h * fx;
+      vy += sp.h * fy;
+      vz += sp.h * fz;
+    }
+    if (ENERGY) acc1 += 0.5 * sp.mass * (vx * vx + vy * vy + vz * vz) * MB_MVV2E;
+    if (sp.drift) {
+      vx += sp.h * fx;
+      vy += sp.h * fy;
+      vz += sp.h * fz;
+      const double nx = xi + sp.dt * vx, ny = yi + sp.dt * vy, nz = zi + sp.dt * vz;
+      if (is_site) {
+        st_site(L.n + i, nx, ny, nz, 0.0);
+        conv_check(g, sp, s, cx, y, z, nx, ny, nz);
+        if (g.images)
+          for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
+            st_site(L.n + idx, nx + ox, ny + oy, nz + oz, 0.0);
+          });
+      } else {
+        I.nx[job] = nx;
+        I.ny[job] = ny;
+        I.nz[job] = nz;
+      }
+    }
+    vxp[vi] = vx;
+    vyp[vi] = vy;
+    vzp[vi] = vz;
+  }
+  // last step's marks came off before this pass: its list takes the next step's
+  if (FORCE && blockIdx.x == 0 && threadIdx.x == 0) *I.old_count = 0;
+  if (ENERGY) {
+    const double t0 = block_sum(acc0);
+    if (threadIdx.x == 0) e0[blockIdx.x] = t0;
+    if (FORCE) {
+      const double t1 = block_sum(acc1);
+      if (threadIdx.x == 0) e1[blockIdx.x] = t1;
     }
   }
-  if (ENERGY) {
-    const double t1 = block_sum(ep_acc);
-    if (threadIdx.x == 0) e_pair[blockIdx.x] = t1;
-    const double t2 = block_sum(ek_acc);
-    if (threadIdx.x == 0) e_kin[blockIdx.x] = t2;
+}
+
+static int itl_blocks(int n) { return n < 4 * device_sm_count() ? n : 4 * device_sm_count(); }
+
+int launch_itl_mark64(const Geom &g, const Lattice64 &L, const Itl64 &I, int clear, cudaStream_t s, int z0, int z1) {
+  if (z1 < 0) z1 = g.bz;
+  const int nmax = I.nd ? I.cap : I.n;
+  if (nmax <= 0 || z0 >= z1) return MB_OK;
+  const int marks = itl_blocks(nmax);
+  int clears = clear ? (I.cap_flag + MB_ITL_THREADS - 1) / MB_ITL_THREADS : 0;
+  if (clears > device_sm_count()) clears = device_sm_count();
+  k_itl_mark<<<marks + clears, MB_ITL_THREADS, 0, s>>>(g, L, I, marks, z0, z1);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
+__global__ void k_itl_reset(const Lattice64 L, const Itl64 I) {
+  const int both = MB_FLAG_ITL(0) | MB_FLAG_ITL(1);
+  for (int l = 0; l < 2; l++) {
+    const int *list = l ? I.old_list : I.flag_list;
+    const int n = min(l ? *I.old_count : *I.flag_count, I.cap_flag);
+    for (int k = threadIdx.x; k < n; k += blockDim.x) code_bit_off(L.code + list[k], both);
   }
+  __syncthreads();
+  if (threadIdx.x == 0) *I.flag_count = *I.old_count = 0;
 }
 
-int launch_itl_mark64(const Geom &g, const Lattice64 &L, const Itl64 &I, cudaStream_t s) {
-  int grid = (I.cap_flag + 255) / 256;
-  if (grid > 4 * device_sm_count()) grid = 4 * device_sm_count();
-  k_itl_clear<<<grid, 256, 0, s>>>(L, I);
-  MB_CUDA(cudaGetLastError());
-  MB_CUDA(cudaMemsetAsync(I.flag_count, 0, sizeof(int), s));
-  const int nmax = I.nd ? I.cap : I.n;
-  if (nmax > 0)
-    k_itl_mark<<<(nmax * 32 + MB_ITL_THREADS - 1) / MB_ITL_THREADS, MB_ITL_THREADS, 0, s>>>(g, L, I, 0, g.bz);
+int launch_itl_reset64(const Lattice64 &L, const Itl64 &I, cudaStream_t s) {
+  k_itl_reset<<<1, 1024, 0, s>>>(L, I);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }
 
-int launch_itl_mark_slab64(const Geom &g, const Lattice64 &L, const Itl64 &I, int z0, int z1, cudaStream_t s) {
-  const int nmax = I.nd ? I.cap : I.n;
-  if (nmax > 0 && z0 < z1)
-    k_itl_mark<<<(nmax * 32 + MB_ITL_THREADS - 1) / MB_ITL_THREADS, MB_ITL_THREADS, 0, s>>>(g, L, I, z0, z1);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
-}
-
-static int itl_grid(const Itl64 &I) {
-  const long long warps = (long long)I.cap_flag + (I.nd ? I.cap : I.n);
-  long long ctas = (warps * 32 + MB_ITL_THREADS - 1) / MB_ITL_THREADS;
-  const long long cap = 4LL * device_sm_count();
-  if (ctas > cap) ctas = cap;
-  if (ctas > MB_EPART_CAP) ctas = MB_EPART_CAP;
-  return (int)(ctas > 0 ? ctas : 1);
-}
-
-int launch_itl_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, const Itl64 &I,
-                     double rc2, double *e_partial, int energy, cudaStream_t s, int z0, int z1) {
+template <bool FORCE>
+static int launch_items(const Geom &g, const DevPot &pot, const Lattice64 &L, const Itl64 &I, const StepParams &sp,
+                        double *e0, double *e1, int energy, cudaStream_t s, int z0, int z1) {
   if (!I.nd && I.n == 0) return MB_OK;
   if (z1 < 0) z1 = g.bz;
-  const int grid = itl_grid(I);
+  const int grid = itl_blocks((I.nd ? I.cap : I.n) + (I.cap_flag + 31) / 32);
   if (energy)
-    k_itl_rho64<true><<<grid, MB_ITL_THREADS, 0, s>>>(st, g, pot, L, I, rc2, e_partial + 3 * MB_EPART_CAP, z0, z1);
+    k_itl_items64<FORCE, true><<<grid, MB_ITL_THREADS, 0, s>>>(g, pot, L, I, sp, e0, e1, z0, z1);
   else
-    k_itl_rho64<false><<<grid, MB_ITL_THREADS, 0, s>>>(st, g, pot, L, I, rc2, nullptr, z0, z1);
+    k_itl_items64<FORCE, false><<<grid, MB_ITL_THREADS, 0, s>>>(g, pot, L, I, sp, nullptr, nullptr, z0, z1);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }
 
-int launch_itl_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, const Itl64 &I,
-                       const StepParams &sp, double *e_partial, int energy, cudaStream_t s, int z0, int z1) {
-  if (!I.nd && I.n == 0) return MB_OK;
-  if (z1 < 0) z1 = g.bz;
-  const int grid = itl_grid(I);
-  if (energy)
-    k_itl_force64<true><<<grid, MB_ITL_THREADS, 0, s>>>(st, g, pot, L, I, sp, e_partial + 4 * MB_EPART_CAP,
-                                                         e_partial + 5 * MB_EPART_CAP, z0, z1);
-  else
-    k_itl_force64<false><<<grid, MB_ITL_THREADS, 0, s>>>(st, g, pot, L, I, sp, nullptr, nullptr, z0, z1);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
+int launch_itl_rho64(const Geom &g, const DevPot &pot, const Lattice64 &L, const Itl64 &I, double rc2,
+                     double *e_partial, int energy, cudaStream_t s, int z0, int z1) {
+  StepParams sp{};
+  sp.rc2 = rc2;
+  return launch_items<false>(g, pot, L, I, sp, energy ? e_partial + 3 * MB_EPART_CAP : nullptr, nullptr, energy, s, z0,
+                             z1);
+}
+
+int launch_itl_force64(const Geom &g, const DevPot &pot, const Lattice64 &L, const Itl64 &I, const StepParams &sp,
+                       double *e_partial, int energy, cudaStream_t s, int z0, int z1) {
+  return launch_items<true>(g, pot, L, I, sp, energy ? e_partial + 4 * MB_EPART_CAP : nullptr,
+                            energy ? e_partial + 5 * MB_EPART_CAP : nullptr, energy, s, z0, z1);
 }
 
 // ------------------------------------------ lattice <-> interstitial bookkeeping
@@ -1073,7 +991,7 @@ __global__ void __launch_bounds__(MB_CONV_THREADS, 1)
     I.fz[k] = L.fz[i];
     I.rho[k] = L.rho ? L.rho[i] : 0.0;
     I.df[k] = L.p[i].w;
-    I.type[k] = (int8_t)(L.code[i] & 0x3F);
+    I.type[k] = (int8_t)(L.code[i] & MB_TYPE_MASK);
     I.id[k] = site_id[t];
     // vacant: both position buffers far away (the pair loops reject vacancies by
     // position, and the buffer of this step comes back as the next step's drift target)
@@ -1251,7 +1169,7 @@ __global__ void k_images64(const Geom g, const Lattice64 L, int what, long long 
         L.p[idx].x = x0 + ox;
         L.p[idx].y = y0 + oy;
         L.p[idx].z = z0 + oz;
-        L.code[idx] = (int8_t)(c < 0 ? c : (c & 0x3F));
+        L.code[idx] = (int8_t)(c < 0 ? c : (c & MB_TYPE_MASK));
       });
     }
     if (what & 2) {
@@ -1332,31 +1250,26 @@ int launch_kick_drift64(const Geom &g, const Lattice64 &L, const Itl64 &I, const
 }
 
 // Sum of each energy region in a fixed order: out[0] = pe, out[1] = ke.
-__global__ void k_reduce_energy(const double *part, double *out) {
-  __shared__ double acc[2][256];
+__global__ void __launch_bounds__(1024) k_reduce_energy(const double *part, double *out) {
   double pe = 0.0, ke = 0.0;
-  for (int k = threadIdx.x; k < MB_EPART_CAP; k += blockDim.x) {
+#pragma unroll
+  for (int r = 0; r < MB_EPART_CAP / 1024; r++) {
+    const int k = r * 1024 + threadIdx.x;
     pe += part[0 * MB_EPART_CAP + k] + part[1 * MB_EPART_CAP + k] + part[3 * MB_EPART_CAP + k] +
           part[4 * MB_EPART_CAP + k];
     ke += part[2 * MB_EPART_CAP + k] + part[5 * MB_EPART_CAP + k];
   }
-  acc[0][threadIdx.x] = pe;
-  acc[1][threadIdx.x] = ke;
-  __syncthreads();
+  pe = block_sum(pe);
+  ke = block_sum(ke);
   if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0;
-    for (int k = 0; k < 256; k++) {
-      a += acc[0][k];
-      b += acc[1][k];
-    }
-    out[0] = a;
-    out[1] = b;
+    out[0] = pe;
+    out[1] = ke;
   }
 }
 
 int launch_reduce(const double *partials, int n, double *out, cudaStream_t s) {
   (void)n;
-  k_reduce_energy<<<1, 256, 0, s>>>(partials, out);
+  k_reduce_energy<<<1, 1024, 0, s>>>(partials, out);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }

@@ -112,7 +112,7 @@ __global__ void k_pack_box(const Geom g, mb_atom_element *aos, const Lattice64 L
     mb_atom_element a;
     const int c = L.code[i];
     a.id = ids ? ids[t] : t;
-    a.type = c < 0 ? -1 : (c & 0x3F);
+    a.type = c < 0 ? -1 : (c & MB_TYPE_MASK);
     a.pad_ = 0;
     if (c < 0) {
       for (int k = 0; k < 3; k++) a.x[k] = a.v[k] = a.f[k] = 0.0;
@@ -162,7 +162,7 @@ __global__ void k_df_from_rho(const Geom g, const DevPot P, Lattice64 L) {
     int m;
     double p;
     spl_loc(L.rho[i], P.rdrho, P.nrho, m, p);
-    const double4 d = ldg4(&P.F_der[(size_t)(c & 0x3F) * P.nrho + m]);
+    const double4 d = ldg4(&P.F_der[(size_t)(c & MB_TYPE_MASK) * P.nrho + m]);
     L.p[i].w = (d.z * p + d.y) * p + d.x;
   }
 }

@@ -33,7 +33,7 @@ struct LatticeArgs {
   int w0, n_items;       // items [w0, n_items)
   double rc2, rc2m;      // squared cutoff; a hair above it for the outer-entry masks
   int rc2_hi;            // high word of rc2
-  int skip_flagged;
+  int flag;              // code bit of the sites an interstitial pass finishes (0: none)
   uint2 *outer;          // per item: the outer entries some lane has inside rc2m (or null)
   double *e0, *e1;       // CTA partials: density pass F(rho); force pass pair and kinetic energy
   StepParams sp;
@@ -259,9 +259,13 @@ __device__ __forceinline__ void decode_site(const Geom &g, int i, int &s, int &c
 
 // df = F'(rho), its ghost images; returns F(rho) with ENERGY.
 template <bool ENERGY>
-__device__ __forceinline__ double rho_finish64(const Geom &g, const DevPot &P, const Lattice64 &L, int ti, int ref,
-                                               double rho) {
-  const int i = ref & MB_SITE_INDEX;
+__device__ __forceinline__ double rho_finish64(const Geom &g, const DevPot &P, const Lattice64 &L, int code, int flag,
+                                               int ref, double rho) {
+  const int i = ref & MB_SITE_INDEX, ti = code & MB_TYPE_MASK;
+  if (code & flag) { // the interstitial pass adds its pairs to this sum
+    L.rho[i] = rho;
+    return 0.0;
+  }
   const double df = dF64(P, ti, rho);
   L.p[i].w = df;
   L.rho[i] = rho;
@@ -288,14 +292,14 @@ __device__ __forceinline__ void conv_check(const Geom &g, const StepParams &sp, 
 // Force of a site: stores it, closes the previous step, drifts to the next positions (and
 // their ghost images); returns the kinetic energy with ENERGY.
 template <bool ENERGY>
-__device__ __forceinline__ double force_finish64(const Geom &g, const Lattice64 &L, const StepParams &sp, int ref,
-                                                 const Site64 &c, double fx, double fy, double fz) {
+__device__ __forceinline__ double force_finish64(const Geom &g, const Lattice64 &L, const StepParams &sp, bool flagged,
+                                                 int ref, const Site64 &c, double fx, double fy, double fz) {
   double ek = 0.0;
   const int i = ref & MB_SITE_INDEX;
   L.fx[i] = fx;
   L.fy[i] = fy;
   L.fz[i] = fz;
-  if (!L.vx) return ek;
+  if (flagged || !L.vx) return ek; // flagged: the interstitial pass adds its pairs and integrates
   double vx = L.vx[i], vy = L.vy[i], vz = L.vz[i];
   if (sp.kick_pre) {
     vx = __fma_rn(sp.h, fx, vx);

@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(MB_SHELL_RHO_THREADS, 1)
           if (SH) rho = L.rho[i];
         }
         unsigned long long near = 0;
-        if (!(code < 0 || (a.skip_flagged && (code & MB_FLAG_ITL)))) {
+        if (code >= 0) {
           const Site64 c{L.p + i, st.off[i >= (int)a.g.E], own.x, own.y, own.z, 0.0};
           const Bases64 bs = site_bases(a.g, L.p, i);
           static_for<SH, END>([&](auto hc) { rho_shell<decltype(hc)::value>(a, W, c, bs, pl, rw, rho); });
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(MB_SHELL_RHO_THREADS, 1)
               rho = __dadd_rn(rho, rho_outer(a, c, k0, min(k0 + MB_OUT_RUN, st.n), m));
               near |= (unsigned long long)m << (k0 - n_near);
             }
-            const double e = rho_finish64<ENERGY>(a.g, a.P, L, code & 0x3F, ref, rho);
+            const double e = rho_finish64<ENERGY>(a.g, a.P, L, code, a.flag, ref, rho);
             if (ENERGY) e_acc += e;
           }
         }
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(MB_SHELL_FORCE_THREADS, 1)
           fy = L.fy[i];
           fz = L.fz[i];
         }
-        if (code < 0 || (a.skip_flagged && (code & MB_FLAG_ITL))) continue;
+        if (code < 0) continue;
         const Site64 c{L.p + i, st.off[i >= (int)a.g.E], own.x, own.y, own.z, own.w};
         force_shell<SH, ENERGY>(a, W, c, site_bases(a.g, L.p, i), pl, rw, fx, fy, fz, e_pair);
         if (SH + 1 < NEAR) {
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(MB_SHELL_FORCE_THREADS, 1)
             fy = __dadd_rn(fy, ty);
             fz = __dadd_rn(fz, tz);
           }
-          const double ek = force_finish64<ENERGY>(a.g, L, a.sp, ref, c, fx, fy, fz);
+          const double ek = force_finish64<ENERGY>(a.g, L, a.sp, code & a.flag, ref, c, fx, fy, fz);
           if (ENERGY) e_kin += ek;
         }
       }

@@ -43,7 +43,8 @@ struct mb_sim {
   double *ipos[2][3] = {}, *iv[3] = {}, *ifr[3] = {}, *irho = nullptr, *idf = nullptr;
   int8_t *itype = nullptr;
   int64_t *iid = nullptr;
-  int *flag_list = nullptr, *flag_count = nullptr;
+  int *flag_list = nullptr, *flag_count = nullptr; // a list per buffer; counts [2], overflow
+  int flag_last = -1;                              // buffer of the last step with interstitial passes
   int *d_nitl = nullptr; // device-resident interstitial count (conversions change it)
   // lattice <-> interstitial conversion (off while conv_d == 0)
   double conv_d = 0.0, rec_d = 0.0;
@@ -130,8 +131,12 @@ Itl64 sim_itl(mb_sim *s, int which) {
   I.df = s->idf;
   I.type = s->itype;
   I.id = s->iid;
-  I.flag_list = s->flag_list;
-  I.flag_count = s->flag_count;
+  I.flag = MB_FLAG_ITL(which);
+  I.flag_list = s->flag_list + (size_t)which * s->cap_flag;
+  I.flag_count = s->flag_count + which;
+  I.old_list = s->flag_list + (size_t)(which ^ 1) * s->cap_flag;
+  I.old_count = s->flag_count + (which ^ 1);
+  I.overflow = s->flag_count + 2;
   I.a0 = s->cfg.lattice_const;
   I.reach = s->cfg.cutoff + s->cfg.stencil_skin;
   return I;
@@ -166,16 +171,22 @@ static int step64(mb_sim *s, int energy, int kick_pre, int drift, int timed) {
   StepParams sp = sim_params(s, kick_pre, drift);
   double *ep = energy ? s->epart : nullptr;
   if (energy) MB_CUDA(cudaMemsetAsync(s->epart, 0, sizeof(double) * energy_partials_needed(), s->stream));
-  const int itl = itl_active(s);
-  if (itl) MB_TRY(launch_itl_mark64(s->g, L, I, s->stream));
+  const int itl = itl_active(s), flag = itl ? I.flag : 0;
+  if (itl) {
+    // a step after one at the other buffer clears that one's marks; any other state of the
+    // lists (a first step, interstitials that come back) starts from empty ones
+    if (s->flag_last != (s->cur ^ 1)) MB_TRY(launch_itl_reset64(L, I, s->stream));
+    MB_TRY(launch_itl_mark64(s->g, L, I, 1, s->stream));
+  }
+  s->flag_last = itl ? s->cur : -1;
   if (timed) MB_CUDA(cudaEventRecord(s->ev[4], s->stream));
-  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, ep, energy, itl, s->stream, 0, -1, s->outer, &s->plan));
+  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, ep, energy, flag, s->stream, 0, -1, s->outer, &s->plan));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[5], s->stream));
-  if (itl) MB_TRY(launch_itl_rho64(s->g, s->st, P, L, I, sp.rc2, ep, energy, s->stream));
+  if (itl) MB_TRY(launch_itl_rho64(s->g, P, L, I, sp.rc2, ep, energy, s->stream));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[6], s->stream));
-  MB_TRY(launch_force64(s->g, s->st, P, L, sp, ep, energy, itl, s->stream, 0, -1, s->outer, &s->plan));
+  MB_TRY(launch_force64(s->g, s->st, P, L, sp, ep, energy, flag, s->stream, 0, -1, s->outer, &s->plan));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[7], s->stream));
-  if (itl) MB_TRY(launch_itl_force64(s->g, s->st, P, L, I, sp, ep, energy, s->stream));
+  if (itl) MB_TRY(launch_itl_force64(s->g, P, L, I, sp, ep, energy, s->stream));
   if (sp.conv2 > 0.0)
     MB_TRY(launch_convert64(s->g, L, I, sp, s->rec_d * s->rec_d, s->id, s->d_nitl, s->d_conv_counters, s->stream));
   return MB_OK;
@@ -476,8 +487,8 @@ static int create_sim(const mb_sim_config *cfg, const mb_eam_tables *pot, int z_
   const double R = reach;
   const int per = (int)(2.0 * 4.18879 * R * R * R / (0.5 * pow(cfg->lattice_const, 3))) + 64;
   s->cap_flag = std::max(1, s->cap_itl * per);
-  if ((rc = dalloc(s, (void **)&s->flag_list, (size_t)s->cap_flag * sizeof(int))) != MB_OK) return cleanup(rc);
-  if ((rc = dalloc(s, (void **)&s->flag_count, 2 * sizeof(int))) != MB_OK) return cleanup(rc);
+  if ((rc = dalloc(s, (void **)&s->flag_list, 2 * (size_t)s->cap_flag * sizeof(int))) != MB_OK) return cleanup(rc);
+  if ((rc = dalloc(s, (void **)&s->flag_count, 3 * sizeof(int))) != MB_OK) return cleanup(rc);
   if ((rc = dalloc(s, (void **)&s->d_nitl, sizeof(int))) != MB_OK) return cleanup(rc);
   if ((rc = dalloc(s, (void **)&s->d_cand, MB_CAND_CAP * sizeof(long long))) != MB_OK) return cleanup(rc);
   if ((rc = dalloc(s, (void **)&s->d_cand_n, sizeof(int))) != MB_OK) return cleanup(rc);
@@ -486,7 +497,7 @@ static int create_sim(const mb_sim_config *cfg, const mb_eam_tables *pot, int z_
       cudaMemsetAsync(s->d_cand_n, 0, sizeof(int), s->stream) != cudaSuccess ||
       cudaMemsetAsync(s->d_conv_counters, 0, 4 * sizeof(long long), s->stream) != cudaSuccess)
     return cleanup(fail(MB_ERR_CUDA, "memset failed"));
-  if (cudaMemsetAsync(s->flag_count, 0, 2 * sizeof(int), s->stream) != cudaSuccess)
+  if (cudaMemsetAsync(s->flag_count, 0, 3 * sizeof(int), s->stream) != cudaSuccess)
     return cleanup(fail(MB_ERR_CUDA, "memset failed"));
   // vacant everywhere until an upload
   if (cudaMemsetAsync(s->code, 0xff, (ne + 3) & ~(size_t)3, s->stream) != cudaSuccess)
@@ -637,13 +648,14 @@ int mb_sim_upload(mb_sim *s, const mb_atom_element *box_atoms, const mb_atom_ele
   s->n_e = 0;
   s->e_steps.clear();
   s->outer_ok = false;
+  s->flag_last = -1;
   MB_TRY(ensure_stage(s, (size_t)s->n_box));
   MB_CUDA(cudaMemcpyAsync(s->stage, box_atoms, (size_t)s->n_box * sizeof(mb_atom_element), cudaMemcpyHostToDevice,
                           s->stream));
   MB_CUDA(cudaMemsetAsync(s->bad, 0, sizeof(int), s->stream));
   // clear interstitial flags and any ghost codes, then load both position buffers
   MB_CUDA(cudaMemsetAsync(s->code, 0xff, ((size_t)s->n_ext + 3) & ~(size_t)3, s->stream));
-  MB_CUDA(cudaMemsetAsync(s->flag_count, 0, 2 * sizeof(int), s->stream));
+  MB_CUDA(cudaMemsetAsync(s->flag_count, 0, 3 * sizeof(int), s->stream));
   for (int b = 0; b < 2; b++) {
     Lattice64 L = sim_lattice(s, b);
     MB_TRY(launch_unpack_box_ids(s->g, s->stage, L, 1, s->bad, s->id, pot_dev(s->pot).n_types, s->stream));
@@ -703,10 +715,10 @@ int mb_sim_sync(mb_sim *s) {
   if (!s) return fail(MB_ERR_ARG, "null sim");
   MB_CUDA(cudaStreamSynchronize(s->stream));
   MB_CUDA(cudaMemcpy(&s->n_itl, s->d_nitl, sizeof(int), cudaMemcpyDeviceToHost));
-  int fc[2] = {0, 0};
+  int fc[3] = {0, 0, 0};
   if (itl_active(s)) {
     MB_CUDA(cudaMemcpy(fc, s->flag_count, sizeof(fc), cudaMemcpyDeviceToHost));
-    if (fc[1]) return fail(MB_ERR_ARG, "interstitial flag list overflowed");
+    if (fc[2]) return fail(MB_ERR_ARG, "interstitial flag list overflowed");
   }
   return MB_OK;
 }
@@ -823,12 +835,16 @@ static int step_host_whole(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
   StepParams sp = sim_params(s, 1, 0);
   MB_TRY(launch_kick_drift64(s->g, L, I, sp, s->stream));
   const DevPot &P = pot_dev(s->pot);
-  const int it = s->n_itl > 0;
-  if (it) MB_TRY(launch_itl_mark64(s->g, L, I, s->stream));
-  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, nullptr, 0, it, s->stream, 0, -1, s->outer, &s->plan));
-  if (it) MB_TRY(launch_itl_rho64(s->g, s->st, P, L, I, sp.rc2, nullptr, 0, s->stream));
-  MB_TRY(launch_force64(s->g, s->st, P, L, sp, nullptr, 0, it, s->stream, 0, -1, s->outer, &s->plan));
-  if (it) MB_TRY(launch_itl_force64(s->g, s->st, P, L, I, sp, nullptr, 0, s->stream));
+  const int it = s->n_itl > 0, flag = it ? I.flag : 0;
+  s->flag_last = -1;
+  if (it) { // the records brought site codes without marks
+    MB_CUDA(cudaMemsetAsync(s->flag_count, 0, 2 * sizeof(int), s->stream));
+    MB_TRY(launch_itl_mark64(s->g, L, I, 0, s->stream));
+  }
+  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, nullptr, 0, flag, s->stream, 0, -1, s->outer, &s->plan));
+  if (it) MB_TRY(launch_itl_rho64(s->g, P, L, I, sp.rc2, nullptr, 0, s->stream));
+  MB_TRY(launch_force64(s->g, s->st, P, L, sp, nullptr, 0, flag, s->stream, 0, -1, s->outer, &s->plan));
+  if (it) MB_TRY(launch_itl_force64(s->g, P, L, I, sp, nullptr, 0, s->stream));
   MB_TRY(launch_pack_box_ids(s->g, s->stage, L, L.p, sp.h, 0, s->id, s->stream));
   MB_CUDA(cudaMemcpyAsync(box_atoms, s->stage, (size_t)s->n_box * sizeof(mb_atom_element), cudaMemcpyDeviceToHost,
                           s->stream));
@@ -871,10 +887,11 @@ static int step_host_slabs(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
   Itl64 I = sim_itl(s, 0);
   const StepParams sp = sim_params(s, 1, 0);
   const DevPot &P = pot_dev(s->pot);
-  const int it = s->n_itl > 0;
+  const int it = s->n_itl > 0, flag = it ? I.flag : 0;
+  s->flag_last = -1;
   auto start = [&]() -> int { // interstitials drift first (their forces came with them); no site is flagged yet
     if (!it) return MB_OK;
-    MB_CUDA(cudaMemsetAsync(s->flag_count, 0, sizeof(int), cs));
+    MB_CUDA(cudaMemsetAsync(s->flag_count, 0, 2 * sizeof(int), cs));
     return launch_kick_drift64(g, L, I, sp, cs, 0, 0, 1);
   };
   auto arrive = [&](int k) -> int {
@@ -882,17 +899,17 @@ static int step_host_slabs(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
     MB_TRY(launch_unpack_box_ids(g, s->stage, L, 1, s->bad, s->id, P.n_types, cs, zb[k], zb[k + 1]));
     MB_TRY(launch_images64(g, L, 1, cs, zb[k], zb[k + 1]));
     MB_TRY(launch_kick_drift64(g, L, I, sp, cs, zb[k], zb[k + 1], 0));
-    if (it) MB_TRY(launch_itl_mark_slab64(g, L, I, zb[k], zb[k + 1], cs));
+    if (it) MB_TRY(launch_itl_mark64(g, L, I, 0, cs, zb[k], zb[k + 1]));
     return MB_OK;
   };
   auto rho = [&](int k) -> int {
-    MB_TRY(launch_rho64(g, s->st, P, L, sp.rc2, nullptr, 0, it, cs, zb[k], zb[k + 1], s->outer, &s->plan));
-    if (it) MB_TRY(launch_itl_rho64(g, s->st, P, L, I, sp.rc2, nullptr, 0, cs, zb[k], zb[k + 1]));
+    MB_TRY(launch_rho64(g, s->st, P, L, sp.rc2, nullptr, 0, flag, cs, zb[k], zb[k + 1], s->outer, &s->plan));
+    if (it) MB_TRY(launch_itl_rho64(g, P, L, I, sp.rc2, nullptr, 0, cs, zb[k], zb[k + 1]));
     return MB_OK;
   };
   auto force = [&](int k) -> int {
-    MB_TRY(launch_force64(g, s->st, P, L, sp, nullptr, 0, it, cs, zb[k], zb[k + 1], s->outer, &s->plan));
-    if (it) MB_TRY(launch_itl_force64(g, s->st, P, L, I, sp, nullptr, 0, cs, zb[k], zb[k + 1]));
+    MB_TRY(launch_force64(g, s->st, P, L, sp, nullptr, 0, flag, cs, zb[k], zb[k + 1], s->outer, &s->plan));
+    if (it) MB_TRY(launch_itl_force64(g, P, L, I, sp, nullptr, 0, cs, zb[k], zb[k + 1]));
     MB_TRY(launch_pack_box_ids(g, s->stage, L, L.p, sp.h, 0, s->id, cs, zb[k], zb[k + 1]));
     MB_CUDA(cudaEventRecord(s->ev_out[k], cs));
     MB_CUDA(cudaStreamWaitEvent(s->cp_out, s->ev_out[k], 0));

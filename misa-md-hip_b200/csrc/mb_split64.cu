@@ -29,7 +29,7 @@ __device__ __forceinline__ void fill_table(double2 *w, const double2 *tab, int w
 
 // A lane's site in item w.
 struct SplitSite {
-  int ref, type;
+  int ref, code;
   Site64 c;
 };
 __device__ __forceinline__ SplitSite split_site(const StencilSet &st, const LatticeArgs &a, int w) {
@@ -37,8 +37,8 @@ __device__ __forceinline__ SplitSite split_site(const StencilSet &st, const Latt
   t.ref = __ldg(a.sites + 32 * (size_t)w + (threadIdx.x & 31));
   const int i = t.ref & MB_SITE_INDEX;
   const int code = t.ref < 0 ? -1 : a.L.code[i];
-  t.type = code & 0x3F;
-  if (code < 0 || (a.skip_flagged && (code & MB_FLAG_ITL))) {
+  t.code = code;
+  if (code < 0) {
     t.ref = -1;
     t.c = Site64{a.L.p, st.off[0], 0.0, 0.0, 0.0, 0.0};
   } else {
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
       if (t.ref >= 0) {
         double rho = 0.0;
         for (int r = 0; r < a.sh.runs; r++) rho = __dadd_rn(rho, sums[r][lane]);
-        const double e = rho_finish64<ENERGY>(a.g, a.P, a.L, t.type, t.ref, rho);
+        const double e = rho_finish64<ENERGY>(a.g, a.P, a.L, t.code, a.flag, t.ref, rho);
         if (ENERGY) e_acc += e;
       }
       if (a.outer && lane == 0) {
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
         fy = __dadd_rn(fy, sum[r * 96 + 32]);
         fz = __dadd_rn(fz, sum[r * 96 + 64]);
       }
-      const double ek = force_finish64<ENERGY>(a.g, a.L, a.sp, t.ref, t.c, fx, fy, fz);
+      const double ek = force_finish64<ENERGY>(a.g, a.L, a.sp, t.code & a.flag, t.ref, t.c, fx, fy, fz);
       if (ENERGY) e_kin += ek;
     }
   }
