@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "mb_ensemble_kernel.cuh"
+#include "mb_host_copy.cuh"
 
 namespace mb {
 
@@ -202,8 +203,12 @@ struct mb_ensemble {
   size_t device_bytes = 0;
   size_t fixed_bytes = 0;
   long long launches = 0;
+  mb::HostCopy copier;               // records to and from pageable buffers
+  mb_atom_element *stage = nullptr;  // records of one lattice on their way (up to MB_STAGE_KEEP)
+  size_t stage_n = 0;
   std::mutex mu;
 };
+#define MB_STAGE_KEEP (64u << 20) // bytes
 
 namespace mb {
 
@@ -217,6 +222,31 @@ static int edalloc(mb_ensemble *e, void **p, size_t bytes) {
   e->device_bytes += bytes;
   e->fixed_bytes += bytes;
   return MB_OK;
+}
+
+// Device records of one lattice (n of them): kept between calls up to MB_STAGE_KEEP, beyond
+// that allocated for the call (drop_stage).
+static int take_stage(mb_ensemble *e, size_t n, mb_atom_element **out) {
+  if (n > e->stage_n || n * sizeof(mb_atom_element) > MB_STAGE_KEEP) {
+    if (n * sizeof(mb_atom_element) <= MB_STAGE_KEEP) {
+      if (e->stage) cudaFree(e->stage);
+      e->stage = nullptr;
+      e->stage_n = 0;
+    }
+    cudaError_t r = cudaMalloc(out, n * sizeof(mb_atom_element));
+    if (r != cudaSuccess) {
+      cudaGetLastError();
+      return fail(MB_ERR_NOMEM, std::string("staging allocation failed: ") + cudaGetErrorString(r));
+    }
+    if (n * sizeof(mb_atom_element) > MB_STAGE_KEEP) return MB_OK;
+    e->stage = *out;
+    e->stage_n = n;
+  }
+  *out = e->stage;
+  return MB_OK;
+}
+static void drop_stage(mb_ensemble *e, mb_atom_element *stage) {
+  if (stage != e->stage) cudaFree(stage);
 }
 
 // Stencil tables of the tile kernel: every BCC site closer than reach, per sublattice.
@@ -936,6 +966,8 @@ int mb_ensemble_destroy(mb_ensemble *e) {
     if (p) cudaFree(p);
   for (auto &ev : e->ev)
     if (ev) cudaEventDestroy(ev);
+  if (e->stage) cudaFree(e->stage);
+  e->copier.release();
   if (e->stream) cudaStreamDestroy(e->stream);
   pot_free(e->pot);
   delete e;
@@ -1065,10 +1097,14 @@ int mb_ensemble_add(mb_ensemble *e, const mb_lattice_spec *spec, const mb_atom_e
   if (cudaMemsetAsync(block, 0, bytes, s) != cudaSuccess) return undo(fail(MB_ERR_CUDA, "memset failed"));
   if (cudaMemsetAsync(d.code, 0xff, n, s) != cudaSuccess) return undo(fail(MB_ERR_CUDA, "memset failed"));
   mb_atom_element *stage = nullptr;
-  if (cudaMalloc(&stage, nb * sizeof(mb_atom_element)) != cudaSuccess)
-    return undo(fail(MB_ERR_NOMEM, "staging allocation failed"));
+  int sc = take_stage(e, nb, &stage);
+  if (sc != MB_OK) return undo(sc);
   cudaMemsetAsync(e->d_bad, 0, sizeof(int), s);
-  cudaMemcpyAsync(stage, box, nb * sizeof(mb_atom_element), cudaMemcpyHostToDevice, s);
+  sc = e->copier.to_device(stage, box, nb * sizeof(mb_atom_element), s);
+  if (sc != MB_OK) {
+    drop_stage(e, stage);
+    return undo(sc);
+  }
   int grid = (int)std::min<size_t>((nb + 255) / 256, 16 * (size_t)device_sm_count());
   k_ens_upload<<<grid, 256, 0, s>>>(d, stage, L.ids, a0, e->d_bad, e->P.P.n_types);
   if (n_itl > 0) {
@@ -1094,7 +1130,7 @@ int mb_ensemble_add(mb_ensemble *e, const mb_lattice_spec *spec, const mb_atom_e
   int bad = 0;
   cudaMemcpyAsync(&bad, e->d_bad, sizeof(int), cudaMemcpyDeviceToHost, s);
   cudaError_t er = cudaStreamSynchronize(s);
-  cudaFree(stage);
+  drop_stage(e, stage);
   if (er != cudaSuccess) return undo(cuda_fail(er, "lattice upload"));
   if (bad) return undo(fail(MB_ERR_ARG, "atom type without a potential table"));
   d.cur = 0;
@@ -1180,13 +1216,12 @@ int mb_ensemble_download(mb_ensemble *e, int32_t slot, mb_atom_element *box, mb_
   const LatDesc &d = L.d;
   const size_t nb = 2 * (size_t)d.bcx * d.by * d.bz;
   mb_atom_element *stage = nullptr;
-  MB_CUDA(cudaMalloc(&stage, nb * sizeof(mb_atom_element)));
+  MB_TRY(take_stage(e, nb, &stage));
   const int grid = (int)std::min<size_t>((nb + 255) / 256, 16 * (size_t)device_sm_count());
   k_ens_pack<<<grid, 256, 0, e->stream>>>(d, stage, L.ids, e->cfg.lattice_const, e->P.h, e->P.dt);
-  cudaError_t r = cudaMemcpyAsync(box, stage, nb * sizeof(mb_atom_element), cudaMemcpyDeviceToHost, e->stream);
-  if (r == cudaSuccess) r = cudaStreamSynchronize(e->stream);
-  cudaFree(stage);
-  if (r != cudaSuccess) return cuda_fail(r, "lattice download");
+  const int rc = e->copier.to_host(box, stage, nb * sizeof(mb_atom_element), e->stream);
+  drop_stage(e, stage);
+  MB_TRY(rc);
   if (n_itl) *n_itl = d.n_itl;
   if (itl && d.n_itl > 0) {
     const int n = d.n_itl, c = d.primed ? (d.cur ^ 1) : d.cur;

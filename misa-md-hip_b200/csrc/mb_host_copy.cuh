@@ -1,0 +1,30 @@
+// Copies between device memory and a caller's pageable buffer (mb_host_copy.cu).
+#pragma once
+
+#include "mb_common.cuh"
+
+namespace mb {
+
+// One per simulation or ensemble: 8 MiB of page-locked memory from the first large copy until
+// release().  Calls on one object must not overlap.
+struct HostCopy {
+  static constexpr int kSlots = 8;
+  static constexpr size_t kChunk = 1u << 20;
+  static constexpr size_t kMinBytes = 2u << 20; // below: one plain copy is as fast
+  char *slots = nullptr;
+  cudaEvent_t ev[kSlots] = {};
+  // `bytes` between dev and host, after the work queued on s; done when it returns.
+  int to_host(void *host, const void *dev, size_t bytes, cudaStream_t s) {
+    return copy(host, const_cast<void *>(dev), bytes, true, s);
+  }
+  int to_device(void *dev, const void *host, size_t bytes, cudaStream_t s) {
+    return copy(const_cast<void *>(host), dev, bytes, false, s);
+  }
+  void release();
+
+ private:
+  int ensure();
+  int copy(void *host, void *dev, size_t bytes, bool to_host, cudaStream_t s);
+};
+
+} // namespace mb

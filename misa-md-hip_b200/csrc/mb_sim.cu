@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "mb_common.cuh"
+#include "mb_host_copy.cuh"
 
 #define MB_SLAB_MAX 32 // z-slabs of the pipelined host-buffer step
 
@@ -58,6 +59,7 @@ struct mb_sim {
   // staging
   mb_atom_element *stage = nullptr;
   size_t stage_n = 0;
+  mb::HostCopy copier; // records to and from pageable buffers
   int *bad = nullptr;
   // state
   int cur = 0;
@@ -547,6 +549,7 @@ int mb_sim_destroy(mb_sim *s) {
     cudaStreamSynchronize(s->cp_out);
     cudaStreamDestroy(s->cp_out);
   }
+  s->copier.release();
   if (s->stream) cudaStreamDestroy(s->stream);
   pot_free(s->pot);
   delete s;
@@ -650,8 +653,7 @@ int mb_sim_upload(mb_sim *s, const mb_atom_element *box_atoms, const mb_atom_ele
   s->outer_ok = false;
   s->flag_last = -1;
   MB_TRY(ensure_stage(s, (size_t)s->n_box));
-  MB_CUDA(cudaMemcpyAsync(s->stage, box_atoms, (size_t)s->n_box * sizeof(mb_atom_element), cudaMemcpyHostToDevice,
-                          s->stream));
+  MB_TRY(s->copier.to_device(s->stage, box_atoms, (size_t)s->n_box * sizeof(mb_atom_element), s->stream));
   MB_CUDA(cudaMemsetAsync(s->bad, 0, sizeof(int), s->stream));
   // clear interstitial flags and any ghost codes, then load both position buffers
   MB_CUDA(cudaMemsetAsync(s->code, 0xff, ((size_t)s->n_ext + 3) & ~(size_t)3, s->stream));
@@ -681,9 +683,7 @@ int mb_sim_download(mb_sim *s, mb_atom_element *box_atoms, mb_atom_element *itl,
   const int unkick = s->primed ? 1 : 0;
   Lattice64 L = sim_lattice(s, s->cur);
   MB_TRY(launch_pack_box_ids(s->g, s->stage, L, s->pos[which], sim_params(s, 0, 0).h, unkick, s->id, s->stream));
-  MB_CUDA(cudaMemcpyAsync(box_atoms, s->stage, (size_t)s->n_box * sizeof(mb_atom_element), cudaMemcpyDeviceToHost,
-                          s->stream));
-  MB_CUDA(cudaStreamSynchronize(s->stream));
+  MB_TRY(s->copier.to_host(box_atoms, s->stage, (size_t)s->n_box * sizeof(mb_atom_element), s->stream));
   MB_CUDA(cudaMemcpy(&s->n_itl, s->d_nitl, sizeof(int), cudaMemcpyDeviceToHost));
   if (n_itl) *n_itl = s->n_itl;
   if (itl) MB_TRY(download_itl(s, itl, which, unkick));
