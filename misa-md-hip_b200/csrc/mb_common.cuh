@@ -91,9 +91,10 @@ struct DevPot {
   const double4 *phi_val; // [np][nr]
   const double4 *phi_der; // [np][nr]
   const double2 *force1;  // single type: [nr][3] {f d0, phi d0}, {f d1, phi d1}, {f d2, phi d2}
-  // single type, knot form: an interval reads its d0 and d2 and the next knot's d0
-  const double2 *f_ys;    // [nr] {y, s} of f (a cubic Hermite piece takes two knots)
-  const double2 *force2;  // [nr][2] {f d0, phi d0}, {f d2, phi d2}
+  // knot form: an interval takes its own knot and the next one
+  const double2 *f_ys;    // [nr][nt] {y, s} of f (a cubic Hermite piece)
+  const double2 *force2;  // one type: [nr][2] {f d0, phi d0}, {f d2, phi d2}; several:
+                          // [nr][nt + np] {f d0, f d2} per type, {phi d0, phi d2} per pair
   // single precision copies for the mixed path
   const float4 *f_val32;   // [nt][nr]  {y, s, c2, c3}
   const float2 *force32;   // single type: [nr][3] {f d0, phi d0}, {f d1, phi d1}, {f d2, phi d2}
@@ -149,7 +150,7 @@ int stencil_generate(double a0, double reach, int ext_x, int ext_y, int64_t *eve
 int stencil_sort_by_distance(double a0, double cutoff, int ext_x, int ext_y, int64_t *even, int64_t *odd, int n,
                              int *n_near, double *dist = nullptr);
 
-// Shell windows and summation runs of a one-type stencil whose near entries are BCC shells
+// Shell windows and summation runs of a stencil whose near entries are BCC shells
 // (mb_pair64.cuh, mb_shell64.cu): near shell h looks up the table intervals lo[h] ..
 // lo[h] + cnt[h] - 1 of the density window and of the force window; run r holds the
 // entries [kb[r], kb[r + 1]), the first near_runs of them near ones of shell[r].
@@ -159,6 +160,7 @@ int stencil_sort_by_distance(double a0, double cutoff, int ext_x, int ext_y, int
 #define MB_OUT_RUN 16 // outer entries per run
 struct Windows64 {
   int lo[MB_NEAR_SHELLS], cnt[MB_NEAR_SHELLS];
+  int copies; // of every word in shared memory
 };
 struct Shells64 {
   int n, runs, near_runs;
@@ -177,7 +179,11 @@ bool plan64_shells(const DevPot &P, const Geom &g, double a0, double cutoff, con
 int plan64_plane_items(const Geom &g); // work items of one (z, sublattice) plane
 int plan64_items(const Geom &g);       // ... of the box
 int plan64_sites(const Geom &g, int *sites, cudaStream_t s);
-bool split64_fits(const Shells64 &sh);
+bool split64_fits(const DevPot &P, const Shells64 &sh);
+// 16-byte words per knot of the force tables (DevPot::force2).
+__host__ __device__ __forceinline__ int force_words(int n_types) {
+  return n_types == 1 ? 2 : n_types + n_types * (n_types + 1) / 2;
+}
 
 // ------------------------------------------------------ kernel arguments
 struct Lattice64 {

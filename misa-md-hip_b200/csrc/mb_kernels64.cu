@@ -520,11 +520,17 @@ int launch_split_force64(const StencilSet &st, const LatticeArgs &a, int energy,
 // (mb_split64.cu); larger ones take shell windows (mb_shell64.cu).  Measured on one B200 (a
 // pass, launch gap included): density 20 us a split round of 4 items per SM and 8.7 us each
 // further one against 44-52 us for up to 32 items per SM in shell windows, so the line lies
-// at 5 rounds; force 20 + 11.7 us against 47-57 us, 4 rounds.  The environment variables
-// MB_SPLIT_RHO_ITEMS and MB_SPLIT_FORCE_ITEMS override the lines (0: shell windows always).
+// at 5 rounds; force 20 + 11.7 us against 47-57 us, 4 rounds.  With several types the split
+// kernels' table loads cost more (force, 3 types: 38 us at 5.8 items per SM and 79 us at 9.3,
+// shell windows 51 and 70 us; density 43 against 45 us at 9.3, 48 us both at 13.8).  The
+// environment variables MB_SPLIT_RHO_ITEMS and MB_SPLIT_FORCE_ITEMS override the lines (0:
+// shell windows always).
 #define MB_SPLIT_RHO_ITEMS 20
 #define MB_SPLIT_FORCE_ITEMS 16
-static bool split_launch(const char *name, int per_sm, const LatticeArgs &a) {
+#define MB_MULTI_SPLIT_RHO_ITEMS 12
+#define MB_MULTI_SPLIT_FORCE_ITEMS 7
+static bool split_launch(const char *name, int one, int multi, const LatticeArgs &a) {
+  int per_sm = a.P.n_types == 1 ? one : multi;
   if (const char *v = getenv(name)) per_sm = atoi(v);
   return a.n_items - a.w0 <= per_sm * device_sm_count();
 }
@@ -559,7 +565,8 @@ int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const L
     if (z0 < 0 || z0 >= z1 || z1 > g.bz) return z0 == z1 ? MB_OK : fail(MB_ERR_ARG, "z-slab outside the box");
     LatticeArgs a = lattice_args(g, pot, L, rc2, flag, outer, *plan, z0, z1);
     a.e0 = e_partial;
-    if (split_launch("MB_SPLIT_RHO_ITEMS", MB_SPLIT_RHO_ITEMS, a)) return launch_split_rho64(st, a, energy, s);
+    if (split_launch("MB_SPLIT_RHO_ITEMS", MB_SPLIT_RHO_ITEMS, MB_MULTI_SPLIT_RHO_ITEMS, a))
+      return launch_split_rho64(st, a, energy, s);
     return launch_shell_rho64(st, a, energy, s);
   }
   RhoArgs a;
@@ -612,7 +619,8 @@ int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const
     a.sp = sp;
     a.e0 = e_partial ? e_partial + MB_EPART_CAP : nullptr;
     a.e1 = e_partial ? e_partial + 2 * MB_EPART_CAP : nullptr;
-    if (split_launch("MB_SPLIT_FORCE_ITEMS", MB_SPLIT_FORCE_ITEMS, a)) return launch_split_force64(st, a, energy, s);
+    if (split_launch("MB_SPLIT_FORCE_ITEMS", MB_SPLIT_FORCE_ITEMS, MB_MULTI_SPLIT_FORCE_ITEMS, a))
+      return launch_split_force64(st, a, energy, s);
     return launch_shell_force64(st, a, energy, s);
   }
   ForceArgs a;

@@ -1,4 +1,4 @@
-// One-type FP64 pair terms of the lattice passes, shared by the shell-window kernels
+// FP64 pair terms of the lattice passes, shared by the shell-window kernels
 // (mb_shell64.cu, large launches) and the entry-split kernels (mb_split64.cu, small ones).
 //
 // Both sum a site's stencil in the same fixed order, so a lattice gives the same bits
@@ -33,6 +33,7 @@ struct LatticeArgs {
   int w0, n_items;       // items [w0, n_items)
   double rc2, rc2m;      // squared cutoff; a hair above it for the outer-entry masks
   int rc2_hi;            // high word of rc2
+  int copies;            // table copies of a shell window (several types)
   int flag;              // code bit of the sites an interstitial pass finishes (0: none)
   uint2 *outer;          // per item: the outer entries some lane has inside rc2m (or null)
   double *e0, *e1;       // CTA partials: density pass F(rho); force pass pair and kinetic energy
@@ -80,83 +81,133 @@ __device__ __forceinline__ double hermite64(double2 k0, double2 k1, double p) {
   return __fma_rn(__fma_rn(__fma_rn(c3, p, __dsub_rn(u, c3)), p, k0.y), p, k0.x);
 }
 
-// {f', phi'} on an interval from its end values d0, d1 and quadratic coefficients c.
-__device__ __forceinline__ double2 slopes(double2 d0, double2 c, double2 d1, double p) {
-  return make_double2(__fma_rn(__fma_rn(c.x, p, __dsub_rn(__dsub_rn(d1.x, d0.x), c.x)), p, d0.x),
-                      __fma_rn(__fma_rn(c.y, p, __dsub_rn(__dsub_rn(d1.y, d0.y), c.y)), p, d0.y));
+// Spline derivative on an interval from its end values d0, d1 and quadratic coefficient c.
+__device__ __forceinline__ double slope64(double d0, double c, double d1, double p) {
+  return __fma_rn(__fma_rn(c, p, __dsub_rn(__dsub_rn(d1, d0), c)), p, d0);
 }
 
-// Table window in shared memory: one (density) or two (force) 16-byte words per knot,
-// COPIES interleaved copies of every word, lane l reading copy l % COPIES; k0 is the window's first knot.  With 8 copies
-// the 8 lanes that a wavefront of 16-byte loads serves read 8 different bank groups,
-// whatever their knots.
+// Table window in shared memory: `words` 16-byte words per knot, interleaved copies of every
+// word, lane l reading copy l % copies; w is the window's first knot.  With 8 copies the 8
+// lanes that a wavefront of 16-byte loads serves read 8 different bank groups, whatever
+// their knots.
+// One type (COPIES > 0): one word {y, s} (density) or two, {f', phi'} at the knot and their
+// quadratic coefficients (force).  Several (COPIES == 0, copies at run time): per type
+// {y, s}, or {f', coefficient}, then per pair of types {phi', coefficient}.
 template <int COPIES>
 struct Window64 {
   const double2 *w; // this lane's copy of the window's first knot
   double base;      // MB_FLOOR - first knot
   unsigned n;       // intervals
+  int words, copies; // COPIES == 0 only
 };
+
+// Word of a pair of types among `nt` (the packed upper triangle, after the nt types).
+__device__ __forceinline__ int pair_word(int a, int b, int nt) {
+  const int lo = min(a, b), hi = max(a, b);
+  return nt + lo * nt - lo * (lo + 1) / 2 + hi;
+}
 
 // Whether a pair outside its window may be inside the cutoff (vacant sites are far away).
 __device__ __forceinline__ bool maybe_in(const LatticeArgs &a, double d2) { return __double2hiint(d2) <= a.rc2_hi; }
 
-// Density term of a pair; false outside the window.
+// Density term of a pair with an atom of type tj; false outside the window.
 template <int COPIES>
-__device__ __forceinline__ bool rho_pair64(const Window64<COPIES> &W, const DevPot &P, double d2, double &v) {
+__device__ __forceinline__ bool rho_pair64(const Window64<COPIES> &W, const DevPot &P, double d2, int tj, double &v) {
   double r, rinv, p;
   unsigned k;
   root64(d2, r, rinv);
   const bool ok = window_locate(r, P.rdr, W.base, W.n, k, p);
-  const double2 *q = W.w + min(k, W.n - 1) * COPIES;
-  v = hermite64(q[0], q[COPIES], p);
+  k = min(k, W.n - 1);
+  if constexpr (COPIES > 0) {
+    const double2 *q = W.w + k * COPIES;
+    v = hermite64(q[0], q[COPIES], p);
+  } else {
+    const double2 *q = W.w + (k * W.words + tj) * W.copies;
+    v = hermite64(q[0], q[W.words * W.copies], p);
+  }
   return ok;
 }
-__device__ __forceinline__ double rho_table64(const DevPot &P, double d2) {
+__device__ __forceinline__ double rho_table64(const DevPot &P, double d2, int tj) {
   double r, rinv, p;
   int m;
   root64(d2, r, rinv);
   table_locate(r, P, m, p);
-  return hermite64(__ldg(P.f_ys + m), __ldg(P.f_ys + m + 1), p);
+  const double2 *q = P.f_ys + (size_t)m * P.n_types + tj;
+  return hermite64(__ldg(q), __ldg(q + P.n_types), p);
 }
 
-// fpair = -((df_i + df_j) f'(r) + phi'(r)) / r of a pair; false outside the window.  With
-// ENERGY e is half its pair energy (inside the window).
-template <bool ENERGY>
-__device__ __forceinline__ double half_phi64(const DevPot &P, int m, double p) {
-  const double4 v = ldg4(P.phi_val + m);
+// fpair = -(df_i f'_tj + df_j f'_ti + phi'_titj) / r of a pair; false outside the window.
+// With ENERGY e is half its pair energy (inside the window).
+__device__ __forceinline__ double half_phi64(const DevPot &P, int ti, int tj, int m, double p) {
+  const double4 v = ldg4(P.phi_val + (size_t)pair_idx(ti, tj, P.n_types) * P.nr + m);
   return __dmul_rn(0.5, __fma_rn(__fma_rn(__fma_rn(v.w, p, v.z), p, v.y), p, v.x));
 }
+// ... from the words of the pair's interval at q (several types), `step` to the next word and
+// `knot` to the next knot.
+template <class Load>
+__device__ __forceinline__ double force_words64(const double2 *q, int step, int knot, int nt, int ti, int tj,
+                                                double dfi, double dfj, double p, Load load) {
+  auto slope = [&](int word) {
+    const double2 a = load(q + word * step), b = load(q + word * step + knot);
+    return slope64(a.x, a.y, b.x, p);
+  };
+  const double fj = slope(tj), fi = slope(ti), ph = slope(pair_word(ti, tj, nt));
+  return __fma_rn(dfi, fj, __fma_rn(dfj, fi, ph));
+}
 template <int COPIES, bool ENERGY>
-__device__ __forceinline__ bool force_pair64(const Window64<COPIES> &W, const DevPot &P, double d2, double dfs,
-                                             double &f, double &e) {
+__device__ __forceinline__ bool force_pair64(const Window64<COPIES> &W, const DevPot &P, double d2, int ti, int tj,
+                                             double dfi, double dfj, double &f, double &e) {
   double r, rinv, p;
   unsigned k;
   root64(d2, r, rinv);
   const bool ok = window_locate(r, P.rdr, W.base, W.n, k, p);
-  const double2 *q = W.w + min(k, W.n - 1) * (2 * COPIES);
-  const double2 s = slopes(q[0], q[COPIES], q[2 * COPIES], p);
-  f = __dmul_rn(-__fma_rn(dfs, s.x, s.y), rinv);
-  if (ENERGY && ok) e = half_phi64<true>(P, (int)k + (int)(MB_FLOOR - W.base), p);
+  const unsigned kk = min(k, W.n - 1);
+  double g;
+  if constexpr (COPIES > 0) {
+    const double2 *q = W.w + kk * (2 * COPIES);
+    const double2 d0 = q[0], c = q[COPIES], d1 = q[2 * COPIES];
+    g = __fma_rn(__dadd_rn(dfi, dfj), slope64(d0.x, c.x, d1.x, p), slope64(d0.y, c.y, d1.y, p));
+  } else {
+    g = force_words64(W.w + kk * (W.words * W.copies), W.copies, W.words * W.copies, P.n_types, ti, tj, dfi, dfj, p,
+                      [](const double2 *x) { return *x; });
+  }
+  f = __dmul_rn(-g, rinv);
+  if (ENERGY && ok) e = half_phi64(P, ti, tj, (int)k + (int)(MB_FLOOR - W.base), p);
   return ok;
 }
 template <bool ENERGY>
-__device__ __forceinline__ double force_table64(const DevPot &P, double d2, double dfs, double &e) {
-  double r, rinv, p;
+__device__ __forceinline__ double force_table64(const DevPot &P, double d2, int ti, int tj, double dfi, double dfj,
+                                                double &e) {
+  double r, rinv, p, g;
   int m;
   root64(d2, r, rinv);
   table_locate(r, P, m, p);
-  const double2 *t = P.force2 + 2 * (size_t)m;
-  const double2 s = slopes(__ldg(t), __ldg(t + 1), __ldg(t + 2), p);
-  if (ENERGY) e = half_phi64<true>(P, m, p);
-  return __dmul_rn(-__fma_rn(dfs, s.x, s.y), rinv);
+  if (P.n_types == 1) {
+    const double2 *t = P.force2 + 2 * (size_t)m;
+    const double2 d0 = __ldg(t), c = __ldg(t + 1), d1 = __ldg(t + 2);
+    g = __fma_rn(__dadd_rn(dfi, dfj), slope64(d0.x, c.x, d1.x, p), slope64(d0.y, c.y, d1.y, p));
+  } else {
+    const int words = P.n_types + P.n_types * (P.n_types + 1) / 2;
+    g = force_words64(P.force2 + (size_t)m * words, 1, words, P.n_types, ti, tj, dfi, dfj, p,
+                      [](const double2 *x) { return __ldg(x); });
+  }
+  if (ENERGY) e = half_phi64(P, ti, tj, m, p);
+  return __dmul_rn(-g, rinv);
 }
 
-// A site at work: its record, F' and stencil offsets.
+// A site at work: its record and code, F' and stencil offsets.
 struct Site64 {
   const double4 *p;  // its record
+  const int8_t *c;   // its code
   const int *off;    // the stencil of its sublattice
   double x, y, z, w; // position and F'
+  int type;
 };
+// Type of the site whose code is *c, of nt (vacant sites: any; the distance rejects them).
+__device__ __forceinline__ int type_at(const int8_t *c, int nt) { return min(*c & MB_TYPE_MASK, nt - 1); }
+__device__ __forceinline__ int far_type(const LatticeArgs &a, const Site64 &c, int k) {
+  return a.P.n_types == 1 ? 0 : type_at(c.c + c.off[k], a.P.n_types);
+}
 
 // ------------------------------------------------------------------ runs
 // The pairs of a run that fell outside their window: entries k0 + b for the bits b of `far`.
@@ -166,7 +217,7 @@ __device__ __forceinline__ void rho_far(const LatticeArgs &a, const Site64 &c, i
     far &= far - 1;
     const double4 q = ld_site(c.p + c.off[k]);
     const double d2 = len2(c.x - q.x, c.y - q.y, c.z - q.z);
-    if (d2 < a.rc2) t = __dadd_rn(t, rho_table64(a.P, d2));
+    if (d2 < a.rc2) t = __dadd_rn(t, rho_table64(a.P, d2, far_type(a, c, k)));
   }
 }
 template <bool ENERGY>
@@ -179,7 +230,7 @@ __device__ __forceinline__ void force_far(const LatticeArgs &a, const Site64 &c,
     const double dx = c.x - q.x, dy = c.y - q.y, dz = c.z - q.z, d2 = len2(dx, dy, dz);
     if (d2 < a.rc2) {
       double e;
-      const double f = force_table64<ENERGY>(a.P, d2, __dadd_rn(c.w, q.w), e);
+      const double f = force_table64<ENERGY>(a.P, d2, c.type, far_type(a, c, k), c.w, q.w, e);
       fx = __fma_rn(dx, f, fx);
       fy = __fma_rn(dy, f, fy);
       fz = __fma_rn(dz, f, fz);
@@ -188,23 +239,23 @@ __device__ __forceinline__ void force_far(const LatticeArgs &a, const Site64 &c,
   }
 }
 
-// One near entry of a run (bit: its place in the run), q the neighbour's record.
+// One near entry of a run (bit: its place in the run), q the neighbour's record, tj its type.
 template <int COPIES>
 __device__ __forceinline__ void rho_near(const LatticeArgs &a, const Window64<COPIES> &W, const Site64 &c,
-                                         const double4 &q, int bit, double &t, unsigned &far) {
+                                         const double4 &q, int tj, int bit, double &t, unsigned &far) {
   const double d2 = len2(c.x - q.x, c.y - q.y, c.z - q.z);
   double v;
-  const bool ok = rho_pair64(W, a.P, d2, v);
+  const bool ok = rho_pair64(W, a.P, d2, tj, v);
   if (ok) t = __dadd_rn(t, v);
   if (!ok && maybe_in(a, d2)) far |= 1u << bit;
 }
 template <int COPIES, bool ENERGY>
 __device__ __forceinline__ void force_near(const LatticeArgs &a, const Window64<COPIES> &W, const Site64 &c,
-                                           const double4 &q, int bit, double &fx, double &fy, double &fz,
+                                           const double4 &q, int tj, int bit, double &fx, double &fy, double &fz,
                                            double &ep, unsigned &far) {
   const double dx = c.x - q.x, dy = c.y - q.y, dz = c.z - q.z, d2 = len2(dx, dy, dz);
   double f, e;
-  const bool ok = force_pair64<COPIES, ENERGY>(W, a.P, d2, __dadd_rn(c.w, q.w), f, e);
+  const bool ok = force_pair64<COPIES, ENERGY>(W, a.P, d2, c.type, tj, c.w, q.w, f, e);
   if (ok) {
     fx = __fma_rn(dx, f, fx);
     fy = __fma_rn(dy, f, fy);

@@ -142,7 +142,7 @@ int pot_build(const mb_eam_tables *t, PotHost **out) {
 
   std::vector<double4> f_val((size_t)nt * nr), f_der((size_t)nt * nr), F_val((size_t)nt * nrho),
       F_der((size_t)nt * nrho), phi_val((size_t)np * nr), phi_der((size_t)np * nr);
-  std::vector<double2> force1((size_t)nr * 3), force2((size_t)nr * 2), f_ys((size_t)nr);
+  std::vector<double2> force1((size_t)nr * 3), force2((size_t)nr * force_words(nt)), f_ys((size_t)nr * nt);
   std::vector<float4> f_val32((size_t)nt * nr), phi_val32((size_t)nr);
   std::vector<float2> force32((size_t)nr * 3);
   std::vector<double> c7;
@@ -172,9 +172,19 @@ int pot_build(const mb_eam_tables *t, PotHost **out) {
     force32[(size_t)m * 3 + 0] = make_float2((float)fd.x, (float)pd.x);
     force32[(size_t)m * 3 + 1] = make_float2((float)fd.y, (float)pd.y);
     force32[(size_t)m * 3 + 2] = make_float2((float)fd.z, (float)pd.z);
-    f_ys[m] = make_double2(f_val[m].x, f_val[m].y);
-    force2[2 * (size_t)m] = make_double2(fd.x, pd.x);
-    force2[2 * (size_t)m + 1] = make_double2(fd.z, pd.z);
+    for (int a = 0; a < nt; a++) {
+      const double4 v = f_val[(size_t)a * nr + m];
+      f_ys[(size_t)m * nt + a] = make_double2(v.x, v.y);
+    }
+    double2 *w = &force2[(size_t)m * force_words(nt)];
+    if (nt == 1) {
+      w[0] = make_double2(fd.x, pd.x);
+      w[1] = make_double2(fd.z, pd.z);
+    } else {
+      for (int a = 0; a < nt; a++) w[a] = make_double2(f_der[(size_t)a * nr + m].x, f_der[(size_t)a * nr + m].z);
+      for (int q = 0; q < np; q++)
+        w[nt + q] = make_double2(phi_der[(size_t)q * nr + m].x, phi_der[(size_t)q * nr + m].z);
+    }
     const double4 pv = phi_val[m];
     phi_val32[m] = make_float4((float)pv.x, (float)pv.y, (float)pv.z, (float)pv.w);
   }

@@ -1,4 +1,4 @@
-// FP64 lattice passes with one-type tables for large launches: shell by shell, each with
+// FP64 lattice passes for large launches: shell by shell, each with
 // its own replicated table window in shared memory.
 //
 // What bounds a pass with one copy of the table is the SM's 128-byte/clock data stage: in
@@ -10,6 +10,7 @@
 // one shell after the other; the partial sums of the sites rest in their rho / force
 // arrays (L2) in between.  The shells are built into the code (mb_ensemble_shells.cuh), so
 // that a neighbour costs one 32-byte load with an immediate column offset.
+// With several types a window holds the words of every type and pair of types.
 // Measured on one B200, 96^3 cells at 300 K: step 1.04 -> 0.79 ms; bank conflicts 94 M + 141
 // M -> none, instructions per 32-site item 6,250 -> 3,290 (density) and 5,460 -> 3,800
 // (force).  The density pass is now at 88% of the L1TEX data stage, the force pass waits on
@@ -26,6 +27,7 @@ namespace mb {
 #ifndef MB_SHELL_FORCE_THREADS
 #define MB_SHELL_FORCE_THREADS 768 // 896 and 1024 (spills): step at 96^3 cells 1% and 4% slower
 #endif
+#define MB_MULTI_FORCE_THREADS 640 // several types (768: spills, 512: step 2% and 6% slower)
 #ifndef MB_SHELL_ROUNDS
 #define MB_SHELL_ROUNDS 12 // items per warp in a batch (6: 3%, 24: 1% slower)
 #endif
@@ -40,6 +42,11 @@ namespace mb {
 #ifndef MB_FORCE_WINDOW
 #define MB_FORCE_WINDOW 648
 #endif
+// Several types: windows of as many intervals, in as many copies (8, 4, 2, 1) as take at most
+// these bytes; the rest is L1.  Step at 48x40x44 cells, 3 types, 2,000 knots, 600 K: 171 us;
+// two copies of the force window (187 KB) 196 us, of a narrower one (133 KB) 191 us; windows
+// of +-0.57 and +-0.36 A in more copies 186 us.
+#define MB_COPIES_BYTES (130 * 1024 + 512)
 
 // The density pass visits neighbouring shells that share a window together: first shell of
 // each visit (the force pass, with twice the bytes per knot, visits them one by one).
@@ -49,33 +56,47 @@ struct RhoVisits {
   static constexpr int first[5] = {0, 2, 3, 5, 6};
 };
 
-// Fills the window with knots [lo, lo + n] of PER 16-byte words each, every word 8 times:
-// a thread reads a word once and lane l starts with copy l % 8, so that the stores of 8
-// lanes fall into 8 bank groups.
-template <int PER>
-__device__ __forceinline__ void fill_window(double2 *w, const double2 *tab, int lo, int n) {
-  const double2 *src = tab + PER * (size_t)lo;
-  const int words = (n + 1) * PER;
+// Fills the window with `words` 16-byte words from src, every word `copies` times: a thread
+// reads a word once and lane l starts with copy l % copies, so that the stores of 8 lanes
+// fall into 8 bank groups.
+__device__ __forceinline__ void fill_window(double2 *w, const double2 *src, int words, int copies) {
 #pragma unroll 2
   for (int k = threadIdx.x; k < words; k += blockDim.x) {
     const double2 v = __ldg(src + k);
 #pragma unroll
-    for (int c = 0; c < MB_COPIES; c++) w[k * MB_COPIES + ((c + threadIdx.x) & (MB_COPIES - 1))] = v;
+    for (int c = 0; c < MB_COPIES; c++)
+      if (c < copies) w[k * copies + ((c + threadIdx.x) & (copies - 1))] = v;
   }
+}
+// The window of knots [lo, lo + cnt] of a table of `words` words per knot.
+template <int COPIES>
+__device__ __forceinline__ Window64<COPIES> take_window(double2 *s_w, const double2 *tab, int words, int copies, int lo,
+                                                        int cnt) {
+  if (COPIES > 0) copies = COPIES;
+  __syncthreads();
+  fill_window(s_w, tab + (size_t)words * lo, (cnt + 1) * words, copies);
+  __syncthreads();
+  return Window64<COPIES>{s_w + (threadIdx.x & (copies - 1)), MB_FLOOR - lo, (unsigned)cnt, words, copies};
 }
 
 // Bases of a site's neighbours: even vectors, and odd ones (on the other sublattice).
 struct Bases64 {
   const double4 *be, *bo;
+  const int8_t *ce, *co; // codes (several types)
 };
-__device__ __forceinline__ Bases64 site_bases(const Geom &g, const double4 *p, int i) {
+__device__ __forceinline__ Bases64 site_bases(const Geom &g, const Lattice64 &L, int i) {
   const int odd = i < (int)g.E ? (int)g.E : -(int)g.E + g.ey * g.ecx + g.ecx + 1;
-  return Bases64{p + i, p + i + odd};
+  return Bases64{L.p + i, L.p + i + odd, L.code + i, L.code + i + odd};
 }
 template <int K>
 __device__ __forceinline__ double4 ld_neighbour(const Bases64 &b, int pl, int rw) {
   using T = HStore<K>;
   return ld_site((T::odd ? b.bo : b.be) + (T::dz * pl + T::dy * rw) + T::dx);
+}
+template <int K, int COPIES>
+__device__ __forceinline__ int neighbour_type(const Bases64 &b, int pl, int rw, int nt) {
+  using T = HStore<K>;
+  return COPIES > 0 ? 0 : type_at((T::odd ? b.co : b.ce) + (T::dz * pl + T::dy * rw) + T::dx, nt);
 }
 
 // Items of a launch in rounds: of the CTA's warps as many take an item in each round as
@@ -109,8 +130,8 @@ __device__ __forceinline__ int item_ref(const LatticeArgs &a, int w, int hi) {
 }
 
 // Density sums of shell SH's runs.
-template <int SH>
-__device__ __forceinline__ void rho_shell(const LatticeArgs &a, const Window64<MB_COPIES> &W, const Site64 &c,
+template <int SH, int COPIES>
+__device__ __forceinline__ void rho_shell(const LatticeArgs &a, const Window64<COPIES> &W, const Site64 &c,
                                           const Bases64 &b, int pl, int rw, double &rho) {
   constexpr int first = kBcc.start[SH], end = kBcc.start[SH + 1];
   static_for<0, (end - first + MB_RUN - 1) / MB_RUN>([&](auto rc) {
@@ -120,10 +141,15 @@ __device__ __forceinline__ void rho_shell(const LatticeArgs &a, const Window64<M
     static_for<0, (k1 - k0 + MB_AHEAD - 1) / MB_AHEAD>([&](auto cc) {
       constexpr int c0 = k0 + decltype(cc)::value * MB_AHEAD, c1 = c0 + MB_AHEAD < k1 ? c0 + MB_AHEAD : k1;
       double4 q[MB_AHEAD];
-      static_for<c0, c1>([&](auto kc) { q[decltype(kc)::value - c0] = ld_neighbour<decltype(kc)::value>(b, pl, rw); });
+      int tj[MB_AHEAD];
       static_for<c0, c1>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
-        rho_near(a, W, c, q[k - c0], k - k0, t, far);
+        q[k - c0] = ld_neighbour<k>(b, pl, rw);
+        tj[k - c0] = neighbour_type<k, COPIES>(b, pl, rw, a.P.n_types);
+      });
+      static_for<c0, c1>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        rho_near(a, W, c, q[k - c0], tj[k - c0], k - k0, t, far);
       });
     });
     rho_far(a, c, k0, far, t);
@@ -131,8 +157,8 @@ __device__ __forceinline__ void rho_shell(const LatticeArgs &a, const Window64<M
   });
 }
 
-template <int SH, bool ENERGY>
-__device__ __forceinline__ void force_shell(const LatticeArgs &a, const Window64<MB_COPIES> &W, const Site64 &c,
+template <int SH, int COPIES, bool ENERGY>
+__device__ __forceinline__ void force_shell(const LatticeArgs &a, const Window64<COPIES> &W, const Site64 &c,
                                             const Bases64 &b, int pl, int rw, double &fx, double &fy, double &fz,
                                             double &ep) {
   constexpr int first = kBcc.start[SH], end = kBcc.start[SH + 1];
@@ -143,10 +169,15 @@ __device__ __forceinline__ void force_shell(const LatticeArgs &a, const Window64
     static_for<0, (k1 - k0 + MB_AHEAD - 1) / MB_AHEAD>([&](auto cc) {
       constexpr int c0 = k0 + decltype(cc)::value * MB_AHEAD, c1 = c0 + MB_AHEAD < k1 ? c0 + MB_AHEAD : k1;
       double4 q[MB_AHEAD];
-      static_for<c0, c1>([&](auto kc) { q[decltype(kc)::value - c0] = ld_neighbour<decltype(kc)::value>(b, pl, rw); });
+      int tj[MB_AHEAD];
       static_for<c0, c1>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
-        force_near<MB_COPIES, ENERGY>(a, W, c, q[k - c0], k - k0, tx, ty, tz, ep, far);
+        q[k - c0] = ld_neighbour<k>(b, pl, rw);
+        tj[k - c0] = neighbour_type<k, COPIES>(b, pl, rw, a.P.n_types);
+      });
+      static_for<c0, c1>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        force_near<COPIES, ENERGY>(a, W, c, q[k - c0], tj[k - c0], k - k0, tx, ty, tz, ep, far);
       });
     });
     force_far<ENERGY>(a, c, k0, far, tx, ty, tz, ep);
@@ -156,8 +187,8 @@ __device__ __forceinline__ void force_shell(const LatticeArgs &a, const Window64
   });
 }
 
-// NEAR: shells inside the cutoff at the ideal lattice.
-template <bool ENERGY, int NEAR>
+// NEAR: shells inside the cutoff at the ideal lattice.  COPIES: table copies; 0 with several types.
+template <bool ENERGY, int NEAR, int COPIES>
 __global__ void __launch_bounds__(MB_SHELL_RHO_THREADS, 1)
     k_shell_rho64(const __grid_constant__ StencilSet st, const __grid_constant__ LatticeArgs a) {
   extern __shared__ double2 s_w[];
@@ -171,10 +202,8 @@ __global__ void __launch_bounds__(MB_SHELL_RHO_THREADS, 1)
     static_for<0, RhoVisits<NEAR>::n>([&](auto vc) {
       constexpr int V = decltype(vc)::value, SH = RhoVisits<NEAR>::first[V], END = RhoVisits<NEAR>::first[V + 1];
       const int lo = a.sh.rho.lo[SH], cnt = a.sh.rho.cnt[SH];
-      __syncthreads();
-      fill_window<1>(s_w, a.P.f_ys, lo, cnt);
-      __syncthreads();
-      const Window64<MB_COPIES> W{s_w + (lane & (MB_COPIES - 1)), MB_FLOOR - lo, (unsigned)cnt};
+      const Window64<COPIES> W =
+          take_window<COPIES>(s_w, a.P.f_ys, COPIES > 0 ? 1 : a.P.n_types, a.copies, lo, cnt);
       int next = item_ref(a, it.lo, it.hi);
       for (int w = it.lo; w < it.hi; w += it.stride) {
         const int ref = next, i = ref & MB_SITE_INDEX;
@@ -189,9 +218,9 @@ __global__ void __launch_bounds__(MB_SHELL_RHO_THREADS, 1)
         }
         unsigned long long near = 0;
         if (code >= 0) {
-          const Site64 c{L.p + i, st.off[i >= (int)a.g.E], own.x, own.y, own.z, 0.0};
-          const Bases64 bs = site_bases(a.g, L.p, i);
-          static_for<SH, END>([&](auto hc) { rho_shell<decltype(hc)::value>(a, W, c, bs, pl, rw, rho); });
+          const Site64 c{L.p + i, L.code + i, st.off[i >= (int)a.g.E], own.x, own.y, own.z, 0.0, 0};
+          const Bases64 bs = site_bases(a.g, L, i);
+          static_for<SH, END>([&](auto hc) { rho_shell<decltype(hc)::value, COPIES>(a, W, c, bs, pl, rw, rho); });
           if (END < NEAR) {
             L.rho[i] = rho;
           } else {
@@ -218,8 +247,8 @@ __global__ void __launch_bounds__(MB_SHELL_RHO_THREADS, 1)
   }
 }
 
-template <bool ENERGY, int NEAR>
-__global__ void __launch_bounds__(MB_SHELL_FORCE_THREADS, 1)
+template <bool ENERGY, int NEAR, int COPIES>
+__global__ void __launch_bounds__(COPIES > 0 ? MB_SHELL_FORCE_THREADS : MB_MULTI_FORCE_THREADS, 1)
     k_shell_force64(const __grid_constant__ StencilSet st, const __grid_constant__ LatticeArgs a) {
   extern __shared__ double2 s_w[];
   const Lattice64 &L = a.L;
@@ -233,10 +262,8 @@ __global__ void __launch_bounds__(MB_SHELL_FORCE_THREADS, 1)
       constexpr int SH = decltype(shc)::value;
       __syncthreads();
       const int lo = a.sh.force.lo[SH], cnt = a.sh.force.cnt[SH];
-      __syncthreads();
-      fill_window<2>(s_w, a.P.force2, lo, cnt);
-      __syncthreads();
-      const Window64<MB_COPIES> W{s_w + (lane & (MB_COPIES - 1)), MB_FLOOR - lo, (unsigned)cnt};
+      const Window64<COPIES> W =
+          take_window<COPIES>(s_w, a.P.force2, COPIES > 0 ? 2 : force_words(a.P.n_types), a.copies, lo, cnt);
       int next = item_ref(a, it.lo, it.hi);
       for (int w = it.lo; w < it.hi; w += it.stride) {
         const int ref = next, i = ref & MB_SITE_INDEX;
@@ -251,8 +278,9 @@ __global__ void __launch_bounds__(MB_SHELL_FORCE_THREADS, 1)
           fz = L.fz[i];
         }
         if (code < 0) continue;
-        const Site64 c{L.p + i, st.off[i >= (int)a.g.E], own.x, own.y, own.z, own.w};
-        force_shell<SH, ENERGY>(a, W, c, site_bases(a.g, L.p, i), pl, rw, fx, fy, fz, e_pair);
+        const Site64 c{L.p + i, L.code + i, st.off[i >= (int)a.g.E], own.x, own.y, own.z, own.w,
+                       COPIES > 0 ? 0 : code & MB_TYPE_MASK};
+        force_shell<SH, COPIES, ENERGY>(a, W, c, site_bases(a.g, L, i), pl, rw, fx, fy, fz, e_pair);
         if (SH + 1 < NEAR) {
           L.fx[i] = fx;
           L.fy[i] = fy;
@@ -286,40 +314,47 @@ __global__ void __launch_bounds__(MB_SHELL_FORCE_THREADS, 1)
   }
 }
 
-static size_t window_bytes(const Windows64 &w, int n, int words) {
+static size_t window_bytes(const Windows64 &w, int n, int words, int copies) {
   int knots = 0;
   for (int h = 0; h < n; h++) knots = w.cnt[h] + 1 > knots ? w.cnt[h] + 1 : knots;
-  return (size_t)knots * words * MB_COPIES * sizeof(double2);
+  return (size_t)knots * words * copies * sizeof(double2);
 }
 
-template <int NEAR>
-static int shell_rho(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
-  MB_SMEM_ATTR((k_shell_rho64<false, NEAR>), (k_shell_rho64<true, NEAR>), MB_SMEM_MAX - 1024);
-  const size_t smem = window_bytes(a.sh.rho, a.sh.n, 1);
+template <int NEAR, int COPIES>
+static int shell_rho(const StencilSet &st, LatticeArgs a, int energy, cudaStream_t s) {
+  MB_SMEM_ATTR((k_shell_rho64<false, NEAR, COPIES>), (k_shell_rho64<true, NEAR, COPIES>), MB_SMEM_MAX - 1024);
+  a.copies = a.sh.rho.copies;
+  const size_t smem = window_bytes(a.sh.rho, a.sh.n, a.P.n_types, a.copies);
   if (energy)
-    k_shell_rho64<true, NEAR><<<device_sm_count(), MB_SHELL_RHO_THREADS, smem, s>>>(st, a);
+    k_shell_rho64<true, NEAR, COPIES><<<device_sm_count(), MB_SHELL_RHO_THREADS, smem, s>>>(st, a);
   else
-    k_shell_rho64<false, NEAR><<<device_sm_count(), MB_SHELL_RHO_THREADS, smem, s>>>(st, a);
+    k_shell_rho64<false, NEAR, COPIES><<<device_sm_count(), MB_SHELL_RHO_THREADS, smem, s>>>(st, a);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }
-template <int NEAR>
-static int shell_force(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
-  MB_SMEM_ATTR((k_shell_force64<false, NEAR>), (k_shell_force64<true, NEAR>), MB_SMEM_MAX - 1024);
-  const size_t smem = window_bytes(a.sh.force, a.sh.n, 2);
+template <int NEAR, int COPIES>
+static int shell_force(const StencilSet &st, LatticeArgs a, int energy, cudaStream_t s) {
+  MB_SMEM_ATTR((k_shell_force64<false, NEAR, COPIES>), (k_shell_force64<true, NEAR, COPIES>), MB_SMEM_MAX - 1024);
+  a.copies = a.sh.force.copies;
+  const size_t smem = window_bytes(a.sh.force, a.sh.n, force_words(a.P.n_types), a.copies);
+  const int threads = COPIES > 0 ? MB_SHELL_FORCE_THREADS : MB_MULTI_FORCE_THREADS;
   if (energy)
-    k_shell_force64<true, NEAR><<<device_sm_count(), MB_SHELL_FORCE_THREADS, smem, s>>>(st, a);
+    k_shell_force64<true, NEAR, COPIES><<<device_sm_count(), threads, smem, s>>>(st, a);
   else
-    k_shell_force64<false, NEAR><<<device_sm_count(), MB_SHELL_FORCE_THREADS, smem, s>>>(st, a);
+    k_shell_force64<false, NEAR, COPIES><<<device_sm_count(), threads, smem, s>>>(st, a);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }
 
 int launch_shell_rho64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
-  return a.sh.n == 5 ? shell_rho<5>(st, a, energy, s) : shell_rho<6>(st, a, energy, s);
+  if (a.P.n_types == 1)
+    return a.sh.n == 5 ? shell_rho<5, MB_COPIES>(st, a, energy, s) : shell_rho<6, MB_COPIES>(st, a, energy, s);
+  return a.sh.n == 5 ? shell_rho<5, 0>(st, a, energy, s) : shell_rho<6, 0>(st, a, energy, s);
 }
 int launch_shell_force64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
-  return a.sh.n == 5 ? shell_force<5>(st, a, energy, s) : shell_force<6>(st, a, energy, s);
+  if (a.P.n_types == 1)
+    return a.sh.n == 5 ? shell_force<5, MB_COPIES>(st, a, energy, s) : shell_force<6, MB_COPIES>(st, a, energy, s);
+  return a.sh.n == 5 ? shell_force<5, 0>(st, a, energy, s) : shell_force<6, 0>(st, a, energy, s);
 }
 
 // ------------------------------------------------------------------ plan
@@ -367,7 +402,7 @@ bool plan64_shells(const DevPot &P, const Geom &g, double a0, double cutoff, con
                    Shells64 &S) {
   S = Shells64{};
   S.n = st.n_near == kBcc.start[5] ? 5 : st.n_near == kBcc.start[6] ? 6 : 0;
-  if (P.n_types != 1 || !S.n || st.n - st.n_near > 64 || g.E > 0x1fffffffLL) return false;
+  if (!S.n || st.n - st.n_near > 64 || g.E > 0x1fffffffLL) return false;
   double r[MB_NEAR_SHELLS];
   for (int h = 0; h < S.n; h++) {
     r[h] = 0.5 * a0 * sqrt((double)kBcc.n2[h]);
@@ -380,21 +415,37 @@ bool plan64_shells(const DevPot &P, const Geom &g, double a0, double cutoff, con
         if (st.off[s][k] != (s2 - s) * (int)g.E + (dz * g.ey + dy) * g.ecx + dx) return false;
       }
     }
-    if (!shell_window(P, cutoff, r[h], r[h], MB_FORCE_WINDOW, S.force.lo[h], S.force.cnt[h])) return false;
     for (int k = kBcc.start[h]; k < kBcc.start[h + 1]; k += MB_RUN) {
       S.shell[S.runs] = (short)h;
       S.kb[S.runs++] = (short)k;
     }
   }
+  // windows: one type as measured; several in the most copies that leave the least margin
   const int *first = RhoVisits<5>::first; // the visits of NEAR = 6 begin with the same shells
-  for (int v = 0; first[v] < S.n; v++)
-    for (int h = first[v]; h < first[v + 1]; h++)
-      if (!shell_window(P, cutoff, r[first[v]], r[first[v + 1] - 1], MB_RHO_WINDOW, S.rho.lo[h], S.rho.cnt[h]))
-        return false;
+  auto windows = [&](Windows64 &w, int words, int most, auto fit) {
+    const int knot = words * (int)sizeof(double2);
+    w.copies = MB_COPIES; // built into the one-type kernels
+    if (P.n_types > 1)
+      while (w.copies > 1 && (most + 1) * knot * w.copies > MB_COPIES_BYTES) w.copies /= 2;
+    const int room = (MB_SMEM_MAX - 2048) / (knot * w.copies) - 1;
+    return fit(room < most ? room : most);
+  };
+  const bool rho = windows(S.rho, P.n_types, MB_RHO_WINDOW, [&](int cap) {
+    for (int v = 0; first[v] < S.n; v++)
+      for (int h = first[v]; h < first[v + 1]; h++)
+        if (!shell_window(P, cutoff, r[first[v]], r[first[v + 1] - 1], cap, S.rho.lo[h], S.rho.cnt[h])) return false;
+    return true;
+  });
+  const bool force = windows(S.force, force_words(P.n_types), MB_FORCE_WINDOW, [&](int cap) {
+    for (int h = 0; h < S.n; h++)
+      if (!shell_window(P, cutoff, r[h], r[h], cap, S.force.lo[h], S.force.cnt[h])) return false;
+    return true;
+  });
+  if (!rho || !force) return false;
   S.near_runs = S.runs;
   for (int k = st.n_near; k < st.n; k += MB_OUT_RUN) S.kb[S.runs++] = (short)k;
   S.kb[S.runs] = (short)st.n;
-  return split64_fits(S);
+  return split64_fits(P, S);
 }
 
 int plan64_sites(const Geom &g, int *sites, cudaStream_t s) {

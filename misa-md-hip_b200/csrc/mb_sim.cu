@@ -424,7 +424,7 @@ static int create_sim(const mb_sim_config *cfg, const mb_eam_tables *pot, int z_
   const int par[2] = {0, 1};
   int n_near = 0;
   double dist[MB_MAX_STENCIL] = {};
-  if (rc == MB_OK && pot->n_types == 1)
+  if (rc == MB_OK)
     rc = stencil_sort_by_distance(cfg->lattice_const, cfg->cutoff, s->ext_x, s->ext_y, even, odd, n, &n_near, dist);
   if (rc == MB_OK) rc = stencil_from_linear(even, n, odd, n, s->ext_x, s->ext_y, g, par, &s->st);
   s->st.n_near = n_near;

@@ -1,13 +1,15 @@
-// FP64 lattice passes with one-type tables for small launches: one item's stencil split
+// FP64 lattice passes for small launches: one item's stencil split
 // over the warps of a group.
 //
 // A launch of a few items per SM leaves most warps idle, and its time is the latency of
 // one warp walking ~90 entries, each a chain of neighbour load, root, table load and sum.
 // Here MB_SPLIT_WARPS warps share an item: each takes whole runs of the site's sum
 // (mb_pair64.cuh), leaves the run sums in shared memory and one warp, another for each item,
-// adds them in order and finishes the sites while the others go on to the next item.  The run sums and their order are those of the
-// shell-window kernels, so both give the same bits.  One copy of the table serves: the
-// warps in flight are too few for bank conflicts to count.
+// adds them in order and finishes the sites while the others go on to the next item.  The
+// run sums and their order are those of the shell-window kernels, so both give the same bits.
+// One copy of the table serves: the warps in flight are too few for bank conflicts to count.
+// The tables of several types that are too wide for shared memory are read where they lie.
+// Measured on one B200, 20^3 cells: step 73 -> 27 us (one type), 81 -> 36 us (three).
 #include "mb_pair64.cuh"
 
 namespace mb {
@@ -40,21 +42,34 @@ __device__ __forceinline__ SplitSite split_site(const StencilSet &st, const Latt
   t.code = code;
   if (code < 0) {
     t.ref = -1;
-    t.c = Site64{a.L.p, st.off[0], 0.0, 0.0, 0.0, 0.0};
+    t.c = Site64{a.L.p, a.L.code, st.off[0], 0.0, 0.0, 0.0, 0.0, 0};
   } else {
     const double4 own = ld_site(a.L.p + i);
-    t.c = Site64{a.L.p + i, st.off[i >= (int)a.g.E], own.x, own.y, own.z, own.w};
+    t.c = Site64{a.L.p + i, a.L.code + i,  st.off[i >= (int)a.g.E],          own.x, own.y, own.z,
+                 own.w,     a.P.n_types == 1 ? 0 : code & MB_TYPE_MASK};
   }
   return t;
 }
 
-template <bool ENERGY>
+template <int COPIES>
+__device__ __forceinline__ int split_type(const Site64 &c, int k, int nt) {
+  return COPIES > 0 ? 0 : type_at(c.c + c.off[k], nt);
+}
+
+// COPIES: 1, or 0 with several types; knots == 0: the table is read where it lies (several
+// types, too wide for shared memory).
+template <bool ENERGY, int COPIES>
 __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
     k_split_rho64(const __grid_constant__ StencilSet st, const __grid_constant__ LatticeArgs a, int lo, int knots) {
   extern __shared__ double2 s_w[];
   __shared__ double s_sum[MB_SPLIT_GROUPS][2][MB_RUNS_MAX][32]; // two items' sums, in turn
   __shared__ unsigned s_near[MB_SPLIT_GROUPS][2][MB_RUNS_MAX];
-  fill_table(s_w, a.P.f_ys + lo, knots);
+  const int words = COPIES > 0 ? 1 : a.P.n_types;
+  const double2 *tab = a.P.f_ys + (size_t)words * lo;
+  if (COPIES > 0 || knots > 0) {
+    fill_table(s_w, tab, words * knots);
+    tab = s_w;
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % MB_SPLIT_WARPS,
             group = threadIdx.x / (32 * MB_SPLIT_WARPS);
@@ -72,10 +87,11 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
         if (r < a.sh.near_runs) {
           const int h = a.sh.shell[r];
           const int wl = a.sh.rho.lo[h];
-          const Window64<1> W{s_w + (wl - lo), MB_FLOOR - wl, (unsigned)a.sh.rho.cnt[h]};
+          const Window64<COPIES> W{tab + words * (wl - lo), MB_FLOOR - wl, (unsigned)a.sh.rho.cnt[h], words, 1};
           unsigned far = 0;
 #pragma unroll 4
-          for (int k = k0; k < k1; k++) rho_near(a, W, t.c, ld_site(t.c.p + t.c.off[k]), k - k0, sum, far);
+          for (int k = k0; k < k1; k++)
+            rho_near(a, W, t.c, ld_site(t.c.p + t.c.off[k]), split_type<COPIES>(t.c, k, a.P.n_types), k - k0, sum, far);
           rho_far(a, t.c, k0, far, sum);
         } else {
           sum = rho_outer(a, t.c, k0, k1, near);
@@ -110,15 +126,20 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
   }
 }
 
-template <bool ENERGY>
+template <bool ENERGY, int COPIES>
 __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
     k_split_force64(const __grid_constant__ StencilSet st, const __grid_constant__ LatticeArgs a, int lo, int knots) {
   extern __shared__ double2 s_w[]; // table, then the run sums
-  fill_table(s_w, a.P.force2 + 2 * (size_t)lo, 2 * knots);
+  const int words = COPIES > 0 ? 2 : force_words(a.P.n_types);
+  const double2 *tab = a.P.force2 + (size_t)words * lo;
+  if (COPIES > 0 || knots > 0) {
+    fill_table(s_w, tab, words * knots);
+    tab = s_w;
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % MB_SPLIT_WARPS,
             group = threadIdx.x / (32 * MB_SPLIT_WARPS);
-  double *sums = reinterpret_cast<double *>(s_w + 2 * knots) + (size_t)group * 2 * a.sh.runs * 96 + lane;
+  double *sums = reinterpret_cast<double *>(s_w + words * knots) + (size_t)group * 2 * a.sh.runs * 96 + lane;
   double e_pair = 0.0, e_kin = 0.0;
   int turn = 0;
   for (int w = a.w0 + blockIdx.x * MB_SPLIT_GROUPS + group; w < a.n_items; w += gridDim.x * MB_SPLIT_GROUPS, turn++) {
@@ -136,11 +157,12 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
         if (r < a.sh.near_runs) {
           const int h = a.sh.shell[r];
           const int wl = a.sh.force.lo[h];
-          const Window64<1> W{s_w + 2 * (wl - lo), MB_FLOOR - wl, (unsigned)a.sh.force.cnt[h]};
+          const Window64<COPIES> W{tab + words * (wl - lo), MB_FLOOR - wl, (unsigned)a.sh.force.cnt[h], words, 1};
           unsigned far = 0;
 #pragma unroll 4
           for (int k = k0; k < k1; k++)
-            force_near<1, ENERGY>(a, W, t.c, ld_site(t.c.p + t.c.off[k]), k - k0, fx, fy, fz, e_pair, far);
+            force_near<COPIES, ENERGY>(a, W, t.c, ld_site(t.c.p + t.c.off[k]), split_type<COPIES>(t.c, k, a.P.n_types), k - k0, fx, fy,
+                                       fz, e_pair, far);
           force_far<ENERGY>(a, t.c, k0, far, fx, fy, fz, e_pair);
         } else {
           force_outer<ENERGY>(a, t.c, k0, k1, (unsigned)(mask >> (k0 - a.sh.kb[a.sh.near_runs])), fx, fy, fz, e_pair);
@@ -181,45 +203,63 @@ static void table_range(const Windows64 &w, int n, int &lo, int &knots) {
 }
 
 static size_t run_sum_bytes(const Shells64 &sh) { return sizeof(double) * 2 * 96 * MB_SPLIT_GROUPS * sh.runs; }
-static const int kSplitSmem = MB_SMEM_MAX - 40 * 1024; // beside the density kernel's run sums
+static const int kRhoSmem = MB_SMEM_MAX - 40 * 1024; // beside its static run sums
+static const int kForceSmem = MB_SMEM_MAX - 2 * 1024;
 
-// Whether the windows' union fits the shared memory of the entry-split kernels.
-bool split64_fits(const Shells64 &sh) {
+// Knots of the union of the windows that shared memory takes with `used` bytes taken; 0: too
+// many.
+static int smem_knots(int knots, int words, size_t used, int most) {
+  return used + (size_t)knots * words * sizeof(double2) <= (size_t)most ? knots : 0;
+}
+static int split_grid(const LatticeArgs &a) {
+  const int grid = (a.n_items - a.w0 + MB_SPLIT_GROUPS - 1) / MB_SPLIT_GROUPS;
+  return grid < device_sm_count() ? grid : device_sm_count();
+}
+
+// Whether the entry-split kernels take the plan's tables.
+bool split64_fits(const DevPot &P, const Shells64 &sh) {
+  int lo, rho, force;
+  table_range(sh.rho, sh.n, lo, rho);
+  table_range(sh.force, sh.n, lo, force);
+  return run_sum_bytes(sh) <= (size_t)kForceSmem &&
+         (P.n_types > 1 || (smem_knots(rho, 1, 0, kRhoSmem) && smem_knots(force, 2, run_sum_bytes(sh), kForceSmem)));
+}
+
+template <int COPIES>
+static int split_rho(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
   int lo, knots;
-  table_range(sh.rho, sh.n, lo, knots);
-  const size_t rho = (size_t)knots * sizeof(double2);
-  table_range(sh.force, sh.n, lo, knots);
-  return rho <= (size_t)kSplitSmem && (size_t)knots * 2 * sizeof(double2) + run_sum_bytes(sh) <= (size_t)kSplitSmem;
+  table_range(a.sh.rho, a.sh.n, lo, knots);
+  knots = smem_knots(knots, a.P.n_types, 0, kRhoSmem);
+  const size_t smem = (size_t)knots * a.P.n_types * sizeof(double2);
+  MB_SMEM_ATTR((k_split_rho64<false, COPIES>), (k_split_rho64<true, COPIES>), kRhoSmem);
+  if (energy)
+    k_split_rho64<true, COPIES><<<split_grid(a), MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
+  else
+    k_split_rho64<false, COPIES><<<split_grid(a), MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
+template <int COPIES>
+static int split_force(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
+  int lo, knots;
+  table_range(a.sh.force, a.sh.n, lo, knots);
+  knots = smem_knots(knots, force_words(a.P.n_types), run_sum_bytes(a.sh), kForceSmem);
+  const size_t smem = (size_t)knots * force_words(a.P.n_types) * sizeof(double2) + run_sum_bytes(a.sh);
+  MB_SMEM_ATTR((k_split_force64<false, COPIES>), (k_split_force64<true, COPIES>), kForceSmem);
+  if (energy)
+    k_split_force64<true, COPIES><<<split_grid(a), MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
+  else
+    k_split_force64<false, COPIES><<<split_grid(a), MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
 }
 
 int launch_split_rho64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
-  int lo, knots;
-  table_range(a.sh.rho, a.sh.n, lo, knots);
-  const size_t smem = (size_t)knots * sizeof(double2);
-  MB_SMEM_ATTR((k_split_rho64<false>), (k_split_rho64<true>), kSplitSmem);
-  int grid = (a.n_items - a.w0 + MB_SPLIT_GROUPS - 1) / MB_SPLIT_GROUPS;
-  if (grid > device_sm_count()) grid = device_sm_count();
-  if (energy)
-    k_split_rho64<true><<<grid, MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
-  else
-    k_split_rho64<false><<<grid, MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
+  return a.P.n_types == 1 ? split_rho<1>(st, a, energy, s) : split_rho<0>(st, a, energy, s);
 }
-
 int launch_split_force64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
-  int lo, knots;
-  table_range(a.sh.force, a.sh.n, lo, knots);
-  const size_t smem = (size_t)knots * 2 * sizeof(double2) + run_sum_bytes(a.sh);
-  MB_SMEM_ATTR((k_split_force64<false>), (k_split_force64<true>), kSplitSmem);
-  int grid = (a.n_items - a.w0 + MB_SPLIT_GROUPS - 1) / MB_SPLIT_GROUPS;
-  if (grid > device_sm_count()) grid = device_sm_count();
-  if (energy)
-    k_split_force64<true><<<grid, MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
-  else
-    k_split_force64<false><<<grid, MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
+  return a.P.n_types == 1 ? split_force<1>(st, a, energy, s) : split_force<0>(st, a, energy, s);
 }
 
 } // namespace mb
