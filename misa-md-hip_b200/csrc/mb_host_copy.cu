@@ -2,9 +2,9 @@
 //
 // cudaMemcpyAsync on pageable memory goes through the driver's own staging buffer on one
 // thread: 4.7 GB/s into freshly allocated pages, so that reading 4.2 M records (436 MB) back
-// took 92 ms, as long as 45 timesteps.  Here a few host threads share the copy in chunks, each with a page-locked
-// slot: the chunk crosses PCIe into the slot while the other threads move (and first touch)
-// their parts of the caller's buffer.
+// took 92 ms, as long as 45 timesteps.  Here a few host threads share the copy in chunks,
+// each with a page-locked slot: the chunk crosses PCIe into the slot while the other threads
+// move (and first touch) their parts of the caller's buffer.
 #include <string.h>
 
 #include <algorithm>
@@ -43,13 +43,16 @@ void HostCopy::release() {
     if (e) cudaEventDestroy(e), e = nullptr;
 }
 
-// Fewer than kMinBytes, or a page-locked buffer: one plain copy.
+// Fewer than kMinBytes, a page-locked buffer, or too little moved yet to pay for the slots:
+// one plain copy.
 int HostCopy::copy(void *host, void *dev, size_t bytes, bool to_host, cudaStream_t s) {
   const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
   unsigned hw = std::thread::hardware_concurrency();
   const int n_chunks = (int)((bytes + kChunk - 1) / kChunk);
   const int workers = std::min({kSlots, n_chunks, (int)std::max(1u, hw / 2)});
-  if (bytes < kMinBytes || workers < 2 || page_locked(host) || ensure() != MB_OK) {
+  bool plain = bytes < kMinBytes || workers < 2 || page_locked(host);
+  if (!plain && !slots) plain = (moved += bytes) < kSlotBytes || ensure() != MB_OK;
+  if (plain) {
     cudaGetLastError();
     MB_CUDA(to_host ? cudaMemcpyAsync(host, dev, bytes, kind, s) : cudaMemcpyAsync(dev, host, bytes, kind, s));
     MB_CUDA(cudaStreamSynchronize(s));
