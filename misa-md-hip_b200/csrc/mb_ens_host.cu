@@ -740,11 +740,11 @@ static const char *mx_stencil(const mb_ensemble *e, const LatDesc &d, MxStencil 
   for (int k = 0; k < MX_SHELLS; k++) Q.w[k] = (float)(rc * rc - h * h * n2s[k]);
   for (int gi = 0; gi < 2; gi++) {
     Q.g[gi].rds = (float)(1.0 / grid_ds[gi]);
-    Q.g[gi].mmax = (float)(grid_n[gi] - 1);
+    Q.g[gi].mmax = grid_n[gi] - 1;
     for (int k = 0; k < MX_SHELLS; k++) {
       const double x = h * h * n2s[k] / grid_ds[gi], fl = floor(x);
       Q.g[gi].fr[k] = (float)(x - fl);
-      Q.g[gi].kb[k] = (float)fl;
+      Q.g[gi].kb[k] = (int)fl - MX_FLOOR_BITS;
     }
   }
   Q.a0 = (float)a0;

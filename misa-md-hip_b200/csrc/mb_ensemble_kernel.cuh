@@ -164,10 +164,14 @@ struct MxWalk {
 // 8th and 9th shell, e.g. skin 1.3).  Only per-shell and per-lattice scalars are runtime
 // values.
 #define MX_SHELLS 8
+// Added with rounding down, 1.5 * 2^23 leaves the floor of a float in its low bits.
+#define MX_FLOOR 12582912.0f
+#define MX_FLOOR_BITS 0x4B400000
 struct MxGrid {
-  float rds, mmax;     // 1 / ds, last interval
+  float rds;           // 1 / ds
+  int mmax;            // last interval
   float fr[MX_SHELLS]; // frac(R^2 / ds)
-  float kb[MX_SHELLS]; // floor(R^2 / ds)
+  int kb[MX_SHELLS];   // floor(R^2 / ds) - bits of MX_FLOOR
 };
 struct MxShells {
   float w[MX_SHELLS];  // rc^2 - R^2
