@@ -96,7 +96,7 @@ template <int K>
 __device__ __forceinline__ float4 mxc_load(const MxSite &b) {
   using T = HStore<K>;
   const float4 *base = T::odd ? b.bo : b.be;
-  return __ldg(base + (T::dz * b.pl + T::dy * b.rw) + T::dx);
+  return ld_u4(base + (T::dz * b.pl + T::dy * b.rw) + T::dx);
 }
 
 // num = r^2 - R^2 = |e|^2 - a0 (h . e), e = u_i - u_j (ma0 = -a0).

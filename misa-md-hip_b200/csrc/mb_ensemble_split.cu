@@ -88,7 +88,7 @@ __device__ __forceinline__ MxPair mx_pair(const MxEntry E, float fr, float kb, f
 
 __device__ __forceinline__ float mx_rho_term(const MxEntry E, float rds, float mmax, const float4 &u,
                                              const float4 *base, const float2 *tab) {
-  const float4 nb = __ldg(base + E.off);
+  const float4 nb = ld_u4(base + E.off);
   const MxPair g = mx_pair(E, E.t.w, E.kb, rds, mmax, u, nb);
   const float2 c = tab[g.m];
   const float v = fmaf(c.y, g.q, c.x);
@@ -101,7 +101,7 @@ template <bool ENERGY>
 __device__ __forceinline__ float mx_force_term(const MxEntry E, float rds, float mmax, const float4 &u,
                                                const float4 *base, const float2 *tab, const float4 *ptab,
                                                float2 &dxy, float &dz, float &e) {
-  const float4 nb = __ldg(base + E.off);
+  const float4 nb = ld_u4(base + E.off);
   const MxPair g = mx_pair(E, E.fr_f, E.kb_f, rds, mmax, u, nb);
   const float2 ab = mx_ab(tab, g.m, g.q);
   const float fp = -fmaf(u.w + nb.w, ab.x, ab.y);
@@ -230,7 +230,7 @@ __device__ __forceinline__ double mx_rho_site(const EnsParams &P, const MxStenci
   if (code < 0) return 0.0;
   const float4 *u4 = d.u4[d.cur];
   float4 *uw = d.u4[d.cur];
-  const float4 u = __ldg(u4 + i);
+  const float4 u = ld_u4(u4 + i);
   float rs = 0.f, rc = 0.f;
   if constexpr (FIXED) {
     const MxShells &Q = S.sh;
@@ -271,7 +271,7 @@ __device__ __forceinline__ double mx_rho_site(const EnsParams &P, const MxStenci
     for (int k = 0; k < S.n_far; k++) {
       const MxEntry E = S.far[k];
       const float4 *bb = (E.odd & s) ? bo : be;
-      const float4 nb = __ldg(bb + E.off);
+      const float4 nb = ld_u4(bb + E.off);
       const MxPair g = mx_pair(E, E.t.w, E.kb, rds, mmax, u, nb);
       if (!g.in) continue;
       const float2 t = s_f[g.m];
@@ -306,7 +306,7 @@ __device__ __forceinline__ void mx_force_site(const EnsParams &P, const MxStenci
   const float4 *u4 = d.u4[d.cur];
   float4 *un = d.u4[d.cur ^ 1];
   const float4 *ptab = P.P.ps32;
-  const float4 u = __ldg(u4 + i);
+  const float4 u = ld_u4(u4 + i);
   float2 fs = make_float2(0.f, 0.f), fc = fs;
   float zs = 0.f, zc = 0.f, ps = 0.f, pc = 0.f;
   auto add2 = [&](float2 d0, float z0, float f0, float e0, float2 d1, float z1, float f1, float e1) {
@@ -369,7 +369,7 @@ __device__ __forceinline__ void mx_force_site(const EnsParams &P, const MxStenci
     for (int k = 0; k < S.n_far; k++) {
       const MxEntry E = S.far[k];
       const float4 *bb = (E.odd & s) ? bo : be;
-      const float4 nb = __ldg(bb + E.off);
+      const float4 nb = ld_u4(bb + E.off);
       const MxPair g = mx_pair(E, E.fr_f, E.kb_f, rds, mmax, u, nb);
       if (!g.in) continue;
       float2 d0;
@@ -418,7 +418,10 @@ template <bool ENERGY, int FIXED, int WALK>
 __global__ void __launch_bounds__(MX_RHO_THREADS, 1)
     k_mx_rho(const __grid_constant__ EnsParams P, const MxStencil S, int lat) {
   extern __shared__ float2 s_f[];
+  chain_next();
   for (int k = threadIdx.x; k < S.n_rs; k += blockDim.x) s_f[k] = P.P.fs32[k];
+  unsigned k0 = threadIdx.x >> 5;
+  chain_wait(k0);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const unsigned nwarps = blockDim.x >> 5;
@@ -426,7 +429,7 @@ __global__ void __launch_bounds__(MX_RHO_THREADS, 1)
   unsigned first, count;
   mx_items<WALK>(S.walk, first, count);
   MxAt at{-1, 1u, 0u};
-  for (unsigned k = threadIdx.x >> 5;; k += nwarps) {
+  for (unsigned k = k0;; k += nwarps) {
     const unsigned item = mx_next<WALK>(S.walk, k, first, count);
     if (item == ~0u) break;
     int s = 0, cx = 0, y = 0, z = 0;
@@ -454,7 +457,10 @@ template <bool ENERGY, int FIXED, int WALK>
 __global__ void __launch_bounds__(MX_FORCE_THREADS, 1)
     k_mx_force(const __grid_constant__ EnsParams P, const MxStencil S, int lat) {
   extern __shared__ float2 s_ab[];
+  chain_next();
   for (int k = threadIdx.x; k <= S.n_fs; k += blockDim.x) s_ab[k] = P.P.ab32[k];
+  unsigned k0 = threadIdx.x >> 5;
+  chain_wait(k0);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const unsigned nwarps = blockDim.x >> 5;
@@ -462,7 +468,7 @@ __global__ void __launch_bounds__(MX_FORCE_THREADS, 1)
   unsigned first, count;
   mx_items<WALK>(S.walk, first, count);
   MxAt at{-1, 1u, 0u};
-  for (unsigned k = threadIdx.x >> 5;; k += nwarps) {
+  for (unsigned k = k0;; k += nwarps) {
     const unsigned item = mx_next<WALK>(S.walk, k, first, count);
     if (item == ~0u) break;
     int s = 0, cx = 0, y = 0, z = 0;
@@ -547,6 +553,8 @@ __device__ void mx_itl_bin(const LatDesc &d) {
 }
 
 __global__ void __launch_bounds__(MX_BIN_THREADS, 1) k_mx_itl_prep(const __grid_constant__ EnsParams P) {
+  chain_next();
+  chain_wait();
   const int bins = P.n_itl_lats;
   if ((int)blockIdx.x < bins) {
     mx_itl_bin(P.lats[P.itl_lats[blockIdx.x]]);
@@ -566,6 +574,8 @@ __global__ void __launch_bounds__(MX_BIN_THREADS, 1) k_mx_itl_prep(const __grid_
 #define MX_ITL_THREADS 256
 template <bool FORCE, bool ENERGY>
 __global__ void __launch_bounds__(MX_ITL_THREADS, 3) k_mx_itl_items(const __grid_constant__ EnsParams P) {
+  chain_next();
+  chain_wait();
   __shared__ double red[4][32];
   itl_block_items<FORCE, ENERGY>(P, red);
 }
@@ -577,6 +587,8 @@ __global__ void __launch_bounds__(MX_ITL_THREADS, 3) k_mx_itl_items(const __grid
 // of a vacant site take it (lowest list index first) and the list is compacted in order.
 #define MX_CONV_THREADS 1024
 __global__ void __launch_bounds__(MX_CONV_THREADS, 1) k_mx_convert(const __grid_constant__ EnsParams P) {
+  chain_next();
+  chain_wait();
   __shared__ long long key[MB_CAND_CAP];
   __shared__ unsigned removed[MB_CONV_ITL_MAX / 32];
   __shared__ int s_scan[MX_CONV_THREADS / 32];
@@ -764,6 +776,8 @@ __global__ void __launch_bounds__(MX_CONV_THREADS, 1) k_mx_convert(const __grid_
 }
 
 __global__ void k_mx_bookkeeping(const __grid_constant__ EnsParams P) {
+  chain_next();
+  chain_wait();
   for (int l = threadIdx.x; l < P.n_lats; l += blockDim.x) {
     LatDesc *d = const_cast<LatDesc *>(&P.lats[l]);
     if (!lat_active(*d)) continue;
@@ -787,32 +801,23 @@ static int mx_set_attrs() {
 }
 
 template <int FIXED, int WALK>
-static void mx_pass(const EnsParams &P, const MxStencil &S, int lat, int energy, cudaStream_t s, int which,
-                    size_t smem) {
-  const int sms = device_sm_count();
-  if (which == 0) {
-    if (energy)
-      k_mx_rho<true, FIXED, WALK><<<sms, MX_RHO_THREADS, smem, s>>>(P, S, lat);
-    else
-      k_mx_rho<false, FIXED, WALK><<<sms, MX_RHO_THREADS, smem, s>>>(P, S, lat);
-  } else {
-    if (energy)
-      k_mx_force<true, FIXED, WALK><<<sms, MX_FORCE_THREADS, smem, s>>>(P, S, lat);
-    else
-      k_mx_force<false, FIXED, WALK><<<sms, MX_FORCE_THREADS, smem, s>>>(P, S, lat);
-  }
+static int mx_pass(const EnsParams &P, const MxStencil &S, int lat, int energy, cudaStream_t s, int which, size_t smem,
+                   bool chain) {
+  if (which == 0)
+    return launch_chained(chain, energy ? k_mx_rho<true, FIXED, WALK> : k_mx_rho<false, FIXED, WALK>,
+                          device_sm_count(), MX_RHO_THREADS, smem, s, P, S, lat);
+  return launch_chained(chain, energy ? k_mx_force<true, FIXED, WALK> : k_mx_force<false, FIXED, WALK>,
+                        device_sm_count(), MX_FORCE_THREADS, smem, s, P, S, lat);
 }
 
-static void mx_passes(const EnsParams &P, const MxStencil &S, int lat, int energy, cudaStream_t s, int which,
-                      size_t smem) {
+static int mx_passes(const EnsParams &P, const MxStencil &S, int lat, int energy, cudaStream_t s, int which,
+                     size_t smem, bool chain) {
   if (S.walk.linear)
-    S.fixed == 8 ? mx_pass<8, 1>(P, S, lat, energy, s, which, smem) : mx_pass<7, 1>(P, S, lat, energy, s, which, smem);
-  else if (S.fixed == 8)
-    mx_pass<8, 0>(P, S, lat, energy, s, which, smem);
-  else if (S.fixed)
-    mx_pass<7, 0>(P, S, lat, energy, s, which, smem);
-  else
-    mx_pass<0, 0>(P, S, lat, energy, s, which, smem);
+    return S.fixed == 8 ? mx_pass<8, 1>(P, S, lat, energy, s, which, smem, chain)
+                        : mx_pass<7, 1>(P, S, lat, energy, s, which, smem, chain);
+  if (S.fixed == 8) return mx_pass<8, 0>(P, S, lat, energy, s, which, smem, chain);
+  if (S.fixed) return mx_pass<7, 0>(P, S, lat, energy, s, which, smem, chain);
+  return mx_pass<0, 0>(P, S, lat, energy, s, which, smem, chain);
 }
 
 // Per-lattice energies of an energy step: block l sums the partials of lattice l's items
@@ -855,32 +860,28 @@ int mx_launch_step(const EnsParams &P, const MxStencil &S, int lat, int energy, 
     attr = true;
   }
   const int itl_grid = 3 * sms;
-  if (P.n_itl_lats > 0) k_mx_itl_prep<<<P.n_itl_lats + sms, MX_BIN_THREADS, 0, s>>>(P);
+  const bool chain = !ev && chain_on(); // events take the kernels one by one
+  if (P.n_itl_lats > 0) MB_TRY(launch_chained(chain, k_mx_itl_prep, P.n_itl_lats + sms, MX_BIN_THREADS, 0, s, P));
   if (ev) MB_CUDA(cudaEventRecord(ev[0], s));
-  mx_passes(P, S, lat, energy, s, 0, rho_smem);
+  MB_TRY(mx_passes(P, S, lat, energy, s, 0, rho_smem, chain));
   if (ev) MB_CUDA(cudaEventRecord(ev[1], s));
-  if (P.n_itl_lats > 0) {
-    if (energy)
-      k_mx_itl_items<false, true><<<itl_grid, MX_ITL_THREADS, 0, s>>>(P);
-    else
-      k_mx_itl_items<false, false><<<itl_grid, MX_ITL_THREADS, 0, s>>>(P);
-  }
+  if (P.n_itl_lats > 0)
+    MB_TRY(launch_chained(chain, energy ? k_mx_itl_items<false, true> : k_mx_itl_items<false, false>, itl_grid,
+                          MX_ITL_THREADS, 0, s, P));
   if (ev) MB_CUDA(cudaEventRecord(ev[2], s));
-  mx_passes(P, S, lat, energy, s, 1, force_smem);
+  MB_TRY(mx_passes(P, S, lat, energy, s, 1, force_smem, chain));
   if (ev) MB_CUDA(cudaEventRecord(ev[3], s));
   if (P.n_itl_lats > 0) {
-    if (energy)
-      k_mx_itl_items<true, true><<<itl_grid, MX_ITL_THREADS, 0, s>>>(P);
-    else
-      k_mx_itl_items<true, false><<<itl_grid, MX_ITL_THREADS, 0, s>>>(P);
-    if (P.conv2 > 0.0) k_mx_convert<<<P.n_itl_lats, MX_CONV_THREADS, 0, s>>>(P);
+    MB_TRY(launch_chained(chain, energy ? k_mx_itl_items<true, true> : k_mx_itl_items<true, false>, itl_grid,
+                          MX_ITL_THREADS, 0, s, P));
+    if (P.conv2 > 0.0) MB_TRY(launch_chained(chain, k_mx_convert, P.n_itl_lats, MX_CONV_THREADS, 0, s, P));
   }
   if (energy) {
     const int nl = S.walk.linear ? S.walk.n_lats : 1;
     k_mx_energy<<<nl, 256, 0, s>>>(S.walk.linear ? P.lats : P.lats + lat, nl,
                                    S.walk.linear ? S.walk.item_first : nullptr, S.walk.n_items, P.epart, out);
   }
-  k_mx_bookkeeping<<<1, 128, 0, s>>>(P);
+  MB_TRY(launch_chained(chain, k_mx_bookkeeping, 1, 128, 0, s, P));
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }

@@ -544,6 +544,7 @@ static LatticeArgs lattice_args(const Geom &g, const DevPot &pot, const Lattice6
   a.L = L;
   a.sh = plan.sh;
   a.sites = plan.sites;
+  a.chain = plan.chain;
   const int per_layer = 2 * plan64_plane_items(g);
   a.w0 = z0 * per_layer;
   a.n_items = z1 * per_layer;
@@ -680,6 +681,8 @@ int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const
 // step's marks, which are another bit, off.
 __global__ void __launch_bounds__(MB_ITL_THREADS)
     k_itl_mark(const Geom g, const Lattice64 L, const Itl64 I, int n_mark, int z0, int z1) {
+  chain_next();
+  chain_wait();
   if ((int)blockIdx.x >= n_mark) {
     const int n = min(*I.old_count, I.cap_flag);
     const int old = MB_FLAG_ITL(0) ^ MB_FLAG_ITL(1) ^ I.flag;
@@ -727,10 +730,13 @@ __global__ void __launch_bounds__(MB_ITL_THREADS)
                   double *e1, int z0, int z1) {
   __shared__ double red[4][MB_ITL_THREADS / 32];
   const bool all_z = z0 <= 0 && z1 >= g.bz; // else only items in box layers [z0, z1)
+  int job0 = blockIdx.x;
+  chain_next();
+  chain_wait(job0);
   const int nflag = min(*I.flag_count, I.cap_flag), n_itl = itl_n(I), l8 = threadIdx.x & 7;
   const int jobs = n_itl + (nflag + MB_ITL_THREADS / 8 - 1) / (MB_ITL_THREADS / 8);
   double acc0 = 0.0, acc1 = 0.0;
-  for (int job = blockIdx.x; job < jobs; job += gridDim.x) {
+  for (int job = job0; job < jobs; job += gridDim.x) {
     const bool is_site = job >= n_itl;
     long long i = 0;
     int s = 0, cx = 0, y = 0, z = 0, ti = 0;
@@ -889,16 +895,15 @@ __global__ void __launch_bounds__(MB_ITL_THREADS)
 
 static int itl_blocks(int n) { return n < 4 * device_sm_count() ? n : 4 * device_sm_count(); }
 
-int launch_itl_mark64(const Geom &g, const Lattice64 &L, const Itl64 &I, int clear, cudaStream_t s, int z0, int z1) {
+int launch_itl_mark64(const Geom &g, const Lattice64 &L, const Itl64 &I, int clear, cudaStream_t s, int z0, int z1,
+                      bool chain) {
   if (z1 < 0) z1 = g.bz;
   const int nmax = I.nd ? I.cap : I.n;
   if (nmax <= 0 || z0 >= z1) return MB_OK;
   const int marks = itl_blocks(nmax);
   int clears = clear ? (I.cap_flag + MB_ITL_THREADS - 1) / MB_ITL_THREADS : 0;
   if (clears > device_sm_count()) clears = device_sm_count();
-  k_itl_mark<<<marks + clears, MB_ITL_THREADS, 0, s>>>(g, L, I, marks, z0, z1);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
+  return launch_chained(chain, k_itl_mark, marks + clears, MB_ITL_THREADS, 0, s, g, L, I, marks, z0, z1);
 }
 
 __global__ void k_itl_reset(const Lattice64 L, const Itl64 I) {
@@ -920,30 +925,26 @@ int launch_itl_reset64(const Lattice64 &L, const Itl64 &I, cudaStream_t s) {
 
 template <bool FORCE>
 static int launch_items(const Geom &g, const DevPot &pot, const Lattice64 &L, const Itl64 &I, const StepParams &sp,
-                        double *e0, double *e1, int energy, cudaStream_t s, int z0, int z1) {
+                        double *e0, double *e1, int energy, cudaStream_t s, int z0, int z1, bool chain) {
   if (!I.nd && I.n == 0) return MB_OK;
   if (z1 < 0) z1 = g.bz;
   const int grid = itl_blocks((I.nd ? I.cap : I.n) + (I.cap_flag + 31) / 32);
-  if (energy)
-    k_itl_items64<FORCE, true><<<grid, MB_ITL_THREADS, 0, s>>>(g, pot, L, I, sp, e0, e1, z0, z1);
-  else
-    k_itl_items64<FORCE, false><<<grid, MB_ITL_THREADS, 0, s>>>(g, pot, L, I, sp, nullptr, nullptr, z0, z1);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
+  return launch_chained(chain, energy ? k_itl_items64<FORCE, true> : k_itl_items64<FORCE, false>, grid, MB_ITL_THREADS,
+                        0, s, g, pot, L, I, sp, energy ? e0 : nullptr, energy ? e1 : nullptr, z0, z1);
 }
 
 int launch_itl_rho64(const Geom &g, const DevPot &pot, const Lattice64 &L, const Itl64 &I, double rc2,
-                     double *e_partial, int energy, cudaStream_t s, int z0, int z1) {
+                     double *e_partial, int energy, cudaStream_t s, int z0, int z1, bool chain) {
   StepParams sp{};
   sp.rc2 = rc2;
   return launch_items<false>(g, pot, L, I, sp, energy ? e_partial + 3 * MB_EPART_CAP : nullptr, nullptr, energy, s, z0,
-                             z1);
+                             z1, chain);
 }
 
 int launch_itl_force64(const Geom &g, const DevPot &pot, const Lattice64 &L, const Itl64 &I, const StepParams &sp,
-                       double *e_partial, int energy, cudaStream_t s, int z0, int z1) {
+                       double *e_partial, int energy, cudaStream_t s, int z0, int z1, bool chain) {
   return launch_items<true>(g, pot, L, I, sp, energy ? e_partial + 4 * MB_EPART_CAP : nullptr,
-                            energy ? e_partial + 5 * MB_EPART_CAP : nullptr, energy, s, z0, z1);
+                            energy ? e_partial + 5 * MB_EPART_CAP : nullptr, energy, s, z0, z1, chain);
 }
 
 // ------------------------------------------ lattice <-> interstitial bookkeeping

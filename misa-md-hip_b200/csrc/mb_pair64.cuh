@@ -34,6 +34,7 @@ struct LatticeArgs {
   double rc2, rc2m;      // squared cutoff; a hair above it for the outer-entry masks
   int rc2_hi;            // high word of rc2
   int copies;            // table copies of a shell window (several types)
+  bool chain;            // see launch_chained
   int flag;              // code bit of the sites an interstitial pass finishes (0: none)
   uint2 *outer;          // per item: the outer entries some lane has inside rc2m (or null)
   double *e0, *e1;       // CTA partials: density pass F(rho); force pass pair and kinetic energy

@@ -68,13 +68,15 @@ __device__ __forceinline__ void fill_window(double2 *w, const double2 *src, int 
       if (c < copies) w[k * copies + ((c + threadIdx.x) & (copies - 1))] = v;
   }
 }
-// The window of knots [lo, lo + cnt] of a table of `words` words per knot.
-template <int COPIES>
+// The window of knots [lo, lo + cnt] of a table of `words` words per knot; the first one (SH
+// == 0) is filled while the kernel before drains.
+template <int COPIES, int SH>
 __device__ __forceinline__ Window64<COPIES> take_window(double2 *s_w, const double2 *tab, int words, int copies, int lo,
-                                                        int cnt) {
+                                                        int cnt, int &first) {
   if (COPIES > 0) copies = COPIES;
   __syncthreads();
   fill_window(s_w, tab + (size_t)words * lo, (cnt + 1) * words, copies);
+  if (SH == 0) chain_wait(first);
   __syncthreads();
   return Window64<COPIES>{s_w + (threadIdx.x & (copies - 1)), MB_FLOOR - lo, (unsigned)cnt, words, copies};
 }
@@ -195,15 +197,16 @@ __global__ void __launch_bounds__(MB_SHELL_RHO_THREADS, 1)
   const Lattice64 &L = a.L;
   constexpr int n_near = kBcc.start[NEAR];
   const int lane = threadIdx.x & 31, pl = a.g.ey * a.g.ecx, rw = a.g.ecx;
+  chain_next();
   const Rounds64 rd = launch_rounds(a);
   double e_acc = 0.0;
   for (int b = 0; b < rd.batches; b++) {
-    const BatchItems it = batch_items(a, b, rd);
+    BatchItems it = batch_items(a, b, rd);
     static_for<0, RhoVisits<NEAR>::n>([&](auto vc) {
       constexpr int V = decltype(vc)::value, SH = RhoVisits<NEAR>::first[V], END = RhoVisits<NEAR>::first[V + 1];
       const int lo = a.sh.rho.lo[SH], cnt = a.sh.rho.cnt[SH];
       const Window64<COPIES> W =
-          take_window<COPIES>(s_w, a.P.f_ys, COPIES > 0 ? 1 : a.P.n_types, a.copies, lo, cnt);
+          take_window<COPIES, SH>(s_w, a.P.f_ys, COPIES > 0 ? 1 : a.P.n_types, a.copies, lo, cnt, it.lo);
       int next = item_ref(a, it.lo, it.hi);
       for (int w = it.lo; w < it.hi; w += it.stride) {
         const int ref = next, i = ref & MB_SITE_INDEX;
@@ -254,16 +257,16 @@ __global__ void __launch_bounds__(COPIES > 0 ? MB_SHELL_FORCE_THREADS : MB_MULTI
   const Lattice64 &L = a.L;
   constexpr int n_near = kBcc.start[NEAR];
   const int lane = threadIdx.x & 31, pl = a.g.ey * a.g.ecx, rw = a.g.ecx;
+  chain_next();
   const Rounds64 rd = launch_rounds(a);
   double e_pair = 0.0, e_kin = 0.0;
   for (int b = 0; b < rd.batches; b++) {
-    const BatchItems it = batch_items(a, b, rd);
+    BatchItems it = batch_items(a, b, rd);
     static_for<0, NEAR>([&](auto shc) {
       constexpr int SH = decltype(shc)::value;
-      __syncthreads();
       const int lo = a.sh.force.lo[SH], cnt = a.sh.force.cnt[SH];
       const Window64<COPIES> W =
-          take_window<COPIES>(s_w, a.P.force2, COPIES > 0 ? 2 : force_words(a.P.n_types), a.copies, lo, cnt);
+          take_window<COPIES, SH>(s_w, a.P.force2, COPIES > 0 ? 2 : force_words(a.P.n_types), a.copies, lo, cnt, it.lo);
       int next = item_ref(a, it.lo, it.hi);
       for (int w = it.lo; w < it.hi; w += it.stride) {
         const int ref = next, i = ref & MB_SITE_INDEX;
@@ -325,12 +328,8 @@ static int shell_rho(const StencilSet &st, LatticeArgs a, int energy, cudaStream
   MB_SMEM_ATTR((k_shell_rho64<false, NEAR, COPIES>), (k_shell_rho64<true, NEAR, COPIES>), MB_SMEM_MAX - 1024);
   a.copies = a.sh.rho.copies;
   const size_t smem = window_bytes(a.sh.rho, a.sh.n, a.P.n_types, a.copies);
-  if (energy)
-    k_shell_rho64<true, NEAR, COPIES><<<device_sm_count(), MB_SHELL_RHO_THREADS, smem, s>>>(st, a);
-  else
-    k_shell_rho64<false, NEAR, COPIES><<<device_sm_count(), MB_SHELL_RHO_THREADS, smem, s>>>(st, a);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
+  return launch_chained(a.chain, energy ? k_shell_rho64<true, NEAR, COPIES> : k_shell_rho64<false, NEAR, COPIES>,
+                        device_sm_count(), MB_SHELL_RHO_THREADS, smem, s, st, a);
 }
 template <int NEAR, int COPIES>
 static int shell_force(const StencilSet &st, LatticeArgs a, int energy, cudaStream_t s) {
@@ -338,12 +337,8 @@ static int shell_force(const StencilSet &st, LatticeArgs a, int energy, cudaStre
   a.copies = a.sh.force.copies;
   const size_t smem = window_bytes(a.sh.force, a.sh.n, force_words(a.P.n_types), a.copies);
   const int threads = COPIES > 0 ? MB_SHELL_FORCE_THREADS : MB_MULTI_FORCE_THREADS;
-  if (energy)
-    k_shell_force64<true, NEAR, COPIES><<<device_sm_count(), threads, smem, s>>>(st, a);
-  else
-    k_shell_force64<false, NEAR, COPIES><<<device_sm_count(), threads, smem, s>>>(st, a);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
+  return launch_chained(a.chain, energy ? k_shell_force64<true, NEAR, COPIES> : k_shell_force64<false, NEAR, COPIES>,
+                        device_sm_count(), threads, smem, s, st, a);
 }
 
 int launch_shell_rho64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {

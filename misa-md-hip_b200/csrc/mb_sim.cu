@@ -174,21 +174,24 @@ static int step64(mb_sim *s, int energy, int kick_pre, int drift, int timed) {
   double *ep = energy ? s->epart : nullptr;
   if (energy) MB_CUDA(cudaMemsetAsync(s->epart, 0, sizeof(double) * energy_partials_needed(), s->stream));
   const int itl = itl_active(s), flag = itl ? I.flag : 0;
+  const bool chain = !timed && chain_on();
+  Plan64 plan = s->plan;
+  plan.chain = chain;
   if (itl) {
     // a step after one at the other buffer clears that one's marks; any other state of the
     // lists (a first step, interstitials that come back) starts from empty ones
     if (s->flag_last != (s->cur ^ 1)) MB_TRY(launch_itl_reset64(L, I, s->stream));
-    MB_TRY(launch_itl_mark64(s->g, L, I, 1, s->stream));
+    MB_TRY(launch_itl_mark64(s->g, L, I, 1, s->stream, 0, -1, chain));
   }
   s->flag_last = itl ? s->cur : -1;
   if (timed) MB_CUDA(cudaEventRecord(s->ev[4], s->stream));
-  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, ep, energy, flag, s->stream, 0, -1, s->outer, &s->plan));
+  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, ep, energy, flag, s->stream, 0, -1, s->outer, &plan));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[5], s->stream));
-  if (itl) MB_TRY(launch_itl_rho64(s->g, P, L, I, sp.rc2, ep, energy, s->stream));
+  if (itl) MB_TRY(launch_itl_rho64(s->g, P, L, I, sp.rc2, ep, energy, s->stream, 0, -1, chain));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[6], s->stream));
-  MB_TRY(launch_force64(s->g, s->st, P, L, sp, ep, energy, flag, s->stream, 0, -1, s->outer, &s->plan));
+  MB_TRY(launch_force64(s->g, s->st, P, L, sp, ep, energy, flag, s->stream, 0, -1, s->outer, &plan));
   if (timed) MB_CUDA(cudaEventRecord(s->ev[7], s->stream));
-  if (itl) MB_TRY(launch_itl_force64(s->g, P, L, I, sp, ep, energy, s->stream));
+  if (itl) MB_TRY(launch_itl_force64(s->g, P, L, I, sp, ep, energy, s->stream, 0, -1, chain));
   if (sp.conv2 > 0.0)
     MB_TRY(launch_convert64(s->g, L, I, sp, s->rec_d * s->rec_d, s->id, s->d_nitl, s->d_conv_counters, s->stream));
   return MB_OK;

@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
   extern __shared__ double2 s_w[];
   __shared__ double s_sum[MB_SPLIT_GROUPS][2][MB_RUNS_MAX][32]; // two items' sums, in turn
   __shared__ unsigned s_near[MB_SPLIT_GROUPS][2][MB_RUNS_MAX];
+  chain_next();
   const int words = COPIES > 0 ? 1 : a.P.n_types;
   const double2 *tab = a.P.f_ys + (size_t)words * lo;
   if (COPIES > 0 || knots > 0) {
@@ -74,8 +75,9 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % MB_SPLIT_WARPS,
             group = threadIdx.x / (32 * MB_SPLIT_WARPS);
   double e_acc = 0.0;
-  int turn = 0;
-  for (int w = a.w0 + blockIdx.x * MB_SPLIT_GROUPS + group; w < a.n_items; w += gridDim.x * MB_SPLIT_GROUPS, turn++) {
+  int turn = 0, w0 = a.w0 + blockIdx.x * MB_SPLIT_GROUPS + group;
+  chain_wait(w0);
+  for (int w = w0; w < a.n_items; w += gridDim.x * MB_SPLIT_GROUPS, turn++) {
     double(*sums)[32] = s_sum[group][turn & 1];
     unsigned *nears = s_near[group][turn & 1];
     const SplitSite t = split_site(st, a, w);
@@ -130,6 +132,7 @@ template <bool ENERGY, int COPIES>
 __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
     k_split_force64(const __grid_constant__ StencilSet st, const __grid_constant__ LatticeArgs a, int lo, int knots) {
   extern __shared__ double2 s_w[]; // table, then the run sums
+  chain_next();
   const int words = COPIES > 0 ? 2 : force_words(a.P.n_types);
   const double2 *tab = a.P.force2 + (size_t)words * lo;
   if (COPIES > 0 || knots > 0) {
@@ -141,8 +144,9 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
             group = threadIdx.x / (32 * MB_SPLIT_WARPS);
   double *sums = reinterpret_cast<double *>(s_w + words * knots) + (size_t)group * 2 * a.sh.runs * 96 + lane;
   double e_pair = 0.0, e_kin = 0.0;
-  int turn = 0;
-  for (int w = a.w0 + blockIdx.x * MB_SPLIT_GROUPS + group; w < a.n_items; w += gridDim.x * MB_SPLIT_GROUPS, turn++) {
+  int turn = 0, w0 = a.w0 + blockIdx.x * MB_SPLIT_GROUPS + group;
+  chain_wait(w0);
+  for (int w = w0; w < a.n_items; w += gridDim.x * MB_SPLIT_GROUPS, turn++) {
     double *sum = sums + (turn & 1) * a.sh.runs * 96;
     const SplitSite t = split_site(st, a, w);
     unsigned long long mask = ~0ull;
@@ -232,12 +236,8 @@ static int split_rho(const StencilSet &st, const LatticeArgs &a, int energy, cud
   knots = smem_knots(knots, a.P.n_types, 0, kRhoSmem);
   const size_t smem = (size_t)knots * a.P.n_types * sizeof(double2);
   MB_SMEM_ATTR((k_split_rho64<false, COPIES>), (k_split_rho64<true, COPIES>), kRhoSmem);
-  if (energy)
-    k_split_rho64<true, COPIES><<<split_grid(a), MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
-  else
-    k_split_rho64<false, COPIES><<<split_grid(a), MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
+  return launch_chained(a.chain, energy ? k_split_rho64<true, COPIES> : k_split_rho64<false, COPIES>, split_grid(a),
+                        MB_SPLIT_THREADS, smem, s, st, a, lo, knots);
 }
 
 template <int COPIES>
@@ -247,12 +247,8 @@ static int split_force(const StencilSet &st, const LatticeArgs &a, int energy, c
   knots = smem_knots(knots, force_words(a.P.n_types), run_sum_bytes(a.sh), kForceSmem);
   const size_t smem = (size_t)knots * force_words(a.P.n_types) * sizeof(double2) + run_sum_bytes(a.sh);
   MB_SMEM_ATTR((k_split_force64<false, COPIES>), (k_split_force64<true, COPIES>), kForceSmem);
-  if (energy)
-    k_split_force64<true, COPIES><<<split_grid(a), MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
-  else
-    k_split_force64<false, COPIES><<<split_grid(a), MB_SPLIT_THREADS, smem, s>>>(st, a, lo, knots);
-  MB_CUDA(cudaGetLastError());
-  return MB_OK;
+  return launch_chained(a.chain, energy ? k_split_force64<true, COPIES> : k_split_force64<false, COPIES>, split_grid(a),
+                        MB_SPLIT_THREADS, smem, s, st, a, lo, knots);
 }
 
 int launch_split_rho64(const StencilSet &st, const LatticeArgs &a, int energy, cudaStream_t s) {
