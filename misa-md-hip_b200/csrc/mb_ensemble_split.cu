@@ -219,6 +219,60 @@ __device__ __forceinline__ void mx_unpack(unsigned p, int &s, int &cx, int &y, i
 // pass.
 #define MX_MASK_MARGIN 1e-3f
 
+// The end of a site's density pass: rho = rs + rc, df to the site and its images; returns
+// F(rho) for the energy.
+template <bool ENERGY>
+__device__ __forceinline__ double mx_rho_finish(const EnsParams &P, const LatDesc &d, long long i, unsigned pos,
+                                                int code, float rs, float rc) {
+  float4 *uw = d.u4[d.cur];
+  const double rho = (double)rs + (double)rc;
+  d.rho[i] = (float)rho;
+  if (code & MB_FLAG_ITL(d.cur)) return 0.0; // lattice part only: the interstitial items finish the site
+  const double df = dF64(P.P, code & MB_TYPE_MASK, rho);
+  reinterpret_cast<float *>(uw + i)[3] = (float)df;
+  int sx, cx, y, z;
+  mx_unpack(pos, sx, cx, y, z);
+  const Geom g = lat_geom(d);
+  for_images(g, sx, cx, y, z,
+             [&](long long idx, double, double, double) { reinterpret_cast<float *>(uw + idx)[3] = (float)df; });
+  return ENERGY ? F64(P.P, code & MB_TYPE_MASK, rho) : 0.0;
+}
+
+// The end of a site's force pass: forces, closing kick, opening kick and drift, images.
+template <bool ENERGY>
+__device__ __forceinline__ void mx_force_finish(const EnsParams &P, const LatDesc &d, long long i, unsigned pos,
+                                                int code, double fx, double fy, double fz, double &e_kin) {
+  float4 *un = d.u4[d.cur ^ 1];
+  d.fx[i] = (float)fx;
+  d.fy[i] = (float)fy;
+  d.fz[i] = (float)fz;
+  if (code & MB_FLAG_ITL(d.cur)) return; // lattice part only: the interstitial items integrate the site
+  double vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
+  if (d.primed) {
+    vx += P.h * fx;
+    vy += P.h * fy;
+    vz += P.h * fz;
+  }
+  if (ENERGY) e_kin += 0.5 * P.mass * (vx * vx + vy * vy + vz * vz) * MB_MVV2E;
+  vx += P.h * fx;
+  vy += P.h * fy;
+  vz += P.h * fz;
+  const double nx = d.ux[i] + P.dt * vx, ny = d.uy[i] + P.dt * vy, nz = d.uz[i] + P.dt * vz;
+  d.vx[i] = vx;
+  d.vy[i] = vy;
+  d.vz[i] = vz;
+  d.ux[i] = nx;
+  d.uy[i] = ny;
+  d.uz[i] = nz;
+  const float4 nu = make_float4((float)nx, (float)ny, (float)nz, 0.f);
+  un[i] = nu;
+  int sx, cx, y, z;
+  mx_unpack(pos, sx, cx, y, z);
+  ens_conv_check(P, d, sx, cx, y, z, nx, ny, nz);
+  const Geom g = lat_geom(d);
+  for_images(g, sx, cx, y, z, [&](long long idx, double, double, double) { un[idx] = nu; });
+}
+
 // near: bit k - 64 set when branch-walked built-in entry k (shells 7 and 8) is inside
 // the cutoff (plus MX_MASK_MARGIN) for this site.
 template <bool ENERGY, int FIXED>
@@ -229,7 +283,6 @@ __device__ __forceinline__ double mx_rho_site(const EnsParams &P, const MxStenci
   const int code = d.code[i];
   if (code < 0) return 0.0;
   const float4 *u4 = d.u4[d.cur];
-  float4 *uw = d.u4[d.cur];
   const float4 u = ld_u4(u4 + i);
   float rs = 0.f, rc = 0.f;
   if constexpr (FIXED) {
@@ -278,17 +331,7 @@ __device__ __forceinline__ double mx_rho_site(const EnsParams &P, const MxStenci
       two_sum(rs, rc, fmaf(t.y, g.q, t.x));
     }
   }
-  const double rho = (double)rs + (double)rc;
-  d.rho[i] = (float)rho;
-  if (code & MB_FLAG_ITL(d.cur)) return 0.0; // lattice part only: the interstitial items finish the site
-  const double df = dF64(P.P, code & MB_TYPE_MASK, rho);
-  reinterpret_cast<float *>(uw + i)[3] = (float)df;
-  int sx, cx, y, z;
-  mx_unpack(pos, sx, cx, y, z);
-  const Geom g = lat_geom(d);
-  for_images(g, sx, cx, y, z,
-             [&](long long idx, double, double, double) { reinterpret_cast<float *>(uw + idx)[3] = (float)df; });
-  return ENERGY ? F64(P.P, code & MB_TYPE_MASK, rho) : 0.0;
+  return mx_rho_finish<ENERGY>(P, d, i, pos, code, rs, rc);
 }
 
 // Force + velocity-Verlet of one site; adds pair energy and kinetic energy.  Pair terms
@@ -304,7 +347,6 @@ __device__ __forceinline__ void mx_force_site(const EnsParams &P, const MxStenci
   const int code = d.code[i];
   if (code < 0) return;
   const float4 *u4 = d.u4[d.cur];
-  float4 *un = d.u4[d.cur ^ 1];
   const float4 *ptab = P.P.ps32;
   const float4 u = ld_u4(u4 + i);
   float2 fs = make_float2(0.f, 0.f), fc = fs;
@@ -316,7 +358,7 @@ __device__ __forceinline__ void mx_force_site(const EnsParams &P, const MxStenci
   };
   auto add1 = [&](float2 d0, float z0, float f0, float e0) {
     two_sum2(fs, fc, __fmul2_rn(d0, make_float2(f0, f0)));
-    two_sum(zs, zc, z0 * f0);
+    two_sum(zs, zc, __fmul_rn(z0, f0)); // rounded like x and y, not contracted into the sum
     if (ENERGY) two_sum(ps, pc, e0);
   };
   if constexpr (FIXED) {
@@ -381,35 +423,8 @@ __device__ __forceinline__ void mx_force_site(const EnsParams &P, const MxStenci
   const double fx = (double)fs.x + (double)fc.x;
   const double fy = (double)fs.y + (double)fc.y;
   const double fz = (double)zs + (double)zc;
-  d.fx[i] = (float)fx;
-  d.fy[i] = (float)fy;
-  d.fz[i] = (float)fz;
   if (ENERGY) e_pair += (double)ps + (double)pc;
-  if (code & MB_FLAG_ITL(d.cur)) return; // lattice part only: the interstitial items integrate the site
-  double vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
-  if (d.primed) {
-    vx += P.h * fx;
-    vy += P.h * fy;
-    vz += P.h * fz;
-  }
-  if (ENERGY) e_kin += 0.5 * P.mass * (vx * vx + vy * vy + vz * vz) * MB_MVV2E;
-  vx += P.h * fx;
-  vy += P.h * fy;
-  vz += P.h * fz;
-  const double nx = d.ux[i] + P.dt * vx, ny = d.uy[i] + P.dt * vy, nz = d.uz[i] + P.dt * vz;
-  d.vx[i] = vx;
-  d.vy[i] = vy;
-  d.vz[i] = vz;
-  d.ux[i] = nx;
-  d.uy[i] = ny;
-  d.uz[i] = nz;
-  const float4 nu = make_float4((float)nx, (float)ny, (float)nz, 0.f);
-  un[i] = nu;
-  int sx, cx, y, z;
-  mx_unpack(pos, sx, cx, y, z);
-  ens_conv_check(P, d, sx, cx, y, z, nx, ny, nz);
-  const Geom g = lat_geom(d);
-  for_images(g, sx, cx, y, z, [&](long long idx, double, double, double) { un[idx] = nu; });
+  mx_force_finish<ENERGY>(P, d, i, pos, code, fx, fy, fz, e_kin);
 }
 
 // Density pass.  FIXED: the built-in BCC shells (MxShells), else the runtime stencil
@@ -491,6 +506,181 @@ __global__ void __launch_bounds__(MX_FORCE_THREADS, 1)
         P.epart[2 * (size_t)item + 1] = ek;
       }
     }
+  }
+}
+
+// ------------------------------------------------- small launches: an item's pairs split
+// A launch of a few items per SM is the latency of one warp walking ~90 entries after its
+// CTA filled 200 KB of table.  Here the 8 warps of a CTA share an item: each computes a few
+// entry pairs, with the tables read where they lie (L2, L1), leaves their sums in shared
+// memory and one warp adds them in the order of the kernels above, so that the results are
+// the same bits.  Measured on one B200, step: 8^3 cells 36.6 -> 18.4 us, 16^3 40 -> 22, 20^3
+// 40 -> 29.
+#define MX_ONE_WARPS 8
+#define MX_ONE_THREADS (32 * MX_ONE_WARPS)
+#define MX_PAIRS 32 // pairs of the 64 entries walked without a branch
+template <int FIXED>
+struct MxOne {
+  static constexpr int outer = kBcc.start[FIXED] - 2 * MX_PAIRS, terms = MX_PAIRS + outer;
+  static constexpr int pairs_w = MX_PAIRS / MX_ONE_WARPS, outer_w = outer / MX_ONE_WARPS;
+  static_assert(outer % MX_ONE_WARPS == 0, "outer entries shared evenly");
+};
+
+// A lane's site of linear item `item`, found by the whole warp.
+__device__ __forceinline__ bool mx_one_site(const EnsParams &P, const MxWalk &W, unsigned item, int lane, int &l,
+                                            long long &i, unsigned &pos) {
+  unsigned n = 0; // lattices that begin at or before the item
+  for (int b = 0; b < W.n_lats; b += 32)
+    n += __popc(__ballot_sync(0xffffffffu, b + lane < W.n_lats && __ldg(W.item_first + b + lane) <= item));
+  l = (int)n - 1;
+  MxAt at{l, __ldg(W.item_first + l), __ldg(W.item_first + n)};
+  int s = 0, cx = 0, y = 0, z = 0;
+  const bool ok = mx_locate<1>(P, W, 0, item, lane, at, s, cx, y, z, i);
+  pos = mx_pack(s, cx, y, z);
+  return ok && lat_active(P.lats[l]);
+}
+
+// Runs f with the calling warp's number as a constant.
+template <class F>
+__device__ __forceinline__ void by_warp(int warp, F f) {
+  static_for<0, MX_ONE_WARPS>([&](auto w) {
+    if (warp == decltype(w)::value) f(w);
+  });
+}
+
+template <int FIXED>
+__global__ void __launch_bounds__(MX_ONE_THREADS, 4)
+    k_mx_one_rho(const __grid_constant__ EnsParams P, const __grid_constant__ MxStencil S) {
+  using One = MxOne<FIXED>;
+  __shared__ float s_t[One::terms][32];
+  __shared__ unsigned s_near[MX_ONE_WARPS][2];
+  chain_next();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float ma0 = -S.sh.a0;
+  const float2 *tab = P.P.fs32;
+  unsigned item = blockIdx.x;
+  chain_wait(item);
+  for (int turn = 0; item < S.walk.n_items; item += gridDim.x, turn++) {
+    int l;
+    long long i = 0;
+    unsigned pos;
+    bool ok = mx_one_site(P, S.walk, item, lane, l, i, pos);
+    const LatDesc &d = P.lats[l];
+    const int code = ok ? d.code[i] : -1;
+    ok = ok && code >= 0;
+    unsigned long long near = 0;
+    if (ok) {
+      const MxShells &Q = S.sh;
+      const float4 *u4 = d.u4[d.cur];
+      const float4 u = ld_u4(u4 + i);
+      const MxSite b = mx_site_bases(d, u4, i, (int)(pos >> 31));
+      by_warp(warp, [&](auto wc) {
+        constexpr int w = decltype(wc)::value;
+        static_for<0, One::pairs_w>([&](auto pc) {
+          constexpr int p = w * One::pairs_w + decltype(pc)::value;
+          s_t[p][lane] = mxc_rho<2 * p>(Q, ma0, b, u, tab) + mxc_rho<2 * p + 1>(Q, ma0, b, u, tab);
+        });
+        static_for<0, One::outer_w>([&](auto oc) {
+          constexpr int o = w * One::outer_w + decltype(oc)::value, k = 2 * MX_PAIRS + o;
+          const float4 nb = mxc_load<k>(b);
+          float2 exy;
+          float ez, q, v = 0.f;
+          const float num = mxc_num<k>(ma0, u, nb, exy, ez);
+          near |= (unsigned long long)(num < Q.w[HStore<k>::sh] + MX_MASK_MARGIN) << o;
+          if (num < Q.w[HStore<k>::sh]) {
+            const float2 t = tab[mxc_index<k, 0>(Q, num, q)];
+            v = fmaf(t.y, q, t.x);
+          }
+          s_t[MX_PAIRS + o][lane] = v;
+        });
+      });
+    }
+    const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)near);
+    const unsigned hi = __reduce_or_sync(0xffffffffu, (unsigned)(near >> 32));
+    if (lane == 0) s_near[warp][0] = lo, s_near[warp][1] = hi;
+    __syncthreads();
+    if (warp == turn % MX_ONE_WARPS) {
+      if (ok) {
+        float rs = 0.f, rc = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < One::terms; k++) two_sum(rs, rc, s_t[k][lane]);
+        mx_rho_finish<false>(P, d, i, pos, code, rs, rc);
+      }
+      if (P.outer && lane == 0) {
+        uint2 m = make_uint2(0u, 0u);
+        for (int k = 0; k < MX_ONE_WARPS; k++) m.x |= s_near[k][0], m.y |= s_near[k][1];
+        P.outer[item] = m;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <int FIXED>
+__global__ void __launch_bounds__(MX_ONE_THREADS, 3)
+    k_mx_one_force(const __grid_constant__ EnsParams P, const __grid_constant__ MxStencil S) {
+  using One = MxOne<FIXED>;
+  __shared__ float2 s_xy[One::terms][32];
+  __shared__ float s_z[One::terms][32];
+  chain_next();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float ma0 = -S.sh.a0;
+  const float2 *tab = P.P.ab32;
+  unsigned item = blockIdx.x;
+  chain_wait(item);
+  for (int turn = 0; item < S.walk.n_items; item += gridDim.x, turn++) {
+    int l;
+    long long i = 0;
+    unsigned pos;
+    bool ok = mx_one_site(P, S.walk, item, lane, l, i, pos);
+    const LatDesc &d = P.lats[l];
+    const int code = ok ? d.code[i] : -1;
+    ok = ok && code >= 0;
+    unsigned long long outer = ~0ull;
+    if (P.outer) {
+      const uint2 m2 = P.outer[item];
+      outer = (unsigned long long)m2.x | ((unsigned long long)m2.y << 32);
+    }
+    if (ok) {
+      const MxShells &Q = S.sh;
+      const float4 *u4 = d.u4[d.cur];
+      const float4 u = ld_u4(u4 + i);
+      const MxSite b = mx_site_bases(d, u4, i, (int)(pos >> 31));
+      by_warp(warp, [&](auto wc) {
+        constexpr int w = decltype(wc)::value;
+        static_for<0, One::pairs_w>([&](auto pc) {
+          constexpr int p = w * One::pairs_w + decltype(pc)::value;
+          float2 d0, d1;
+          float z0, z1, e;
+          const float f0 = mxc_force<2 * p, false>(Q, ma0, b, u, tab, nullptr, d0, z0, e);
+          const float f1 = mxc_force<2 * p + 1, false>(Q, ma0, b, u, tab, nullptr, d1, z1, e);
+          s_xy[p][lane] = __ffma2_rn(d1, make_float2(f1, f1), __fmul2_rn(d0, make_float2(f0, f0)));
+          s_z[p][lane] = fmaf(z1, f1, z0 * f0);
+        });
+        static_for<0, One::outer_w>([&](auto oc) {
+          constexpr int o = w * One::outer_w + decltype(oc)::value, k = 2 * MX_PAIRS + o;
+          float2 d0 = make_float2(0.f, 0.f);
+          float z0 = 0.f, f0 = 0.f, e;
+          if ((outer >> o) & 1ull) f0 = mxc_force<k, false>(Q, ma0, b, u, tab, nullptr, d0, z0, e);
+          s_xy[MX_PAIRS + o][lane] = __fmul2_rn(d0, make_float2(f0, f0));
+          s_z[MX_PAIRS + o][lane] = __fmul_rn(z0, f0);
+        });
+      });
+    }
+    __syncthreads();
+    if (warp == turn % MX_ONE_WARPS && ok) {
+      float2 fs = make_float2(0.f, 0.f), fc = fs;
+      float zs = 0.f, zc = 0.f;
+#pragma unroll 8
+      for (int k = 0; k < One::terms; k++) {
+        two_sum2(fs, fc, s_xy[k][lane]);
+        two_sum(zs, zc, s_z[k][lane]);
+      }
+      double e_kin = 0.0;
+      mx_force_finish<false>(P, d, i, pos, code, (double)fs.x + (double)fc.x, (double)fs.y + (double)fc.y,
+                             (double)zs + (double)zc, e_kin);
+    }
+    __syncthreads();
   }
 }
 
@@ -810,8 +1000,29 @@ static int mx_pass(const EnsParams &P, const MxStencil &S, int lat, int energy, 
                         device_sm_count(), MX_FORCE_THREADS, smem, s, P, S, lat);
 }
 
+// Linear launches of up to this many items per SM split each item's pairs over a CTA; energy
+// steps, which need the pair energies too, do not.  Step with split / whole items: 16^3 cells
+// (1.7 items per SM) 22 / 40 us, 20^3 (3.4) 29 / 40, 24^3 (5.8) 35 / 39, 28^3 (9.3) 53 / 41; at
+// 5.8 the density pass alone gains 9 us, the force pass, with 2.5 times the table bytes per
+// pair from L2, nothing.  MB_MX_ONE_ITEMS overrides both lines (0: never).
+#define MX_ONE_RHO_ITEMS 7
+#define MX_ONE_FORCE_ITEMS 4
+static bool mx_one(const MxStencil &S, int energy, int which) {
+  int per_sm = which == 0 ? MX_ONE_RHO_ITEMS : MX_ONE_FORCE_ITEMS;
+  if (const char *v = getenv("MB_MX_ONE_ITEMS")) per_sm = atoi(v);
+  return S.walk.linear && !energy && (long long)S.walk.n_items <= (long long)per_sm * device_sm_count();
+}
+template <int FIXED>
+static int mx_one_pass(const EnsParams &P, const MxStencil &S, cudaStream_t s, int which, bool chain) {
+  const int most = (which == 0 ? 4 : 3) * device_sm_count(), n = (int)S.walk.n_items;
+  return launch_chained(chain, which == 0 ? k_mx_one_rho<FIXED> : k_mx_one_force<FIXED>, n < most ? n : most,
+                        MX_ONE_THREADS, 0, s, P, S);
+}
+
 static int mx_passes(const EnsParams &P, const MxStencil &S, int lat, int energy, cudaStream_t s, int which,
                      size_t smem, bool chain) {
+  if (mx_one(S, energy, which))
+    return S.fixed == 8 ? mx_one_pass<8>(P, S, s, which, chain) : mx_one_pass<7>(P, S, s, which, chain);
   if (S.walk.linear)
     return S.fixed == 8 ? mx_pass<8, 1>(P, S, lat, energy, s, which, smem, chain)
                         : mx_pass<7, 1>(P, S, lat, energy, s, which, smem, chain);
