@@ -218,6 +218,7 @@ struct Shells64 {
 };
 struct Plan64 {
   bool ok; // the stencil and tables suit the shell-window and entry-split kernels
+  bool entries; // every entry is tested, items are always split (plan64_entries); no site list
   bool chain; // launches join the chain of a resident step (launch_chained)
   Shells64 sh;
   int *sites; // site list of the work items
@@ -226,6 +227,7 @@ struct Plan64 {
 struct StencilSet;
 bool plan64_shells(const DevPot &P, const Geom &g, double a0, double cutoff, const double *R, const StencilSet &st,
                    Shells64 &S);
+bool plan64_entries(const StencilSet &st, Shells64 &S);
 int plan64_plane_items(const Geom &g); // work items of one (z, sublattice) plane
 int plan64_items(const Geom &g);       // ... of the box
 int plan64_sites(const Geom &g, int *sites, cudaStream_t s);

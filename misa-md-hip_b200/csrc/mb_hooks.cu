@@ -115,15 +115,33 @@ static int require_ready(const HookCtx &c) {
   return MB_OK;
 }
 
+// Passes over boxes of up to this many work items per SM split each item over several warps
+// (mb_split64.cu); larger ones take the row walk, whose pass costs 45 us however few items a
+// slab has.  Measured on one B200, pass with copies, split / rows: 12 x 14 x 16 cells 0.105 /
+// 0.133 ms, 30 x 27 x 33 (11 items per SM) 0.36 / 0.38 in one piece and 0.31 / 0.38 in four
+// slabs, 44 x 40 x 48 (36 per SM) 0.70 / 0.69.  The line looks at the whole box, not at the
+// slab, so that every slab count gives the same bits.  MB_HOOK_SPLIT_ITEMS overrides it (0:
+// never).
+#define MB_HOOK_SPLIT_ITEMS 24
+static Plan64 hook_plan(const HookCtx &c) {
+  Plan64 plan{};
+  int per_sm = MB_HOOK_SPLIT_ITEMS;
+  if (const char *v = getenv("MB_HOOK_SPLIT_ITEMS")) per_sm = atoi(v);
+  plan.entries = plan64_entries(c.st, plan.sh) && (long long)plan64_items(c.g) <= (long long)per_sm * device_sm_count();
+  plan.ok = plan.entries;
+  return plan;
+}
+
 // Slabs of a streamed hook pass: the -b/--batches count when the host set one above 1,
 // else as many as give each slab at least 4 MiB of records, at most 16 (measured on
-// 128^3 cells: 16 slabs 11.0 ms per pass, 32 slabs 11.4, 8 slabs 11.3, one piece 18.5);
-// never more than one per box layer; 1 = one piece.
-static int hook_slabs(const HookCtx &c) {
+// 128^3 cells: 16 slabs 11.0 ms per pass, 32 slabs 11.4, 8 slabs 11.3, one piece 18.5), or
+// 1.75 MiB when items are split (a slab then costs 25 us besides its copies: 8.1 MB in 1 / 2 /
+// 4 / 6 slabs 0.36 / 0.33 / 0.31 / 0.32 ms); never more than one per box layer; 1 = one piece.
+static int hook_slabs(const HookCtx &c, bool split) {
   const mb_device_domain &d = c.dom;
   if (d.ext_size_z != d.box_size_z + 2 * d.ghost_size_z) return 1;
   long long n = c.batches > 1 ? (long long)c.batches
-                              : std::min<long long>(16, (long long)(c.n_ext * sizeof(mb_atom_element) / (4u << 20)));
+                              : std::min<long long>(16, (long long)(c.n_ext * sizeof(mb_atom_element) / (split ? 7u << 18 : 4u << 20)));
   n = std::min<long long>(std::min<long long>(n, MB_HOOK_SLAB_MAX), d.box_size_z);
   return n < 2 ? 1 : (int)n;
 }
@@ -132,7 +150,7 @@ static int hook_slabs(const HookCtx &c) {
 // copy the box rows out; in z-slabs when `sliced` and more than one slab is planned.
 // kernel_ms / copy_ms: the span of the device work, and the rest of the call.
 template <class Body>
-static int run_hook(HookCtx &c, mb_atom_element *atoms, int with_df, int pack_what, bool sliced, Body body) {
+static int run_hook(HookCtx &c, mb_atom_element *atoms, int with_df, int pack_what, bool sliced, bool split, Body body) {
   if (!atoms) return fail(MB_ERR_ARG, "null atoms array");
   MB_TRY(require_ready(c));
   MB_TRY(ensure_buffers(c));
@@ -143,7 +161,7 @@ static int run_hook(HookCtx &c, mb_atom_element *atoms, int with_df, int pack_wh
   auto row1 = [&](int z) { return row0(z) + ((size_t)d.box_size_y - 1) * ex + d.box_size_x - 1; };
   cudaStream_t s = c.stream;
   const int n_types = pot_dev(c.potp).n_types;
-  const int nsl = sliced ? hook_slabs(c) : 1;
+  const int nsl = sliced ? hook_slabs(c, split) : 1;
   MB_CUDA(cudaMemsetAsync(c.bad, 0, sizeof(int), s));
   MB_CUDA(cudaEventRecord(c.ev[0], s));
   Lattice64 L = lattice_view(c);
@@ -402,8 +420,10 @@ int mb_eam_rho_calc(mb_atom_element *atoms, double cutoff_radius) {
   HookCtx &c = g_ctx;
   if (!(cutoff_radius > 0)) return fail(MB_ERR_ARG, "cutoff must be > 0");
   if (c.half) return run_half(c, atoms, false, cutoff_radius * cutoff_radius);
-  return run_hook(c, atoms, 0, 1, true, [&](Lattice64 &L, cudaStream_t s, int z0, int z1) {
-    return launch_rho64(c.g, c.st, pot_dev(c.potp), L, cutoff_radius * cutoff_radius, nullptr, 0, 0, s, z0, z1);
+  const Plan64 plan = hook_plan(c);
+  return run_hook(c, atoms, 0, 1, true, plan.entries, [&](Lattice64 &L, cudaStream_t s, int z0, int z1) {
+    return launch_rho64(c.g, c.st, pot_dev(c.potp), L, cutoff_radius * cutoff_radius, nullptr, 0, 0, s, z0, z1, nullptr,
+                        &plan);
   });
 }
 
@@ -417,7 +437,7 @@ int mb_eam_df_calc(mb_atom_element *atoms, double cutoff_radius) {
   std::lock_guard<std::mutex> lk(g_mu);
   HookCtx &c = g_ctx;
   if (!c.half) return require_ready(c);
-  return run_hook(c, atoms, 2, 3, false, [&](Lattice64 &L, cudaStream_t s, int, int) {
+  return run_hook(c, atoms, 2, 3, false, false, [&](Lattice64 &L, cudaStream_t s, int, int) {
     return launch_df_from_rho(c.g, pot_dev(c.potp), L, s);
   });
 }
@@ -425,7 +445,7 @@ int mb_eam_df_calc(mb_atom_element *atoms, double cutoff_radius) {
 int mb_eam_df_from_rho(mb_atom_element *atoms) {
   std::lock_guard<std::mutex> lk(g_mu);
   HookCtx &c = g_ctx;
-  return run_hook(c, atoms, 2, 3, false, [&](Lattice64 &L, cudaStream_t s, int, int) {
+  return run_hook(c, atoms, 2, 3, false, false, [&](Lattice64 &L, cudaStream_t s, int, int) {
     return launch_df_from_rho(c.g, pot_dev(c.potp), L, s);
   });
 }
@@ -436,12 +456,13 @@ int mb_eam_force_calc(mb_atom_element *atoms, double cutoff_radius) {
   HookCtx &c = g_ctx;
   if (!(cutoff_radius > 0)) return fail(MB_ERR_ARG, "cutoff must be > 0");
   if (c.half) return run_half(c, atoms, true, cutoff_radius * cutoff_radius);
-  return run_hook(c, atoms, 1, 2, true, [&](Lattice64 &L, cudaStream_t s, int z0, int z1) {
+  const Plan64 plan = hook_plan(c);
+  return run_hook(c, atoms, 1, 2, true, plan.entries, [&](Lattice64 &L, cudaStream_t s, int z0, int z1) {
     StepParams sp{};
     sp.rc2 = cutoff_radius * cutoff_radius;
     Lattice64 Lf = L;
     Lf.vx = Lf.vy = Lf.vz = nullptr; // forces only, no integration in drop-in mode
-    return launch_force64(c.g, c.st, pot_dev(c.potp), Lf, sp, nullptr, 0, 0, s, z0, z1);
+    return launch_force64(c.g, c.st, pot_dev(c.potp), Lf, sp, nullptr, 0, 0, s, z0, z1, nullptr, &plan);
   });
 }
 
@@ -585,7 +606,10 @@ extern "C" int mb_eam_rho_calc_noalloc(mb_atom_element *atoms, double cutoff_rad
     return e == cudaSuccess ? MB_OK : cuda_fail(e, "cudaStreamSynchronize");
   };
   int rc = launch_unpack_ext(c.g, aos, d.ext_size_x, d.ext_size_y, d.ext_size_z, L, 0, bad, pot_dev(c.potp).n_types, s);
-  if (rc == MB_OK) rc = launch_rho64(c.g, c.st, pot_dev(c.potp), L, cutoff_radius * cutoff_radius, nullptr, 0, 0, s);
+  const Plan64 plan = hook_plan(c);
+  if (rc == MB_OK)
+    rc = launch_rho64(c.g, c.st, pot_dev(c.potp), L, cutoff_radius * cutoff_radius, nullptr, 0, 0, s, 0, -1, nullptr,
+                      &plan);
   int flag = 0;
   if (rc == MB_OK && cudaMemcpyAsync(&flag, bad, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess)
     rc = cuda_fail(cudaGetLastError(), "cudaMemcpyAsync");

@@ -566,7 +566,7 @@ int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const L
     if (z0 < 0 || z0 >= z1 || z1 > g.bz) return z0 == z1 ? MB_OK : fail(MB_ERR_ARG, "z-slab outside the box");
     LatticeArgs a = lattice_args(g, pot, L, rc2, flag, outer, *plan, z0, z1);
     a.e0 = e_partial;
-    if (split_launch("MB_SPLIT_RHO_ITEMS", MB_SPLIT_RHO_ITEMS, MB_MULTI_SPLIT_RHO_ITEMS, a))
+    if (plan->entries || split_launch("MB_SPLIT_RHO_ITEMS", MB_SPLIT_RHO_ITEMS, MB_MULTI_SPLIT_RHO_ITEMS, a))
       return launch_split_rho64(st, a, energy, s);
     return launch_shell_rho64(st, a, energy, s);
   }
@@ -620,7 +620,7 @@ int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const
     a.sp = sp;
     a.e0 = e_partial ? e_partial + MB_EPART_CAP : nullptr;
     a.e1 = e_partial ? e_partial + 2 * MB_EPART_CAP : nullptr;
-    if (split_launch("MB_SPLIT_FORCE_ITEMS", MB_SPLIT_FORCE_ITEMS, MB_MULTI_SPLIT_FORCE_ITEMS, a))
+    if (plan->entries || split_launch("MB_SPLIT_FORCE_ITEMS", MB_SPLIT_FORCE_ITEMS, MB_MULTI_SPLIT_FORCE_ITEMS, a))
       return launch_split_force64(st, a, energy, s);
     return launch_shell_force64(st, a, energy, s);
   }

@@ -196,6 +196,17 @@ __device__ __forceinline__ double force_table64(const DevPot &P, double d2, int 
   return __dmul_rn(-g, rinv);
 }
 
+// Lane `lane`'s site of item w: index and MB_SITE_FACE, -1 past the end of the plane.
+__device__ __forceinline__ int site_ref64(const Geom &g, int w, int lane) {
+  const int cpp = (g.bcx * g.by + 31) / 32, p = w / cpp, b = (w - p * cpp) * 32 + lane;
+  const int y = b / g.bcx, cx = b - y * g.bcx, s = p & 1, z = p >> 1;
+  if (y >= g.by) return -1;
+  int ref = (int)ext_index(g, s, cx, y, z);
+  if (cx < g.gcx || cx >= g.bcx - g.gcx || y < g.gy || y >= g.by - g.gy || z < g.gz || z >= g.bz - g.gz)
+    ref |= MB_SITE_FACE;
+  return ref;
+}
+
 // A site at work: its record and code, F' and stencil offsets.
 struct Site64 {
   const double4 *p;  // its record
@@ -281,19 +292,27 @@ __device__ __forceinline__ double rho_outer(const LatticeArgs &a, const Site64 &
   return t;
 }
 
-// The outer entries [k0, k1) of a force whose bit k - k0 of `bits` is set (the others are
-// beyond the cutoff for every lane of the item).
+// The outer entries [k0, k1) of a force: those whose bit k - k0 of `bits` is set (the others
+// are beyond the cutoff for every lane of the item), or all (`all`).
 template <bool ENERGY>
-__device__ __forceinline__ void force_outer(const LatticeArgs &a, const Site64 &c, int k0, int k1, unsigned bits,
-                                            double &fx, double &fy, double &fz, double &ep) {
+__device__ __forceinline__ void force_outer(const LatticeArgs &a, const Site64 &c, int k0, int k1, bool all,
+                                            unsigned bits, double &fx, double &fy, double &fz, double &ep) {
   fx = fy = fz = 0.0;
-  bits &= (1u << (k1 - k0)) - 1u;
   unsigned in = 0;
-  while (bits) {
-    const int b = __ffs(bits) - 1;
-    bits &= bits - 1;
-    const double4 q = ld_site(c.p + c.off[k0 + b]);
-    in |= (unsigned)(len2(c.x - q.x, c.y - q.y, c.z - q.z) < a.rc2) << b;
+  if (all) {
+#pragma unroll 4
+    for (int k = k0; k < k1; k++) {
+      const double4 q = ld_site(c.p + c.off[k]);
+      in |= (unsigned)(len2(c.x - q.x, c.y - q.y, c.z - q.z) < a.rc2) << (k - k0);
+    }
+  } else {
+    bits &= (1u << (k1 - k0)) - 1u;
+    while (bits) {
+      const int b = __ffs(bits) - 1;
+      bits &= bits - 1;
+      const double4 q = ld_site(c.p + c.off[k0 + b]);
+      in |= (unsigned)(len2(c.x - q.x, c.y - q.y, c.z - q.z) < a.rc2) << b;
+    }
   }
   force_far<ENERGY>(a, c, k0, in, fx, fy, fz, ep);
 }

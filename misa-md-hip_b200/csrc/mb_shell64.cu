@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(COPIES > 0 ? MB_SHELL_FORCE_THREADS : MB_MULTI
             const unsigned bits = (unsigned)(mask >> (k0 - n_near)) & ((1u << MB_OUT_RUN) - 1u);
             if (!bits) continue;
             double tx, ty, tz;
-            force_outer<ENERGY>(a, c, k0, min(k0 + MB_OUT_RUN, st.n), bits, tx, ty, tz, e_pair);
+            force_outer<ENERGY>(a, c, k0, min(k0 + MB_OUT_RUN, st.n), false, bits, tx, ty, tz, e_pair);
             fx = __dadd_rn(fx, tx);
             fy = __dadd_rn(fy, ty);
             fz = __dadd_rn(fz, tz);
@@ -373,17 +373,8 @@ static bool shell_window(const DevPot &P, double cutoff, double r0, double r1, i
 
 __global__ void k_site_list(const Geom g, int cpp, int *sites) {
   const long long n = 64LL * g.bz * cpp;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int p = (int)(t / (32LL * cpp)), b = (int)(t - (long long)p * 32 * cpp);
-    const int y = b / g.bcx, cx = b - y * g.bcx, s = p & 1, z = p >> 1;
-    int ref = -1;
-    if (y < g.by) {
-      ref = (int)ext_index(g, s, cx, y, z);
-      if (cx < g.gcx || cx >= g.bcx - g.gcx || y < g.gy || y >= g.by - g.gy || z < g.gz || z >= g.bz - g.gz)
-        ref |= MB_SITE_FACE;
-    }
-    sites[t] = ref;
-  }
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
+    sites[t] = site_ref64(g, (int)(t >> 5), (int)(t & 31));
 }
 
 int plan64_items(const Geom &g) { return 2 * g.bz * plan64_plane_items(g); }

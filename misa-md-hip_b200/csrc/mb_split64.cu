@@ -36,7 +36,7 @@ struct SplitSite {
 };
 __device__ __forceinline__ SplitSite split_site(const StencilSet &st, const LatticeArgs &a, int w) {
   SplitSite t;
-  t.ref = __ldg(a.sites + 32 * (size_t)w + (threadIdx.x & 31));
+  t.ref = a.sites ? __ldg(a.sites + 32 * (size_t)w + (threadIdx.x & 31)) : site_ref64(a.g, w, threadIdx.x & 31);
   const int i = t.ref & MB_SITE_INDEX;
   const int code = t.ref < 0 ? -1 : a.L.code[i];
   t.code = code;
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
   for (int w = w0; w < a.n_items; w += gridDim.x * MB_SPLIT_GROUPS, turn++) {
     double *sum = sums + (turn & 1) * a.sh.runs * 96;
     const SplitSite t = split_site(st, a, w);
-    unsigned long long mask = ~0ull;
+    unsigned long long mask = 0;
     if (a.outer) {
       const uint2 m2 = a.outer[w];
       mask = (unsigned long long)m2.x | ((unsigned long long)m2.y << 32);
@@ -165,11 +165,12 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
           unsigned far = 0;
 #pragma unroll 4
           for (int k = k0; k < k1; k++)
-            force_near<COPIES, ENERGY>(a, W, t.c, ld_site(t.c.p + t.c.off[k]), split_type<COPIES>(t.c, k, a.P.n_types), k - k0, fx, fy,
-                                       fz, e_pair, far);
+            force_near<COPIES, ENERGY>(a, W, t.c, ld_site(t.c.p + t.c.off[k]),
+                                       split_type<COPIES>(t.c, k, a.P.n_types), k - k0, fx, fy, fz, e_pair, far);
           force_far<ENERGY>(a, t.c, k0, far, fx, fy, fz, e_pair);
         } else {
-          force_outer<ENERGY>(a, t.c, k0, k1, (unsigned)(mask >> (k0 - a.sh.kb[a.sh.near_runs])), fx, fy, fz, e_pair);
+          const unsigned bits = a.outer ? (unsigned)(mask >> (k0 - a.sh.kb[a.sh.near_runs])) : 0u;
+          force_outer<ENERGY>(a, t.c, k0, k1, !a.outer, bits, fx, fy, fz, e_pair);
         }
       }
       sum[r * 96] = fx;
@@ -198,6 +199,10 @@ __global__ void __launch_bounds__(MB_SPLIT_THREADS, 1)
 
 static void table_range(const Windows64 &w, int n, int &lo, int &knots) {
   int hi = 0;
+  if (n == 0) { // an entry plan: no windows
+    lo = knots = 0;
+    return;
+  }
   lo = 1 << 30;
   for (int h = 0; h < n; h++) {
     lo = w.lo[h] < lo ? w.lo[h] : lo;
@@ -218,6 +223,16 @@ static int smem_knots(int knots, int words, size_t used, int most) {
 static int split_grid(const LatticeArgs &a) {
   const int grid = (a.n_items - a.w0 + MB_SPLIT_GROUPS - 1) / MB_SPLIT_GROUPS;
   return grid < device_sm_count() ? grid : device_sm_count();
+}
+
+// Plan of a stencil in no order and of no known lattice (the hooks): every entry is tested,
+// MB_OUT_RUN to a run, and the tables are read where they lie.
+bool plan64_entries(const StencilSet &st, Shells64 &S) {
+  if (st.n < 1 || st.n > MB_OUT_RUN * MB_RUNS_MAX) return false;
+  S = Shells64{};
+  for (int k = 0; k < st.n; k += MB_OUT_RUN) S.kb[S.runs++] = (short)k;
+  S.kb[S.runs] = (short)st.n;
+  return true;
 }
 
 // Whether the entry-split kernels take the plan's tables.
