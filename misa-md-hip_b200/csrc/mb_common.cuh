@@ -333,8 +333,7 @@ int launch_images64(const Geom &g, const Lattice64 &L, int what, cudaStream_t s,
 // [1] recombinations, [2] refused conversions (list full), [3] dropped candidates.
 int launch_convert64(const Geom &g, const Lattice64 &L, const Itl64 &I, const StepParams &sp, double rec2,
                      int64_t *site_id, int *nd, long long *counters, cudaStream_t s);
-int launch_kick_drift64(const Geom &g, const Lattice64 &L, const Itl64 &I, const StepParams &sp, cudaStream_t s,
-                        int z0 = 0, int z1 = -1, int with_itl = 1);
+int launch_itl_kick_drift64(const Itl64 &I, const StepParams &sp, cudaStream_t s);
 int launch_reduce(const double *partials, int n, double *out, cudaStream_t s);
 int energy_partials_needed();
 
@@ -350,6 +349,12 @@ int launch_unpack_box(const Geom &g, const mb_atom_element *aos, Lattice64 L, in
                       int n_types, cudaStream_t s);
 int launch_pack_box(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double4 *pos, double h, int unkick,
                     cudaStream_t s);
+// Records of a host step as they arrive: unpacked, kicked and drifted, ghost images written.
+int launch_arrive64(const Geom &g, const mb_atom_element *aos, const Lattice64 &L, const StepParams &sp, int *bad_type,
+                    int64_t *ids, int n_types, cudaStream_t s, int z0 = 0, int z1 = -1);
+// Interstitial records in (setting the device count) and out.
+int launch_unpack_itl(const Itl64 &I, const mb_atom_element *aos, int n, int *nd, cudaStream_t s);
+int launch_pack_itl(const Itl64 &I, mb_atom_element *aos, int n, double h, int unkick, cudaStream_t s);
 int launch_unpack_box_ids(const Geom &g, const mb_atom_element *aos, Lattice64 L, int with_f, int *bad_type,
                           int64_t *ids, int n_types, cudaStream_t s, int z0 = 0, int z1 = -1);
 int launch_pack_box_ids(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double4 *pos, double h,

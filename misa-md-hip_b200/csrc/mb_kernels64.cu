@@ -21,6 +21,7 @@
 //  * sites near the domain faces write their periodic ghost images themselves
 //    (no separate ghost-exchange pass), and the force pass closes the previous
 //    velocity-Verlet step and drifts to the next positions (double-buffered).
+#include <algorithm>
 #include <limits.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -1200,60 +1201,24 @@ int launch_images64(const Geom &g, const Lattice64 &L, int what, cudaStream_t s,
   return MB_OK;
 }
 
-// First half of a velocity-Verlet step in place (used when the state arrives
-// from the host each step): v += h f ; x += dt v, then refresh ghost images.
-// Lattice sites [t0, t1) (numbered as in k_images64), then the interstitials when
-// with_itl is set.
-__global__ void k_kick_drift64(const Geom g, const Lattice64 L, const Itl64 I, const StepParams sp, long long t0,
-                               long long t1, int with_itl) {
-  const long long n = t1 - t0;
-  const int n_itl = with_itl ? itl_n(I) : 0;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n + n_itl;
-       q += (long long)gridDim.x * blockDim.x) {
-    const long long t = t0 + q;
-    if (q >= n) {
-      const int it = (int)(q - n);
-      I.vx[it] += sp.h * I.fx[it];
-      I.vy[it] += sp.h * I.fy[it];
-      I.vz[it] += sp.h * I.fz[it];
-      I.px[it] += sp.dt * I.vx[it];
-      I.py[it] += sp.dt * I.vy[it];
-      I.pz[it] += sp.dt * I.vz[it];
-      continue;
-    }
-    const int cx = (int)(t % g.bcx);
-    long long r = t / g.bcx;
-    const int y = (int)(r % g.by);
-    r /= g.by;
-    const int s = (int)(r & 1);
-    const int z = (int)(r >> 1);
-    const long long i = ext_index(g, s, cx, y, z);
-    if (L.code[i] < 0) continue;
-    const double vx = L.vx[i] + sp.h * L.fx[i], vy = L.vy[i] + sp.h * L.fy[i], vz = L.vz[i] + sp.h * L.fz[i];
-    const double x0 = L.p[i].x + sp.dt * vx, y0 = L.p[i].y + sp.dt * vy, z0 = L.p[i].z + sp.dt * vz;
-    L.vx[i] = vx;
-    L.vy[i] = vy;
-    L.vz[i] = vz;
-    L.p[i].x = x0;
-    L.p[i].y = y0;
-    L.p[i].z = z0;
-    for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
-      L.p[idx].x = x0 + ox;
-      L.p[idx].y = y0 + oy;
-      L.p[idx].z = z0 + oz;
-    });
+// First half of a velocity-Verlet step of the interstitials in place (used when the state
+// arrives from the host each step): v += h f ; x += dt v.
+__global__ void k_itl_kick_drift64(const Itl64 I, const StepParams sp) {
+  const int n = itl_n(I);
+  for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n; it += gridDim.x * blockDim.x) {
+    I.vx[it] += sp.h * I.fx[it];
+    I.vy[it] += sp.h * I.fy[it];
+    I.vz[it] += sp.h * I.fz[it];
+    I.px[it] += sp.dt * I.vx[it];
+    I.py[it] += sp.dt * I.vy[it];
+    I.pz[it] += sp.dt * I.vz[it];
   }
 }
 
-int launch_kick_drift64(const Geom &g, const Lattice64 &L, const Itl64 &I, const StepParams &sp, cudaStream_t s,
-                        int z0, int z1, int with_itl) {
-  if (z1 < 0) z1 = g.bz;
-  const long long layer = 2LL * g.bcx * g.by;
-  const long long n = layer * (z1 - z0) + (with_itl ? (I.nd ? I.cap : I.n) : 0);
+int launch_itl_kick_drift64(const Itl64 &I, const StepParams &sp, cudaStream_t s) {
+  const int n = I.nd ? I.cap : I.n;
   if (n <= 0) return MB_OK;
-  int grid = (int)((n + 255) / 256);
-  if (grid > 8 * device_sm_count()) grid = 8 * device_sm_count();
-  k_kick_drift64<<<grid, 256, 0, s>>>(g, L, I, sp, layer * z0, layer * z1, with_itl);
+  k_itl_kick_drift64<<<std::min((n + 255) / 256, 8 * device_sm_count()), 256, 0, s>>>(I, sp);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }

@@ -2,6 +2,7 @@
 // reference's _cuAtomElement, src/kernel_types.h:40-48) and the device's
 // sublattice-split SoA arrays.
 #include "mb_common.cuh"
+#include "mb_device.cuh"
 
 namespace mb {
 
@@ -96,6 +97,88 @@ __global__ void k_unpack_box(const Geom g, const mb_atom_element *aos, Lattice64
     }
     if (ids) ids[t] = a.id;
   }
+}
+
+// Records [t0, t1) of a host step as they arrive: unpacked, the first half of a
+// velocity-Verlet step (v += h f ; x += dt v) and the ghost images, in one pass over the
+// records.  Bound by the record reads (104 bytes of which every sector is used); as three
+// kernels the step's slabs took two launches and 190 bytes per site more.
+__global__ void k_arrive64(const Geom g, const mb_atom_element *aos, const Lattice64 L, const StepParams sp,
+                           int *bad_type, int64_t *ids, int n_types, long long t0, long long t1) {
+  const int bxd = 2 * g.bcx;
+  for (long long t = t0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; t < t1;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int bx = (int)(t % bxd);
+    const long long r = t / bxd;
+    const int y = (int)(r % g.by), z = (int)(r / g.by), s = bx & 1, cx = bx >> 1;
+    const long long i = ext_index(g, s, cx, y, z);
+    const mb_atom_element &a = aos[t];
+    int type = a.type;
+    if (type >= n_types) { // no table for it: flagged, and kept out of the pair loops
+      *bad_type = 1;
+      type = -1;
+    }
+    const bool vac = type < 0;
+    const int8_t code = (int8_t)(vac ? -1 : type);
+    double p[3], v[3], f[3];
+    for (int k = 0; k < 3; k++) {
+      f[k] = vac ? 0.0 : a.f[k];
+      v[k] = vac ? 0.0 : a.v[k] + sp.h * f[k];
+      p[k] = vac ? MB_VACANT_POS : a.x[k] + sp.dt * v[k];
+    }
+    L.code[i] = code;
+    st_site(L.p + i, p[0], p[1], p[2], 0.0);
+    L.vx[i] = v[0];
+    L.vy[i] = v[1];
+    L.vz[i] = v[2];
+    L.fx[i] = f[0];
+    L.fy[i] = f[1];
+    L.fz[i] = f[2];
+    ids[t] = a.id;
+    for_images(g, s, cx, y, z, [&](long long idx, double ox, double oy, double oz) {
+      st_site(L.p + idx, p[0] + ox, p[1] + oy, p[2] + oz, 0.0);
+      L.code[idx] = code;
+    });
+  }
+}
+
+__global__ void k_unpack_itl(const Itl64 I, const mb_atom_element *aos, int n, int *nd) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k == 0) *nd = n;
+  if (k >= n) return;
+  const mb_atom_element &a = aos[k];
+  I.px[k] = a.x[0];
+  I.py[k] = a.x[1];
+  I.pz[k] = a.x[2];
+  I.vx[k] = a.v[0];
+  I.vy[k] = a.v[1];
+  I.vz[k] = a.v[2];
+  I.fx[k] = a.f[0];
+  I.fy[k] = a.f[1];
+  I.fz[k] = a.f[2];
+  I.type[k] = (int8_t)a.type;
+  I.id[k] = a.id;
+}
+
+__global__ void k_pack_itl(const Itl64 I, mb_atom_element *aos, int n, double h, int unkick) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  mb_atom_element a;
+  a.id = I.id[k];
+  a.type = I.type[k];
+  a.pad_ = 0;
+  a.x[0] = I.px[k];
+  a.x[1] = I.py[k];
+  a.x[2] = I.pz[k];
+  a.f[0] = I.fx[k];
+  a.f[1] = I.fy[k];
+  a.f[2] = I.fz[k];
+  a.v[0] = I.vx[k] - (unkick ? h * a.f[0] : 0.0);
+  a.v[1] = I.vy[k] - (unkick ? h * a.f[1] : 0.0);
+  a.v[2] = I.vz[k] - (unkick ? h * a.f[2] : 0.0);
+  a.rho = I.rho[k];
+  a.df = I.df[k];
+  aos[k] = a;
 }
 
 // Box-order records of the synchronised state.  pos: positions and F' of the step; unkick: v is stored half a step ahead and is brought back by h*f.
@@ -203,6 +286,29 @@ int launch_unpack_box_ids(const Geom &g, const mb_atom_element *aos, Lattice64 L
   if (z1 <= z0) return MB_OK;
   k_unpack_box<<<flat_grid(layer * (z1 - z0)), 256, 0, s>>>(g, aos, L, with_f, bad_type, ids, n_types, layer * z0,
                                                              layer * z1);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
+int launch_arrive64(const Geom &g, const mb_atom_element *aos, const Lattice64 &L, const StepParams &sp, int *bad_type,
+                    int64_t *ids, int n_types, cudaStream_t s, int z0, int z1) {
+  if (z1 < 0) z1 = g.bz;
+  const long long layer = 2LL * g.bcx * g.by;
+  if (z1 <= z0) return MB_OK;
+  k_arrive64<<<flat_grid(layer * (z1 - z0)), 256, 0, s>>>(g, aos, L, sp, bad_type, ids, n_types, layer * z0,
+                                                           layer * z1);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
+int launch_unpack_itl(const Itl64 &I, const mb_atom_element *aos, int n, int *nd, cudaStream_t s) {
+  k_unpack_itl<<<(n + 127) / 128, 128, 0, s>>>(I, aos, n, nd);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
+int launch_pack_itl(const Itl64 &I, mb_atom_element *aos, int n, double h, int unkick, cudaStream_t s) {
+  k_pack_itl<<<(n + 127) / 128, 128, 0, s>>>(I, aos, n, h, unkick);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }

@@ -44,6 +44,7 @@ struct mb_sim {
   double *ipos[2][3] = {}, *iv[3] = {}, *ifr[3] = {}, *irho = nullptr, *idf = nullptr;
   int8_t *itype = nullptr;
   int64_t *iid = nullptr;
+  mb_atom_element *istage = nullptr; // interstitial records on their way in or out
   int *flag_list = nullptr, *flag_count = nullptr; // a list per buffer; counts [2], overflow
   int flag_last = -1;                              // buffer of the last step with interstitial passes
   int *d_nitl = nullptr; // device-resident interstitial count (conversions change it)
@@ -165,6 +166,12 @@ StepParams sim_params(const mb_sim *s, int kick_pre, int drift) {
 // them (the count itself lives on the device).
 static bool itl_active(const mb_sim *s) { return s->n_itl > 0 || s->conv_d > 0.0; }
 
+static Plan64 chained_plan(const mb_sim *s) {
+  Plan64 plan = s->plan;
+  plan.chain = chain_on();
+  return plan;
+}
+
 // One FP64 step at positions pos[cur] (forces, closing kick, drift to pos[cur^1]).
 static int step64(mb_sim *s, int energy, int kick_pre, int drift, int timed) {
   const DevPot &P = pot_dev(s->pot);
@@ -174,9 +181,9 @@ static int step64(mb_sim *s, int energy, int kick_pre, int drift, int timed) {
   double *ep = energy ? s->epart : nullptr;
   if (energy) MB_CUDA(cudaMemsetAsync(s->epart, 0, sizeof(double) * energy_partials_needed(), s->stream));
   const int itl = itl_active(s), flag = itl ? I.flag : 0;
-  const bool chain = !timed && chain_on();
-  Plan64 plan = s->plan;
-  plan.chain = chain;
+  Plan64 plan = chained_plan(s);
+  if (timed) plan.chain = false; // events take the kernels one by one
+  const bool chain = plan.chain;
   if (itl) {
     // a step after one at the other buffer clears that one's marks; any other state of the
     // lists (a first step, interstitials that come back) starts from empty ones
@@ -488,6 +495,7 @@ static int create_sim(const mb_sim_config *cfg, const mb_eam_tables *pot, int z_
   if ((rc = dalloc(s, (void **)&s->idf, ci * sizeof(double))) != MB_OK) return cleanup(rc);
   if ((rc = dalloc(s, (void **)&s->itype, ci)) != MB_OK) return cleanup(rc);
   if ((rc = dalloc(s, (void **)&s->iid, ci * sizeof(int64_t))) != MB_OK) return cleanup(rc);
+  if ((rc = dalloc(s, (void **)&s->istage, ci * sizeof(mb_atom_element))) != MB_OK) return cleanup(rc);
   // sites in reach of one interstitial: the window sphere holds < 2 * (4/3 pi R^3) / (a0^3 / 2)
   const double R = reach;
   const int per = (int)(2.0 * 4.18879 * R * R * R / (0.5 * pow(cfg->lattice_const, 3))) + 64;
@@ -523,7 +531,7 @@ int mb_sim_destroy(mb_sim *s) {
   drop_graph(s);
   if (s->ens) mb_ensemble_destroy(s->ens);
   void *ptrs[] = {s->code, s->rho, s->outer, s->plan.sites, s->id, s->epart, s->eout, s->stage, s->bad, s->irho, s->idf, s->itype,
-                  s->iid, s->flag_list, s->flag_count, s->d_nitl, s->d_cand, s->d_cand_n, s->d_conv_counters};
+                  s->iid, s->istage, s->flag_list, s->flag_count, s->d_nitl, s->d_cand, s->d_cand_n, s->d_conv_counters};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (int b = 0; b < 2; b++) {
@@ -572,73 +580,31 @@ static int ensure_stage(mb_sim *s, size_t n) {
   return MB_OK;
 }
 
-static int upload_itl(mb_sim *s, const mb_atom_element *itl, int32_t n_itl, int with_f) {
+// Interstitial records to the device: one copy and one kernel, queued on the stream (the
+// caller's records may be in use until it is synchronised).
+static int upload_itl(mb_sim *s, const mb_atom_element *itl, int32_t n_itl) {
   if (n_itl < 0 || n_itl > s->cap_itl) return fail(MB_ERR_ARG, "n_itl exceeds max_interstitials");
   if (n_itl > 0 && !itl) return fail(MB_ERR_ARG, "null interstitial array");
-  s->n_itl = n_itl;
-  MB_CUDA(cudaStreamSynchronize(s->stream));
-  MB_CUDA(cudaMemcpy(s->d_nitl, &s->n_itl, sizeof(int), cudaMemcpyHostToDevice));
-  MB_CUDA(cudaMemsetAsync(s->d_cand_n, 0, sizeof(int), s->stream));
-  if (n_itl == 0) return MB_OK;
-  std::vector<double> buf((size_t)n_itl);
-  std::vector<int8_t> t((size_t)n_itl);
-  std::vector<int64_t> ids((size_t)n_itl);
-  for (int k = 0; k < n_itl; k++) {
+  for (int k = 0; k < n_itl; k++)
     if (itl[k].type < 0 || itl[k].type >= pot_dev(s->pot).n_types)
       return fail(MB_ERR_ARG, "interstitial type without a potential table");
-    t[k] = (int8_t)itl[k].type;
-    ids[k] = itl[k].id;
-  }
-  auto put = [&](double *dst, auto get) -> int {
-    for (int k = 0; k < n_itl; k++) buf[k] = get(itl[k]);
-    MB_CUDA(cudaMemcpyAsync(dst, buf.data(), sizeof(double) * n_itl, cudaMemcpyHostToDevice, s->stream));
-    MB_CUDA(cudaStreamSynchronize(s->stream));
+  s->n_itl = n_itl;
+  MB_CUDA(cudaMemsetAsync(s->d_cand_n, 0, sizeof(int), s->stream));
+  if (n_itl == 0) {
+    MB_CUDA(cudaMemsetAsync(s->d_nitl, 0, sizeof(int), s->stream));
     return MB_OK;
-  };
-  for (int c = 0; c < 3; c++) {
-    MB_TRY(put(s->ipos[s->cur][c], [c](const mb_atom_element &a) { return a.x[c]; }));
-    MB_TRY(put(s->iv[c], [c](const mb_atom_element &a) { return a.v[c]; }));
-    MB_TRY(put(s->ifr[c], [c, with_f](const mb_atom_element &a) { return with_f ? a.f[c] : 0.0; }));
   }
-  MB_CUDA(cudaMemcpyAsync(s->itype, t.data(), n_itl, cudaMemcpyHostToDevice, s->stream));
-  MB_CUDA(cudaMemcpyAsync(s->iid, ids.data(), sizeof(int64_t) * n_itl, cudaMemcpyHostToDevice, s->stream));
-  MB_CUDA(cudaStreamSynchronize(s->stream));
-  return MB_OK;
+  MB_CUDA(cudaMemcpyAsync(s->istage, itl, (size_t)n_itl * sizeof(mb_atom_element), cudaMemcpyHostToDevice, s->stream));
+  return launch_unpack_itl(sim_itl(s, s->cur), s->istage, n_itl, s->d_nitl, s->stream);
 }
 
+// Positions of buffer `which`; unkick: see launch_pack_box_ids.
 static int download_itl(mb_sim *s, mb_atom_element *itl, int which, int unkick) {
   const int n = s->n_itl;
   if (n == 0) return MB_OK;
-  std::vector<double> x[3], v[3], f[3], rho(n), df(n);
-  std::vector<int8_t> t(n);
-  std::vector<int64_t> ids(n);
-  for (int c = 0; c < 3; c++) {
-    x[c].resize(n);
-    v[c].resize(n);
-    f[c].resize(n);
-    MB_CUDA(cudaMemcpyAsync(x[c].data(), s->ipos[which][c], sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream));
-    MB_CUDA(cudaMemcpyAsync(v[c].data(), s->iv[c], sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream));
-    MB_CUDA(cudaMemcpyAsync(f[c].data(), s->ifr[c], sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream));
-  }
-  MB_CUDA(cudaMemcpyAsync(rho.data(), s->irho, sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream));
-  MB_CUDA(cudaMemcpyAsync(df.data(), s->idf, sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream));
-  MB_CUDA(cudaMemcpyAsync(t.data(), s->itype, n, cudaMemcpyDeviceToHost, s->stream));
-  MB_CUDA(cudaMemcpyAsync(ids.data(), s->iid, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, s->stream));
+  MB_TRY(launch_pack_itl(sim_itl(s, which), s->istage, n, sim_params(s, 0, 0).h, unkick, s->stream));
+  MB_CUDA(cudaMemcpyAsync(itl, s->istage, (size_t)n * sizeof(mb_atom_element), cudaMemcpyDeviceToHost, s->stream));
   MB_CUDA(cudaStreamSynchronize(s->stream));
-  const double h = sim_params(s, 0, 0).h;
-  for (int k = 0; k < n; k++) {
-    mb_atom_element &a = itl[k];
-    a.id = ids[k];
-    a.type = t[k];
-    a.pad_ = 0;
-    for (int c = 0; c < 3; c++) {
-      a.x[c] = x[c][k];
-      a.f[c] = f[c][k];
-      a.v[c] = v[c][k] - (unkick ? h * f[c][k] : 0.0);
-    }
-    a.rho = rho[k];
-    a.df = df[k];
-  }
   return MB_OK;
 }
 
@@ -670,7 +636,8 @@ int mb_sim_upload(mb_sim *s, const mb_atom_element *box_atoms, const mb_atom_ele
   MB_CUDA(cudaMemcpyAsync(&bad, s->bad, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   MB_CUDA(cudaStreamSynchronize(s->stream));
   if (bad) return fail(MB_ERR_ARG, "atom type without a potential table");
-  MB_TRY(upload_itl(s, itl, n_itl, 1));
+  MB_TRY(upload_itl(s, itl, n_itl));
+  MB_CUDA(cudaStreamSynchronize(s->stream));
   return MB_OK;
 }
 
@@ -831,23 +798,27 @@ static int step_host_whole(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
                           s->stream));
   Lattice64 L = sim_lattice(s, 0);
   L.n = nullptr;
-  MB_TRY(launch_unpack_box_ids(s->g, s->stage, L, 1, s->bad, s->id, pot_dev(s->pot).n_types, s->stream));
-  MB_TRY(launch_images64(s->g, L, 1, s->stream));
-  MB_TRY(upload_itl(s, itl, n_itl, 1));
+  const int urc = upload_itl(s, itl, n_itl);
+  if (urc != MB_OK) {
+    cudaStreamSynchronize(s->stream); // the caller's records are not in use after a refusal
+    return urc;
+  }
   Itl64 I = sim_itl(s, 0);
   StepParams sp = sim_params(s, 1, 0);
-  MB_TRY(launch_kick_drift64(s->g, L, I, sp, s->stream));
   const DevPot &P = pot_dev(s->pot);
+  MB_TRY(launch_arrive64(s->g, s->stage, L, sp, s->bad, s->id, P.n_types, s->stream));
+  MB_TRY(launch_itl_kick_drift64(I, sp, s->stream));
   const int it = s->n_itl > 0, flag = it ? I.flag : 0;
   s->flag_last = -1;
   if (it) { // the records brought site codes without marks
     MB_CUDA(cudaMemsetAsync(s->flag_count, 0, 2 * sizeof(int), s->stream));
     MB_TRY(launch_itl_mark64(s->g, L, I, 0, s->stream));
   }
-  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, nullptr, 0, flag, s->stream, 0, -1, s->outer, &s->plan));
-  if (it) MB_TRY(launch_itl_rho64(s->g, P, L, I, sp.rc2, nullptr, 0, s->stream));
-  MB_TRY(launch_force64(s->g, s->st, P, L, sp, nullptr, 0, flag, s->stream, 0, -1, s->outer, &s->plan));
-  if (it) MB_TRY(launch_itl_force64(s->g, P, L, I, sp, nullptr, 0, s->stream));
+  const Plan64 plan = chained_plan(s);
+  MB_TRY(launch_rho64(s->g, s->st, P, L, sp.rc2, nullptr, 0, flag, s->stream, 0, -1, s->outer, &plan));
+  if (it) MB_TRY(launch_itl_rho64(s->g, P, L, I, sp.rc2, nullptr, 0, s->stream, 0, -1, plan.chain));
+  MB_TRY(launch_force64(s->g, s->st, P, L, sp, nullptr, 0, flag, s->stream, 0, -1, s->outer, &plan));
+  if (it) MB_TRY(launch_itl_force64(s->g, P, L, I, sp, nullptr, 0, s->stream, 0, -1, plan.chain));
   MB_TRY(launch_pack_box_ids(s->g, s->stage, L, L.p, sp.h, 0, s->id, s->stream));
   MB_CUDA(cudaMemcpyAsync(box_atoms, s->stage, (size_t)s->n_box * sizeof(mb_atom_element), cudaMemcpyDeviceToHost,
                           s->stream));
@@ -871,19 +842,15 @@ static int step_host_slabs(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
   const long long layer = 2LL * g.bcx * g.by; // records per box layer
   const size_t rec = sizeof(mb_atom_element);
   cudaStream_t cs = s->stream;
-  // the slabs start travelling at once (the stage is free: the last call ended synced) ...
+  // the interstitials first: behind the slabs their copy would wait for all of them
+  MB_TRY(upload_itl(s, itl, n_itl));
+  // the slabs start travelling at once (the stage is free: the last call ended synced)
   MB_CUDA(cudaEventRecord(s->ev_go, cs));
   MB_CUDA(cudaStreamWaitEvent(s->cp_in, s->ev_go, 0));
   for (int k = 0; k < n; k++) {
     const long long r0 = zb[k] * layer, r1 = zb[k + 1] * layer;
     MB_CUDA(cudaMemcpyAsync(s->stage + r0, box_atoms + r0, (size_t)(r1 - r0) * rec, cudaMemcpyHostToDevice, s->cp_in));
     MB_CUDA(cudaEventRecord(s->ev_in[k], s->cp_in));
-  }
-  // ... while the interstitials go up on the compute stream
-  const int urc = upload_itl(s, itl, n_itl, 1);
-  if (urc != MB_OK) {
-    cudaStreamSynchronize(s->cp_in); // the caller's records are not in use after a refusal
-    return urc;
   }
   Lattice64 L = sim_lattice(s, 0);
   L.n = nullptr;
@@ -892,27 +859,27 @@ static int step_host_slabs(mb_sim *s, mb_atom_element *box_atoms, mb_atom_elemen
   const DevPot &P = pot_dev(s->pot);
   const int it = s->n_itl > 0, flag = it ? I.flag : 0;
   s->flag_last = -1;
+  // of a slab's kernels only arrive follows an event, and it is no link of the chain
+  const Plan64 plan = chained_plan(s);
   auto start = [&]() -> int { // interstitials drift first (their forces came with them); no site is flagged yet
     if (!it) return MB_OK;
     MB_CUDA(cudaMemsetAsync(s->flag_count, 0, 2 * sizeof(int), cs));
-    return launch_kick_drift64(g, L, I, sp, cs, 0, 0, 1);
+    return launch_itl_kick_drift64(I, sp, cs);
   };
   auto arrive = [&](int k) -> int {
     MB_CUDA(cudaStreamWaitEvent(cs, s->ev_in[k], 0));
-    MB_TRY(launch_unpack_box_ids(g, s->stage, L, 1, s->bad, s->id, P.n_types, cs, zb[k], zb[k + 1]));
-    MB_TRY(launch_images64(g, L, 1, cs, zb[k], zb[k + 1]));
-    MB_TRY(launch_kick_drift64(g, L, I, sp, cs, zb[k], zb[k + 1], 0));
+    MB_TRY(launch_arrive64(g, s->stage, L, sp, s->bad, s->id, P.n_types, cs, zb[k], zb[k + 1]));
     if (it) MB_TRY(launch_itl_mark64(g, L, I, 0, cs, zb[k], zb[k + 1]));
     return MB_OK;
   };
   auto rho = [&](int k) -> int {
-    MB_TRY(launch_rho64(g, s->st, P, L, sp.rc2, nullptr, 0, flag, cs, zb[k], zb[k + 1], s->outer, &s->plan));
-    if (it) MB_TRY(launch_itl_rho64(g, P, L, I, sp.rc2, nullptr, 0, cs, zb[k], zb[k + 1]));
+    MB_TRY(launch_rho64(g, s->st, P, L, sp.rc2, nullptr, 0, flag, cs, zb[k], zb[k + 1], s->outer, &plan));
+    if (it) MB_TRY(launch_itl_rho64(g, P, L, I, sp.rc2, nullptr, 0, cs, zb[k], zb[k + 1], plan.chain));
     return MB_OK;
   };
   auto force = [&](int k) -> int {
-    MB_TRY(launch_force64(g, s->st, P, L, sp, nullptr, 0, flag, cs, zb[k], zb[k + 1], s->outer, &s->plan));
-    if (it) MB_TRY(launch_itl_force64(g, P, L, I, sp, nullptr, 0, cs, zb[k], zb[k + 1]));
+    MB_TRY(launch_force64(g, s->st, P, L, sp, nullptr, 0, flag, cs, zb[k], zb[k + 1], s->outer, &plan));
+    if (it) MB_TRY(launch_itl_force64(g, P, L, I, sp, nullptr, 0, cs, zb[k], zb[k + 1], plan.chain));
     MB_TRY(launch_pack_box_ids(g, s->stage, L, L.p, sp.h, 0, s->id, cs, zb[k], zb[k + 1]));
     MB_CUDA(cudaEventRecord(s->ev_out[k], cs));
     MB_CUDA(cudaStreamWaitEvent(s->cp_out, s->ev_out[k], 0));

@@ -35,3 +35,36 @@ def test_uploaded_records_come_back(cells, kind):
     assert np.array_equal(got["id"], sc.box["id"]) and np.array_equal(got["type"], sc.box["type"])
     for k in fields[2:]:
         assert np.max(np.abs(got[k][live] - sc.box[k][live])) <= tol, k
+
+
+@pytest.mark.parametrize("slabs", [1, 5])
+@pytest.mark.parametrize("cells,n_itl", [((6, 7, 24), 0), ((9, 8, 27), 6)])
+def test_host_steps_match_resident_steps(cells, n_itl, slabs, monkeypatch):
+    # records in, drifted and given their ghost images by one kernel, kernels chained or one by one
+    sc = make(cells=cells, vacancy=0.02, n_itl=n_itl, seed=82)
+    kw = dict(lattice_const=A0, mass=MASS, dt=1.0, cutoff=sc.cutoff, stencil_skin=sc.skin, max_interstitials=8)
+    with mb.Sim(sc.cells, sc.tables, **kw) as sim:
+        sim.upload(sc.box, sc.itl if n_itl else None)
+        sim.run(0)
+        start = sim.download()
+        sim.run(1)
+        want = sim.download()
+    got = {}
+    for chain in ("1", "0"):
+        monkeypatch.setenv("MB_CHAIN", chain)
+        box, itl = start[0].copy(), start[1].copy()
+        with mb.Sim(sc.cells, sc.tables, **kw) as sim:
+            sim.set_host_slabs(slabs)
+            sim.step_host(box, itl if n_itl else None)
+        got[chain] = box, itl
+    for k in ("id", "type", "x", "f", "rho", "df", "v"):
+        assert np.array_equal(got["0"][0][k], got["1"][0][k]) and np.array_equal(got["0"][1][k], got["1"][1][k]), k
+    live = want[0]["type"] >= 0
+    assert np.array_equal(got["1"][0]["id"], want[0]["id"]) and np.array_equal(got["1"][0]["type"], want[0]["type"])
+    # one drift from the same records: positions to the rounding of the half-step velocity,
+    # forces to that of the positions
+    assert np.max(np.abs(got["1"][0]["x"][live] - want[0]["x"][live])) < 1e-12
+    assert np.max(np.abs(got["1"][0]["f"][live] - want[0]["f"][live])) < 1e-10 * np.max(np.abs(want[0]["f"][live]))
+    if n_itl:
+        assert np.max(np.abs(got["1"][1]["x"] - want[1]["x"])) < 1e-12
+        assert np.array_equal(got["1"][1]["type"], want[1]["type"]) and np.array_equal(got["1"][1]["id"], want[1]["id"])
