@@ -696,6 +696,10 @@ __global__ void __launch_bounds__(MX_ONE_THREADS, 3)
 // occupied cell gets its start and count.  The order (cell, index) does not depend on
 // thread timing.
 #define MX_BIN_THREADS 1024
+// Up to this many interstitials are walked as a list: a site's 27 cells are four dependent
+// rounds of loads, more than its eighth of a short list.  Step at 33 x 70 x 41 cells by cells /
+// list: 16 interstitials 105.6 / 100.7 us, 48 107.9 / 104.1, 96 109.2 / 108.4, 200 123 / 135.
+#define MX_ICELL_MIN 64
 #define MX_MARK_THREADS 256
 __device__ void mx_itl_bin(const LatDesc &d) {
   __shared__ long long key[MX_ICELL_MAX];
@@ -704,7 +708,7 @@ __device__ void mx_itl_bin(const LatDesc &d) {
   const int nold = d.iflag[1];
   for (int k = tid; k < nold; k += blockDim.x) d.icount[d.icell_of[k]] = 0;
   __syncthreads();
-  if (n > MX_ICELL_MAX) { // too many for the shared-memory sort: items walk the whole list
+  if (n <= MX_ICELL_MIN || n > MX_ICELL_MAX) { // few, or too many to sort: items walk the whole list
     if (tid == 0) {
       d.iflag[0] = 0;
       d.iflag[1] = 0;

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 import misa_b200 as mb
+from oracle import oracle as orc
 from scenarios import A0, MASS, make
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +55,24 @@ def test_split_items_of_many_lattices_give_the_same_bits(monkeypatch):
     for a, b in zip(got["0"], got["1000000"]):
         for k in FIELDS:
             assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n_itl", [64, 65])
+def test_interstitials_as_a_list_and_in_cells_match_the_oracle(n_itl):
+    # up to 64 interstitials are walked as a list, more through the cell list
+    sc = make(cells=(16, 15, 14), temperature=900.0, vacancy=0.01, n_itl=n_itl, seed=103, jitter=0.1)
+    with mb.Sim(sc.cells, sc.tables, lattice_const=A0, mass=MASS, dt=1.0, cutoff=sc.cutoff, stencil_skin=sc.skin,
+                precision=mb.MB_PREC_MIXED, max_interstitials=n_itl) as sim:
+        sim.upload(sc.box, sc.itl)
+        sim.run(0)
+        box, itl = sim.download()
+    even, odd = sc.stencil()
+    ext, il = sc.ext().view(orc.ATOM), sc.itl.view(orc.ATOM).copy()
+    orc.compute_forces(sc.orc_pot(), sc.orc_domain(), ext, il, even, odd, sc.md_params())
+    ref = mb.lattice.ext_to_box(ext, sc.cells, sc.ghost)
+    live = ref["type"] >= 0
+    got = np.concatenate([box["f"][live], itl["f"]])
+    want = np.concatenate([ref["f"][live], il["f"]])
+    assert np.sqrt(np.mean((got - want) ** 2)) < 1e-6 * np.sqrt(np.mean(want**2))
+    got, want = np.concatenate([box["rho"][live], itl["rho"]]), np.concatenate([ref["rho"][live], il["rho"]])
+    assert np.sqrt(np.mean((got - want) ** 2)) < 1e-6 * np.sqrt(np.mean(want**2))
