@@ -89,6 +89,8 @@ int HostCopy::copy(void *host, void *dev, size_t bytes, bool to_host, cudaStream
   };
   std::vector<std::thread> threads;
   std::vector<int> own{0}; // shares of this thread: its own, and of threads that did not start
+  threads.reserve(workers);
+  own.reserve(workers);
   for (int t = 1; t < workers; t++) {
     try {
       threads.emplace_back(worker, t);

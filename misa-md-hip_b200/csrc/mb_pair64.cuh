@@ -69,6 +69,10 @@ __device__ __forceinline__ bool window_locate(double r, double rdr, double base,
 __device__ __forceinline__ void table_locate(double r, const DevPot &P, int &m, double &p) {
   m = min((int)__dmul_rd(r, P.rdr), P.nr - 2);
   p = __fma_rn(r, P.rdr, -(double)m);
+  if (P.n_types > 1 && r != r) { // coincident atoms: as spl_locate
+    m = P.nr - 2;
+    p = 1.0;
+  }
 }
 
 // Squared length of d, summed as x, y, z.

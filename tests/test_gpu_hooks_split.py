@@ -71,3 +71,33 @@ def test_hook_passes_match_the_oracle(hooks, name, monkeypatch):
         assert rel_err(got["rho"][live], want["rho"][live]) < 1e-12
         assert rel_err(got["df"][live], want["df"][live]) < 1e-12
         assert rel_err(got["f"][live], want["f"][live]) < 1e-10
+
+
+@pytest.mark.parametrize("n_types", [1, 3])
+def test_degenerate_positions_as_in_the_row_walk(hooks, n_types, monkeypatch):
+    # coincident atoms, infinite and undefined coordinates: finite where the row walk is finite
+    sc = make(cells=(7, 6, 6), seed=112, n_types=n_types, jitter=0.05)
+    dom = mb.lattice.domain(sc.cells, sc.ghost, (0, 0, 0))
+    even, odd = mb.lattice.stencil_linear(A0, sc.reach, dom.ext_size_x, dom.ext_size_y)
+    hooks.domain_init(dom)
+    hooks.nei_offset_init(even, odd)
+    hooks.pot_init(sc.tables)
+    ext = sc.ext()
+    mid = ext.shape[0] // 2 + 3
+    ext["x"][mid] = ext["x"][mid + 1]
+    ext["x"][mid + 40, 1] = np.inf
+    ext["x"][mid - 40, 2] = np.nan
+    got = {}
+    for items in ("0", "1000000"):
+        monkeypatch.setenv("MB_HOOK_SPLIT_ITEMS", items)
+        e = ext.copy()
+        hooks.rho_calc(e, sc.cutoff)
+        # the pair that coincides has no finite df in one type: keep the force pass's own case apart
+        e["df"] = np.where(np.isfinite(e["df"]), e["df"], 0.0)
+        hooks.force_calc(e, sc.cutoff)
+        got[items] = e
+    for k, tol in (("rho", 1e-12), ("f", 1e-10)):
+        a, b = got["0"][k], got["1000000"][k]
+        fin = np.isfinite(a)
+        assert np.array_equal(fin, np.isfinite(b)), k
+        assert np.max(np.abs(a[fin] - b[fin])) <= tol * max(1.0, np.max(np.abs(a[fin]))), k
