@@ -333,7 +333,7 @@ def run_ours(args, mb, wl, world, rank, local, pg) -> None:
     if probe.mb_probe_fma_peaks(C.byref(f64), C.byref(f32)) != 0:
         raise RuntimeError("the FMA peak probe failed")
     if precision == mb.MB_PREC_FP64:
-        kname, kbytes, kflops, kms = "k_force64 (force + velocity-Verlet)", BYTES_FORCE * n_atoms, FLOP_FORCE, force_ms
+        kname, kbytes, kflops, kms = "k_shell_force64 (force + velocity-Verlet)", BYTES_FORCE * n_atoms, FLOP_FORCE, force_ms
         fpeak, fname = f64.value, "fp64"
     elif rho_ms > 0:
         # split kernels (one large lattice): density pass, then force + integration
@@ -359,7 +359,7 @@ def run_ours(args, mb, wl, world, rank, local, pg) -> None:
     }
     if rho_ms > 0:
         rb = BYTES_RHO if precision == mb.MB_PREC_FP64 else BYTES_MIXED_RHO
-        roofline["rho_kernel"] = {"kernel": "k_rho64" if precision == mb.MB_PREC_FP64 else "k_mx_rho",
+        roofline["rho_kernel"] = {"kernel": "k_shell_rho64" if precision == mb.MB_PREC_FP64 else "k_mx_rho",
                                   "launch_ms": rho_ms, "achieved_gbs": rb * n_atoms / (rho_ms * 1e-3) / 1e9,
                                   "achieved_tflops": FLOP_RHO * n_atoms / (rho_ms * 1e-3) / 1e12}
 
@@ -417,9 +417,9 @@ def run_ours(args, mb, wl, world, rank, local, pg) -> None:
         except Exception as e:
             serving = {"error": str(e)[:300]}
     if precision == mb.MB_PREC_FP64:
-        launches_per_step = 6 if n_itl else 2  # itl clear, itl mark, rho, itl rho, force, itl force
-    elif rho_ms > 0:  # split: itl clear, bin, mark, rho, itl rho, force, itl force, bookkeeping
-        launches_per_step = 8 if n_itl else 3
+        launches_per_step = 5 if n_itl else 2  # itl mark, rho, itl rho, force, itl force
+    elif rho_ms > 0:  # split: itl preparation, rho, itl rho, force, itl force, bookkeeping
+        launches_per_step = 6 if n_itl else 3
     else:
         launches_per_step = 1
     if rank == 0:

@@ -337,7 +337,7 @@ int mb_ensemble_set_graphs(mb_ensemble *e, int enable);
  * first poll that finds the barrier still closed.  For failure-detection tests. */
 int mb_ensemble_set_wait_limit(mb_ensemble *e, int64_t barrier_polls);
 /* Kernel structure: 0 (default) runs the separate density and force kernels ("split":
- * one CUDA graph of up to 8 launches per step, every lattice in each launch) whenever
+ * one CUDA graph of up to 7 launches per step, every lattice in each launch) whenever
  * their built-in BCC stencil applies and the persistent one-launch-per-step tile
  * kernel otherwise; 1 always the persistent kernel; 2 always split (MB_ERR_UNSUPPORTED
  * at the next launch if it cannot apply). */

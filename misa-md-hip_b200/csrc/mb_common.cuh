@@ -1,6 +1,6 @@
 // Shared declarations of the misa_b200 library (host + device).
 //
-// Device layout ("sublattice-split SoA"): the reference indexes a BCC lattice
+// Device layout (split by sublattice): the reference indexes a BCC lattice
 // with x doubled, so neighbouring memory cells alternate between the two
 // simple-cubic sublattices and every warp mixes two stencils
 // (src/kernels/kernel_itl.hpp:82,86).  Here each sublattice s in {0,1} is its own

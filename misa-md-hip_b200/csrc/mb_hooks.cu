@@ -6,7 +6,7 @@
 // with a fresh pair of streams per call (src/double-buffer/*).  Here the rho and
 // force hooks stream the array in z-slabs too, on two long-lived copy streams: the
 // ext layers slab k needs come in on one while the compute stream converts them to
-// the split SoA layout, runs the pass over slab k's box layers and converts back, and
+// the split layout, runs the pass over slab k's box layers and converts back, and
 // slab k's box rows go out on the other while later slabs still come in.  The host
 // fills the ghosts, so slab k depends on nothing after its own ext layers and the
 // slabs need no particular thickness.  Same results (bitwise, for every slab count),

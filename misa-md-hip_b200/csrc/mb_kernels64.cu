@@ -9,15 +9,16 @@
 // (src/kernels/kernel_pairs.hpp:39-60).
 //
 // B200 design:
-//  * sublattice-split SoA: a warp is 32 consecutive sites of one sublattice row,
-//    so every stencil entry is one contiguous, coalesced 256-byte row fetch per
-//    coordinate, and the stencil offset is warp-uniform (read from the kernel's
-//    parameter bank);
+//  * records {x, y, z, F'} of 32 bytes per site, split by sublattice: a warp is 32
+//    consecutive sites of one sublattice row, so every stencil entry is one coalesced
+//    256-bit load per lane, and the stencil offset is warp-uniform (read from the
+//    kernel's parameter bank);
 //  * vacant sites carry a far-away position, so the r^2 test rejects them with no
 //    type fetch;
-//  * the spline pieces of the hot function live in shared memory (loaded once per
-//    persistent CTA): random per-lane knot gathers are served by shared-memory
-//    banks instead of L1 tag lookups;
+//  * lattices with BCC shells take the shell-window kernels (mb_shell64.cu) or, in small
+//    launches, the entry-split ones (mb_split64.cu); the row walk here serves the hooks of
+//    larger boxes, other stencils and tables that the windows do not take: the spline pieces
+//    of the hot function live in shared memory, loaded once per persistent CTA;
 //  * sites near the domain faces write their periodic ghost images themselves
 //    (no separate ghost-exchange pass), and the force pass closes the previous
 //    velocity-Verlet step and drifts to the next positions (double-buffered).

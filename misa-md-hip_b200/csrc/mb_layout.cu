@@ -1,6 +1,6 @@
 // Conversion between the host's AoS lattice records (mb_atom_element, the
 // reference's _cuAtomElement, src/kernel_types.h:40-48) and the device's
-// sublattice-split SoA arrays.
+// sublattice-split arrays.
 #include "mb_common.cuh"
 #include "mb_device.cuh"
 

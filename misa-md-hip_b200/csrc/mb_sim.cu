@@ -6,7 +6,8 @@
 //   items) -> force + velocity-Verlet (lattice) -> force + VV (interstitial items)
 // where the force passes close step n (v += h f) and drift to step n+1 into the
 // second position buffer, and every site near a face writes its own periodic ghost
-// images.  The steady-state step pair is captured once into a CUDA graph.
+// images.  The steady-state step pair is captured once into a CUDA graph; its kernels are
+// chained, each starting while the one before drains.
 #include <math.h>
 #include <string.h>
 
