@@ -51,7 +51,8 @@ int HostCopy::copy(void *host, void *dev, size_t bytes, bool to_host, cudaStream
   const int n_chunks = (int)((bytes + kChunk - 1) / kChunk);
   const int workers = std::min({kSlots, n_chunks, (int)std::max(1u, hw / 2)});
   bool plain = bytes < kMinBytes || workers < 2 || page_locked(host);
-  if (!plain && !slots) plain = (moved += bytes) < kSlotBytes || ensure() != MB_OK;
+  if (!plain && !slots)
+    plain = (moved += bytes) < (bytes >= kBigBytes ? kSlotBytes : kSlotBytesSmall) || ensure() != MB_OK;
   if (plain) {
     cudaGetLastError();
     MB_CUDA(to_host ? cudaMemcpyAsync(host, dev, bytes, kind, s) : cudaMemcpyAsync(dev, host, bytes, kind, s));

@@ -5,15 +5,16 @@
 
 namespace mb {
 
-// One per simulation or ensemble: 8 MiB of page-locked memory from the time that large copies
-// have moved kSlotBytes until release().  Calls on one object must not overlap.
+// One per simulation or ensemble: 8 MiB of page-locked memory from the time that its copies
+// have moved enough for it to pay until release().  Calls on one object must not overlap.
 struct HostCopy {
   static constexpr int kSlots = 8;
   static constexpr size_t kChunk = 1u << 20;
   static constexpr size_t kMinBytes = 2u << 20; // below: one plain copy is as fast
-  // The slots are taken once this much has been moved: to lock 8 MiB takes 6.5 ms, a plain
-  // copy of 18 MiB 1.3 ms (8 ms into fresh pages).
-  static constexpr size_t kSlotBytes = 64u << 20;
+  // The slots are taken once this much has been moved by an object's copies: to lock 8 MiB
+  // takes 6.5 ms, and they save 8 ms of a copy of 54 MiB into fresh pages but 0.3 ms of one of
+  // 17 MiB (2.0 against 2.3 ms).
+  static constexpr size_t kBigBytes = 32u << 20, kSlotBytes = 64u << 20, kSlotBytesSmall = 512u << 20;
   size_t moved = 0;
   char *slots = nullptr;
   cudaEvent_t ev[kSlots] = {};

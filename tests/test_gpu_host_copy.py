@@ -11,7 +11,7 @@ from scenarios import A0, MASS, make
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("cells", [(6, 5, 7), (21, 21, 22), (32, 32, 32), (40, 41, 43)])
+@pytest.mark.parametrize("cells", [(6, 5, 7), (21, 21, 22), (32, 32, 32), (40, 41, 43), (56, 57, 55)])
 @pytest.mark.parametrize("kind", ["fp64", "ensemble"])
 def test_uploaded_records_come_back(cells, kind):
     sc = make(cells=cells, vacancy=0.01, seed=81)
