@@ -20,12 +20,15 @@ __device__ __forceinline__ void spl_locate(double x, double rdx, int n, int &m, 
   p = fmin(pp - (double)mm, 1.0);
   m = mm;
 }
-// spl_locate for x inside the table's range (x < (n - 1) / rdx, which every pair inside
+// spl_locate for x >= 0 inside the table's range (x < (n - 1) / rdx, which every pair inside
 // a cutoff within the table satisfies): the same m and p there; past the range m is
-// clamped and p is meaningless, for terms the caller masks out.
+// clamped and p is meaningless, for terms the caller masks out.  x may be undefined
+// (coincident atoms: d2 * rsqrt(d2) at d2 = 0; undefined coordinates): the conversion of a
+// NaN gives the most negative integer, so the clamp compares unsigned (m = n - 2), and p is
+// undefined, as what follows from it.
 __device__ __forceinline__ void spl_locate_in(double x, double rdx, int n, int &m, double &p) {
   const double pp = x * rdx;
-  m = min((int)pp, n - 2);
+  m = (int)min((unsigned)(int)pp, (unsigned)(n - 2));
   p = pp - (double)m;
 }
 __device__ __forceinline__ double cubic(const double4 c, double p) { return ((c.w * p + c.z) * p + c.y) * p + c.x; }
