@@ -161,6 +161,7 @@ struct LatHost {
   CUtensorMap tmap[2];
   std::vector<double> e_step, e_pe, e_ke;
   int policy_shape = -1;
+  bool marks = false; // interstitial passes may have left marks in the site codes
 };
 
 } // namespace mb
@@ -390,6 +391,19 @@ static bool bricks_pay(const LatDesc &d, const MxWalk &w) {
   return 100 * bricks * sms * warps <= 106 * items;
 }
 
+// Takes off the marks of a lattice that gets no more interstitial passes (its last
+// interstitial recombined and conversion went off) and empties both lists: the lattice passes
+// would leave a site that is still marked to them.
+__global__ void k_ens_unmark(LatDesc d) {
+  for (int l = 0; l < 2; l++) {
+    const int n = min(d.flag_count[l], d.cap_flag);
+    for (int k = threadIdx.x; k < n; k += blockDim.x)
+      code_bit_off(d.code + d.flag_list[(size_t)l * d.cap_flag + k], MB_FLAG_ITL(0) | MB_FLAG_ITL(1));
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) d.flag_count[threadIdx.x] = 0;
+}
+
 // Rebuild descriptors, tile lists and tensor maps after slots or shapes change.
 static const char *mx_stencil(const mb_ensemble *e, const LatDesc &d, MxStencil &S);
 
@@ -428,7 +442,14 @@ static int rebuild(mb_ensemble *e) {
                              ((unsigned)(tz * kShapes[shape][2]) << 22));
         }
     (void)nt;
-    if (L.d.n_itl > 0 || (e->conv_d > 0.0 && L.d.cap_itl > 0)) itl_lats.push_back(c);
+    if (L.d.n_itl > 0 || (e->conv_d > 0.0 && L.d.cap_itl > 0)) {
+      itl_lats.push_back(c);
+      L.marks = true;
+    } else if (L.marks) {
+      k_ens_unmark<<<1, 1024, 0, e->stream>>>(L.d);
+      MB_CUDA(cudaGetLastError());
+      L.marks = false;
+    }
     descs[c] = L.d;
   }
   tile_first[nl] = (int)tile_lat.size();
