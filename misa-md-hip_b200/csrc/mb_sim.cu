@@ -950,6 +950,8 @@ int mb_sim_set_conversion(mb_sim *s, double convert_distance, double recombine_d
     return fail(MB_ERR_ARG, "max_interstitials above the conversion limit (65536)");
   if (convert_distance > 0 && s->cap_itl < 1) return fail(MB_ERR_ARG, "conversion needs max_interstitials > 0");
   MB_CUDA(cudaStreamSynchronize(s->stream));
+  // steps so far may have changed the count, which decides whether interstitials are passed over
+  MB_CUDA(cudaMemcpy(&s->n_itl, s->d_nitl, sizeof(int), cudaMemcpyDeviceToHost));
   s->conv_d = convert_distance;
   s->rec_d = convert_distance > 0 ? recombine_distance : 0.0;
   drop_graph(s); // the captured step pair changes

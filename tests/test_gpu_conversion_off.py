@@ -1,6 +1,7 @@
 """Conversion switched off in mid-run: what the last step with it left on the device (marks of
-sites near an interstitial that has since recombined) must not change the steps that follow.
-Against runs in which nothing is left over, bitwise."""
+sites near an interstitial that has since recombined; interstitials that the host has not
+counted yet) must not change the steps that follow.  Against runs in which nothing is left
+over, bitwise."""
 from __future__ import annotations
 
 import numpy as np
@@ -53,3 +54,22 @@ def test_off_after_the_last_recombination(precision, steps_before):
             out[off, "on again"] = sim.download()
     _same(out[True], out[False])
     _same(out[True, "on again"], out[False, "on again"])
+
+
+def test_off_before_the_host_has_counted_the_interstitials():
+    sc = make(cells=CELLS, temperature=300.0, seed=132)
+    site = ((4 * CELLS[1]) + 3) * 2 * CELLS[0] + 6
+    sc.box["x"][site] = mb.lattice.bcc_box(CELLS, A0)["x"][site] + np.array([0.55, 0.35, 0.0])
+    out = {}
+    for counted in (True, False):
+        with _sim(sc, mb.MB_PREC_FP64) as sim:
+            sim.upload(sc.box)
+            sim.set_conversion(0.6, 0.3)
+            sim.time_steps(1)  # steps without a synchronisation of the host's count
+            if counted:
+                sim.sync()
+            sim.set_conversion(0.0, 0.0)
+            sim.run(5)
+            out[counted] = sim.download()
+    assert len(out[True][1]) == 1
+    _same(out[True], out[False])
