@@ -26,13 +26,20 @@ static bool page_locked(const void *host) {
   return a.type != cudaMemoryTypeUnregistered;
 }
 
+// All of it or nothing: a later copy finds the slots with their events, or tries again.
 int HostCopy::ensure() {
   if (slots) return MB_OK;
   void *p = nullptr;
   MB_CUDA(cudaHostAlloc(&p, kSlots * kChunk, cudaHostAllocDefault));
   slots = (char *)p;
-  for (auto &e : ev)
-    if (!e) MB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  for (auto &e : ev) {
+    const cudaError_t r = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    if (r != cudaSuccess) {
+      e = nullptr;
+      release();
+      return cuda_fail(r, "cudaEventCreateWithFlags");
+    }
+  }
   return MB_OK;
 }
 

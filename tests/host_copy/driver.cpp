@@ -1,0 +1,82 @@
+// The shared host copies (csrc/mb_host_copy.cu) on a stand-in CUDA runtime without a device:
+// "device" memory is host memory, copies are done at once, and a call can be made to fail.
+// Usage: driver SCENARIO; prints one line per copy: its status and whether the bytes are right.
+#include <stdio.h>
+#include <string.h>
+
+#include <string>
+#include <vector>
+
+template <class T>
+T __ldg(const T *p) { return *p; } // named by device code of the header
+#include "mb_host_copy.cuh"
+
+static int events_made = 0, event_to_fail = -1; // the event creation that fails
+static int events_open = 0, slots_open = 0;
+
+extern "C" {
+void **__cudaRegisterFatBinary(void *) { return nullptr; }
+void __cudaRegisterFatBinaryEnd(void **) {}
+void __cudaUnregisterFatBinary(void **) {}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+  if (events_made++ == event_to_fail) return cudaErrorMemoryAllocation;
+  events_open++;
+  *e = (cudaEvent_t) new char;
+  return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+  events_open--;
+  delete (char *)e;
+  return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return e ? cudaSuccess : cudaErrorInvalidResourceHandle; }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) { return e ? cudaSuccess : cudaErrorInvalidResourceHandle; }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
+  slots_open++;
+  *p = new char[n];
+  return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void *p) {
+  slots_open--;
+  delete[](char *)p;
+  return cudaSuccess;
+}
+cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
+  a->type = cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  memcpy(d, s, n);
+  return cudaSuccess;
+}
+}
+namespace mb {
+int cuda_fail(cudaError_t e, const char *) { return 1000 + (int)e; }
+} // namespace mb
+
+static void copies(mb::HostCopy &c, int times, size_t bytes) {
+  std::vector<char> host(bytes), dev(bytes);
+  for (int k = 0; k < times; k++) {
+    for (size_t i = 0; i < bytes; i++) host[i] = (char)(i * 31 + i / 4096 + k), dev[i] = 0;
+    const int up = c.to_device(dev.data(), host.data(), bytes, nullptr);
+    const bool up_ok = host == dev;
+    memset(host.data(), 0, bytes);
+    const int down = c.to_host(host.data(), dev.data(), bytes, nullptr);
+    printf("%d %d %d %d\n", up, (int)up_ok, down, (int)(host == dev));
+  }
+}
+
+int main(int, char **argv) {
+  const std::string scenario = argv[1];
+  mb::HostCopy c;
+  const size_t big = 40u << 20;
+  if (scenario == "event") event_to_fail = 2; // the slots are taken, the third event is not
+  copies(c, 3, big);
+  c.release();
+  printf("left %d %d\n", events_open, slots_open);
+  return 0;
+}

@@ -1,0 +1,35 @@
+"""The shared host copies when a call under them fails, on a stand-in CUDA runtime (no device):
+every copy still succeeds with the right bytes, and all that was taken is given back."""
+from __future__ import annotations
+
+import pathlib
+import shutil
+import subprocess
+
+import pytest
+
+import misa_b200 as mb
+
+ROOT = pathlib.Path(__file__).resolve().parents[1]
+PKG = ROOT / "misa-md-hip_b200"
+
+
+@pytest.fixture(scope="module")
+def driver(tmp_path_factory):
+    out = tmp_path_factory.mktemp("host_copy") / "driver"
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    include = pathlib.Path(nvcc).resolve().parents[1] / "include"
+    mb.build()
+    subprocess.run(["g++", "-std=c++17", "-O1", f"-I{PKG / 'csrc'}", f"-I{ROOT / 'include'}", f"-I{include}",
+                    str(ROOT / "tests" / "host_copy" / "driver.cpp"), str(PKG / "_build" / "mb_host_copy.o"),
+                    "-lpthread", "-ldl", "-o", str(out)], check=True, capture_output=True, text=True)
+    return out
+
+
+@pytest.mark.parametrize("scenario", ["none", "event"])
+def test_copies_survive_a_failing_call(driver, scenario):
+    r = subprocess.run([str(driver), scenario], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    lines = r.stdout.split("\n")
+    assert lines[:3] == ["0 1 0 1"] * 3, lines
+    assert lines[3] == "left 0 0"
