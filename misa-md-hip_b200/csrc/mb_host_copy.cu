@@ -9,9 +9,7 @@
 
 #include <algorithm>
 #include <mutex>
-#include <system_error>
 #include <thread>
-#include <vector>
 
 #include "mb_host_copy.cuh"
 
@@ -95,19 +93,21 @@ int HostCopy::copy(void *host, void *dev, size_t bytes, bool to_host, cudaStream
       if (first == cudaSuccess) first = r;
     }
   };
-  std::vector<std::thread> threads;
-  std::vector<int> own{0}; // shares of this thread: its own, and of threads that did not start
-  threads.reserve(workers);
-  own.reserve(workers);
+  // No allocation here but a thread's own, and no exception leaves: a share whose thread
+  // does not start (no thread, no memory) is done by this one.
+  std::thread threads[kSlots];
+  bool own[kSlots] = {true};
   for (int t = 1; t < workers; t++) {
     try {
-      threads.emplace_back(worker, t);
-    } catch (const std::system_error &) {
-      own.push_back(t);
+      threads[t] = std::thread(worker, t);
+    } catch (...) {
+      own[t] = true;
     }
   }
-  for (int t : own) worker(t);
-  for (auto &th : threads) th.join();
+  for (int t = 0; t < workers; t++)
+    if (own[t]) worker(t);
+  for (auto &th : threads)
+    if (th.joinable()) th.join();
   const cudaError_t end = cudaStreamSynchronize(s); // the slots are free again
   MB_CUDA(first);
   MB_CUDA(end);

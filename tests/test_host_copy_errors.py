@@ -1,4 +1,4 @@
-"""The shared host copies when a call under them fails, on a stand-in CUDA runtime (no device):
+"""The shared host copies when a call or an allocation under them fails, on a stand-in CUDA runtime (no device):
 every copy still succeeds with the right bytes, and all that was taken is given back."""
 from __future__ import annotations
 
@@ -26,9 +26,9 @@ def driver(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("scenario", ["none", "event"])
+@pytest.mark.parametrize("scenario", ["none", "event", "memory 0", "memory 1", "memory 2", "memory 4"])
 def test_copies_survive_a_failing_call(driver, scenario):
-    r = subprocess.run([str(driver), scenario], capture_output=True, text=True, timeout=60)
+    r = subprocess.run([str(driver), *scenario.split()], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stderr
     lines = r.stdout.split("\n")
     assert lines[:3] == ["0 1 0 1"] * 3, lines
