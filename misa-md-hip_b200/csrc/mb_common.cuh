@@ -14,6 +14,7 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -380,14 +381,29 @@ int launch_half64(bool force, mb_atom_element *aos, const mb_device_domain &d, c
 // ------------------------------------------------------------ utilities
 int device_sm_count();
 #define MB_SMEM_MAX (227 * 1024)
-// Lets two kernels use `bytes` of dynamic shared memory (once per process).
+// Something done once for each device that the process uses (kernel attributes belong to a
+// device).  Two threads may do it at once.
+class DeviceOnce {
+  std::atomic<unsigned long long> devices{0};
+
+ public:
+  // The current device's bit while it is still to be done, else 0.
+  unsigned long long todo() const {
+    int d = 0;
+    if (cudaGetDevice(&d) != cudaSuccess) cudaGetLastError();
+    const unsigned long long bit = 1ull << (d & 63);
+    return devices.load() & bit ? 0 : bit;
+  }
+  void done(unsigned long long bit) { devices |= bit; }
+};
+// Lets two kernels use `bytes` of dynamic shared memory.
 #define MB_SMEM_ATTR(k0, k1, bytes)                                                                            \
   do {                                                                                                         \
-    static bool done_ = false;                                                                                 \
-    if (!done_) {                                                                                              \
+    static ::mb::DeviceOnce once_;                                                                             \
+    if (const unsigned long long bit_ = once_.todo()) {                                                        \
       MB_CUDA(cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes)));            \
       MB_CUDA(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes)));            \
-      done_ = true;                                                                                            \
+      once_.done(bit_);                                                                                        \
     }                                                                                                          \
   } while (0)
 

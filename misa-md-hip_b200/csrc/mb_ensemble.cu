@@ -424,12 +424,7 @@ size_t ens_smem_bytes(int nsm) {
 
 int ens_launch(const EnsParams &P, int grid, cudaStream_t s) {
   const size_t smem = ens_smem_bytes(P.nsm);
-  static bool attr = false;
-  if (!attr) {
-    MB_CUDA(cudaFuncSetAttribute(k_ens_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MB_CUDA(cudaFuncSetAttribute(k_ens_step<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  MB_SMEM_ATTR(k_ens_step<false>, k_ens_step<true>, smem);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(ENS_THREADS);

@@ -985,18 +985,10 @@ __global__ void k_mx_bookkeeping(const __grid_constant__ EnsParams P) {
 }
 
 template <int FIXED, int WALK>
-static int mx_set_attrs() {
-  MB_CUDA(cudaFuncSetAttribute(k_mx_rho<false, FIXED, WALK>, cudaFuncAttributeMaxDynamicSharedMemorySize, MX_SMEM_MAX));
-  MB_CUDA(cudaFuncSetAttribute(k_mx_rho<true, FIXED, WALK>, cudaFuncAttributeMaxDynamicSharedMemorySize, MX_SMEM_MAX));
-  MB_CUDA(
-      cudaFuncSetAttribute(k_mx_force<false, FIXED, WALK>, cudaFuncAttributeMaxDynamicSharedMemorySize, MX_SMEM_MAX));
-  MB_CUDA(cudaFuncSetAttribute(k_mx_force<true, FIXED, WALK>, cudaFuncAttributeMaxDynamicSharedMemorySize, MX_SMEM_MAX));
-  return MB_OK;
-}
-
-template <int FIXED, int WALK>
 static int mx_pass(const EnsParams &P, const MxStencil &S, int lat, int energy, cudaStream_t s, int which, size_t smem,
                    bool chain) {
+  MB_SMEM_ATTR((k_mx_rho<false, FIXED, WALK>), (k_mx_rho<true, FIXED, WALK>), MX_SMEM_MAX);
+  MB_SMEM_ATTR((k_mx_force<false, FIXED, WALK>), (k_mx_force<true, FIXED, WALK>), MX_SMEM_MAX);
   if (which == 0)
     return launch_chained(chain, energy ? k_mx_rho<true, FIXED, WALK> : k_mx_rho<false, FIXED, WALK>,
                           device_sm_count(), MX_RHO_THREADS, smem, s, P, S, lat);
@@ -1065,15 +1057,6 @@ int mx_launch_step(const EnsParams &P, const MxStencil &S, int lat, int energy, 
   if (force_smem > MX_SMEM_MAX || rho_smem > MX_SMEM_MAX)
     return fail(MB_ERR_ARG, "squared-distance table larger than shared memory");
   if (S.walk.linear && !S.fixed) return fail(MB_ERR_STATE, "linear walk needs the built-in shells");
-  static bool attr = false;
-  if (!attr) {
-    MB_TRY((mx_set_attrs<0, 0>()));
-    MB_TRY((mx_set_attrs<7, 0>()));
-    MB_TRY((mx_set_attrs<7, 1>()));
-    MB_TRY((mx_set_attrs<8, 0>()));
-    MB_TRY((mx_set_attrs<8, 1>()));
-    attr = true;
-  }
   const int itl_grid = 3 * sms;
   const bool chain = !ev && chain_on(); // events take the kernels one by one
   if (P.n_itl_lats > 0) MB_TRY(launch_chained(chain, k_mx_itl_prep, P.n_itl_lats + sms, MX_BIN_THREADS, 0, s, P));

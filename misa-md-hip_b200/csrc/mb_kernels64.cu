@@ -590,12 +590,7 @@ int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const L
   set_walk(g, z0, z1, kRhoBrick, a.walk, a.w0, a.n_items);
   const size_t smem = (size_t)nsm * sizeof(double4);
   const int grid = grid_for(a.n_items - a.w0, MB_RHO_THREADS);
-  static bool attr_done = false;
-  if (!attr_done) {
-    MB_CUDA(cudaFuncSetAttribute(k_rho64<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap));
-    MB_CUDA(cudaFuncSetAttribute(k_rho64<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap));
-    attr_done = true;
-  }
+  MB_SMEM_ATTR((k_rho64<false, true>), (k_rho64<true, true>), kSmemCap);
   if (one) {
     if (energy)
       k_rho64<true, true><<<grid, MB_RHO_THREADS, smem, s>>>(st, a);
@@ -644,12 +639,7 @@ int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const
   set_walk(g, z0, z1, kForceBrick, a.walk, a.w0, a.n_items);
   const size_t smem = (size_t)nsm * 3 * sizeof(double2);
   const int grid = grid_for(a.n_items - a.w0, MB_FORCE_THREADS);
-  static bool attr_done = false;
-  if (!attr_done) {
-    MB_CUDA(cudaFuncSetAttribute(k_force64<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap));
-    MB_CUDA(cudaFuncSetAttribute(k_force64<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap));
-    attr_done = true;
-  }
+  MB_SMEM_ATTR((k_force64<false, true>), (k_force64<true, true>), kSmemCap);
   if (one) {
     if (energy)
       k_force64<true, true><<<grid, MB_FORCE_THREADS, smem, s>>>(st, a);
