@@ -422,9 +422,13 @@ size_t ens_smem_bytes(int nsm) {
   return tab + 2 * ENS_TILE_MAX_BYTES + 4 * sizeof(uint64_t);
 }
 
+// The kernel's limit is the same whichever ensemble launches it: ensembles of larger and
+// smaller tables may be used in turn.
+static const int kEnsSmemMost = MB_SMEM_MAX - 2048 + 128;
+
 int ens_launch(const EnsParams &P, int grid, cudaStream_t s) {
   const size_t smem = ens_smem_bytes(P.nsm);
-  MB_SMEM_ATTR(k_ens_step<false>, k_ens_step<true>, smem);
+  MB_SMEM_ATTR(k_ens_step<false>, k_ens_step<true>, kEnsSmemMost);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(ENS_THREADS);
@@ -445,7 +449,7 @@ int ens_launch(const EnsParams &P, int grid, cudaStream_t s) {
 int ens_max_grid(int nsm) {
   int per_sm = 0;
   const size_t smem = ens_smem_bytes(nsm);
-  if (cudaFuncSetAttribute(k_ens_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(k_ens_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kEnsSmemMost) != cudaSuccess)
     return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ens_step<false>, ENS_THREADS, smem) != cudaSuccess)
     return 0;

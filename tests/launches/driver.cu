@@ -12,6 +12,8 @@ extern int device;
 namespace mb {
 int mx_launch_step(const EnsParams &P, const MxStencil &S, int lat, int energy, cudaStream_t s, cudaEvent_t *ev,
                    double *out);
+int ens_launch(const EnsParams &P, int grid, cudaStream_t s);
+int ens_max_grid(int nsm);
 } // namespace mb
 using namespace mb;
 
@@ -68,6 +70,20 @@ static void mixed(int fixed, bool linear) {
     printf("%d mixed%d_%d %d\n", device, fixed, (int)linear, mx_launch_step(P, S, 0, energy, nullptr, nullptr, nullptr));
 }
 
+// The persistent kernel with few knots in shared memory and with many, an ensemble of each.
+static void persistent() {
+  const int knots[2] = {100, 3000};
+  for (int k : knots) printf("%d persistent_grid%d %d\n", device, k, ens_max_grid(k) == 148 ? 0 : 1);
+  for (int first = 0; first < 2; first++) // either of them made last
+    for (int k = 0; k < 2; k++) {
+      ens_max_grid(knots[first]);
+      EnsParams P{};
+      P.nsm = knots[k];
+      P.energy = first;
+      printf("%d persistent%d_%d %d\n", device, knots[k], first, ens_launch(P, 148, nullptr));
+    }
+}
+
 int main() {
   for (device = 0; device < 2; device++) {
     for (int n_types : {1, 3}) {
@@ -78,6 +94,7 @@ int main() {
     for (int fixed : {0, 7, 8})
       for (bool linear : {false, true})
         if (fixed || !linear) mixed(fixed, linear);
+    persistent();
   }
   return 0;
 }

@@ -52,6 +52,9 @@ cudaError_t cudaGetLastError() {
   last = cudaSuccess;
   return r;
 }
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *f, int, size_t smem, unsigned) {
+  return *n = 1, launch(f, smem);
+}
 const char *cudaGetErrorString(cudaError_t) { return "refused"; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 }

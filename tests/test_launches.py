@@ -1,6 +1,6 @@
 """Launchers of the lattice passes on a stand-in CUDA runtime (no device): every pass launches
 on the first device that a process uses and on the next one, whose kernels start with their
-own limits of shared memory."""
+own limits of shared memory; and whatever table the last ensemble was made with."""
 from __future__ import annotations
 
 import pathlib
@@ -13,7 +13,7 @@ import misa_b200 as mb
 
 ROOT = pathlib.Path(__file__).resolve().parents[1]
 PKG = ROOT / "misa-md-hip_b200"
-OBJECTS = ("mb_kernels64", "mb_split64", "mb_shell64", "mb_geometry", "mb_ensemble_split")
+OBJECTS = ("mb_kernels64", "mb_split64", "mb_shell64", "mb_geometry", "mb_ensemble_split", "mb_ensemble")
 
 
 @pytest.fixture(scope="module")
@@ -34,5 +34,5 @@ def lines(tmp_path_factory):
 @pytest.mark.parametrize("device", ["0", "1"])
 def test_every_pass_launches_on_every_device(lines, device):
     got = [(name, status) for d, name, status in lines if d == device]
-    assert len(got) == 34
+    assert len(got) == 40
     assert all(status == "0" for _, status in got), [g for g in got if g[1] != "0"]
