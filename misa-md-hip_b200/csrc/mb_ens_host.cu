@@ -205,7 +205,7 @@ struct mb_ensemble {
   size_t fixed_bytes = 0;
   long long launches = 0;
   mb::HostCopy copier;               // records to and from pageable buffers
-  mb_atom_element *stage = nullptr;  // records of one lattice on their way (up to MB_STAGE_KEEP)
+  mb_atom_element *stage = nullptr;  // records of one lattice on their way (up to MB_STAGE_KEEP), counted
   size_t stage_n = 0;
   std::mutex mu;
 };
@@ -225,25 +225,46 @@ static int edalloc(mb_ensemble *e, void **p, size_t bytes) {
   return MB_OK;
 }
 
-// Device records of one lattice (n of them): kept between calls up to MB_STAGE_KEEP, beyond
-// that allocated for the call (drop_stage).
+// The records kept between calls count like the rest of the ensemble's memory; they give way
+// to whatever else the budget has room for.
+static bool over_budget(const mb_ensemble *e, size_t more) {
+  return e->cfg.hbm_budget_bytes > 0 && e->device_bytes + more > (size_t)e->cfg.hbm_budget_bytes;
+}
+static void free_stage(mb_ensemble *e) {
+  if (!e->stage) return;
+  cudaFree(e->stage);
+  e->device_bytes -= e->stage_n * sizeof(mb_atom_element);
+  e->fixed_bytes -= e->stage_n * sizeof(mb_atom_element);
+  e->stage = nullptr;
+  e->stage_n = 0;
+}
+
+// Device records of one lattice (n of them): kept between calls up to MB_STAGE_KEEP and the
+// budget, beyond that allocated for the call (drop_stage).
 static int take_stage(mb_ensemble *e, size_t n, mb_atom_element **out) {
-  if (n > e->stage_n || n * sizeof(mb_atom_element) > MB_STAGE_KEEP) {
-    if (n * sizeof(mb_atom_element) <= MB_STAGE_KEEP) {
-      if (e->stage) cudaFree(e->stage);
-      e->stage = nullptr;
-      e->stage_n = 0;
-    }
-    cudaError_t r = cudaMalloc(out, n * sizeof(mb_atom_element));
-    if (r != cudaSuccess) {
-      cudaGetLastError();
-      return fail(MB_ERR_NOMEM, std::string("staging allocation failed: ") + cudaGetErrorString(r));
-    }
-    if (n * sizeof(mb_atom_element) > MB_STAGE_KEEP) return MB_OK;
+  const size_t bytes = n * sizeof(mb_atom_element);
+  if (n <= e->stage_n) {
+    *out = e->stage;
+    return MB_OK;
+  }
+  const bool keep = bytes <= MB_STAGE_KEEP && !over_budget(e, bytes - e->stage_n * sizeof(mb_atom_element));
+  if (keep) free_stage(e);
+  cudaError_t r = cudaMalloc(out, bytes);
+  if (r != cudaSuccess && e->stage) { // the kept records make room
+    cudaGetLastError();
+    free_stage(e);
+    r = cudaMalloc(out, bytes);
+  }
+  if (r != cudaSuccess) {
+    cudaGetLastError();
+    return fail(MB_ERR_NOMEM, std::string("staging allocation failed: ") + cudaGetErrorString(r));
+  }
+  if (keep) {
     e->stage = *out;
     e->stage_n = n;
+    e->device_bytes += bytes;
+    e->fixed_bytes += bytes;
   }
-  *out = e->stage;
   return MB_OK;
 }
 static void drop_stage(mb_ensemble *e, mb_atom_element *stage) {
@@ -642,6 +663,7 @@ static int rebuild(mb_ensemble *e) {
     P.epart = e->d_epart_items;
     P.outer = outer_masks_on() ? e->d_outer_items : nullptr;
   }
+  if (over_budget(e, 0)) free_stage(e); // the arrays above have grown
   e->dirty = false;
   return MB_OK;
 }
@@ -987,7 +1009,7 @@ int mb_ensemble_destroy(mb_ensemble *e) {
     if (p) cudaFree(p);
   for (auto &ev : e->ev)
     if (ev) cudaEventDestroy(ev);
-  if (e->stage) cudaFree(e->stage);
+  free_stage(e);
   e->copier.release();
   if (e->stream) cudaStreamDestroy(e->stream);
   pot_free(e->pot);
@@ -1018,7 +1040,8 @@ int mb_ensemble_add(mb_ensemble *e, const mb_lattice_spec *spec, const mb_atom_e
   for (int k = 0; k < n_itl; k++)
     if (itl[k].type != 0) return fail(MB_ERR_ARG, "interstitial type must be 0 (one-type potential)");
   const size_t bytes = lattice_bytes(cx, cy, cz, spec->max_interstitials);
-  if (e->cfg.hbm_budget_bytes > 0 && e->device_bytes + bytes > (size_t)e->cfg.hbm_budget_bytes)
+  if (over_budget(e, bytes)) free_stage(e);
+  if (over_budget(e, bytes))
     return fail(MB_ERR_NOMEM, "HBM budget exceeded: " + std::to_string(e->device_bytes + bytes) + " > " +
                                   std::to_string(e->cfg.hbm_budget_bytes) + " bytes");
   if (e->cfg.max_lattices > 0) {
@@ -1040,6 +1063,11 @@ int mb_ensemble_add(mb_ensemble *e, const mb_lattice_spec *spec, const mb_atom_e
   LatHost &L = e->slots[slot];
   void *block = nullptr;
   cudaError_t r = cudaMalloc(&block, bytes);
+  if (r != cudaSuccess && e->stage) {
+    cudaGetLastError();
+    free_stage(e);
+    r = cudaMalloc(&block, bytes);
+  }
   if (r != cudaSuccess) return fail(MB_ERR_NOMEM, std::string("device allocation failed: ") + cudaGetErrorString(r));
   L.used = true;
   L.block = block;
