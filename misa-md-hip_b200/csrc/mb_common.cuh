@@ -346,10 +346,6 @@ int launch_unpack_ext(const Geom &g, const mb_atom_element *aos, int ext_x, int 
                       int with_df, int *bad_type, int n_types, cudaStream_t s, long long t0 = 0, long long t1 = -1);
 int launch_pack_ext(const Geom &g, mb_atom_element *aos, int ext_x, int ext_y, const Lattice64 &L, int what,
                     cudaStream_t s, int z0 = 0, int z1 = -1); // what: 1 rho+df, 2 force, 3 df only
-int launch_unpack_box(const Geom &g, const mb_atom_element *aos, Lattice64 L, int with_f, int *bad_type,
-                      int n_types, cudaStream_t s);
-int launch_pack_box(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double4 *pos, double h, int unkick,
-                    cudaStream_t s);
 // Records of a host step as they arrive: unpacked, kicked and drifted, ghost images written.
 int launch_arrive64(const Geom &g, const mb_atom_element *aos, const Lattice64 &L, const StepParams &sp, int *bad_type,
                     int64_t *ids, int n_types, cudaStream_t s, int z0 = 0, int z1 = -1);

@@ -95,7 +95,7 @@ __global__ void k_unpack_box(const Geom g, const mb_atom_element *aos, Lattice64
       L.fy[i] = vac ? 0.0 : a.f[1];
       L.fz[i] = vac ? 0.0 : a.f[2];
     }
-    if (ids) ids[t] = a.id;
+    ids[t] = a.id;
   }
 }
 
@@ -194,7 +194,7 @@ __global__ void k_pack_box(const Geom g, mb_atom_element *aos, const Lattice64 L
                         (bx >> 1) + g.gcx;
     mb_atom_element a;
     const int c = L.code[i];
-    a.id = ids ? ids[t] : t;
+    a.id = ids[t];
     a.type = c < 0 ? -1 : (c & MB_TYPE_MASK);
     a.pad_ = 0;
     if (c < 0) {
@@ -313,11 +313,6 @@ int launch_pack_itl(const Itl64 &I, mb_atom_element *aos, int n, double h, int u
   return MB_OK;
 }
 
-int launch_unpack_box(const Geom &g, const mb_atom_element *aos, Lattice64 L, int with_f, int *bad_type,
-                      int n_types, cudaStream_t s) {
-  return launch_unpack_box_ids(g, aos, L, with_f, bad_type, nullptr, n_types, s);
-}
-
 int launch_pack_box_ids(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double4 *pos, double h,
                         int unkick, const int64_t *ids, cudaStream_t s, int z0, int z1) {
   if (z1 < 0) z1 = g.bz;
@@ -326,11 +321,6 @@ int launch_pack_box_ids(const Geom &g, mb_atom_element *aos, const Lattice64 &L,
   k_pack_box<<<flat_grid(layer * (z1 - z0)), 256, 0, s>>>(g, aos, L, pos, h, unkick, ids, layer * z0, layer * z1);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
-}
-
-int launch_pack_box(const Geom &g, mb_atom_element *aos, const Lattice64 &L, const double4 *pos, double h, int unkick,
-                    cudaStream_t s) {
-  return launch_pack_box_ids(g, aos, L, pos, h, unkick, nullptr, s);
 }
 
 int launch_df_from_rho(const Geom &g, const DevPot &pot, const Lattice64 &L, cudaStream_t s) {
