@@ -227,6 +227,16 @@ int mb_sim_host_slabs(mb_sim *sim, int32_t *n_slabs);
  * takes (mixed precision: as mb_ensemble_kernel_times). */
 int mb_sim_kernel_times(mb_sim *sim, float *rho_ms, float *force_ms);
 int mb_sim_info(mb_sim *sim, int64_t *n_sites, int64_t *n_stencil, int64_t *device_bytes);
+/* Kernels of the density and force passes of the sim's next step without energies, which
+ * the library chooses by stencil, tables and size: */
+#define MB_PASS_ROWS 0         /* FP64: row walk (any stencil and tables) */
+#define MB_PASS_SHELLS 1       /* FP64: shell windows (large launches) */
+#define MB_PASS_SPLIT 2        /* FP64: items split over warps (small launches) */
+#define MB_PASS_TILES 3        /* mixed: the persistent tile kernel, both passes in one */
+#define MB_PASS_BRICKS 4       /* mixed: brick walk */
+#define MB_PASS_LINEAR 5       /* mixed: linear items, one to a warp */
+#define MB_PASS_LINEAR_SPLIT 6 /* mixed: linear items, one to a CTA (small launches) */
+int mb_sim_pass_kinds(mb_sim *sim, int32_t *rho, int32_t *force);
 /* CUDA graph capture of the steady-state step (on by default). */
 int mb_sim_set_graphs(mb_sim *sim, int enable);
 /* Lattice <-> interstitial bookkeeping of the device-resident run.  MISA-MD keeps atoms

@@ -181,6 +181,13 @@ class Sim:
         check(lib().mb_sim_info(self._h, C.byref(a), C.byref(b), C.byref(c)))
         return {"n_sites": a.value, "n_stencil": b.value, "device_bytes": c.value}
 
+    def pass_kinds(self) -> tuple[str, str]:
+        """Kernels of the density and force passes of the next step (mb_sim_pass_kinds)."""
+        names = ("rows", "shells", "split", "tiles", "bricks", "linear", "linear_split")
+        r, f = C.c_int32(), C.c_int32()
+        check(lib().mb_sim_pass_kinds(self._h, C.byref(r), C.byref(f)))
+        return names[r.value], names[f.value]
+
     def set_graphs(self, enable: bool) -> None:
         check(lib().mb_sim_set_graphs(self._h, int(enable)))
 

@@ -107,6 +107,7 @@ SIGNATURES: dict[str, tuple] = {
     "mb_sim_host_slabs": (_I, [_P, C.POINTER(C.c_int32)]),
     "mb_sim_kernel_times": (_I, [_P, _PF, _PF]),
     "mb_sim_info": (_I, [_P, _PI64, _PI64, _PI64]),
+    "mb_sim_pass_kinds": (_I, [_P, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "mb_sim_set_graphs": (_I, [_P, _I]),
     "mb_sim_set_conversion": (_I, [_P, _D, _D]),
     "mb_sim_conversion_stats": (_I, [_P, _PI64, C.POINTER(C.c_int32)]),

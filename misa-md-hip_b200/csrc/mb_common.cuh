@@ -301,6 +301,8 @@ __host__ __device__ __forceinline__ void site_ideal(int s, int cx, int y, int z,
 // box (items_per_box).  The density pass writes them; a force pass given them walks only
 // those entries, so it must run on the positions of the density pass that wrote them
 // (null: the force pass walks every entry).
+// pass_kind64: the kernels that a pass takes (MB_PASS_*).
+int pass_kind64(const Geom &g, const DevPot &pot, const Plan64 *plan, double rc2, bool force, int z0 = 0, int z1 = -1);
 int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, double rc2,
                  double *e_partial, int energy, int flag, cudaStream_t s, int z0 = 0, int z1 = -1,
                  uint2 *outer = nullptr, const Plan64 *plan = nullptr);

@@ -25,6 +25,7 @@ int ens_energy_launch(const LatDesc *lats, int n, const int *tile_first, const d
                       cudaStream_t s);
 int mx_launch_step(const EnsParams &P, const MxStencil &S, int lat, int energy, cudaStream_t s, cudaEvent_t *ev,
                    double *out);
+int mx_pass_kind(const MxStencil &S, int which);
 
 
 static const int kShapes[ENS_NSHAPE][3] = {{16, 4, 4}, {8, 8, 4}, {8, 4, 8}, {4, 8, 8}};
@@ -405,7 +406,9 @@ static void drop_graph(mb_ensemble *e) {
 // bricks, linear items spread evenly but cost 6% more each (the warps of a CTA share fewer
 // rows in L1).  Measured on one B200, step by bricks / linear: 32^3 174 / 46 us, 33 x 70 x
 // 41 177 / 84, 64^3 177 / 161, 100^3 809 / 617, 96^3 510 / 541, 128^3 1167 / 1228 us.
+// The environment variable MB_MX_BRICKS overrides the line (0: never, else always).
 static bool bricks_pay(const LatDesc &d, const MxWalk &w) {
+  if (const char *v = getenv("MB_MX_BRICKS")) return atoi(v) != 0;
   const long long sms = device_sm_count(), warps = 32;
   const long long bricks = (w.n_units + sms - 1) / sms * ((w.bitems + warps - 1) / warps);
   const long long items = 2LL * d.bz * (((long long)d.bcx * d.by + 31) / 32);
@@ -931,6 +934,14 @@ static int push_targets(mb_ensemble *e) {
     MB_CUDA(cudaMemcpyAsync(e->d_lats, descs.data(), sizeof(LatDesc) * descs.size(), cudaMemcpyHostToDevice,
                             e->stream));
   MB_CUDA(cudaStreamSynchronize(e->stream));
+  return MB_OK;
+}
+
+int ens_pass_kinds(mb_ensemble *e, int32_t *rho, int32_t *force) {
+  std::lock_guard<std::mutex> lk(e->mu);
+  if (e->dirty) MB_TRY(rebuild(e));
+  *rho = e->split ? mx_pass_kind(e->mxs, 0) : MB_PASS_TILES;
+  *force = e->split ? mx_pass_kind(e->mxs, 1) : MB_PASS_TILES;
   return MB_OK;
 }
 

@@ -1008,6 +1008,9 @@ static bool mx_one(const MxStencil &S, int energy, int which) {
   if (const char *v = getenv("MB_MX_ONE_ITEMS")) per_sm = atoi(v);
   return S.walk.linear && !energy && (long long)S.walk.n_items <= (long long)per_sm * device_sm_count();
 }
+int mx_pass_kind(const MxStencil &S, int which) {
+  return mx_one(S, 0, which) ? MB_PASS_LINEAR_SPLIT : S.walk.linear ? MB_PASS_LINEAR : MB_PASS_BRICKS;
+}
 template <int FIXED>
 static int mx_one_pass(const EnsParams &P, const MxStencil &S, cudaStream_t s, int which, bool chain) {
   const int most = (which == 0 ? 4 : 3) * device_sm_count(), n = (int)S.walk.n_items;

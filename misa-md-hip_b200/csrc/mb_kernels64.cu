@@ -531,10 +531,14 @@ int launch_split_force64(const StencilSet &st, const LatticeArgs &a, int energy,
 #define MB_SPLIT_FORCE_ITEMS 16
 #define MB_MULTI_SPLIT_RHO_ITEMS 12
 #define MB_MULTI_SPLIT_FORCE_ITEMS 7
-static bool split_launch(const char *name, int one, int multi, const LatticeArgs &a) {
-  int per_sm = a.P.n_types == 1 ? one : multi;
-  if (const char *v = getenv(name)) per_sm = atoi(v);
-  return a.n_items - a.w0 <= per_sm * device_sm_count();
+int pass_kind64(const Geom &g, const DevPot &pot, const Plan64 *plan, double rc2, bool force, int z0, int z1) {
+  if (!plan || !plan->ok || !cutoff_in_table(pot, rc2)) return MB_PASS_ROWS;
+  if (plan->entries) return MB_PASS_SPLIT;
+  int per_sm = force ? (pot.n_types == 1 ? MB_SPLIT_FORCE_ITEMS : MB_MULTI_SPLIT_FORCE_ITEMS)
+                     : (pot.n_types == 1 ? MB_SPLIT_RHO_ITEMS : MB_MULTI_SPLIT_RHO_ITEMS);
+  if (const char *v = getenv(force ? "MB_SPLIT_FORCE_ITEMS" : "MB_SPLIT_RHO_ITEMS")) per_sm = atoi(v);
+  const int items = ((z1 < 0 ? g.bz : z1) - z0) * 2 * plan64_plane_items(g);
+  return items <= per_sm * device_sm_count() ? MB_PASS_SPLIT : MB_PASS_SHELLS;
 }
 
 // Arguments of a planned pass over box layers [z0, z1).
@@ -563,14 +567,13 @@ static LatticeArgs lattice_args(const Geom &g, const DevPot &pot, const Lattice6
 int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, double rc2,
                  double *e_partial, int energy, int flag, cudaStream_t s, int z0, int z1, uint2 *outer,
                  const Plan64 *plan) {
-  if (plan && plan->ok && L.rho && cutoff_in_table(pot, rc2)) {
+  const int kind = L.rho ? pass_kind64(g, pot, plan, rc2, false, z0, z1) : MB_PASS_ROWS;
+  if (kind != MB_PASS_ROWS) {
     if (z1 < 0) z1 = g.bz;
     if (z0 < 0 || z0 >= z1 || z1 > g.bz) return z0 == z1 ? MB_OK : fail(MB_ERR_ARG, "z-slab outside the box");
     LatticeArgs a = lattice_args(g, pot, L, rc2, flag, outer, *plan, z0, z1);
     a.e0 = e_partial;
-    if (plan->entries || split_launch("MB_SPLIT_RHO_ITEMS", MB_SPLIT_RHO_ITEMS, MB_MULTI_SPLIT_RHO_ITEMS, a))
-      return launch_split_rho64(st, a, energy, s);
-    return launch_shell_rho64(st, a, energy, s);
+    return kind == MB_PASS_SPLIT ? launch_split_rho64(st, a, energy, s) : launch_shell_rho64(st, a, energy, s);
   }
   RhoArgs a;
   a.g = g;
@@ -609,7 +612,8 @@ int launch_rho64(const Geom &g, const StencilSet &st, const DevPot &pot, const L
 int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const Lattice64 &L, const StepParams &sp,
                    double *e_partial, int energy, int flag, cudaStream_t s, int z0, int z1,
                    const uint2 *outer, const Plan64 *plan) {
-  if (plan && plan->ok && L.fx && cutoff_in_table(pot, sp.rc2)) {
+  const int kind = L.fx ? pass_kind64(g, pot, plan, sp.rc2, true, z0, z1) : MB_PASS_ROWS;
+  if (kind != MB_PASS_ROWS) {
     if (z1 < 0) z1 = g.bz;
     if (z0 < 0 || z0 >= z1 || z1 > g.bz) return z0 == z1 ? MB_OK : fail(MB_ERR_ARG, "z-slab outside the box");
     LatticeArgs a =
@@ -617,9 +621,7 @@ int launch_force64(const Geom &g, const StencilSet &st, const DevPot &pot, const
     a.sp = sp;
     a.e0 = e_partial ? e_partial + MB_EPART_CAP : nullptr;
     a.e1 = e_partial ? e_partial + 2 * MB_EPART_CAP : nullptr;
-    if (plan->entries || split_launch("MB_SPLIT_FORCE_ITEMS", MB_SPLIT_FORCE_ITEMS, MB_MULTI_SPLIT_FORCE_ITEMS, a))
-      return launch_split_force64(st, a, energy, s);
-    return launch_shell_force64(st, a, energy, s);
+    return kind == MB_PASS_SPLIT ? launch_split_force64(st, a, energy, s) : launch_shell_force64(st, a, energy, s);
   }
   ForceArgs a;
   a.g = g;

@@ -98,6 +98,8 @@ static int dalloc(mb_sim *s, void **p, size_t bytes) {
   return MB_OK;
 }
 
+int ens_pass_kinds(mb_ensemble *e, int32_t *rho, int32_t *force); // mb_ens_host.cu
+
 Lattice64 sim_lattice(mb_sim *s, int which) {
   Lattice64 L{};
   L.p = s->pos[which];
@@ -985,6 +987,18 @@ int mb_sim_info(mb_sim *s, int64_t *n_sites, int64_t *n_stencil, int64_t *device
   if (n_sites) *n_sites = s->n_box;
   if (n_stencil) *n_stencil = s->st.n;
   if (device_bytes) *device_bytes = (int64_t)s->device_bytes;
+  return MB_OK;
+}
+
+int mb_sim_pass_kinds(mb_sim *s, int32_t *rho, int32_t *force) {
+  if (!s || !rho || !force) return fail(MB_ERR_ARG, "null argument");
+  if (s->ens) {
+    MB_TRY(mixed_need_slot(s));
+    return ens_pass_kinds(s->ens, rho, force);
+  }
+  const double rc2 = s->cfg.cutoff * s->cfg.cutoff;
+  *rho = pass_kind64(s->g, pot_dev(s->pot), &s->plan, rc2, false);
+  *force = pass_kind64(s->g, pot_dev(s->pot), &s->plan, rc2, true);
   return MB_OK;
 }
 

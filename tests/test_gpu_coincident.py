@@ -69,6 +69,7 @@ def test_resident_passes_with_coincident_atoms(kind, n_types, monkeypatch):
     monkeypatch.setenv("MB_SPLIT_RHO_ITEMS", items)
     monkeypatch.setenv("MB_SPLIT_FORCE_ITEMS", items)
     with mb.Sim(sc.cells, sc.tables, lattice_const=A0, mass=MASS, dt=1.0, cutoff=sc.cutoff, stencil_skin=sc.skin) as sim:
+        assert sim.pass_kinds() == ({"shell": "shells"}.get(kind, kind),) * 2
         sim.upload(sc.box)
         sim.run(0, 1)
         first = sim.download()[0]
