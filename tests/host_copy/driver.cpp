@@ -5,6 +5,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
 #include <new>
 #include <string>
 #include <vector>
@@ -15,6 +16,7 @@ T __ldg(const T *p) { return *p; } // named by device code of the header
 
 static int events_made = 0, event_to_fail = -1; // the event creation that fails
 static int events_open = 0, slots_open = 0;
+static std::atomic<int> pieces{0}; // copies that crossed to the device and back
 static thread_local int news_left = -1; // allocations of this thread until one fails (< 0: none does)
 
 void *operator new(size_t n) {
@@ -61,6 +63,7 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  pieces++;
   memcpy(d, s, n);
   return cudaSuccess;
 }
@@ -91,6 +94,12 @@ int main(int, char **argv) {
   if (scenario == "event") event_to_fail = 2; // the slots are taken, the third event is not
   // "memory N": every allocation of a copy but the first N fails
   copies(c, 3, big, scenario == "memory" ? atoi(argv[2]) : -1);
+  if (scenario == "sizes") // in bytes beyond argv[2], argv[3], ... MiB
+    for (int k = 2; argv[k]; k++) {
+      pieces = 0;
+      copies(c, 1, ((size_t)atoi(argv[k]) << 20) + 12345, -1);
+      printf("pieces %d\n", pieces.load());
+    }
   c.release();
   printf("left %d %d\n", events_open, slots_open);
   return 0;

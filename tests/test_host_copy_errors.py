@@ -1,7 +1,9 @@
-"""The shared host copies when a call or an allocation under them fails, on a stand-in CUDA runtime (no device):
-every copy still succeeds with the right bytes, and all that was taken is given back."""
+"""The shared host copies on a stand-in CUDA runtime (no device): when a call or an allocation
+under them fails every copy still succeeds with the right bytes, and all that was taken is
+given back; copies of every size from 2 MiB on go through the slots once they are there."""
 from __future__ import annotations
 
+import os
 import pathlib
 import shutil
 import subprocess
@@ -33,3 +35,14 @@ def test_copies_survive_a_failing_call(driver, scenario):
     lines = r.stdout.split("\n")
     assert lines[:3] == ["0 1 0 1"] * 3, lines
     assert lines[3] == "left 0 0"
+
+
+@pytest.mark.skipif((os.cpu_count() or 1) < 4, reason="one thread copies plainly")
+def test_copies_of_every_size_take_the_slots_that_are_there(driver):
+    sizes = [2, 3, 7, 8, 14, 31]  # MiB and a short last chunk: fewer chunks than slots, as many, more
+    r = subprocess.run([str(driver), "sizes", *map(str, sizes)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    lines = r.stdout.split("\n")
+    for k, mib in enumerate(sizes):
+        assert lines[3 + 2 * k] == "0 1 0 1", mib
+        assert lines[4 + 2 * k] == f"pieces {2 * (mib + 1)}", mib  # up and down
