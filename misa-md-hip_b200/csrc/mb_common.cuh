@@ -228,7 +228,7 @@ struct Plan64 {
 struct StencilSet;
 bool plan64_shells(const DevPot &P, const Geom &g, double a0, double cutoff, const double *R, const StencilSet &st,
                    Shells64 &S);
-bool plan64_entries(const StencilSet &st, Shells64 &S);
+bool plan64_entries(const Geom &g, const StencilSet &st, Shells64 &S);
 int plan64_plane_items(const Geom &g); // work items of one (z, sublattice) plane
 int plan64_items(const Geom &g);       // ... of the box
 int plan64_sites(const Geom &g, int *sites, cudaStream_t s);

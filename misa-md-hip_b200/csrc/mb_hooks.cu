@@ -127,7 +127,7 @@ static Plan64 hook_plan(const HookCtx &c) {
   Plan64 plan{};
   int per_sm = MB_HOOK_SPLIT_ITEMS;
   if (const char *v = getenv("MB_HOOK_SPLIT_ITEMS")) per_sm = atoi(v);
-  plan.entries = plan64_entries(c.st, plan.sh) && (long long)plan64_items(c.g) <= (long long)per_sm * device_sm_count();
+  plan.entries = plan64_entries(c.g, c.st, plan.sh) && (long long)plan64_items(c.g) <= (long long)per_sm * device_sm_count();
   plan.ok = plan.entries;
   return plan;
 }

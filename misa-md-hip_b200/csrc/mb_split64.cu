@@ -226,9 +226,10 @@ static int split_grid(const LatticeArgs &a) {
 }
 
 // Plan of a stencil in no order and of no known lattice (the hooks): every entry is tested,
-// MB_OUT_RUN to a run, and the tables are read where they lie.
-bool plan64_entries(const StencilSet &st, Shells64 &S) {
-  if (st.n < 1 || st.n > MB_OUT_RUN * MB_RUNS_MAX) return false;
+// MB_OUT_RUN to a run, and the tables are read where they lie.  A site's index leaves the top
+// two bits free (MB_SITE_FACE, no site), which the hooks' own limit does not ask for.
+bool plan64_entries(const Geom &g, const StencilSet &st, Shells64 &S) {
+  if (st.n < 1 || st.n > MB_OUT_RUN * MB_RUNS_MAX || 2 * g.E > MB_SITE_INDEX) return false;
   S = Shells64{};
   for (int k = 0; k < st.n; k += MB_OUT_RUN) S.kb[S.runs++] = (short)k;
   S.kb[S.runs] = (short)st.n;

@@ -84,6 +84,20 @@ static void persistent() {
     }
 }
 
+// Hooks split items only where a site's index leaves two bits free; a small box inside a wide
+// frame of ghosts reaches beyond that.
+static void wide_ghosts(int width, bool splits) {
+  Geom g{};
+  g.bcx = g.by = g.bz = 8;
+  g.gcx = g.gy = g.gz = width;
+  g.ecx = g.ey = g.ez = 8 + 2 * width;
+  g.E = (long long)g.ecx * g.ey * g.ez;
+  StencilSet st{};
+  st.n = 88;
+  Shells64 S;
+  printf("%d ghosts%d %d\n", device, width, plan64_entries(g, st, S) == splits ? 0 : 1);
+}
+
 int main() {
   for (device = 0; device < 2; device++) {
     for (int n_types : {1, 3}) {
@@ -95,6 +109,10 @@ int main() {
       for (bool linear : {false, true})
         if (fixed || !linear) mixed(fixed, linear);
     persistent();
+    wide_ghosts(400, true);
+    wide_ghosts(402, true);
+    wide_ghosts(403, false); // 2 x 814^3 sites
+    wide_ghosts(500, false);
   }
   return 0;
 }

@@ -34,5 +34,5 @@ def lines(tmp_path_factory):
 @pytest.mark.parametrize("device", ["0", "1"])
 def test_every_pass_launches_on_every_device(lines, device):
     got = [(name, status) for d, name, status in lines if d == device]
-    assert len(got) == 40
+    assert len(got) == 44
     assert all(status == "0" for _, status in got), [g for g in got if g[1] != "0"]
