@@ -154,7 +154,8 @@ int mb_release_atoms_mem(void *atoms, int *released);
  * value, the number of z-slabs the rho and force hooks stream the array in (as the
  * reference's double buffer does, src/double-buffer/double_buffer.cpp:12-47, with the
  * layers split evenly; at most 32).  1, the reference's default, lets the library
- * choose (slabs of at least 4 MiB of records, at most 16).  The results are bitwise the
+ * choose (at most 16 slabs, of at least 4 MiB of records, or 1.75 MiB where a small box
+ * takes split items).  The results are bitwise the
  * same for every count. */
 int mb_cli_set_batches(unsigned int batches);
 unsigned int mb_cli_batches(void);

@@ -11,10 +11,11 @@
 // arrays (L2) in between.  The shells are built into the code (mb_ensemble_shells.cuh), so
 // that a neighbour costs one 32-byte load with an immediate column offset.
 // With several types a window holds the words of every type and pair of types.
-// Measured on one B200, 96^3 cells at 300 K: step 1.04 -> 0.79 ms; bank conflicts 94 M + 141
-// M -> none, instructions per 32-site item 6,250 -> 3,290 (density) and 5,460 -> 3,800
-// (force).  The density pass is now at 88% of the L1TEX data stage, the force pass waits on
-// neighbour loads (24 warps per SM, 80 registers).
+// Measured on one B200, 96^3 cells at 300 K: step 1.04 -> 0.79 ms; bank conflicts 0.15 M of
+// 27.5 M shared wavefronts (density) and 0.47 M of 42.6 M (force), with one table copy over
+// half; instructions per 32-site item 6,250 -> 3,820 and 5,460 -> 4,840.  The density pass is
+// now at 83% of the L1TEX data stage, the force pass (63%) waits on neighbour loads (24 warps
+// per SM, 80 registers).
 #include <math.h>
 
 #include "mb_pair64.cuh"
